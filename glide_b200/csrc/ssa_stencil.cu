@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
     const T* __restrict__ mask, const T* __restrict__ gamma, Geo g, Phys<T> p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
-    const int wid = blockIdx.x * (256 / 32) + threadIdx.x / 32;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= n_warps) return;  // whole warp
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
     const T* __restrict__ mask, Geo g, Phys<T> p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
-    const int wid = blockIdx.x * (256 / 32) + threadIdx.x / 32;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= n_warps) return;  // whole warp
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
     const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H, int exact_boundary, Geo g,
     Phys<T> p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
-    const int wid = blockIdx.x * (VS_NT / 32) + threadIdx.x / 32;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= n_warps) return;  // whole warp
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
@@ -789,20 +789,33 @@ __global__ void grad_beta_kernel(T* __restrict__ grad, const T* __restrict__ u, 
 // launchers
 // --------------------------------------------------------------------------
 
-// strips of SW columns, row chunks sized for ~32 warps per SM
+// Strips of SW columns and chunks of rows.  A warp's march is one serial chain
+// (two preparatory rows, then its rows), so a grid that leaves schedulers idle
+// takes chunks of as few rows as one warp per scheduler allows: the chunk's
+// time falls with its length and the repeated preparatory rows run on units
+// that had nothing to do.  From 8 rows on, chunks are sized for ~32 warps per
+// SM.  Chunks of at least 8 rows took 28-29 us for the FP64 VJP at every size
+// from 32^2 to 256^2, and two FP64 adjoint V-cycles at 256^2 22.9 ms; with this
+// rule the same cycles take 13.2 ms.  Warps are spread over the SMs in CTAs no larger
+// than that needs.
 struct StreamShape {
-    int n_strips, rows, n_warps;
+    int n_strips, rows, n_warps, threads;
+    unsigned blocks;
 };
 // 32-bit element offsets suffice when every field of one problem has fewer
 // than 2^31 elements (u and v have (ny+1)(nx+1) at most)
 static inline bool index32(const Geo& g) { return int64_t(g.ny + 1) * (g.nx + 1) < (int64_t(1) << 31); }
 
-static inline StreamShape stream_shape(const Geo& g) {
+static inline StreamShape stream_shape(const Geo& g, int max_threads) {
     StreamShape sh;
     sh.n_strips = (g.nx + SW - 1) / SW;
-    int rows = int((int64_t(g.ny) * sh.n_strips * g.nb + 148 * 32 - 1) / (148 * 32));
-    sh.rows = rows < 8 ? 8 : (rows > 128 ? 128 : rows);
+    const int64_t units = int64_t(g.ny) * sh.n_strips * g.nb;
+    const int64_t few = (units + 148 * 4 - 1) / (148 * 4), many = (units + 148 * 32 - 1) / (148 * 32);
+    sh.rows = int(few < 8 ? few : many < 8 ? 8 : many > 128 ? 128 : many);
     sh.n_warps = sh.n_strips * ((g.ny + sh.rows - 1) / sh.rows);
+    const int64_t per_sm = (int64_t(sh.n_warps) * g.nb + 147) / 148;
+    sh.threads = 32 * int(per_sm < max_threads / 32 ? per_sm : max_threads / 32);
+    sh.blocks = unsigned((sh.n_warps + sh.threads / 32 - 1) / (sh.threads / 32));
     return sh;
 }
 
@@ -811,10 +824,10 @@ int launch_residual(const GlideLevelArgs* a, const void* f_u, const void* f_v, c
                     void* r_H, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
     Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
-    const StreamShape sh = stream_shape(g);
-    const dim3 grid((sh.n_warps + 7) / 8, g.nb);
+    const StreamShape sh = stream_shape(g, 256);
+    const dim3 grid(sh.blocks, g.nb);
     auto go = [&](auto kernel) {
-        glide::count_launch(), kernel<<<grid, 256, 0, s>>>(
+        glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
             (T*)r_u, (T*)r_v, (T*)r_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u,
             (const T*)f_v, (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
             (const T*)a->gamma, g, p, sh.n_strips, sh.rows, sh.n_warps);
@@ -832,10 +845,10 @@ int launch_jvp(const GlideLevelArgs* a, const void* d_u, const void* d_v, const 
                const void* base_v, const void* base_H, void* j_u, void* j_v, void* j_H, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
     Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
-    const StreamShape sh = stream_shape(g);
-    const dim3 grid((sh.n_warps + 7) / 8, g.nb);
+    const StreamShape sh = stream_shape(g, 256);
+    const dim3 grid(sh.blocks, g.nb);
     auto go = [&](auto kernel) {
-        glide::count_launch(), kernel<<<grid, 256, 0, s>>>(
+        glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
             (T*)j_u, (T*)j_v, (T*)j_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)d_u,
             (const T*)d_v, (const T*)d_H, (const T*)base_u, (const T*)base_v, (const T*)base_H, (const T*)a->bed,
             (const T*)a->B, (const T*)a->beta, (const T*)a->mask, g, p, sh.n_strips, sh.rows, sh.n_warps);
@@ -854,10 +867,10 @@ int launch_vjp(const GlideLevelArgs* a, const void* l_u, const void* l_v, const 
                cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
     Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
-    const StreamShape sh = stream_shape(g);
-    const dim3 grid((sh.n_warps + VS_NT / 32 - 1) / (VS_NT / 32), g.nb);
+    const StreamShape sh = stream_shape(g, VS_NT);
+    const dim3 grid(sh.blocks, g.nb);
     auto go = [&](auto kernel) {
-        glide::count_launch(), kernel<<<grid, VS_NT, 0, s>>>(
+        glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
             (T*)o_u, (T*)o_v, (T*)o_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)l_u,
             (const T*)l_v, (const T*)l_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
             (const T*)f_u, (const T*)f_v, (const T*)f_H, exact_boundary, g, p, sh.n_strips, sh.rows, sh.n_warps);
