@@ -24,56 +24,19 @@
 #include <stdint.h>
 
 #include "glide_b200.h"
+#include "tc_common.cuh"
 
 namespace glide {
 void count_launch();
+int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W, const void* Wt,
+                  int ldw, void* out, int ldc, int N, const float* bias, int relu, int out_mode, int* err,
+                  cudaStream_t s);
 }
 
 namespace glide {
 
 constexpr int GM = 128, GN = 64, GK = 64, GTHREADS = 128;
 constexpr uint32_t TMEM_COLS = 64;
-constexpr long long WAIT_CYCLES = 2000000000LL;  // ~1 s at 2 GHz
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-// UMMA shared-memory matrix descriptor, K-major, no swizzle (SM100 version 1).
-__device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-    uint64_t d = 0;
-    d |= uint64_t((saddr >> 4) & 0x3FFFu);
-    d |= uint64_t((lbo_bytes >> 4) & 0x3FFFu) << 16;
-    d |= uint64_t((sbo_bytes >> 4) & 0x3FFFu) << 32;
-    d |= uint64_t(1) << 46;
-    return d;
-}
-
-// Instruction descriptor: D = F32, A = B = BF16, both K-major, M x N.
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(addr), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ bool mbar_wait_bounded(uint32_t addr, uint32_t parity) {
-    const long long t0 = clock64();
-    while (!mbar_try(addr, parity)) {
-        if (clock64() - t0 > WAIT_CYCLES) return false;
-    }
-    return true;
-}
-
 // offset of element (row, k) inside a [rows x GK] canonical tile
 __device__ __forceinline__ uint32_t tile_off(int row, int kc) {
     return uint32_t((row >> 3) * 1024 + kc * 128 + (row & 7) * 16);
@@ -179,21 +142,10 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_kernel(const __nv_bfloat16* 
         if (threadIdx.x == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-            for (int s = 0; s < GK / 16; s++) {
-                const uint64_t da = umma_desc(a_base + s * 256, 128, 1024);
-                const uint64_t db = umma_desc(b_base + s * 256, 128, 1024);
-                const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                    :
-                    : "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             mbar_addr)
-                         : "memory");
+            for (int s = 0; s < GK / 16; s++)
+                mma_bf16(tmem, umma_desc(a_base + s * 256, 128, 1024), umma_desc(b_base + s * 256, 128, 1024), idesc,
+                         ch > 0 || s > 0);
+            mma_commit(&mbar);
         }
         // every thread waits for the MMAs that read the staged tile; the
         // outcome is made uniform so all threads leave the loop together
@@ -259,16 +211,6 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_kernel(const __nv_bfloat16* 
 // store where the row allows it.
 // --------------------------------------------------------------------------
 constexpr int PSTAGES_MAX = 4;
-
-__device__ __forceinline__ void cp_async16(uint32_t saddr, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(saddr), "l"(src), "r"(src_bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 
 template <bool CONV, int BN, int PSTAGES>
 __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloat16* __restrict__ A, int lda,
@@ -384,21 +326,10 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloa
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t st = sbase + uint32_t((ch % PSTAGES) * STAGE);
 #pragma unroll
-            for (int s = 0; s < GK / 16; s++) {
-                const uint64_t da = umma_desc(st + s * 256, 128, 1024);
-                const uint64_t db = umma_desc(st + A_BYTES + s * 256, 128, 1024);
-                const uint32_t acc = (ch > 0 || s > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n\t.reg .pred p;\n\t"
-                    "setp.ne.b32 p, %4, 0;\n\t"
-                    "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-                    :
-                    : "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
-                    : "memory");
-            }
-            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                             smem_u32(&mbar[ch % PSTAGES]))
-                         : "memory");
+            for (int s = 0; s < GK / 16; s++)
+                mma_bf16(tmem, umma_desc(st + s * 256, 128, 1024), umma_desc(st + A_BYTES + s * 256, 128, 1024), idesc,
+                         ch > 0 || s > 0);
+            mma_commit(&mbar[ch % PSTAGES]);
         }
         issued = ch + 1;
     }
@@ -527,6 +458,9 @@ extern "C" int glide_conv3x3_bf16(const void* x, int Bn, int H, int W, int C, co
     const int64_t M64 = int64_t(Bn) * H * W;
     if (M64 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
     const int M = int(M64), K = 9 * C;
+    const int rc = glide::try_conv_rows(x, C, 0, nullptr, 0, Bn, H, W, Wt, ldw, out, ldc, N, bias, relu, out_mode, err,
+                                        (cudaStream_t)stream);
+    if (rc != -1000) return rc;
     if (ldw % 8 == 0 && glide::al16(Wt))
         return glide::launch_pipe_n<true>((const __nv_bfloat16*)x, 0, (const __nv_bfloat16*)Wt, ldw, out, ldc, M, N, K,
                                           bias, relu, out_mode, err, glide::ConvShape{Bn, H, W, C},
