@@ -143,8 +143,8 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
                 for (int k = tid; k < items; k += CR_ROLE) {
                     const int sx = xs - 1 + px;
                     const bool in = yin && sx >= 0 && sx < a.Wd;
-                    const __nv_bfloat16* src = c < c08 ? r0 + int64_t(a.up0 ? sx >> 1 : sx) * a.C0 + c * 8
-                                                       : r1 + int64_t(sx) * a.C1 + (c - c08) * 8;
+                    const __nv_bfloat16* src =
+                        c < c08 ? r0 + ((a.up0 ? sx >> 1 : sx) * a.C0 + c * 8) : r1 + (sx * a.C1 + (c - c08) * 8);
                     cp_async16(st + uint32_t(c) * CR_PLANE + uint32_t(px) * 16, in ? src : a.x0, in ? 16u : 0u);
                     px += dpx;
                     c += dc;
@@ -172,59 +172,67 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
         cp_async_wait<0>();
         if (ok) publish(n_in - 1);
     } else if (warp == 8) {
-        // ---------------------------------------------------------------- products
-        if (lane == 0) {
-            const uint32_t idesc = idesc_bf16_f32(128, BN);
-            for (int r = 0; r < n_in && ok; r++) {
-                if (!mbar_wait_bounded(smem_u32(&full[r % S]), uint32_t((r / S) & 1))) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t st = sA + uint32_t(r % S) * stage_bytes;
-                if constexpr (C8) {
-                    const int slot = r % CR_ACC;
-                    if (r >= CR_ACC && !mbar_wait_bounded(smem_u32(&acc_empty[slot]), uint32_t((r / CR_ACC - 1) & 1))) {
-                        ok = false;
-                        break;
-                    }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    for (int s = 0; s < CR_PLANES8 / 2; s++)
-                        mma_bf16(tmem + slot * BN, umma_desc(st + uint32_t(s) * 2 * CR_PLANE8, CR_PLANE8, 128),
-                                 umma_desc(sB + uint32_t(s) * 2 * BN * 16, BN * 16, 128), idesc, s > 0);
-                    mma_commit(&acc_full[slot]);
-                } else {
-                    // ky = 2 finishes output row r-2 of the chunk, ky = 1 continues r-1, ky = 0 opens r
-                    for (int ky = 2; ky >= 0; ky--) {
-                        const int yo = r - ky;
-                        if (yo < 0 || yo >= y1 - y0) continue;
-                        const int slot = yo % CR_ACC;
-                        if (ky == 0 && yo >= CR_ACC) {
-                            if (!mbar_wait_bounded(smem_u32(&acc_empty[slot]), uint32_t((yo / CR_ACC - 1) & 1))) {
-                                ok = false;
-                                break;
-                            }
-                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        }
-                        for (int kx = 0; kx < 3; kx++) {
-                            const uint32_t wb = sB + uint32_t((ky * 3 + kx) * (C / 8)) * BN * 16;
-                            for (int s = 0; s < C / 16; s++)
-                                mma_bf16(tmem + slot * BN,
-                                         umma_desc(st + uint32_t(s) * 2 * CR_PLANE + uint32_t(kx) * 16, CR_PLANE, 128),
-                                         umma_desc(wb + uint32_t(s) * 2 * BN * 16, BN * 16, 128), idesc,
-                                         ky > 0 || kx > 0 || s > 0);
-                        }
-                        if (ky == 2) mma_commit(&acc_full[slot]);
-                    }
+        // ---------------------------------------------------------------- products (the whole warp, lane 0 issues)
+        const uint32_t idesc = idesc_bf16_f32(128, BN), lead = lane == 0;
+        const uint32_t a_hi = umma_hi(128), b_hi = umma_hi(128);
+        for (int r = 0; r < n_in && ok; r++) {
+            if (!mbar_wait_bounded(smem_u32(&full[r % S]), uint32_t((r / S) & 1))) { ok = false; break; }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t st = sA + uint32_t(r % S) * stage_bytes;
+            if constexpr (C8) {
+                const int slot = r % CR_ACC;
+                if (r >= CR_ACC && !mbar_wait_bounded(smem_u32(&acc_empty[slot]), uint32_t((r / CR_ACC - 1) & 1))) {
+                    ok = false;
+                    break;
                 }
-                mma_commit(&empty[r % S]);
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t a0 = umma_lo(st, CR_PLANE8), b0 = umma_lo(sB, BN * 16);
+#pragma unroll
+                for (int s = 0; s < CR_PLANES8 / 2; s++)
+                    mma_bf16_lead(tmem + slot * BN, a0 + s * (2 * CR_PLANE8 / 16), a_hi, b0 + s * (2 * BN), b_hi, idesc,
+                                  s > 0, lead);
+                mma_commit_lead(&acc_full[slot], lead);
+            } else {
+                // ky = 2 finishes output row r-2 of the chunk, ky = 1 continues r-1, ky = 0 opens r
+                for (int ky = 2; ky >= 0; ky--) {
+                    const int yo = r - ky;
+                    if (yo < 0 || yo >= y1 - y0) continue;
+                    const int slot = yo % CR_ACC;
+                    if (ky == 0 && yo >= CR_ACC) {
+                        if (!mbar_wait_bounded(smem_u32(&acc_empty[slot]), uint32_t((yo / CR_ACC - 1) & 1))) {
+                            ok = false;
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    }
+                    uint32_t b_lo = umma_lo(sB + uint32_t(ky * 3 * (C / 8)) * BN * 16, BN * 16);
+                    uint32_t acc = ky > 0;
+                    for (int kx = 0; kx < 3; kx++) {
+                        uint32_t a_lo = umma_lo(st + uint32_t(kx) * 16, CR_PLANE);
+#pragma unroll 2
+                        for (int s = 0; s < C / 16; s++) {
+                            mma_bf16_lead(tmem + slot * BN, a_lo, a_hi, b_lo, b_hi, idesc, acc, lead);
+                            a_lo += 2 * CR_PLANE / 16;
+                            b_lo += 2 * BN;
+                            acc = 1;
+                        }
+                    }
+                    if (ky == 2) mma_commit_lead(&acc_full[slot], lead);
+                }
             }
-            // the MMAs in flight read shared memory: they end before the CTA does
-            mma_commit(&drain);
-            if (!mbar_wait_bounded(smem_u32(&drain), 0)) ok = false;
+            mma_commit_lead(&empty[r % S], lead);
         }
+        // the MMAs in flight read shared memory: they end before the CTA does
+        mma_commit_lead(&drain, lead);
+        if (!mbar_wait_bounded(smem_u32(&drain), 0)) ok = false;
         __syncwarp();
     } else {
         // ---------------------------------------------------------------- store finished rows
         const int w = warp - 4, m = w * 32 + lane, x = xs + m;
         const bool vec = (a.ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
+        float bias[BN];
+#pragma unroll
+        for (int e = 0; e < BN; e++) bias[e] = a.bias && n0 + e < a.N ? __ldg(a.bias + n0 + e) : 0.0f;
         for (int yo = 0; yo < y1 - y0; yo++) {
             const int slot = yo % CR_ACC;
             if (!mbar_wait_bounded(smem_u32(&acc_full[slot]), uint32_t((yo / CR_ACC) & 1))) { ok = false; break; }
@@ -238,7 +246,7 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
             const int64_t o = ((int64_t(img) * a.H + y0 + yo) * a.Wd + x) * a.ldc + n0;
 #pragma unroll
             for (int e = 0; e < BN; e++) {
-                if (a.bias && n0 + e < a.N) v[e] += __ldg(a.bias + n0 + e);
+                if (a.bias) v[e] += bias[e];
                 if (a.relu) v[e] = fmaxf(v[e], 0.0f);
             }
 #pragma unroll
