@@ -3,6 +3,11 @@
 //
 //   out[p, n] = act(bias[n] + sum_{ky,kx,c} x[y+ky-1, x+kx-1, c] W[n, (ky*3+kx)*C + c])
 //
+// What bounds it: the issue of narrow MMAs and, per row, the copy -> product ->
+// store latency that the ring and the resident CTAs have to cover.  1024^2,
+// 32 -> 32: 226 us as an implicit GEMM, 54 us here (134 MB, 2.5 TB/s); 512^2,
+// 64 -> 64: 163 -> 37.
+//
 // The implicit GEMM of tc_gemm.cu gathers nine shifted copies of its 128
 // pixels (73 KB of copies for 8 KB of input at C = 32) and runs load, product
 // and store of a CTA one after the other; at 1024^2 and C = 32 it held the
@@ -61,7 +66,8 @@ struct ConvRows {
     int Bn, H, Wd, strips, rows, chunks, stages;
 };
 
-template <int BN, bool C8>
+// KS: K steps per tap (C / 16) when known at compile time, else 0
+template <int BN, bool C8, int KS>
 __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[CR_MAXST], empty[CR_MAXST], acc_full[CR_ACC], acc_empty[CR_ACC], drain;
@@ -86,7 +92,7 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
     }
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
-            mbar_init(&full[s], 4);
+            mbar_init(&full[s], CR_ROLE);
             mbar_init(&empty[s], 1);
         }
         for (int s = 0; s < CR_ACC; s++) {
@@ -152,32 +158,23 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
                 }
             }
         };
-        auto publish = [&](int r) {   // this warp's copies of row r have landed
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&full[r % S]);
-        };
         for (int r = 0; r < n_in; r++) {
             if (r >= S && !mbar_wait_bounded(smem_u32(&empty[r % S]), uint32_t((r / S - 1) & 1))) {
                 ok = false;
                 break;
             }
             copy_row(r);
-            cp_async_commit();
-            if (r >= 1) {
-                cp_async_wait<1>();
-                publish(r - 1);
-            }
+            cp_async_arrive(&full[r % S]);
         }
+        cp_async_commit();
         cp_async_wait<0>();
-        if (ok) publish(n_in - 1);
     } else if (warp == 8) {
         // ---------------------------------------------------------------- products (the whole warp, lane 0 issues)
         const uint32_t idesc = idesc_bf16_f32(128, BN), lead = lane == 0;
         const uint32_t a_hi = umma_hi(128), b_hi = umma_hi(128);
         for (int r = 0; r < n_in && ok; r++) {
             if (!mbar_wait_bounded(smem_u32(&full[r % S]), uint32_t((r / S) & 1))) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            fence_copied();
             const uint32_t st = sA + uint32_t(r % S) * stage_bytes;
             if constexpr (C8) {
                 const int slot = r % CR_ACC;
@@ -194,6 +191,9 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
                 mma_commit_lead(&acc_full[slot], lead);
             } else {
                 // ky = 2 finishes output row r-2 of the chunk, ky = 1 continues r-1, ky = 0 opens r
+                const uint32_t a0 = umma_lo(st, CR_PLANE), b0 = umma_lo(sB, BN * 16);
+                const int ks = KS ? KS : C / 16;
+#pragma unroll
                 for (int ky = 2; ky >= 0; ky--) {
                     const int yo = r - ky;
                     if (yo < 0 || yo >= y1 - y0) continue;
@@ -205,17 +205,13 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
                         }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     }
-                    uint32_t b_lo = umma_lo(sB + uint32_t(ky * 3 * (C / 8)) * BN * 16, BN * 16);
-                    uint32_t acc = ky > 0;
+#pragma unroll
                     for (int kx = 0; kx < 3; kx++) {
-                        uint32_t a_lo = umma_lo(st + uint32_t(kx) * 16, CR_PLANE);
-#pragma unroll 2
-                        for (int s = 0; s < C / 16; s++) {
-                            mma_bf16_lead(tmem + slot * BN, a_lo, a_hi, b_lo, b_hi, idesc, acc, lead);
-                            a_lo += 2 * CR_PLANE / 16;
-                            b_lo += 2 * BN;
-                            acc = 1;
-                        }
+#pragma unroll
+                        for (int s = 0; s < ks; s++)
+                            mma_bf16_lead(tmem + slot * BN, a0 + kx + s * (2 * CR_PLANE / 16), a_hi,
+                                          b0 + ((ky * 3 + kx) * ks + s) * (2 * BN), b_hi, idesc,
+                                          ky > 0 || kx > 0 || s > 0, lead);
                     }
                     if (ky == 2) mma_commit_lead(&acc_full[slot], lead);
                 }
@@ -282,20 +278,36 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(CR_ACC * BN)));
 }
 
-template <int BN, bool C8> int launch_conv_rows(const ConvRows& a, size_t smem, cudaStream_t s) {
+template <int BN, bool C8, int KS> int launch_conv_rows(const ConvRows& a, size_t smem, cudaStream_t s) {
     static int configured[64] = {0};
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return GLIDE_E_SHAPE;
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(conv_rows_kernel<BN, C8>,
+        const cudaError_t e = cudaFuncSetAttribute(conv_rows_kernel<BN, C8, KS>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, CR_SMEM_MAX);
         if (e != cudaSuccess) return int(e);
         configured[dev] = 1;
     }
     const dim3 grid(unsigned(a.strips) * a.chunks * a.Bn, (a.N + BN - 1) / BN);
-    count_launch(), conv_rows_kernel<BN, C8><<<grid, CR_THREADS, smem, s>>>(a);
+    count_launch(), conv_rows_kernel<BN, C8, KS><<<grid, CR_THREADS, smem, s>>>(a);
     return int(cudaGetLastError());
+}
+
+// The narrow widths of the guess network have their K loop unrolled: with
+// every descriptor an immediate away from two bases the issuing warp comes
+// closer to the tensor pipe (about 90 clocks per MMA in a rolled loop, 40
+// needed; 1024^2, 96 -> 32: 160 -> 129 us).  At 192 channels the unrolled body
+// is slower than the loop (512^2, 192 -> 64: 180 against 138 us).
+template <int BN> int pick_conv_rows(const ConvRows& a, bool c8, size_t smem, cudaStream_t s) {
+    if (c8) return launch_conv_rows<BN, true, 0>(a, smem, s);
+    switch (a.C0 + a.C1) {
+        case 32: return launch_conv_rows<BN, false, 2>(a, smem, s);
+        case 64: return launch_conv_rows<BN, false, 4>(a, smem, s);
+        case 96: return launch_conv_rows<BN, false, 6>(a, smem, s);
+        case 128: return launch_conv_rows<BN, false, 8>(a, smem, s);
+        default: return launch_conv_rows<BN, false, 0>(a, smem, s);
+    }
 }
 
 // Launches the row march and returns its status, or returns -1000 where the
@@ -338,8 +350,7 @@ int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int B
     a.rows = int(rows < H ? rows : H);
     a.chunks = (H + a.rows - 1) / a.rows;
     const size_t smem = weights(bn) + a.stages * stage;
-    if (bn == 64) return c8 ? launch_conv_rows<64, true>(a, smem, s) : launch_conv_rows<64, false>(a, smem, s);
-    return c8 ? launch_conv_rows<32, true>(a, smem, s) : launch_conv_rows<32, false>(a, smem, s);
+    return bn == 64 ? pick_conv_rows<64>(a, c8, smem, s) : pick_conv_rows<32>(a, c8, smem, s);
 }
 
 }  // namespace glide

@@ -49,6 +49,11 @@ __device__ __forceinline__ uint32_t umma_lo(uint32_t saddr, uint32_t lbo_bytes) 
     return ((saddr >> 4) & 0x3FFFu) | (((lbo_bytes >> 4) & 0x3FFFu) << 16);
 }
 __device__ __forceinline__ uint32_t umma_hi(uint32_t sbo_bytes) { return ((sbo_bytes >> 4) & 0x3FFFu) | (1u << 14); }
+// K-major operand of 64 columns in 128-byte rows whose 16-byte entries are
+// permuted (entry ^ row % 8) within groups of 8 rows (1024-byte aligned): a row
+// is one shared-memory line, so cp.async copies of it stay coalesced; a K step
+// of 16 is 32 bytes.
+__device__ __forceinline__ uint32_t umma_hi_sw128() { return (1024u >> 4) | (1u << 14) | (2u << 29); }
 __device__ __forceinline__ void mma_bf16_lead(uint32_t tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                               uint32_t idesc, uint32_t acc, uint32_t lead) {
     asm volatile(
@@ -110,6 +115,19 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// bar gets one arrival of this thread once all its cp.async copies so far have
+// landed.  The thread itself does not wait, and needs no proxy fence: the
+// reader fences after its wait (a fence here would first wait for every copy
+// the thread has in flight, i.e. undo the ring).
+__device__ __forceinline__ void cp_async_arrive(uint64_t* bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// after a wait for copied data: order it before this thread's MMAs
+__device__ __forceinline__ void fence_copied() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
 
 // 32 TMEM columns of the calling warp's 32 lanes, without the wait

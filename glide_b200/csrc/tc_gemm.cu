@@ -11,10 +11,11 @@
 // K halves, SBO = 1024 B between 8-row groups); one elected thread issues
 // four tcgen05.mma (M=128, K=16) per 64-wide K chunk into a TMEM accumulator
 // and commits them to an mbarrier; the epilogue reads TMEM with tcgen05.ld
-// (each warp its 32-lane subpartition).  Two kernels:
-//  * tc_gemm_pipe_kernel (aligned operands, every convolution): a 2-stage
-//    (short K) or 4-stage ring filled by cp.async, N tile 32/64/128 after
-//    the output width;
+// (each warp its 32-lane subpartition).  Three kernels:
+//  * tc_gemm_pipe_kernel (aligned operands, short K): a 2-stage ring filled by
+//    cp.async, N tile 32/64/128 after the output width;
+//  * tc_gemm_ring_kernel (aligned operands, long K or a two-source
+//    convolution): specialised copy and MMA warps on a six-stage ring;
 //  * tc_gemm_kernel (any pitch or K): one 128 x 64 tile staged through
 //    registers per chunk, every thread waiting for its MMAs before the next.
 //
@@ -40,6 +41,11 @@ constexpr uint32_t TMEM_COLS = 64;
 // offset of element (row, k) inside a [rows x GK] canonical tile
 __device__ __forceinline__ uint32_t tile_off(int row, int kc) {
     return uint32_t((row >> 3) * 1024 + kc * 128 + (row & 7) * 16);
+}
+
+// the same element's 16 bytes in 128-byte rows with permuted entries (umma_hi_sw128)
+__device__ __forceinline__ uint32_t sw128_off(int row, int kc) {
+    return uint32_t(row * 128 + ((kc ^ (row & 7)) << 4));
 }
 
 // Stage rows [r0, r0+R) x cols [k0, k0+GK) of a K-major BF16 matrix (ld elements).
@@ -73,6 +79,10 @@ __device__ __forceinline__ void stage_tile(uint8_t* s, const __nv_bfloat16* __re
 // matrix, so the products are bit-identical.
 struct ConvShape {
     int Bn, H, W, C;
+    // second source (tc_gemm_ring_kernel): channels C0.. of a pixel come from x1 at full resolution, channels
+    // 0..C0-1 from x, at half resolution (nearest) with up0
+    const __nv_bfloat16* x1;
+    int C0, up0;
 };
 __device__ __forceinline__ void stage_tile_conv(uint8_t* s, const __nv_bfloat16* __restrict__ x, const ConvShape cs,
                                                 int M, int K, int m0, int k0) {
@@ -212,6 +222,48 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_kernel(const __nv_bfloat16* 
 // --------------------------------------------------------------------------
 constexpr int PSTAGES_MAX = 4;
 
+// Bias, ReLU and store of the 32 rows of one warp (warps 0..3) of a finished tile.
+template <int BN>
+__device__ __forceinline__ void store_tile(uint32_t tmem, int warp, int lane, int m0, int n0, int M, int N, void* C,
+                                           int ldc, const float* __restrict__ bias, int relu, int out_mode) {
+    const int row = m0 + warp * 32 + lane;
+    const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16);
+    const bool vec = out_mode == 1 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += 8) {
+        uint32_t r[8];
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+            : "r"(taddr + uint32_t(c0)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const int col0 = n0 + c0;
+        if (row >= M || col0 >= N) continue;
+        float x[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            x[e] = __uint_as_float(r[e]);
+            if (bias && col0 + e < N) x[e] += bias[col0 + e];
+            if (relu) x[e] = fmaxf(x[e], 0.0f);
+        }
+        const int64_t o = int64_t(row) * ldc + col0;
+        if (vec && col0 + 8 <= N) {
+            __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+            for (int e = 0; e < 8; e++) h[e] = __float2bfloat16(x[e]);
+            *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(C) + o) = *reinterpret_cast<uint4*>(h);
+            continue;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            if (col0 + e >= N) break;
+            if (out_mode == 0) reinterpret_cast<float*>(C)[o + e] = x[e];
+            else if (out_mode == 1) reinterpret_cast<__nv_bfloat16*>(C)[o + e] = __float2bfloat16(x[e]);
+            else reinterpret_cast<float*>(C)[o + e] += x[e];
+        }
+    }
+}
+
 template <bool CONV, int BN, int PSTAGES>
 __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloat16* __restrict__ A, int lda,
                                                                 const __nv_bfloat16* __restrict__ B, int ldb,
@@ -345,48 +397,173 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloa
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
     if (ok && issued == nchunks && nchunks > 0) {
-        const int row = m0 + warp * 32 + lane;
-        const uint32_t taddr = tmem + (uint32_t(warp * 32) << 16);
-        const bool vec = out_mode == 1 && (ldc & 7) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
-#pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 8) {
-            uint32_t r[8];
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                : "r"(taddr + uint32_t(c0)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            const int col0 = n0 + c0;
-            if (row >= M || col0 >= N) continue;
-            float x[8];
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                x[e] = __uint_as_float(r[e]);
-                if (bias && col0 + e < N) x[e] += bias[col0 + e];
-                if (relu) x[e] = fmaxf(x[e], 0.0f);
-            }
-            const int64_t o = int64_t(row) * ldc + col0;
-            if (vec && col0 + 8 <= N) {
-                __align__(16) __nv_bfloat16 h[8];
-#pragma unroll
-                for (int e = 0; e < 8; e++) h[e] = __float2bfloat16(x[e]);
-                *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(C) + o) = *reinterpret_cast<uint4*>(h);
-                continue;
-            }
-#pragma unroll
-            for (int e = 0; e < 8; e++) {
-                if (col0 + e >= N) break;
-                if (out_mode == 0) reinterpret_cast<float*>(C)[o + e] = x[e];
-                else if (out_mode == 1) reinterpret_cast<__nv_bfloat16*>(C)[o + e] = __float2bfloat16(x[e]);
-                else reinterpret_cast<float*>(C)[o + e] += x[e];
-            }
-        }
+        store_tile<BN>(tmem, warp, lane, m0, n0, M, N, C, ldc, bias, relu, out_mode);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(BN)));
     }
+}
+
+// --------------------------------------------------------------------------
+// Long K (more than 8 chunks): the same tile and accumulation order with
+// specialised warps.  Eight warps copy chunks into a ring of six stages and one
+// warp issues the MMAs, synchronised by the stages' mbarriers alone (a stage's
+// copies arrive on its barrier by themselves), so the copies run up to six
+// chunks ahead of the products.  Rows are 128-byte lines (sw128_off): in the
+// 16-byte core-matrix layout every 16-byte copy is a request and a sector of
+// its own, 2x the L2 traffic and 8x the shared-memory writes, and the copies
+// set the pace (256^2, 384 -> 128: 274 us against 127).  The convolution's
+// input may be two tensors (see ConvShape).
+// --------------------------------------------------------------------------
+constexpr int RG_COPY = 256, RG_THREADS = RG_COPY + 32, RG_STAGES = 6;
+
+template <bool CONV, int BN>
+__global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfloat16* __restrict__ A, int lda,
+                                                                  const __nv_bfloat16* __restrict__ B, int ldb, void* C,
+                                                                  int ldc, int M, int N, int K,
+                                                                  const float* __restrict__ bias, int relu,
+                                                                  int out_mode, int* err, ConvShape cs) {
+    constexpr int A_BYTES = GM * GK * 2, B_BYTES = BN * GK * 2, STAGE = A_BYTES + B_BYTES;
+    constexpr int AROWS = GM * 8 / RG_COPY, BROWS = BN * 8 / RG_COPY;   // 16-byte copies per thread and chunk
+    constexpr int STEP = RG_COPY / 8;                                   // rows between a thread's copies
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ __align__(8) uint64_t full[RG_STAGES], empty[RG_STAGES], done;
+    __shared__ uint32_t tmem_slot;
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const int m0 = blockIdx.x * GM, n0 = blockIdx.y * BN;
+    const uint32_t sbase = (smem_u32(smem) + 1023u) & ~1023u;
+    if (warp == RG_COPY / 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                     "r"(uint32_t(BN)));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
+    }
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < RG_STAGES; s++) {
+            mbar_init(&full[s], RG_COPY);
+            mbar_init(&empty[s], 1);
+        }
+        mbar_init(&done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = tmem_slot;
+    const int nchunks = (K + GK - 1) / GK;
+    bool ok = true;
+
+    if (warp < RG_COPY / 32) {
+        const int kc = threadIdx.x & 7, rsub = threadIdx.x >> 3;
+        int a_pix[AROWS], a_y[AROWS], a_x[AROWS], a_lo[AROWS];
+        bool a_ok[AROWS];
+#pragma unroll
+        for (int i = 0; i < AROWS; i++) {
+            const int p = m0 + rsub + STEP * i;
+            a_ok[i] = p < M;
+            a_pix[i] = a_ok[i] ? p : 0;
+            if (CONV) {
+                const int t = a_pix[i] / cs.W;
+                a_x[i] = a_pix[i] - t * cs.W;
+                a_y[i] = t % cs.H;
+                a_lo[i] = (t / cs.H) * (cs.H / 2);   // first row of the image at half resolution
+            }
+        }
+        int tap = 0, c = kc * 8;   // this thread's position within the convolution's K
+        if (CONV)
+            while (c >= cs.C) { c -= cs.C; tap++; }
+        for (int ch = 0; ch < nchunks; ch++) {
+            const int sl = ch % RG_STAGES;
+            if (ch >= RG_STAGES && !mbar_wait_bounded(smem_u32(&empty[sl]), uint32_t((ch / RG_STAGES - 1) & 1))) {
+                ok = false;
+                break;
+            }
+            const uint32_t st = sbase + uint32_t(sl * STAGE);
+            const int k = ch * GK + kc * 8;
+            const bool kin = k < K;
+            if (CONV) {
+                const int ky = tap / 3, dy = ky - 1, dx = tap - 3 * ky - 1;
+                const bool second = c >= cs.C0;
+                const int Cs = second ? cs.C - cs.C0 : cs.C0, cc = second ? c - cs.C0 : c;
+                const __nv_bfloat16* src0 = second ? cs.x1 : A;
+                const bool half = !second && cs.up0;
+#pragma unroll
+                for (int i = 0; i < AROWS; i++) {
+                    const int sy = a_y[i] + dy, sx = a_x[i] + dx;
+                    const bool in = kin && a_ok[i] && sy >= 0 && sy < cs.H && sx >= 0 && sx < cs.W;
+                    const int pix = half ? (a_lo[i] + (sy >> 1)) * (cs.W / 2) + (sx >> 1)
+                                         : a_pix[i] + dy * cs.W + dx;
+                    cp_async16(st + sw128_off(rsub + STEP * i, kc), in ? src0 + int64_t(pix) * Cs + cc : A,
+                               in ? 16u : 0u);
+                }
+                c += GK;
+                while (c >= cs.C) { c -= cs.C; tap++; }
+            } else {
+#pragma unroll
+                for (int i = 0; i < AROWS; i++) {
+                    const bool in = kin && a_ok[i];
+                    cp_async16(st + sw128_off(rsub + STEP * i, kc), in ? A + int64_t(a_pix[i]) * lda + k : A,
+                               in ? 16u : 0u);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < BROWS; i++) {
+                const int n = n0 + rsub + STEP * i;
+                const bool in = kin && n < N;
+                cp_async16(st + A_BYTES + sw128_off(rsub + STEP * i, kc), in ? B + int64_t(n) * ldb + k : B,
+                           in ? 16u : 0u);
+            }
+            cp_async_arrive(&full[sl]);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+    } else {
+        const uint32_t idesc = idesc_bf16_f32(GM, BN), lead = lane == 0, hi = umma_hi_sw128();
+        for (int ch = 0; ch < nchunks; ch++) {
+            const int sl = ch % RG_STAGES;
+            if (!mbar_wait_bounded(smem_u32(&full[sl]), uint32_t((ch / RG_STAGES) & 1))) { ok = false; break; }
+            fence_copied();
+            const uint32_t st = sbase + uint32_t(sl * STAGE);
+            const uint32_t a_lo = umma_lo(st, 16), b_lo = umma_lo(st + A_BYTES, 16);
+#pragma unroll
+            for (int s = 0; s < GK / 16; s++)
+                mma_bf16_lead(tmem, a_lo + s * 2, hi, b_lo + s * 2, hi, idesc, ch > 0 || s > 0, lead);
+            mma_commit_lead(&empty[sl], lead);
+        }
+        mma_commit_lead(&done, lead);
+    }
+    // the accumulator is complete, and no MMA reads shared memory any more
+    if (!mbar_wait_bounded(smem_u32(&done), 0)) ok = false;
+    if (!ok && lane == 0 && err) atomicExch(err, 1);
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ok && warp < 4) store_tile<BN>(tmem, warp, lane, m0, n0, M, N, C, ldc, bias, relu, out_mode);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == RG_COPY / 32) {
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(BN)));
+    }
+}
+
+template <bool CONV, int BN>
+int launch_ring(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, void* C, int ldc, int M, int N,
+                int K, const float* bias, int relu, int out_mode, int* err, ConvShape cs, cudaStream_t s) {
+    constexpr int SMEM = RG_STAGES * (GM * GK * 2 + BN * GK * 2) + 1024;
+    static int configured[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return GLIDE_E_SHAPE;
+    if (!configured[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(tc_gemm_ring_kernel<CONV, BN>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+        if (e != cudaSuccess) return int(e);
+        configured[dev] = 1;
+    }
+    dim3 grid((M + GM - 1) / GM, (N + BN - 1) / BN);
+    count_launch(), tc_gemm_ring_kernel<CONV, BN><<<grid, RG_THREADS, SMEM, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias,
+                                                                                 relu, out_mode, err, cs);
+    return int(cudaGetLastError());
 }
 
 template <bool CONV, int BN, int PSTAGES>
@@ -409,16 +586,17 @@ int launch_pipe(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb
     return int(cudaGetLastError());
 }
 
-// Short K (a few chunks, the convolutions of the guess network) runs a
-// 2-stage ring: half the shared memory, so 2-3x the CTAs per SM hide each
-// CTA's fixed latencies (ncu at 1024^2, C = 32, 4 stages: 2 CTAs and 7.7
-// warps per SM, tensor pipe 3 % active); long K keeps 4 stages.
+// Short K (a few chunks) runs the 2-stage form: half the shared memory, so
+// 2-3x the CTAs per SM hide each CTA's fixed latencies (ncu at 1024^2, C = 32,
+// 4 stages: 2 CTAs and 7.7 warps per SM, tensor pipe 3 % active); long K and
+// two-source inputs run the specialised warps.  256^2, 384 -> 128 channels:
+// 376 -> 127 us; 128^2, 256 -> 256: 134 -> 52.
 template <bool CONV, int BN>
 int launch_pipe_s(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, void* C, int ldc, int M, int N,
                   int K, const float* bias, int relu, int out_mode, int* err, ConvShape cs, cudaStream_t s) {
-    if ((K + GK - 1) / GK <= 8)
+    if ((K + GK - 1) / GK <= 8 && !cs.x1)
         return launch_pipe<CONV, BN, 2>(A, lda, B, ldb, C, ldc, M, N, K, bias, relu, out_mode, err, cs, s);
-    return launch_pipe<CONV, BN, 4>(A, lda, B, ldb, C, ldc, M, N, K, bias, relu, out_mode, err, cs, s);
+    return launch_ring<CONV, BN>(A, lda, B, ldb, C, ldc, M, N, K, bias, relu, out_mode, err, cs, s);
 }
 
 template <bool CONV>
@@ -439,12 +617,12 @@ extern "C" int glide_gemm_bf16(const void* A, int lda, const void* B, int ldb, v
     if (M < 1 || N < 1 || K < 1 || lda < K || ldb < K || ldc < N || out_mode < 0 || out_mode > 2) return GLIDE_E_SHAPE;
     if (K % 8 == 0 && lda % 8 == 0 && ldb % 8 == 0 && glide::al16(A) && glide::al16(B))
         return glide::launch_pipe_n<false>((const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)B, ldb, C, ldc, M, N, K,
-                                           bias, relu, out_mode, err, glide::ConvShape{0, 0, 0, 0},
+                                           bias, relu, out_mode, err, glide::ConvShape{},
                                            (cudaStream_t)stream);
     dim3 grid((M + glide::GM - 1) / glide::GM, (N + glide::GN - 1) / glide::GN);
     glide::count_launch(), glide::tc_gemm_kernel<false><<<grid, glide::GTHREADS, 0, (cudaStream_t)stream>>>(
         (const __nv_bfloat16*)A, lda, (const __nv_bfloat16*)B, ldb, C, ldc, M, N, K, bias, relu, out_mode, err,
-        glide::ConvShape{0, 0, 0, 0});
+        glide::ConvShape{});
     return (int)cudaGetLastError();
 }
 
@@ -463,11 +641,31 @@ extern "C" int glide_conv3x3_bf16(const void* x, int Bn, int H, int W, int C, co
     if (rc != -1000) return rc;
     if (ldw % 8 == 0 && glide::al16(Wt))
         return glide::launch_pipe_n<true>((const __nv_bfloat16*)x, 0, (const __nv_bfloat16*)Wt, ldw, out, ldc, M, N, K,
-                                          bias, relu, out_mode, err, glide::ConvShape{Bn, H, W, C},
+                                          bias, relu, out_mode, err, glide::ConvShape{Bn, H, W, C, nullptr, C, 0},
                                           (cudaStream_t)stream);
     dim3 grid((M + glide::GM - 1) / glide::GM, (N + glide::GN - 1) / glide::GN);
     glide::count_launch(), glide::tc_gemm_kernel<true><<<grid, glide::GTHREADS, 0, (cudaStream_t)stream>>>(
         (const __nv_bfloat16*)x, 0, (const __nv_bfloat16*)Wt, ldw, out, ldc, M, N, K, bias, relu, out_mode, err,
-        glide::ConvShape{Bn, H, W, C});
+        glide::ConvShape{Bn, H, W, C, nullptr, C, 0});
     return (int)cudaGetLastError();
+}
+
+extern "C" int glide_conv3x3_cat_bf16(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W,
+                                      const void* Wt, int ldw, void* out, int ldc, int N, const float* bias, int relu,
+                                      int out_mode, int* err, void* stream) {
+    if (!x0 || !x1 || !Wt || !out) return GLIDE_E_NULL;
+    const int C = C0 + C1;
+    if (Bn < 1 || H < 1 || W < 1 || C0 < 8 || C0 % 8 != 0 || C1 < 8 || C1 % 8 != 0 || N < 1 || ldw < 9 * C || ldc < N ||
+        ldw % 8 != 0 || out_mode < 0 || out_mode > 2 || (up0 && (H % 2 || W % 2)))
+        return GLIDE_E_SHAPE;
+    if (!glide::al16(x0) || !glide::al16(x1) || !glide::al16(Wt)) return GLIDE_E_SHAPE;
+    const int64_t M64 = int64_t(Bn) * H * W;
+    if (M64 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
+    const int rc = glide::try_conv_rows(x0, C0, up0, x1, C1, Bn, H, W, Wt, ldw, out, ldc, N, bias, relu, out_mode, err,
+                                        (cudaStream_t)stream);
+    if (rc != -1000) return rc;
+    return glide::launch_pipe_n<true>((const __nv_bfloat16*)x0, 0, (const __nv_bfloat16*)Wt, ldw, out, ldc, int(M64), N,
+                                      9 * C, bias, relu, out_mode, err,
+                                      glide::ConvShape{Bn, H, W, C, (const __nv_bfloat16*)x1, C0, up0},
+                                      (cudaStream_t)stream);
 }

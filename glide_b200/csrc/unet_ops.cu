@@ -74,6 +74,28 @@ __global__ void transpose_bf16_k(const __nv_bfloat16* __restrict__ src, __nv_bfl
     }
 }
 
+// 2x2 average, 8 channels per thread (glide_b200.guess._pool in one pass)
+__global__ void pool2_k(const uint4* __restrict__ x, uint4* __restrict__ y, int Ho, int Wo, int C8, int64_t total) {
+    const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (idx >= total) return;
+    const int c = int(idx % C8);
+    const int64_t p = idx / C8;
+    const int xo = int(p % Wo);
+    const int64_t row = p / Wo;   // image and output row
+    const uint4* s = x + ((2 * row) * (2 * Wo) + 2 * xo) * C8 + c;
+    const int64_t down = int64_t(2 * Wo) * C8;
+    const uint4 q[4] = {__ldg(s), __ldg(s + C8), __ldg(s + down), __ldg(s + down + C8)};
+    __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) {
+        float v[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(&q[k])[e]);
+        h[e] = __float2bfloat16(((v[0] + v[1]) + (v[2] + v[3])) * 0.25f);
+    }
+    y[idx] = *reinterpret_cast<const uint4*>(h);
+}
+
 static inline unsigned blocks_for(int64_t n) {
     int64_t b = (n + 255) / 256;
     return unsigned(b > 148 * 64 ? 148 * 64 : (b < 1 ? 1 : b));
@@ -103,5 +125,16 @@ extern "C" int glide_transpose_bf16(const void* src, void* dst, int R, int Cc, v
     dim3 grid((Cc + 31) / 32, (R + 31) / 32);
     glide::count_launch(), glide::transpose_bf16_k<<<grid, dim3(32, 8), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)src,
                                                                            (__nv_bfloat16*)dst, R, Cc);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int glide_pool2_bf16(const void* x, void* y, int Bn, int H, int W, int C, void* stream) {
+    if (!x || !y) return GLIDE_E_NULL;
+    if (Bn < 1 || H < 2 || W < 2 || H % 2 || W % 2 || C < 8 || C % 8) return GLIDE_E_SHAPE;
+    if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) return GLIDE_E_SHAPE;
+    const int64_t total = int64_t(Bn) * (H / 2) * (W / 2) * (C / 8);
+    if ((total + 255) / 256 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
+    glide::count_launch(), glide::pool2_k<<<unsigned((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (const uint4*)x, (uint4*)y, H / 2, W / 2, C / 8, total);
     return (int)cudaGetLastError();
 }

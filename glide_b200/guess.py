@@ -50,6 +50,12 @@ def _lib():
                                                                           C.c_int, C.c_void_p, C.c_int, C.c_int,
                                                                           C.c_void_p, C.c_void_p]
         lib.glide_conv3x3_bf16.restype = C.c_int
+        lib.glide_conv3x3_cat_bf16.argtypes = ([C.c_void_p, C.c_int, C.c_int, C.c_void_p] + [C.c_int] * 4 +
+                                               [C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p,
+                                                C.c_int, C.c_int, C.c_void_p, C.c_void_p])
+        lib.glide_conv3x3_cat_bf16.restype = C.c_int
+        lib.glide_pool2_bf16.argtypes = [C.c_void_p, C.c_void_p] + [C.c_int] * 4 + [C.c_void_p]
+        lib.glide_pool2_bf16.restype = C.c_int
         lib._guess_sigs = True
     return lib
 
@@ -129,6 +135,23 @@ def conv3x3_relu(x, W, b, relu=True):
     return y.view(Bn, H, Wd, Cout)
 
 
+def conv3x3_up_cat(x, skip, W, b):
+    """conv3x3_relu(cat([_up(x), skip]), W, b).  Without autograd recording the
+    convolution reads both tensors directly (bit-identical)."""
+    if (torch.is_grad_enabled() and any(t.requires_grad for t in (x, skip, W, b))) or \
+            x.shape[3] % 8 != 0 or skip.shape[3] % 8 != 0:
+        return conv3x3_relu(torch.cat([_up(x), skip], dim=3), W, b)
+    Bn, H, Wd, C1 = skip.shape
+    x, skip = x.contiguous(), skip.contiguous()
+    Wb = W.detach().to(torch.bfloat16).contiguous()
+    y = torch.empty((Bn, H, Wd, W.shape[0]), dtype=torch.bfloat16, device=x.device)
+    rc = _lib().glide_conv3x3_cat_bf16(x.data_ptr(), x.shape[3], 1, skip.data_ptr(), C1, Bn, H, Wd, Wb.data_ptr(),
+                                       Wb.shape[1], y.data_ptr(), y.shape[3], y.shape[3], b.detach().data_ptr(), 1, 1,
+                                       _err_flag(x.device).data_ptr(), N.stream_handle())
+    N.check(rc, "tensor-core conv3x3 (two sources)")
+    return y
+
+
 class Conv3x3ReLU(torch.autograd.Function):
     """y = relu(conv3x3(x, W) + b); x NHWC BF16, W (Cout, 9*Cin) FP32 master."""
 
@@ -198,6 +221,10 @@ class Conv1x1(torch.autograd.Function):
 
 def _pool(x):
     Bn, H, W, Cc = x.shape
+    if not (torch.is_grad_enabled() and x.requires_grad) and Cc % 8 == 0 and x.is_contiguous():
+        y = torch.empty((Bn, H // 2, W // 2, Cc), dtype=torch.bfloat16, device=x.device)
+        N.check(_lib().glide_pool2_bf16(x.data_ptr(), y.data_ptr(), Bn, H, W, Cc, N.stream_handle()), "pool")
+        return y
     return x.view(Bn, H // 2, 2, W // 2, 2, Cc).float().mean((2, 4)).to(torch.bfloat16)
 
 
@@ -246,8 +273,7 @@ class UNet(torch.nn.Module):
                 skips.append(x)
                 x = _pool(x)
         for k in range(self.levels - 2, -1, -1):
-            x = torch.cat([_up(x), skips[k]], dim=3)
-            x = conv3x3_relu(x, self.ws[i], self.bs[i]); i += 1
+            x = conv3x3_up_cat(x, skips[k], self.ws[i], self.bs[i]); i += 1
             x = conv3x3_relu(x, self.ws[i], self.bs[i]); i += 1
         return Conv1x1.apply(x, self.head_w, self.head_b)
 

@@ -304,6 +304,18 @@ int glide_gemm_bf16(const void* A, int lda, const void* B, int ldb, void* C, int
  * glide_gemm_bf16 with Kp = 9C. */
 int glide_conv3x3_bf16(const void* x, int Bn, int H, int W, int C, const void* Wt, int ldw, void* out, int ldc, int N,
                        const float* bias, int relu, int out_mode, int* err, void* stream);
+/* The same convolution on the channel concatenation of two NHWC BF16 tensors,
+ * x0 (C0 channels; with up0 != 0 at half resolution (Bn, H/2, W/2, C0), read
+ * by nearest upsampling) and x1 (Bn, H, W, C1): neither the upsampled nor the
+ * joined tensor is formed.  C0 and C1 multiples of 8, x0, x1 and Wt 16-byte
+ * aligned, ldw a multiple of 8.  Bit-identical to glide_conv3x3_bf16 on the
+ * joined tensor. */
+int glide_conv3x3_cat_bf16(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W,
+                           const void* Wt, int ldw, void* out, int ldc, int N, const float* bias, int relu,
+                           int out_mode, int* err, void* stream);
+/* y (Bn, H/2, W/2, C) = 2x2 averages of NHWC BF16 x (Bn, H, W, C), summed in
+ * FP32; H and W even, C a multiple of 8, 16-byte aligned. */
+int glide_pool2_bf16(const void* x, void* y, int Bn, int H, int W, int C, void* stream);
 /* im2col of a 3x3 same convolution on NHWC BF16 x (Bn,H,W,C) into col (Bn*H*W, Kp), Kp >= 9C (zero pad). */
 int glide_im2col3_bf16(const void* x, void* col, int Bn, int H, int W, int C, int Kp, void* stream);
 /* Transpose of im2col (gather form): dx (Bn,H,W,C) FP32 from dcol (Bn*H*W, Kp) FP32. */

@@ -19,7 +19,7 @@ def _inputs(Bn, H, W, C, N):
 @pytest.mark.parametrize("Bn,H,W,C,N,out_mode", [
     (1, 1, 64, 8, 32, 1), (2, 9, 129, 8, 32, 1), (1, 300, 257, 8, 40, 0), (2, 7, 130, 32, 32, 1),
     (1, 700, 128, 32, 64, 1), (3, 33, 70, 16, 5, 0), (1, 40, 200, 96, 32, 1), (1, 30, 256, 64, 64, 1),
-    (1, 21, 128, 192, 64, 0), (2, 17, 127, 128, 128, 1)])
+    (1, 21, 128, 192, 64, 0), (2, 17, 127, 128, 128, 1), (1, 9, 100, 256, 256, 1), (2, 5, 37, 72, 96, 0)])
 def test_conv_rows_equals_im2col_gemm(Bn, H, W, C, N, out_mode):
     from glide_b200.guess import _err_flag, conv3x3, gemm, im2col3
     x, Wb, bias = _inputs(Bn, H, W, C, N)
@@ -31,3 +31,30 @@ def test_conv_rows_equals_im2col_gemm(Bn, H, W, C, N, out_mode):
     torch.cuda.synchronize()
     assert int(_err_flag(x.device).item()) == 0
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("Bn,H,W,C0,C1,N", [(1, 2, 128, 64, 32, 32), (2, 34, 130, 128, 64, 64), (1, 16, 66, 256, 128, 128),
+                                            (2, 6, 10, 8, 16, 24)])
+def test_two_source_conv_equals_joined(Bn, H, W, C0, C1, N):
+    """Upsampling and concatenation read inside the convolution: the same bits
+    as on the joined tensor (row march, specialised GEMM, narrow images)."""
+    from glide_b200.guess import _up, conv3x3_relu, conv3x3_up_cat
+    g = torch.Generator(device="cuda").manual_seed(H + W + C0)
+    x = torch.randn(Bn, H // 2, W // 2, C0, generator=g, device="cuda").to(torch.bfloat16)
+    skip = torch.randn(Bn, H, W, C1, generator=g, device="cuda").to(torch.bfloat16)
+    Wf = torch.randn(N, 9 * (C0 + C1), generator=g, device="cuda") * 0.1
+    b = torch.randn(N, generator=g, device="cuda")
+    ref = conv3x3_relu(torch.cat([_up(x), skip], dim=3), Wf, b)
+    assert torch.equal(conv3x3_up_cat(x, skip, Wf, b), ref)
+
+
+@pytest.mark.parametrize("shape", [(1, 2, 2, 8), (2, 34, 50, 32), (1, 16, 66, 64)])
+def test_pool_equals_mean(shape):
+    """One-pass pooling against the torch expression (the sums of four BF16
+    values differ by an FP32 rounding at most, i.e. by at most one BF16 step)."""
+    from glide_b200.guess import _pool
+    g = torch.Generator(device="cuda").manual_seed(shape[1])
+    x = torch.randn(shape, generator=g, device="cuda").to(torch.bfloat16)
+    Bn, H, W, Cc = shape
+    ref = x.view(Bn, H // 2, 2, W // 2, 2, Cc).float().mean((2, 4))
+    assert (_pool(x).float() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item()
