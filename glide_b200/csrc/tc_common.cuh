@@ -54,6 +54,11 @@ __device__ __forceinline__ uint32_t umma_hi(uint32_t sbo_bytes) { return ((sbo_b
 // is one shared-memory line, so cp.async copies of it stay coalesced; a K step
 // of 16 is 32 bytes.
 __device__ __forceinline__ uint32_t umma_hi_sw128() { return (1024u >> 4) | (1u << 14) | (2u << 29); }
+// MN-major operand in 64-byte rows of 32 elements, one row per k, entries
+// permuted (entry ^ (row / 2) % 4); groups of 8 rows are 512 bytes apart, the
+// leading offset is the step to the next 32 elements; a K step of 16 is 1024
+// bytes.
+__device__ __forceinline__ uint32_t umma_hi_mn_sw64() { return (512u >> 4) | (1u << 14) | (4u << 29); }
 __device__ __forceinline__ void mma_bf16_lead(uint32_t tmem, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi,
                                               uint32_t idesc, uint32_t acc, uint32_t lead) {
     asm volatile(
@@ -100,6 +105,7 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity) {
 }
 
 __device__ __forceinline__ bool mbar_wait_bounded(uint32_t addr, uint32_t parity) {
+    if (mbar_try(addr, parity)) return true;
     const long long t0 = clock64();
     while (!mbar_try(addr, parity)) {
         if (clock64() - t0 > WAIT_CYCLES) return false;

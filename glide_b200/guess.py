@@ -56,6 +56,12 @@ def _lib():
         lib.glide_conv3x3_cat_bf16.restype = C.c_int
         lib.glide_pool2_bf16.argtypes = [C.c_void_p, C.c_void_p] + [C.c_int] * 4 + [C.c_void_p]
         lib.glide_pool2_bf16.restype = C.c_int
+        lib.glide_conv3x3_wgrad_bf16.argtypes = [C.c_void_p] * 3 + [C.c_int] * 5 + [C.c_void_p, C.c_void_p]
+        lib.glide_conv3x3_wgrad_bf16.restype = C.c_int
+        lib.glide_relu_grad_bf16.argtypes = [C.c_void_p] * 5 + [C.c_int64, C.c_int, C.c_int, C.c_void_p]
+        lib.glide_relu_grad_bf16.restype = C.c_int
+        lib.glide_relu_grad_blocks.argtypes = [C.c_int64, C.c_int]
+        lib.glide_relu_grad_blocks.restype = C.c_int
         lib._guess_sigs = True
     return lib
 
@@ -152,8 +158,25 @@ def conv3x3_up_cat(x, skip, W, b):
     return y
 
 
+def _relu_grad(gy, y, relu):
+    """(gz, db): gy masked by y > 0 in BF16 and its channel sums in FP32, one pass."""
+    P, Cout = y.shape
+    lib = _lib()
+    gz = torch.empty_like(y)
+    db = torch.empty(Cout, dtype=torch.float32, device=y.device)
+    parts = torch.empty(lib.glide_relu_grad_blocks(P, Cout) * Cout, dtype=torch.float32, device=y.device)
+    N.check(lib.glide_relu_grad_bf16(gy.data_ptr(), y.data_ptr(), gz.data_ptr(), db.data_ptr(), parts.data_ptr(), P,
+                                     Cout, int(relu), N.stream_handle()), "relu gradient")
+    return gz, db
+
+
 class Conv3x3ReLU(torch.autograd.Function):
-    """y = relu(conv3x3(x, W) + b); x NHWC BF16, W (Cout, 9*Cin) FP32 master."""
+    """y = relu(conv3x3(x, W) + b); x NHWC BF16, W (Cout, 9*Cin) FP32 master.
+
+    With Cin and Cout multiples of 8 no im2col matrix exists in either
+    direction: the forward product, the data gradient (the convolution of gz
+    with the flipped kernel) and the weight gradient gather their shifted
+    pixels themselves.  Other widths run im2col + GEMM."""
 
     @staticmethod
     def forward(ctx, x, W, b, relu: bool):
@@ -162,26 +185,43 @@ class Conv3x3ReLU(torch.autograd.Function):
         x = x.contiguous()
         Wb = W.to(torch.bfloat16).contiguous()
         y = torch.empty((Bn * H * Wd, Cout), dtype=torch.bfloat16, device=x.device)
-        col = im2col3(x)
-        gemm(col, Wb, y, bias=b, relu=relu, out_mode=1)
-        ctx.save_for_backward(col, Wb, y)
+        ctx.implicit = Cin % 8 == 0 and Cout % 8 == 0 and Cout <= 2048
+        if ctx.implicit:
+            conv3x3(x, Wb, y, bias=b, relu=relu, out_mode=1)
+            ctx.save_for_backward(x, Wb, y)
+        else:
+            col = im2col3(x)
+            gemm(col, Wb, y, bias=b, relu=relu, out_mode=1)
+            ctx.save_for_backward(col, Wb, y)
         ctx.shape = (Bn, H, Wd, Cin)
         ctx.relu = relu
         return y.view(Bn, H, Wd, Cout)
 
     @staticmethod
     def backward(ctx, gy):
-        col, Wb, y = ctx.saved_tensors
+        src, Wb, y = ctx.saved_tensors
         Bn, H, Wd, Cin = ctx.shape
         Cout = Wb.shape[0]
         P = Bn * H * Wd
+        if ctx.implicit:
+            gy = gy.reshape(P, Cout).to(torch.bfloat16).contiguous()
+            gz, db = _relu_grad(gy, y.reshape(P, Cout), ctx.relu)
+            dW = torch.empty((Cout, 9 * Cin), dtype=torch.float32, device=gy.device)
+            N.check(_lib().glide_conv3x3_wgrad_bf16(gz.data_ptr(), src.data_ptr(), dW.data_ptr(), Bn, H, Wd, Cin, Cout,
+                                                    _err_flag(gy.device).data_ptr(), N.stream_handle()),
+                    "weight gradient")
+            # data gradient: gz convolved with the kernel flipped in both directions, channels exchanged
+            Wf = Wb.view(Cout, 3, 3, Cin).flip(1, 2).permute(3, 1, 2, 0).reshape(Cin, 9 * Cout)
+            dx = torch.empty((Bn, H, Wd, Cin), dtype=torch.bfloat16, device=gy.device)
+            conv3x3(gz.view(Bn, H, Wd, Cout), Wf, dx.view(P, Cin), out_mode=1)
+            return dx, dW, db, None
         g = gy.reshape(P, Cout).float()
         if ctx.relu:
             g = g * (y > 0)
         gz = g.to(torch.bfloat16).contiguous()
         # weight gradient: dW (Cout x 9Cin) = gz^T (Cout x P) . col (P x 9Cin)
         dW = torch.zeros((Cout, 9 * Cin), dtype=torch.float32, device=gy.device)
-        gemm(transpose(gz), transpose(col), dW, out_mode=0)
+        gemm(transpose(gz), transpose(src), dW, out_mode=0)
         db = g.sum(0)
         # data gradient: dcol (P x 9Cin) = gz (P x Cout) . W (Cout x 9Cin)
         dcol = torch.empty((P, 9 * Cin), dtype=torch.float32, device=gy.device)

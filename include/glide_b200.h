@@ -313,6 +313,20 @@ int glide_conv3x3_bf16(const void* x, int Bn, int H, int W, int C, const void* W
 int glide_conv3x3_cat_bf16(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W,
                            const void* Wt, int ldw, void* out, int ldc, int N, const float* bias, int relu,
                            int out_mode, int* err, void* stream);
+/* Weight gradient of the same convolution: dW (N, 9C) FP32, dW[n, tap*C + c] =
+ * sum over the pixels p of gz[p, n] * x[p shifted by tap, c] (zero outside the
+ * image); gz (Bn*H*W, N) and x (Bn, H, W, C) BF16, N and C multiples of 8,
+ * 16-byte aligned.  Accumulated in FP32 pixel after pixel: bit-identical to
+ * glide_gemm_bf16 on the transposes of gz and of the im2col matrix. */
+int glide_conv3x3_wgrad_bf16(const void* gz, const void* x, float* dW, int Bn, int H, int W, int C, int N, int* err,
+                             void* stream);
+/* Backward of bias + ReLU of a (P, N) BF16 layer output y: gz = gy where y > 0
+ * (gy itself without relu; y may then be null) and db[n] = the sum of gz over
+ * p.  N a multiple of 8 (at most 2048), 16-byte aligned; parts:
+ * glide_relu_grad_blocks(P, N) * N floats of scratch. */
+int glide_relu_grad_bf16(const void* gy, const void* y, void* gz, float* db, float* parts, int64_t P, int N, int relu,
+                         void* stream);
+int glide_relu_grad_blocks(int64_t P, int N);
 /* y (Bn, H/2, W/2, C) = 2x2 averages of NHWC BF16 x (Bn, H, W, C), summed in
  * FP32; H and W even, C a multiple of 8, 16-byte aligned. */
 int glide_pool2_bf16(const void* x, void* y, int Bn, int H, int W, int C, void* stream);

@@ -58,3 +58,43 @@ def test_pool_equals_mean(shape):
     Bn, H, W, Cc = shape
     ref = x.view(Bn, H // 2, 2, W // 2, 2, Cc).float().mean((2, 4))
     assert (_pool(x).float() - ref).abs().max().item() <= 2.0 ** -8 * ref.abs().max().item()
+
+
+@pytest.mark.parametrize("Bn,H,W,C,N", [(1, 1, 3, 8, 8), (2, 9, 13, 40, 24), (1, 16, 16, 32, 136), (3, 20, 37, 64, 64),
+                                         (2, 3, 128, 32, 32), (1, 7, 384, 40, 24), (3, 8, 32, 96, 160)])
+def test_weight_gradient_equals_transposed_gemm(Bn, H, W, C, N):
+    """Pixels as the contraction, read in place: the same bits as the GEMM on
+    the transposes of gz and of the im2col matrix (ragged pixel count and
+    channel tiles, more than 128 output channels)."""
+    from glide_b200 import _native as NT
+    from glide_b200.guess import _err_flag, _lib, gemm, im2col3, transpose
+    g = torch.Generator(device="cuda").manual_seed(H + W + C + N)
+    x = torch.randn(Bn, H, W, C, generator=g, device="cuda").to(torch.bfloat16)
+    gz = torch.randn(Bn * H * W, N, generator=g, device="cuda").to(torch.bfloat16)
+    P = Bn * H * W
+    # the pixel count padded to a multiple of 8 with zero rows keeps the GEMM on its aligned kernel
+    pad = (-P) % 8
+    zp, cp = (torch.cat([t, t.new_zeros(pad, t.shape[1])]) for t in (gz, im2col3(x)))
+    ref = torch.empty(N, 9 * C, device="cuda")
+    gemm(transpose(zp), transpose(cp), ref)
+    out = torch.full_like(ref, float("nan"))
+    NT.check(_lib().glide_conv3x3_wgrad_bf16(gz.data_ptr(), x.data_ptr(), out.data_ptr(), Bn, H, W, C, N,
+                                             _err_flag(x.device).data_ptr(), NT.stream_handle()), "wgrad")
+    torch.cuda.synchronize()
+    assert int(_err_flag(x.device).item()) == 0
+    assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("P,N,relu", [(1, 8, True), (1000, 24, True), (70000, 256, True), (333, 32, False)])
+def test_relu_gradient_and_bias_sum(P, N, relu):
+    """gz exactly; db within FP32 summation error, P eps of the sum of |gz|
+    (each block adds at most P values in FP32)."""
+    from glide_b200.guess import _relu_grad
+    g = torch.Generator(device="cuda").manual_seed(P)
+    gy = torch.randn(P, N, generator=g, device="cuda").to(torch.bfloat16)
+    y = torch.relu(torch.randn(P, N, generator=g, device="cuda")).to(torch.bfloat16)
+    gz, db = _relu_grad(gy, y, relu)
+    ref = gy.float() * (y > 0) if relu else gy.float()
+    assert torch.equal(gz.float(), ref)
+    err = (db.double() - ref.double().sum(0)).abs()
+    assert bool((err <= min(P, 4096) * 6e-8 * ref.double().abs().sum(0) + 1e-30).all())
