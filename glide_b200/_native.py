@@ -27,7 +27,7 @@ SYMBOLS = [
     "glide_noalloc_scratch_bytes", "glide_vanka_sweeps_ex", "glide_vanka_lu", "glide_vanka_linear",
     "glide_misfit", "glide_tikhonov", "glide_loss_parts", "glide_jvp_add",
     "glide_linear_setup", "glide_linear_vcycle", "glide_vanka_lu_masked", "glide_newton_rhs", "glide_newton_update",
-    "glide_active_mask", "glide_dots", "glide_dots_parts", "glide_combine",
+    "glide_active_mask", "glide_vanka_adjoint_sweeps", "glide_dots", "glide_dots_parts", "glide_combine",
 ]
 
 
@@ -54,9 +54,10 @@ class Level(C.Structure):
                 ("scratch", C.c_void_p), ("flags", C.c_void_p), ("any_active", C.c_void_p),
                 ("ls_tmp", C.c_void_p), ("ls_norms", C.c_void_p), ("norm_parts", C.c_void_p),
                 ("lu", C.c_void_p), ("lin_rhs", C.c_void_p), ("lin_rho", C.c_void_p), ("lin_d", C.c_void_p),
-                ("r_raw", C.c_void_p)]
+                ("r_raw", C.c_void_p), ("adj_factors", C.c_void_p)]
 
 LS_CANDIDATES = 4  # GLIDE_LS_CANDIDATES
+ADJ_FACTORS = 18   # GLIDE_ADJ_FACTORS
 
 
 class SolverConfig(C.Structure):
@@ -104,6 +105,7 @@ def load():
         "glide_error_mask": [LA, vp, vp, vp, d, vp, vp, vp, vp],
         "glide_tile_flags": [LA, vp, vp, vp, vp],
         "glide_vanka_adjoint": [LA, vp, vp, vp, vp, vp, vp, i, d, vp],
+        "glide_vanka_adjoint_sweeps": [LA] + [vp] * 9 + [i, d, i, vp, vp],
         "glide_restrict": [i, i, i, vp, vp, i, i, i, vp],
         "glide_prolong": [i, i, i, i, vp, vp, i, i, i, vp],
         "glide_lincomb": [i, vp, vp, d, vp, d, i64, vp],

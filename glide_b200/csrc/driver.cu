@@ -24,7 +24,9 @@ template <typename T> int launch_vjp(const GlideLevelArgs*, const void*, const v
 template <typename T> int launch_grad_beta(const GlideLevelArgs*, const void*, const void*, void*, int, cudaStream_t);
 template <typename T> int launch_vanka_sweeps(const GlideLevelArgs*, const void*, const void*, const void*, int, int, double, double, const int*, const int*, void*, cudaStream_t, double, int);
 template <typename T> int launch_vanka_lu(const GlideLevelArgs*, const void*, void*, double, cudaStream_t);
-template <typename T> int launch_vanka_linear(const GlideLevelArgs*, const void*, const void*, const void*, const void*, void*, void*, void*, double, void*, cudaStream_t);
+template <typename T> int launch_vanka_linear(const GlideLevelArgs*, const void*, const void*, const void*, const void*, void*, void*, void*, double, cudaStream_t);
+template <typename T> int launch_adjoint_factors(const GlideLevelArgs*, void*, cudaStream_t);
+template <typename T> int launch_adjoint_color(const GlideLevelArgs*, const void*, void*, void*, void*, const void*, const void*, const void*, int, double, cudaStream_t);
 template <typename T> int launch_vanka_cells(const GlideLevelArgs*, const void*, const void*, const void*, int, int, double, const int*, const int*, void*, cudaStream_t, double);
 template <typename T> int launch_error_mask(const GlideLevelArgs*, const void*, const void*, const void*, double, void*, int*, int*, cudaStream_t);
 template <typename T> int launch_tile_flags(const GlideLevelArgs*, const void*, int*, int*, cudaStream_t);
@@ -169,9 +171,8 @@ int glide_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* r
     if (e) return e;
     if (!rho_u || !rho_v || !rho_H || !lu || !d_u || !d_v || !d_H || !scratch) return GLIDE_E_NULL;
     return TDISPATCH(a->dtype,
-                     launch_vanka_linear<float>(a, rho_u, rho_v, rho_H, lu, d_u, d_v, d_H, omega, scratch, S(stream)),
-                     launch_vanka_linear<double>(a, rho_u, rho_v, rho_H, lu, d_u, d_v, d_H, omega, scratch,
-                                                 S(stream)));
+                     launch_vanka_linear<float>(a, rho_u, rho_v, rho_H, lu, d_u, d_v, d_H, omega, S(stream)),
+                     launch_vanka_linear<double>(a, rho_u, rho_v, rho_H, lu, d_u, d_v, d_H, omega, S(stream)));
 }
 
 int glide_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_launch,
@@ -216,6 +217,30 @@ int glide_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H
     if (color != 0 && color != 1) return GLIDE_E_SHAPE;
     return TDISPATCH(a->dtype, launch_vanka_adjoint<float>(a, l_u, l_v, l_H, ra_u, ra_v, ra_H, color, omega, S(stream)),
                      launch_vanka_adjoint<double>(a, l_u, l_v, l_H, ra_u, ra_v, ra_H, color, omega, S(stream)));
+}
+
+int glide_vanka_adjoint_sweeps(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* f_u,
+                               const void* f_v, const void* f_H, void* ra_u, void* ra_v, void* ra_H, int n_iter,
+                               double omega, int exact_boundary, void* factors, void* stream) {
+    int e = check_level(a);
+    if (e) return e;
+    if (!l_u || !l_v || !l_H || !f_u || !f_v || !f_H || !ra_u || !ra_v || !ra_H) return GLIDE_E_NULL;
+    if (n_iter < 0) return GLIDE_E_SHAPE;
+    if (n_iter > 0 && factors &&
+        (e = TDISPATCH(a->dtype, launch_adjoint_factors<float>(a, factors, S(stream)),
+                       launch_adjoint_factors<double>(a, factors, S(stream)))))
+        return e;
+    for (int k = 0; k < 2 * n_iter; k++) {
+        if ((e = glide_vjp(a, l_u, l_v, l_H, f_u, f_v, f_H, ra_u, ra_v, ra_H, exact_boundary, stream))) return e;
+        e = !factors ? glide_vanka_adjoint(a, l_u, l_v, l_H, ra_u, ra_v, ra_H, k & 1, omega, stream)
+                     : TDISPATCH(a->dtype,
+                                 launch_adjoint_color<float>(a, factors, l_u, l_v, l_H, ra_u, ra_v, ra_H, k & 1, omega,
+                                                             S(stream)),
+                                 launch_adjoint_color<double>(a, factors, l_u, l_v, l_H, ra_u, ra_v, ra_H, k & 1, omega,
+                                                              S(stream)));
+        if (e) return e;
+    }
+    return 0;
 }
 
 int glide_restrict(int dtype, int field, int use_max, const void* fine, void* coarse, int nyc, int nxc, int nb,
@@ -439,14 +464,9 @@ int adj_residual(GlideLevel* L, int exact, void* s) {
 
 int vanka_adj(GlideLevel* L, int n_iter, double omega, int exact, void* s) {
     LevelView w = view(L);
-    for (int it = 0; it < n_iter; it++) {
-        for (int color = 0; color < 2; color++) {
-            TRY(adj_residual(L, exact, s));
-            TRY(glide_vanka_adjoint(&L->a, w.u(L->lam), w.v(L->lam), w.H(L->lam), w.u(L->r_adj), w.v(L->r_adj),
-                                    w.H(L->r_adj), color, omega, s));
-        }
-    }
-    return 0;
+    return glide_vanka_adjoint_sweeps(&L->a, w.u(L->lam), w.v(L->lam), w.H(L->lam), w.u(L->f_adj), w.v(L->f_adj),
+                                      w.H(L->f_adj), w.u(L->r_adj), w.v(L->r_adj), w.H(L->r_adj), n_iter, omega, exact,
+                                      L->adj_factors, s);
 }
 
 int restrict_params(GlideLevel* L, GlideLevel* C, void* s) {

@@ -344,32 +344,6 @@ __device__ __forceinline__ EtaIn<T> eta_inputs(const T* __restrict__ u, const T*
     return a;
 }
 
-// Unpivoted Doolittle 5x5 solve, same elimination order as
-// glide/cuda/common.cu:132-175.  A is overwritten.
-template <typename T> __device__ __forceinline__ void lu5_solve(T (&A)[25], const T (&b)[5], T (&x)[5]) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        T inv = T(1) / A[k * 5 + k];
-#pragma unroll
-        for (int i = k + 1; i < 5; i++) {
-            A[i * 5 + k] *= inv;
-#pragma unroll
-            for (int j = k + 1; j < 5; j++) A[i * 5 + j] -= A[i * 5 + k] * A[k * 5 + j];
-        }
-    }
-    T y[5];
-    y[0] = b[0];
-    y[1] = b[1] - A[5] * y[0];
-    y[2] = b[2] - A[10] * y[0] - A[11] * y[1];
-    y[3] = b[3] - A[15] * y[0] - A[16] * y[1] - A[17] * y[2];
-    y[4] = b[4] - A[20] * y[0] - A[21] * y[1] - A[22] * y[2] - A[23] * y[3];
-    x[4] = y[4] / A[24];
-    x[3] = (y[3] - A[19] * x[4]) / A[18];
-    x[2] = (y[2] - A[13] * x[3] - A[14] * x[4]) / A[12];
-    x[1] = (y[1] - A[7] * x[2] - A[8] * x[3] - A[9] * x[4]) / A[6];
-    x[0] = (y[0] - A[1] * x[1] - A[2] * x[2] - A[3] * x[3] - A[4] * x[4]) / A[0];
-}
-
 // error reporting from kernels: set a device flag, never trap
 __device__ __forceinline__ void set_error(int* flag, int code) {
     if (flag) atomicCAS(flag, 0, code);

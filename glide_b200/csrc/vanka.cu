@@ -32,140 +32,6 @@ template <typename T> struct Patch {
     int i, j;
 };
 
-// Local 5x5 Jacobian and residual of cell (i,j) at the local iterate
-// (vanka.cu:56-404).  Row/column order (u_l, u_r, v_t, v_b, H_c).
-// WITH_RES adds the residual and the active-set switch (vanka.cu:104-113);
-// the adjoint variant calls it without.
-template <typename T, bool WITH_RES>
-__device__ __forceinline__ void assemble(const Patch<T>& P, T ul, T ur, T vt, T vb, T Hc, T fu_l, T fu_r, T fv_t,
-                                         T fv_b, T fH, T thklim, int ny, int nx, const Phys<T>& p, T (&J)[25],
-                                         T (&r)[5]) {
-    const int i = P.i, j = P.j;
-    const T dxi = p.dxi;
-#pragma unroll
-    for (int k = 0; k < 25; k++) J[k] = T(0);
-    if (WITH_RES) {
-        r[0] = -fu_l; r[1] = -fu_r; r[2] = -fv_t; r[3] = -fv_b; r[4] = -fH;
-    }
-    const T gc = sigmoid(P.bed_c + rho_ratio<T>() * Hc, p.sig_c);
-
-    // mass row (vanka.cu:67-115)
-    {
-        J[24] = T(1) / p.dt;
-        if (WITH_RES) r[4] += Hc / p.dt;
-        Calving<T> cv = calving_g(Hc, gc, p);
-        J[24] -= cv.d_H;
-        if (WITH_RES) r[4] -= cv.res;
-        Flux<T> ql = upwind_flux(ul, P.Hn[1][0], Hc, j > 0 && j < nx);
-        J[20] -= ql.d_vel * dxi; J[24] -= ql.d_Hb * dxi;
-        if (WITH_RES) r[4] -= ql.res * dxi;
-        Flux<T> qr = upwind_flux(ur, Hc, P.Hn[1][2], j + 1 > 0 && j + 1 < nx);
-        J[21] += qr.d_vel * dxi; J[24] += qr.d_Ha * dxi;
-        if (WITH_RES) r[4] += qr.res * dxi;
-        Flux<T> qt = upwind_flux(vt, Hc, P.Hn[0][1], i > 0 && i < ny);
-        J[22] += qt.d_vel * dxi; J[24] += qt.d_Ha * dxi;
-        if (WITH_RES) r[4] += qt.res * dxi;
-        Flux<T> qb = upwind_flux(vb, P.Hn[2][1], Hc, i + 1 > 0 && i + 1 < ny);
-        J[23] -= qb.d_vel * dxi; J[24] -= qb.d_Hb * dxi;
-        if (WITH_RES) {
-            r[4] -= qb.res * dxi;
-            if ((Hc - p.dt * r[4]) <= thklim) {
-                J[20] = T(0); J[21] = T(0); J[22] = T(0); J[23] = T(0);
-                J[24] = T(1);
-                r[4] = Hc - thklim;
-            }
-        }
-    }
-    const T (&eta)[3][3] = P.eta;
-    // own-cell normal stresses (vanka.cu:117-152)
-    {
-        const T etaH = eta[1][1] * Hc;
-        NormalStress<T> s = normal_stress<T, true>(ul, ur, vt, vb, etaH, dxi, true);
-        const T dH = s.d_etaH * eta[1][1] * dxi;
-        if (WITH_RES) { r[0] += s.res * dxi; r[1] -= s.res * dxi; }
-        J[0] += s.d_ul * dxi; J[1] += s.d_ur * dxi; J[2] += s.d_vt * dxi; J[3] += s.d_vb * dxi; J[4] += dH;
-        J[5] -= s.d_ul * dxi; J[6] -= s.d_ur * dxi; J[7] -= s.d_vt * dxi; J[8] -= s.d_vb * dxi; J[9] -= dH;
-        NormalStress<T> y = normal_stress<T, false>(ul, ur, vt, vb, etaH, dxi, true);
-        const T dHy = y.d_etaH * eta[1][1] * dxi;
-        if (WITH_RES) { r[2] -= y.res * dxi; r[3] += y.res * dxi; }
-        J[10] -= y.d_ul * dxi; J[11] -= y.d_ur * dxi; J[12] -= y.d_vt * dxi; J[13] -= y.d_vb * dxi; J[14] -= dHy;
-        J[15] += y.d_ul * dxi; J[16] += y.d_ur * dxi; J[17] += y.d_vt * dxi; J[18] += y.d_vb * dxi; J[19] += dHy;
-    }
-    // neighbour normal stresses (vanka.cu:154-208)
-    {
-        NormalStress<T> s = normal_stress<T, true>(P.u_ll, ul, P.v_lt, P.v_lb, eta[1][0] * P.Hn[1][0], dxi, j - 1 >= 0);
-        if (WITH_RES) r[0] -= s.res * dxi;
-        J[0] -= s.d_ur * dxi;
-        s = normal_stress<T, true>(ur, P.u_rr, P.v_rt, P.v_rb, eta[1][2] * P.Hn[1][2], dxi, j + 1 < nx);
-        if (WITH_RES) r[1] += s.res * dxi;
-        J[6] += s.d_ul * dxi;
-        s = normal_stress<T, false>(P.u_tl, P.u_tr, P.v_tt, vt, eta[0][1] * P.Hn[0][1], dxi, i - 1 >= 0);
-        if (WITH_RES) r[2] += s.res * dxi;
-        J[12] += s.d_vb * dxi;
-        s = normal_stress<T, false>(P.u_bl, P.u_br, vb, P.v_bb, eta[2][1] * P.Hn[2][1], dxi, i + 1 < ny);
-        if (WITH_RES) r[3] -= s.res * dxi;
-        J[18] -= s.d_vt * dxi;
-    }
-    // corner shear stresses (vanka.cu:211-311)
-    {
-        const T ec = T(0.25) * eta[1][1];
-        // top-left vertex (i,j)
-        T etaH = T(0.25) * (eta[0][0] * P.Hn[0][0] + eta[0][1] * P.Hn[0][1] + eta[1][0] * P.Hn[1][0]) + ec * Hc;
-        ShearStress<T> s = shear_stress(P.u_tl, ul, P.v_lt, vt, etaH, dxi, i > 0 && j > 0);
-        if (WITH_RES) { r[0] += s.res * dxi; r[2] -= s.res * dxi; }
-        J[0] += s.d_ub * dxi; J[4] += s.d_etaH * ec * dxi;
-        J[12] -= s.d_vr * dxi; J[14] -= s.d_etaH * ec * dxi;
-        // top-right vertex (i,j+1)
-        etaH = T(0.25) * (eta[0][1] * P.Hn[0][1] + eta[0][2] * P.Hn[0][2] + eta[1][2] * P.Hn[1][2]) + ec * Hc;
-        s = shear_stress(P.u_tr, ur, vt, P.v_rt, etaH, dxi, i > 0 && j + 1 < nx);
-        if (WITH_RES) { r[1] += s.res * dxi; r[2] += s.res * dxi; }
-        J[6] += s.d_ub * dxi; J[9] += s.d_etaH * ec * dxi;
-        J[12] += s.d_vl * dxi; J[14] += s.d_etaH * ec * dxi;
-        // bottom-left vertex (i+1,j)
-        etaH = T(0.25) * (eta[1][0] * P.Hn[1][0] + eta[2][0] * P.Hn[2][0] + eta[2][1] * P.Hn[2][1]) + ec * Hc;
-        s = shear_stress(ul, P.u_bl, P.v_lb, vb, etaH, dxi, i + 1 < ny && j > 0);
-        if (WITH_RES) { r[0] -= s.res * dxi; r[3] -= s.res * dxi; }
-        J[0] -= s.d_ut * dxi; J[4] -= s.d_etaH * ec * dxi;
-        J[18] -= s.d_vr * dxi; J[19] -= s.d_etaH * ec * dxi;
-        // bottom-right vertex (i+1,j+1)
-        etaH = T(0.25) * (eta[1][2] * P.Hn[1][2] + eta[2][1] * P.Hn[2][1] + eta[2][2] * P.Hn[2][2]) + ec * Hc;
-        s = shear_stress(ur, P.u_br, vb, P.v_rb, etaH, dxi, i + 1 < ny && j + 1 < nx);
-        if (WITH_RES) { r[1] -= s.res * dxi; r[3] += s.res * dxi; }
-        J[6] -= s.d_ut * dxi; J[9] -= s.d_etaH * ec * dxi;
-        J[18] += s.d_vl * dxi; J[19] += s.d_etaH * ec * dxi;
-    }
-    // basal drag (vanka.cu:314-364)
-    {
-        BasalDrag<T> d = basal_drag_g(ul, P.g_l, gc, P.beta_l, P.beta_c, p);
-        if (WITH_RES) r[0] += d.res;
-        J[0] += d.d_vel; J[4] += d.d_H2;
-        d = basal_drag_g(ur, gc, P.g_r, P.beta_c, P.beta_r, p);
-        if (WITH_RES) r[1] += d.res;
-        J[6] += d.d_vel; J[9] += d.d_H1;
-        d = basal_drag_g(vt, P.g_t, gc, P.beta_t, P.beta_c, p);
-        if (WITH_RES) r[2] += d.res;
-        J[12] += d.d_vel; J[14] += d.d_H2;
-        d = basal_drag_g(vb, gc, P.g_b, P.beta_c, P.beta_b, p);
-        if (WITH_RES) r[3] += d.res;
-        J[18] += d.d_vel; J[19] += d.d_H1;
-    }
-    // driving stress (vanka.cu:366-404); y-faces: m = bottom, p = top
-    {
-        Driving<T> d = driving(P.Hn[1][0], Hc, P.bed_l, P.bed_c, dxi, j > 0 && j < nx);
-        if (WITH_RES) r[0] -= d.res;
-        J[4] -= d.d_Hp;
-        d = driving(Hc, P.Hn[1][2], P.bed_c, P.bed_r, dxi, j + 1 < nx);
-        if (WITH_RES) r[1] -= d.res;
-        J[9] -= d.d_Hm;
-        d = driving(Hc, P.Hn[0][1], P.bed_c, P.bed_t, dxi, i > 0 && i < ny);
-        if (WITH_RES) r[2] -= d.res;
-        J[14] -= d.d_Hm;
-        d = driving(P.Hn[2][1], Hc, P.bed_b, P.bed_c, dxi, i + 1 < ny);
-        if (WITH_RES) r[3] -= d.res;
-        J[19] -= d.d_Hp;
-    }
-}
-
 // Fill the eta window of a VYxVX tile (+ ring) and the frozen patch of the
 // calling thread's cell.
 template <typename T>
@@ -547,119 +413,6 @@ __global__ void __launch_bounds__(VNT, sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS
     scratch[4 * nc + ic] = Hc - H0;
 }
 
-// --------------------------------------------------------------------------
-// Linear Vanka for defect correction (no counterpart in the reference): the
-// local 5x5 matrix of each cell at the current state (the same matrix the
-// first Newton iteration of vanka_cells_kernel factors) is factored once and
-// stored; each sweep then solves it against the cell's part of the linear
-// residual rho = r + J d, giving the additive-Vanka update of the correction
-// d with the H >= gamma bound applied to H + d_H.
-// --------------------------------------------------------------------------
-template <typename T>
-__device__ __forceinline__ void lu5_factor(T (&A)[25]) {
-#pragma unroll
-    for (int k = 0; k < 5; k++) {
-        const T inv = M<T>::rcp(A[k * 5 + k]);
-#pragma unroll
-        for (int i = k + 1; i < 5; i++) {
-            A[i * 5 + k] *= inv;
-#pragma unroll
-            for (int j = k + 1; j < 5; j++) A[i * 5 + j] -= A[i * 5 + k] * A[k * 5 + j];
-        }
-        A[k * 5 + k] = inv;  // stored as the reciprocal pivot
-    }
-}
-template <typename T>
-__device__ __forceinline__ void lu5_subst(const T (&A)[25], const T (&b)[5], T (&x)[5]) {
-    T y1 = b[1] - A[5] * b[0];
-    T y2 = b[2] - A[10] * b[0] - A[11] * y1;
-    T y3 = b[3] - A[15] * b[0] - A[16] * y1 - A[17] * y2;
-    T y4 = b[4] - A[20] * b[0] - A[21] * y1 - A[22] * y2 - A[23] * y3;
-    x[4] = y4 * A[24];
-    x[3] = (y3 - A[19] * x[4]) * A[18];
-    x[2] = (y2 - A[13] * x[3] - A[14] * x[4]) * A[12];
-    x[1] = (y1 - A[7] * x[2] - A[8] * x[3] - A[9] * x[4]) * A[6];
-    x[0] = (b[0] - A[1] * x[1] - A[2] * x[2] - A[3] * x[3] - A[4] * x[4]) * A[0];
-}
-
-// lu[k * nc + cell], k = 0..24: factors of the cell's local matrix at U.
-template <typename T>
-__global__ void __launch_bounds__(VNT, sizeof(T) == 4 ? 2 : GLIDE_VANKA64_MIN_BLOCKS) vanka_lu_kernel(
-    T* __restrict__ lu, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
-    const T* __restrict__ f_H, const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
-    const T* __restrict__ gamma, const T* __restrict__ act, T shift, Geo g, Phys<T> p) {
-    __shared__ T s_eta[VY + 2][VX + 2];
-    const int ny = g.ny, nx = g.nx;
-    const int bz = blockIdx.z;
-    u += bz * g.nu(); v += bz * g.nv(); H += bz * g.nc();
-    if (act) act += bz * g.nc(); else f_H += bz * g.nc();
-    bed += bz * g.nc(); B += bz * g.nc(); beta += bz * g.nc(); gamma += bz * g.nc();
-    const int64_t nc = g.nc();
-    lu += bz * 25 * nc;
-    const int i0 = blockIdx.y * VY, j0 = blockIdx.x * VX;
-    const int r = threadIdx.x / VX, c = threadIdx.x % VX;
-    const int i = i0 + r, j = j0 + c;
-    eta_window(s_eta, u, v, B, i0, j0, ny, nx, p);
-    __syncthreads();
-    if (i >= ny || j >= nx) return;
-    Frozen<T> F;
-    {
-        Patch<T> P;
-        load_patch(P, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
-        make_frozen(F, P, ny, nx, p);
-    }
-    const int64_t ic = int64_t(i) * nx + j;
-    const T ul = u[int64_t(i) * (nx + 1) + j], ur = u[int64_t(i) * (nx + 1) + j + 1];
-    const T vt = v[ic], vb = v[int64_t(i + 1) * nx + j];
-    T J[25], rr[5];
-    // the momentum rows do not depend on f; the mass row's active-set switch
-    // (vanka.cu:104-113) needs the local mass residual, hence f_H.  With a
-    // given active set (act) the switch is forced instead: a right-hand side
-    // of -/+1e30 makes H - dt r_H far below / above gamma (r is discarded).
-    const T fH = act ? (act[ic] > T(0.5) ? T(-1e30) : T(1e30)) : f_H[ic];
-    assemble_fast<T>(F, ul, ur, vt, vb, H[ic], T(0), T(0), T(0), T(0), fH, gamma[ic], T(1) / p.dt, p, J, rr);
-    J[0] -= shift; J[6] -= shift; J[12] -= shift; J[18] -= shift; J[24] += shift;  // vanka.cu:406-410
-    lu5_factor(J);
-#pragma unroll
-    for (int k = 0; k < 25; k++) lu[k * nc + ic] = J[k];
-}
-
-// scratch = the additive-Vanka halves of -A^-1 rho (same layout as
-// vanka_cells_kernel), with H + d_H + delta_H >= gamma.
-template <typename T>
-__global__ void vanka_linear_kernel(T* __restrict__ scratch, const T* __restrict__ lu,
-                                    const T* __restrict__ rho_u, const T* __restrict__ rho_v,
-                                    const T* __restrict__ rho_H, const T* __restrict__ H,
-                                    const T* __restrict__ dH, const T* __restrict__ gamma, Geo g) {
-    const int ny = g.ny, nx = g.nx;
-    const int bz = blockIdx.z;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
-    if (i >= ny || j >= nx) return;
-    const int64_t nc = g.nc();
-    rho_u += bz * g.nu(); rho_v += bz * g.nv(); rho_H += bz * nc; H += bz * nc; dH += bz * nc;
-    gamma += bz * nc; lu += bz * 25 * nc; scratch += bz * 5 * nc;
-    const int64_t ic = int64_t(i) * nx + j;
-    T A[25];
-#pragma unroll
-    for (int k = 0; k < 25; k++) A[k] = lu[k * nc + ic];
-    const T b[5] = {rho_u[int64_t(i) * (nx + 1) + j], rho_u[int64_t(i) * (nx + 1) + j + 1], rho_v[ic],
-                    rho_v[int64_t(i + 1) * nx + j], rho_H[ic]};
-    T x[5];
-    lu5_subst(A, b, x);
-    T dHc = -x[4];
-    dHc = M<T>::max(dHc, gamma[ic] - H[ic] - dH[ic]);
-    if (!(isfinite(x[0]) && isfinite(x[1]) && isfinite(x[2]) && isfinite(x[3]) && isfinite(dHc))) {
-        x[0] = x[1] = x[2] = x[3] = T(0);
-        dHc = T(0);
-    }
-    scratch[ic] = T(-0.5) * x[0];
-    scratch[nc + ic] = T(-0.5) * x[1];
-    scratch[2 * nc + ic] = T(-0.5) * x[2];
-    scratch[3 * nc + ic] = T(-0.5) * x[3];
-    scratch[4 * nc + ic] = dHc;
-}
-
 // U += omega * delta, face delta = sum of the two adjacent cells' halves.
 template <typename T, bool LOCAL>
 __global__ void vanka_apply_kernel(T* __restrict__ u, T* __restrict__ v, T* __restrict__ H,
@@ -734,55 +487,6 @@ __global__ void tile_flags_kernel(int* __restrict__ flags, int* __restrict__ any
 }
 
 // --------------------------------------------------------------------------
-// adjoint Vanka, one colour (glide/cuda/vanka.cu:441-840)
-// Solves J^T dlam = r_adj per cell of the colour with the local Jacobian at
-// the current state (mask>0.5 rows replaced by the identity, no shift) and
-// updates lambda in place: each face is adjacent to exactly one cell of a
-// colour, so every lambda entry has a single writer.
-// --------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(VNT) vanka_adjoint_kernel(
-    T* __restrict__ lu, T* __restrict__ lv, T* __restrict__ lH, const T* __restrict__ ra_u,
-    const T* __restrict__ ra_v, const T* __restrict__ ra_H, const T* __restrict__ u, const T* __restrict__ v,
-    const T* __restrict__ H, const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
-    const T* __restrict__ mask, int color, T omega, Geo g, Phys<T> p) {
-    __shared__ T s_eta[VY + 2][VX + 2];
-    const int ny = g.ny, nx = g.nx;
-    const int bz = blockIdx.z;
-    u += bz * g.nu(); v += bz * g.nv(); H += bz * g.nc(); bed += bz * g.nc(); B += bz * g.nc();
-    beta += bz * g.nc(); mask += bz * g.nc(); lu += bz * g.nu(); lv += bz * g.nv(); lH += bz * g.nc();
-    ra_u += bz * g.nu(); ra_v += bz * g.nv(); ra_H += bz * g.nc();
-    const int i0 = blockIdx.y * VY, j0 = blockIdx.x * VX;
-    const int r = threadIdx.x / VX, c = threadIdx.x % VX;
-    const int i = i0 + r, j = j0 + c;
-    eta_window(s_eta, u, v, B, i0, j0, ny, nx, p);
-    __syncthreads();
-    if (i >= ny || j >= nx || ((i + j) & 1) != color) return;
-    Patch<T> P;
-    load_patch(P, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
-    const int64_t iu = int64_t(i) * (nx + 1) + j, ic = int64_t(i) * nx + j, ivb = int64_t(i + 1) * nx + j;
-    T J[25], rr[5];
-    assemble<T, false>(P, u[iu], u[iu + 1], v[ic], v[ivb], H[ic], T(0), T(0), T(0), T(0), T(0), T(0), ny, nx, p,
-                       J, rr);
-    if (mask[ic] > T(0.5)) {
-        J[20] = T(0); J[21] = T(0); J[22] = T(0); J[23] = T(0); J[24] = T(1);
-    }
-    T JT[25];
-#pragma unroll
-    for (int a = 0; a < 5; a++)
-#pragma unroll
-        for (int b = 0; b < 5; b++) JT[a * 5 + b] = J[b * 5 + a];
-    T rhs[5] = {ra_u[iu], ra_u[iu + 1], ra_v[ic], ra_v[ivb], ra_H[ic]};
-    T x[5];
-    lu5_solve(JT, rhs, x);
-    lu[iu] += T(0.5) * omega * x[0];
-    lu[iu + 1] += T(0.5) * omega * x[1];
-    lv[ic] += T(0.5) * omega * x[2];
-    lv[ivb] += T(0.5) * omega * x[3];
-    lH[ic] += omega * x[4];
-}
-
-// --------------------------------------------------------------------------
 // launchers
 // --------------------------------------------------------------------------
 static inline dim3 cell_grid(const Geo& g) { return dim3((g.nx + VX - 1) / VX, (g.ny + VY - 1) / VY, g.nb); }
@@ -838,34 +542,6 @@ int launch_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v
 }
 
 template <typename T>
-int launch_vanka_lu(const GlideLevelArgs* a, const void* f_H, void* lu, double shift, cudaStream_t s) {
-    Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
-    // f_H null: the active set is the level's mask (glide_vanka_lu_masked)
-    glide::count_launch(), vanka_lu_kernel<T><<<cell_grid(g), VNT, 0, s>>>(
-        (T*)lu, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_H, (const T*)a->bed, (const T*)a->B,
-        (const T*)a->beta, (const T*)a->gamma, f_H ? nullptr : (const T*)a->mask, T(shift), g, p);
-    return (int)cudaGetLastError();
-}
-
-// d += omega * (linear Vanka update of rho), n_iter times with a fixed rho is
-// not useful: one sweep per call, rho recomputed by the caller in between.
-template <typename T>
-int launch_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* rho_v, const void* rho_H,
-                        const void* lu, void* d_u, void* d_v, void* d_H, double omega, void* scratch,
-                        cudaStream_t s) {
-    Geo g{a->ny, a->nx, a->nb};
-    dim3 blk(32, 8);
-    dim3 grd((g.nx + 31) / 32, (g.ny + 7) / 8, g.nb);
-    glide::count_launch(), vanka_linear_kernel<T><<<grd, blk, 0, s>>>(
-        (T*)scratch, (const T*)lu, (const T*)rho_u, (const T*)rho_v, (const T*)rho_H, (const T*)a->H,
-        (const T*)d_H, (const T*)a->gamma, g);
-    glide::count_launch(), vanka_apply_kernel<T, false><<<face_grid(g), dim3(32, 8), 0, s>>>(
-        (T*)d_u, (T*)d_v, (T*)d_H, (const T*)scratch, nullptr, nullptr, T(omega), g);
-    return (int)cudaGetLastError();
-}
-
-template <typename T>
 int launch_error_mask(const GlideLevelArgs* a, const void* r_u, const void* r_v, const void* r_H, double threshold,
                       void* err_mask, int* flags, int* any_active, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
@@ -890,18 +566,6 @@ int launch_tile_flags(const GlideLevelArgs* a, const void* err_mask, int* flags,
     return (int)cudaGetLastError();
 }
 
-template <typename T>
-int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
-                         const void* ra_H, int color, double omega, cudaStream_t s) {
-    Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
-    glide::count_launch(), vanka_adjoint_kernel<T><<<cell_grid(g), VNT, 0, s>>>(
-        (T*)l_u, (T*)l_v, (T*)l_H, (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, (const T*)a->u, (const T*)a->v,
-        (const T*)a->H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask, color, T(omega), g,
-        p);
-    return (int)cudaGetLastError();
-}
-
 #define INST(T)                                                                                                  \
     template int launch_vanka_sweeps<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,   \
                                         double, double, const int*, const int*, void*, cudaStream_t, double, int);\
@@ -909,12 +573,7 @@ int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_
                                        double, const int*, const int*, void*, cudaStream_t, double);              \
     template int launch_error_mask<T>(const GlideLevelArgs*, const void*, const void*, const void*, double,       \
                                       void*, int*, int*, cudaStream_t);                                           \
-    template int launch_tile_flags<T>(const GlideLevelArgs*, const void*, int*, int*, cudaStream_t);              \
-    template int launch_vanka_adjoint<T>(const GlideLevelArgs*, void*, void*, void*, const void*, const void*,    \
-                                         const void*, int, double, cudaStream_t);                                 \
-    template int launch_vanka_lu<T>(const GlideLevelArgs*, const void*, void*, double, cudaStream_t);             \
-    template int launch_vanka_linear<T>(const GlideLevelArgs*, const void*, const void*, const void*, const void*, \
-                                        void*, void*, void*, double, void*, cudaStream_t);
+    template int launch_tile_flags<T>(const GlideLevelArgs*, const void*, int*, int*, cudaStream_t);
 INST(float)
 INST(double)
 #undef INST

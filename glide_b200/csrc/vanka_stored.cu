@@ -1,0 +1,399 @@
+// Vanka smoothers that form each cell's local matrix once: the linear sweeps of
+// the defect correction and the adjoint smoother.
+//
+// Neither the state nor the active set changes while such a smoother runs, so
+// the cells' 5x5 systems are formed once per call, in the arrow form of
+// cell_system.cuh, and every sweep only solves them: 14 arrays for the linear
+// sweep (bound by reading them: the factors of an unstructured elimination are
+// 25), 18 for the adjoint (the solved form, without a reciprocal per sweep: its
+// levels are small and wait on latency).
+#include "cell_system.cuh"
+
+namespace glide {
+
+constexpr int SW = 30;          // cell columns per warp of the march
+constexpr int FC_NT = 128;
+constexpr int LU_N = 14;        // D1, D2, p2, c1, c2, e1, e2, j4
+constexpr int ADJ_N = 18;       // i, w1, w2, Cd, k, e, b11, b12, b22, ag, bg, ih
+
+enum { STORE_LU = 0, STORE_ADJOINT = 1, SOLVE_ADJOINT = 2 };
+
+template <typename T> struct StoredArgs {
+    const T *u, *v, *H, *f_H, *bed, *B, *beta, *gamma;
+    const T* act;               // active set; null: tested with f_H
+    T* out;                     // stored arrays
+    T shift;
+    T *l_u, *l_v, *l_H;         // SOLVE_ADJOINT: multiplier, adjoint residual, colour
+    const T *ra_u, *ra_v, *ra_H;
+    T omega;
+    int color;
+    int n_strips, rows, n_warps;
+};
+
+// J^T x = b of one cell in the arrow form: the velocity block is symmetric, the
+// thickness column and the mass row change places (the mass row is stored at
+// half its size).
+template <typename T> __device__ __forceinline__ Arrow<T> transposed(const Arrow<T>& s) {
+    Arrow<T> t = s;
+    t.c1 = s.e1 + s.e1;
+    t.c2 = s.e2 + s.e2;
+    t.e1 = s.c1 + two(s.hxy.x, s.hxy.y);
+    t.e2 = s.c2 + two(s.hxy.x, s.hxy.y);
+    t.hxy = both(T(0));
+    t.j4 = T(2) * s.j4;
+    return t;
+}
+
+// lambda += omega * (half of each face's change, the full thickness change);
+// within one colour every face has one writer
+template <typename T>
+__device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __restrict__ ra_u,
+                                               const T* __restrict__ ra_v, const T* __restrict__ ra_H,
+                                               T* __restrict__ l_u, T* __restrict__ l_v, T* __restrict__ l_H, int i,
+                                               int j, int nx, T omega) {
+    const int iu = i * (nx + 1) + j, ic = i * nx + j;
+    Two<T> x1, x2;
+    T xh;
+    arrow_solve(q, two(ra_u[iu], -ra_v[ic]), two(-ra_u[iu + 1], ra_v[ic + nx]), both(T(0)), ra_H[ic], x1, x2, xh);
+    l_u[iu] -= T(0.5) * omega * x1.x;
+    l_u[iu + 1] += T(0.5) * omega * x2.x;
+    l_v[ic] += T(0.5) * omega * x1.y;
+    l_v[ic + nx] -= T(0.5) * omega * x2.y;
+    l_H[ic] += omega * xh;
+}
+
+// --------------------------------------------------------------------------
+// The march: a warp owns SW cell columns (lane l holds column j0 - 1 + l) and
+// marches down a chunk of rows with the rows in reach in registers and the
+// neighbouring columns in its lanes, as the residual does (ssa_stencil.cu).
+// --------------------------------------------------------------------------
+template <typename T, int MODE>
+__global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
+    stored_cells_kernel(const StoredArgs<T> A, Geo g, Phys<T> p) {
+    const int ny = g.ny, nx = g.nx, b = blockIdx.y;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (wid >= A.n_warps) return;  // whole warp
+    const int lane = threadIdx.x & 31;
+    const unsigned FULL = 0xffffffffu;
+    const int64_t nc = g.nc();
+    const T* __restrict__ u = A.u + b * g.nu();
+    const T* __restrict__ v = A.v + b * g.nv();
+    const T* __restrict__ H = A.H + b * nc;
+    const T* __restrict__ bed = A.bed + b * nc;
+    const T* __restrict__ B = A.B + b * nc;
+    const T* __restrict__ beta = A.beta + b * nc;
+
+    const int strip = wid % A.n_strips, chunk = wid / A.n_strips;
+    const int i0 = chunk * A.rows, i1 = min(i0 + A.rows, ny);
+    const int jc = strip * SW - 1 + lane;
+    const int jcc = clampi(jc, 0, nx - 1), juL = clampi(jc, 0, nx), juR = clampi(jc + 1, 0, nx);
+    const int jvL = clampi(jc - 1, 0, nx - 1), jvR = clampi(jc + 1, 0, nx - 1);
+    const bool first = lane == 0, last = lane == 31;
+    const bool own = lane >= 1 && lane <= SW && jc < nx;
+    const T dxi = p.dxi, d2 = p.dxi * p.dxi, rr = rho_ratio<T>();
+    auto U = [&](int r, int col) -> T { return __ldg(u + (clampi(r, 0, ny - 1) * (nx + 1) + col)); };
+    auto V = [&](int r, int col) -> T { return __ldg(v + (clampi(r, 0, ny) * nx + col)); };
+    auto row = [&](const T* a, int r) -> T { return __ldg(a + (clampi(r, 0, ny - 1) * nx + jcc)); };
+
+    // at the start of iteration i: u rows i-1..i+1, v rows i-1..i+1, cell rows i-1 and i
+    int i = i0 - 2;
+    T um = T(0), u0 = U(i, juL), u1 = U(i + 1, juL);
+    T uR0 = last ? U(i, juR) : T(0), uR1 = last ? U(i + 1, juR) : T(0), uRm = T(0);
+    T vm = T(0), v0 = V(i, jcc), v1 = V(i + 1, jcc);
+    T vL1 = first ? V(i + 1, jvL) : T(0), vR1 = last ? V(i + 1, jvR) : T(0);
+    T Hm = T(0), Zm = T(0), bm = T(0), em = T(0);              // row i-1: H, surface, drag, eta*H
+    T Hc = T(0), Zc = T(0), bc = T(0), ec = T(0), etac = T(0); // row i
+    T bedc = T(0), betac = T(0);
+    for (; i < i1; ++i) {
+        const T u2 = U(i + 2, juL), uR2 = last ? U(i + 2, juR) : T(0);
+        const T v2 = V(i + 2, jcc), vL2 = first ? V(i + 2, jvL) : T(0), vR2 = last ? V(i + 2, jvR) : T(0);
+        const T Hp = row(H, i + 1), bedp = row(bed, i + 1), betap = row(beta, i + 1), Bp = row(B, i + 1);
+        T u0r = __shfl_down_sync(FULL, u0, 1), u1r = __shfl_down_sync(FULL, u1, 1);
+        T u2r = __shfl_down_sync(FULL, u2, 1);
+        T v1l = __shfl_up_sync(FULL, v1, 1), v2l = __shfl_up_sync(FULL, v2, 1);
+        T v1r = __shfl_down_sync(FULL, v1, 1), v2r = __shfl_down_sync(FULL, v2, 1);
+        if (last) { u0r = uR0; u1r = uR1; u2r = uR2; v1r = vR1; v2r = vR2; }
+        if (first) { v1l = vL1; v2l = vL2; }
+        EtaIn<T> a;
+        a.ul = u1;   a.ur = u1r;   a.vt = v1;   a.vb = v2;
+        a.u_tl = u0; a.u_tr = u0r; a.u_bl = u2; a.u_br = u2r;
+        a.v_lt = v1l; a.v_rt = v1r; a.v_lb = v2l; a.v_rb = v2r;
+        const T etap = cell_eta(a, Bp, clampi(i + 1, 0, ny - 1), jcc, ny, nx, p).eta, ep = etap * Hp;
+        const T Zp = M<T>::max(bedp, -rr * Hp) + Hp;
+        const T gp = sigmoid(bedp + rr * Hp, p.sig_c);
+        const T bp = gp * betap + (T(1) - gp) * p.water_drag;
+
+        if (i >= i0) {  // warp-uniform
+            Cell<T> C;
+            const T wl = jc > 0 ? T(1) : T(0), wr = jc + 1 < nx ? T(1) : T(0);
+            const T wt = i > 0 ? T(1) : T(0), wb = i + 1 < ny ? T(1) : T(0);
+            T umr = __shfl_down_sync(FULL, um, 1);
+            if (last) umr = uRm;
+            const T v0l = __shfl_up_sync(FULL, v0, 1), v0r = __shfl_down_sync(FULL, v0, 1);
+            const T eL = __shfl_up_sync(FULL, ec, 1), eR = __shfl_down_sync(FULL, ec, 1);
+            const T emL = __shfl_up_sync(FULL, em, 1), emR = __shfl_down_sync(FULL, em, 1);
+            const T epL = __shfl_up_sync(FULL, ep, 1), epR = __shfl_down_sync(FULL, ep, 1);
+            const T bL = __shfl_up_sync(FULL, bc, 1), bR = __shfl_down_sync(FULL, bc, 1);
+            const T HL = __shfl_up_sync(FULL, Hc, 1), HR = __shfl_down_sync(FULL, Hc, 1);
+            const T ZL = __shfl_up_sync(FULL, Zc, 1), ZR = __shfl_down_sync(FULL, Zc, 1);
+            C.H_1 = two(HL, Hm);
+            C.H_2 = two(HR, Hp);
+            C.Z_1 = two(-ZL, -Zm);
+            C.Z_2 = two(-ZR, -Zp);
+            C.B_1 = two(T(0.5) * bL, T(0.5) * bm);
+            C.B_2 = two(T(0.5) * bR, T(0.5) * bp);
+            C.bed = bedc;
+            C.beta = betac;
+            C.n_1 = two(-u0, v0);
+            C.n_2 = two(u0r, -v1);
+            C.D0 = two(u0r - u0, v0 - v1);
+            C.E = T(2) * d2 * etac;
+            const T e4 = T(0.25) * d2 * etac, q = T(0.25) * d2;
+            C.ew_p = two(e4 * wt * wl, e4 * wb * wr);
+            C.ew_q = two(e4 * wb * wl, e4 * wt * wr);
+            C.S_p = two(q * (emL + em + eL) * wt * wl, q * (eR + ep + epR) * wb * wr);
+            C.S_q = two(q * (eL + epL + ep) * wb * wl, q * (em + emR + eR) * wt * wr);
+            C.X_p = two((um - u0) + (v0 - v0l), (u0r - u1r) + (v1r - v1));
+            C.X_q = two((u1 - u0) + (v1l - v1), (u0r - umr) + (v0 - v0r));
+            C.K_1 = two(T(4) * d2 * eL * wl, T(4) * d2 * em * wt);
+            C.K_2 = two(T(4) * d2 * eR * wr, T(4) * d2 * ep * wb);
+            C.W_1 = two(T(-0.5) * dxi * wl, T(-0.5) * dxi * wt);
+            C.W_2 = two(T(-0.5) * dxi * wr, T(-0.5) * dxi * wb);
+            if (own && (MODE != SOLVE_ADJOINT || ((i + jc) & 1) == A.color)) {
+                const int ic = i * nx + jc;
+                const T* act = A.act ? A.act + b * nc : nullptr;
+                C.f_H = act ? T(0) : __ldg(A.f_H + b * nc + ic);
+                C.thk = __ldg(A.gamma + b * nc + ic);
+                Arrow<T> s;
+                arrow_assemble(C, Hc, A.shift, act ? (__ldg(act + ic) > T(0.5) ? 1 : 0) : -1, p, s);
+                if constexpr (MODE == STORE_LU) {
+                    const Two<T> c1 = s.c1 + s.hxy, c2 = s.c2 + s.hxy;
+                    const T o[LU_N] = {s.D1.x, s.D1.y, s.D2.x, s.D2.y, s.p2, c1.x, c1.y, c2.x, c2.y, s.e1.x, s.e1.y,
+                                       s.e2.x, s.e2.y, s.j4};
+                    T* out = A.out + b * 25 * nc + ic;
+#pragma unroll
+                    for (int k = 0; k < LU_N; k++) out[k * nc] = o[k];
+                } else {
+                    ArrowInv<T> q;
+                    arrow_factor(transposed(s), q);
+                    if constexpr (MODE == STORE_ADJOINT) {
+                        const T o[ADJ_N] = {q.i.x, q.i.y, q.w1.x, q.w1.y, q.w2.x, q.w2.y, q.Cd.x, q.Cd.y, q.k.x,
+                                            q.k.y, q.e.x, q.e.y, q.b11, q.b12, q.b22, q.ag, q.bg, q.ih};
+                        T* out = A.out + b * ADJ_N * nc + ic;
+#pragma unroll
+                        for (int k = 0; k < ADJ_N; k++) out[k * nc] = o[k];
+                    } else {
+                        adjoint_update(q, A.ra_u + b * g.nu(), A.ra_v + b * g.nv(), A.ra_H + b * nc,
+                                       A.l_u + b * g.nu(), A.l_v + b * g.nv(), A.l_H + b * nc, i, jc, nx, A.omega);
+                    }
+                }
+            }
+        }
+        // roll the window one row down
+        um = u0; u0 = u1; u1 = u2; uRm = uR0; uR0 = uR1; uR1 = uR2;
+        vm = v0; v0 = v1; v1 = v2; vL1 = vL2; vR1 = vR2;
+        Hm = Hc; Zm = Zc; bm = bc; em = ec;
+        Hc = Hp; Zc = Zp; bc = bp; ec = ep; etac = etap; bedc = bedp; betac = betap;
+    }
+}
+
+// One colour of the adjoint sweep from stored factors: a thread per cell of the colour.
+template <typename T>
+__global__ void adjoint_color_kernel(const T* __restrict__ f, T* __restrict__ l_u, T* __restrict__ l_v,
+                                     T* __restrict__ l_H, const T* __restrict__ ra_u, const T* __restrict__ ra_v,
+                                     const T* __restrict__ ra_H, int color, T omega, Geo g) {
+    const int ny = g.ny, nx = g.nx, b = blockIdx.z;
+    const int i = blockIdx.y * blockDim.y + threadIdx.y;
+    const int j = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((i + color) & 1);
+    if (i >= ny || j >= nx) return;
+    const int64_t nc = g.nc();
+    f += b * ADJ_N * nc + int64_t(i) * nx + j;
+    T o[ADJ_N];
+#pragma unroll
+    for (int k = 0; k < ADJ_N; k++) o[k] = __ldg(f + k * nc);
+    ArrowInv<T> q;
+    q.i = two(o[0], o[1]); q.w1 = two(o[2], o[3]); q.w2 = two(o[4], o[5]); q.Cd = two(o[6], o[7]);
+    q.k = two(o[8], o[9]); q.e = two(o[10], o[11]);
+    q.b11 = o[12]; q.b12 = o[13]; q.b22 = o[14]; q.ag = o[15]; q.bg = o[16]; q.ih = o[17];
+    adjoint_update(q, ra_u + b * g.nu(), ra_v + b * g.nv(), ra_H + b * nc, l_u + b * g.nu(), l_v + b * g.nv(),
+                   l_H + b * nc, i, j, nx, omega);
+}
+
+// --------------------------------------------------------------------------
+// One additive linear sweep, d += omega * sum of the cells' updates, in one
+// pass: a warp owns 31 face columns (lane 0 is the cell to their left) and
+// marches down, so a face's two cells are this lane and the one to its left,
+// or this row and the one above; no intermediate cell arrays.  A cell's
+// solution needs nothing that another warp writes (the bound H + d_H >= gamma
+// only enters its own d_H).
+// --------------------------------------------------------------------------
+constexpr int LW = 31;
+
+template <typename T>
+__global__ void __launch_bounds__(256) vanka_linear_kernel(T* __restrict__ d_u, T* __restrict__ d_v,
+                                                           T* __restrict__ d_H, const T* __restrict__ lu,
+                                                           const T* __restrict__ rho_u, const T* __restrict__ rho_v,
+                                                           const T* __restrict__ rho_H, const T* __restrict__ H,
+                                                           const T* __restrict__ gamma, T omega, Geo g, int n_strips,
+                                                           int rows, int n_warps) {
+    const int ny = g.ny, nx = g.nx, b = blockIdx.y;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    if (wid >= n_warps) return;  // whole warp
+    const int lane = threadIdx.x & 31;
+    const unsigned FULL = 0xffffffffu;
+    const int64_t nc = g.nc();
+    d_u += b * g.nu(); d_v += b * g.nv(); d_H += b * nc;
+    rho_u += b * g.nu(); rho_v += b * g.nv(); rho_H += b * nc; H += b * nc; gamma += b * nc;
+    lu += b * 25 * nc;
+    const int strip = wid % n_strips, chunk = wid / n_strips;
+    const int i0 = chunk * rows, i1 = min(i0 + rows, ny + 1);   // face rows
+    const int j = strip * LW - 1 + lane;
+    const bool col = j >= 0 && j < nx;
+    const bool own = lane >= 1 && j <= nx;
+    T xb_prev = T(0);   // the row above's change of its lower face
+    T rv = col && i0 > 0 ? __ldg(rho_v + (i0 - 1) * nx + j) : T(0);
+    for (int i = i0 - 1; i < i1; ++i) {
+        const bool cell = col && i >= 0 && i < ny;
+        Two<T> x1 = both(T(0)), x2 = both(T(0));   // outward changes of (l, t) and (r, b)
+        T xh = T(0);
+        const int ic = i * nx + j, iu = i * (nx + 1) + j;
+        if (i < 0 && col) rv = __ldg(rho_v + j);   // becomes row 0's upper face below
+        T rvb = rv;
+        if (cell) {
+            const T* f = lu + ic;
+            T o[LU_N];
+#pragma unroll
+            for (int k = 0; k < LU_N; k++) o[k] = __ldg(f + k * nc);
+            const T ru_l = __ldg(rho_u + iu), ru_r = __ldg(rho_u + iu + 1), rH = __ldg(rho_H + ic);
+            rvb = __ldg(rho_v + ic + nx);
+            Arrow<T> s;
+            s.D1 = two(o[0], o[1]); s.D2 = two(o[2], o[3]); s.p2 = o[4];
+            s.c1 = two(o[5], o[6]); s.c2 = two(o[7], o[8]); s.e1 = two(o[9], o[10]); s.e2 = two(o[11], o[12]);
+            s.j4 = o[13];
+            s.hxy = both(T(0));
+            ArrowInv<T> q;
+            arrow_factor(s, q);
+            arrow_solve(q, two(ru_l, -rv), two(-ru_r, rvb), both(T(0)), T(0.5) * rH, x1, x2, xh);
+            if (!(isfinite(x1.x) && isfinite(x1.y) && isfinite(x2.x) && isfinite(x2.y) && isfinite(xh))) {
+                x1 = x2 = both(T(0));   // a failed local solve leaves its faces and its cell unchanged
+                xh = T(0);
+            } else if (own && i >= i0) {
+                const T dh = __ldg(gamma + ic) - __ldg(H + ic) - d_H[ic];
+                d_H[ic] += omega * M<T>::max(-xh, dh);
+            }
+        }
+        // changes: u_l += x1.x/2, u_r -= x2.x/2, v_t -= x1.y/2, v_b += x2.y/2
+        const T from_left = __shfl_up_sync(FULL, x2.x, 1);
+        if (own && i >= i0) {
+            if (i < ny) d_u[iu] += omega * (T(0.5) * x1.x - T(0.5) * from_left);
+            if (j < nx) d_v[ic] += omega * (T(0.5) * xb_prev - T(0.5) * x1.y);
+        }
+        xb_prev = x2.y;
+        rv = rvb;
+    }
+}
+
+// --------------------------------------------------------------------------
+// launchers
+// --------------------------------------------------------------------------
+// rows per warp and CTA size of a march over `lines` rows of n_strips strips
+struct MarchShape {
+    int rows, n_warps, threads;
+    unsigned blocks;
+};
+static inline MarchShape march_shape(int n_strips, int lines, int nb, int warps_per_sm, int max_threads) {
+    const int64_t units = int64_t(n_strips) * lines * nb;
+    const int64_t few = (units + 148 * 4 - 1) / (148 * 4), many = (units + 148 * warps_per_sm - 1) / (148 * warps_per_sm);
+    MarchShape sh;
+    // short chunks on small grids, as in ssa_stencil.cu
+    sh.rows = int(few < 8 ? few : many < 8 ? 8 : many > 64 ? 64 : many);
+    sh.n_warps = n_strips * ((lines + sh.rows - 1) / sh.rows);
+    const int64_t per_sm = (int64_t(sh.n_warps) * nb + 147) / 148;
+    sh.threads = 32 * int(per_sm < max_threads / 32 ? per_sm : max_threads / 32);
+    sh.blocks = unsigned((sh.n_warps + sh.threads / 32 - 1) / (sh.threads / 32));
+    return sh;
+}
+
+template <typename T, int MODE>
+static int run_stored(const GlideLevelArgs* a, StoredArgs<T> A, cudaStream_t s) {
+    Geo g{a->ny, a->nx, a->nb};
+    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
+    A.u = (const T*)a->u; A.v = (const T*)a->v; A.H = (const T*)a->H;
+    A.bed = (const T*)a->bed; A.B = (const T*)a->B; A.beta = (const T*)a->beta; A.gamma = (const T*)a->gamma;
+    A.n_strips = (g.nx + SW - 1) / SW;
+    const MarchShape sh = march_shape(A.n_strips, g.ny, g.nb, sizeof(T) == 4 ? 16 : 8, FC_NT);
+    A.rows = sh.rows;
+    A.n_warps = sh.n_warps;
+    glide::count_launch(), stored_cells_kernel<T, MODE><<<dim3(sh.blocks, g.nb), sh.threads, 0, s>>>(A, g, p);
+    return (int)cudaGetLastError();
+}
+
+// f_H null: the active set is the level's mask (glide_vanka_lu_masked)
+template <typename T>
+int launch_vanka_lu(const GlideLevelArgs* a, const void* f_H, void* lu, double shift, cudaStream_t s) {
+    StoredArgs<T> A{};
+    A.f_H = (const T*)f_H;
+    A.act = f_H ? nullptr : (const T*)a->mask;
+    A.out = (T*)lu;
+    A.shift = T(shift);
+    return run_stored<T, STORE_LU>(a, A, s);
+}
+
+// one sweep with a given rho = r + J d (recomputed by the caller in between)
+template <typename T>
+int launch_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* rho_v, const void* rho_H,
+                        const void* lu, void* d_u, void* d_v, void* d_H, double omega, cudaStream_t s) {
+    Geo g{a->ny, a->nx, a->nb};
+    const int n_strips = (g.nx + 1 + LW - 1) / LW;
+    const MarchShape sh = march_shape(n_strips, g.ny + 1, g.nb, 32, 256);
+    glide::count_launch(), vanka_linear_kernel<T><<<dim3(sh.blocks, g.nb), sh.threads, 0, s>>>(
+        (T*)d_u, (T*)d_v, (T*)d_H, (const T*)lu, (const T*)rho_u, (const T*)rho_v, (const T*)rho_H, (const T*)a->H,
+        (const T*)a->gamma, T(omega), g, n_strips, sh.rows, sh.n_warps);
+    return (int)cudaGetLastError();
+}
+
+template <typename T>
+int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
+                         const void* ra_H, int color, double omega, cudaStream_t s) {
+    StoredArgs<T> A{};
+    A.act = (const T*)a->mask;
+    A.l_u = (T*)l_u; A.l_v = (T*)l_v; A.l_H = (T*)l_H;
+    A.ra_u = (const T*)ra_u; A.ra_v = (const T*)ra_v; A.ra_H = (const T*)ra_H;
+    A.omega = T(omega);
+    A.color = color;
+    return run_stored<T, SOLVE_ADJOINT>(a, A, s);
+}
+
+template <typename T> int launch_adjoint_factors(const GlideLevelArgs* a, void* factors, cudaStream_t s) {
+    StoredArgs<T> A{};
+    A.act = (const T*)a->mask;
+    A.out = (T*)factors;
+    return run_stored<T, STORE_ADJOINT>(a, A, s);
+}
+
+template <typename T>
+int launch_adjoint_color(const GlideLevelArgs* a, const void* factors, void* l_u, void* l_v, void* l_H,
+                         const void* ra_u, const void* ra_v, const void* ra_H, int color, double omega,
+                         cudaStream_t s) {
+    Geo g{a->ny, a->nx, a->nb};
+    const dim3 blk(32, 4), grd(((g.nx + 1) / 2 + 31) / 32, (g.ny + 3) / 4, g.nb);
+    glide::count_launch(), adjoint_color_kernel<T><<<grd, blk, 0, s>>>(
+        (const T*)factors, (T*)l_u, (T*)l_v, (T*)l_H, (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, color, T(omega),
+        g);
+    return (int)cudaGetLastError();
+}
+
+#define INST(T)                                                                                                     \
+    template int launch_vanka_lu<T>(const GlideLevelArgs*, const void*, void*, double, cudaStream_t);               \
+    template int launch_vanka_linear<T>(const GlideLevelArgs*, const void*, const void*, const void*, const void*,  \
+                                        void*, void*, void*, double, cudaStream_t);                                 \
+    template int launch_vanka_adjoint<T>(const GlideLevelArgs*, void*, void*, void*, const void*, const void*,      \
+                                         const void*, int, double, cudaStream_t);                                   \
+    template int launch_adjoint_factors<T>(const GlideLevelArgs*, void*, cudaStream_t);                             \
+    template int launch_adjoint_color<T>(const GlideLevelArgs*, const void*, void*, void*, void*, const void*,      \
+                                         const void*, const void*, int, double, cudaStream_t);
+INST(float)
+INST(double)
+#undef INST
+
+}  // namespace glide

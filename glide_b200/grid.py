@@ -80,7 +80,7 @@ class Grid:
         self._flags = torch.zeros(nflags, dtype=torch.int32, device=self.device)
         self._any_active = torch.zeros(self.nb, dtype=torch.int32, device=self.device)
         self._norm_out = torch.zeros(3, dtype=torch.float64, device=self.device)
-        self._ls_tmp = self._ls_norms = None
+        self._ls_tmp = self._ls_norms = self._adj_factors = None
         self._norm_parts = torch.zeros(3 * self._lib.glide_norm_parts(max(self.nu, self.nh) * self.nb),
                                        dtype=torch.float64, device=self.device)
 
@@ -117,7 +117,17 @@ class Grid:
                 self._ls_norms = torch.zeros(3 * N.LS_CANDIDATES + 1, dtype=torch.float64, device=self.device)
             L.ls_tmp, L.ls_norms = self._ls_tmp.data_ptr(), self._ls_norms.data_ptr()
             L.norm_parts = self._norm_parts.data_ptr()
+        if self._adj_factors is not None:
+            L.adj_factors = self._adj_factors.data_ptr()
         return L
+
+    def adjoint_factors(self):
+        """Buffer of the adjoint smoother's local systems, made on first use
+        and kept with the level; None while a CUDA graph that would own a new
+        allocation is being captured (the sweeps then form them per colour)."""
+        if self._adj_factors is None and not torch.cuda.is_current_stream_capturing():
+            self._adj_factors = torch.empty(N.ADJ_FACTORS * self.nb * self.nh, dtype=self.dtype, device=self.device)
+        return self._adj_factors
 
     def newton_buffers(self):
         """Buffers of the linear multigrid of the Newton-Krylov finishing
@@ -277,10 +287,13 @@ class Grid:
 
     def vanka_sweep_adjoint(self, n_iter, omega=0.5, exact_boundary=False):
         """glide/grid.py:319-330."""
-        for _ in range(n_iter):
-            for color in (0, 1):
-                self.compute_adjoint_residual(exact_boundary)
-                self.vanka_smooth_adjoint(color, omega)
+        a = self.level_args()
+        factors = self.adjoint_factors()
+        N.check(self._lib.glide_vanka_adjoint_sweeps(
+            C.byref(a), self.lambda_u.data_ptr(), self.lambda_v.data_ptr(), self.lambda_H.data_ptr(),
+            self.f_adj_u.data_ptr(), self.f_adj_v.data_ptr(), self.f_adj_H.data_ptr(), self.r_adj_u.data_ptr(),
+            self.r_adj_v.data_ptr(), self.r_adj_H.data_ptr(), int(n_iter), float(omega), int(exact_boundary),
+            None if factors is None else factors.data_ptr(), self._s()), "adjoint sweeps")
 
     def compute_mask(self, tol=1e-1):
         """mask = H <= gamma + tol (glide/grid.py:332-334)."""

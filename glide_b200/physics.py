@@ -782,6 +782,9 @@ class IcePhysics:
             g.f_adj_H.copy_(-_as_tensor(dL_dH, g.dtype, self.device))
             g.Lambda.zero_()
             cfg = st.native(self.thklim)
+            for level, lg in zip(self._native, self._solve_grids):
+                f = lg.adjoint_factors()
+                level.adj_factors = None if f is None else f.data_ptr()
             if tol is not None and self.adjoint_krylov > 0:
                 from .newton import AdjointKrylov
                 if self._ak is None or self._ak.m != self.adjoint_krylov:

@@ -126,7 +126,7 @@ size_t glide_noalloc_scratch_bytes(void);
  * factors every cell's local 5x5 matrix at the state in a (the matrix of the
  * first local Newton iteration of glide_vanka_sweeps with right-hand side
  * f_H in the mass row's active-set test, diagonal shifted by shift) into lu
- * (25 * ny * nx * nb elements).  glide_vanka_linear makes one
+ * (room for 25 * ny * nx * nb elements; the contents are private).  glide_vanka_linear makes one
  * additive sweep for the correction d of the linear problem r + J d = 0:
  * rho = r + J d is the caller's linear residual; d += omega * (face average
  * of -A^-1 rho), with H + d_H kept >= gamma.  scratch as for the sweeps. */
@@ -148,6 +148,15 @@ int glide_tile_flags(const GlideLevelArgs* a, const void* err_mask, int* flags, 
 /* One colour of the red-black adjoint Vanka; lambda updated in place. */
 int glide_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
                         const void* ra_H, int color, double omega, void* stream);
+/* n_iter adjoint sweeps, each two colours of r_adj = f_adj - lambda^T J (into
+ * ra) followed by glide_vanka_adjoint (glide/grid.py:319-330).  factors: room
+ * for GLIDE_ADJ_FACTORS * ny * nx * nb elements, where the cells' local systems
+ * (fixed while the state and the mask are) are kept for the call; null forms
+ * them for every colour. */
+#define GLIDE_ADJ_FACTORS 18
+int glide_vanka_adjoint_sweeps(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* f_u,
+                               const void* f_v, const void* f_H, void* ra_u, void* ra_v, void* ra_H, int n_iter,
+                               double omega, int exact_boundary, void* factors, void* stream);
 
 /* Transfers.  field: 0 = u faces, 1 = v faces, 2 = cells; sizes of the coarse grid. */
 int glide_restrict(int dtype, int field, int use_max, const void* fine, void* coarse, int nyc, int nxc, int nb,
@@ -190,6 +199,8 @@ typedef struct GlideLevel {
     void* lin_rho;          /* like U: linear residual g + J d */
     void* lin_d;            /* like U: correction d */
     void* r_raw;            /* like U: residual at the linearisation state (active-set test) */
+    /* adjoint smoother (may be null: the local matrices are then formed for every colour) */
+    void* adj_factors;      /* GLIDE_ADJ_FACTORS * nc * nb */
 } GlideLevel;
 
 /* Step sizes tried by the coarse-correction line search, best first on ties. */
