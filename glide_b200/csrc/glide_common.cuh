@@ -69,6 +69,29 @@ template <typename T> struct Phys {
     T dx, dxi, dt;
 };
 
+// Glen's exponent n = 3 in FP64: the viscosity's power is a reciprocal cube
+// root, several times cheaper than the general pow (which is most of an FP64
+// stencil's instructions) and as accurate.  The kernels are instantiated for
+// both; FP32's pow is two hardware approximations either way.  FP64 VJP at
+// 1024^2 with the gradient of beta: 159 us with pow, 129 with the cube root.
+template <typename T> struct PhysCube : Phys<T> {
+    explicit PhysCube(const Phys<T>& p) : Phys<T>(p) {}
+};
+template <typename T> __device__ __forceinline__ T glen_pow(T x, const Phys<T>& p) {
+    return M<T>::pow(x, p.glen_exp);
+}
+__device__ __forceinline__ double glen_pow(double x, const PhysCube<double>&) { return ::rcbrt(x); }
+// go(p) with the parameters in the type the kernels should be instantiated for
+template <typename T, typename F> inline void with_glen(const GlidePhysicsParams& gp, const Phys<T>& p, F&& go) {
+    if constexpr (sizeof(T) == 8) {
+        if (gp.n == 3.0) {
+            go(PhysCube<T>(p));
+            return;
+        }
+    }
+    go(p);
+}
+
 template <typename T>
 inline Phys<T> make_phys(const GlidePhysicsParams& p, double dx, double dt) {
     Phys<T> q;
@@ -283,9 +306,8 @@ template <typename T> struct EtaIn {
 template <typename T> struct EtaOut {
     T eta, eII, exy[4], ux, vy;
 };
-template <typename T>
-__device__ __forceinline__ EtaOut<T> cell_eta(const EtaIn<T>& a, T Bc, int i, int j, int ny, int nx,
-                                              const Phys<T>& p) {
+template <typename T, typename P>
+__device__ __forceinline__ EtaOut<T> cell_eta(const EtaIn<T>& a, T Bc, int i, int j, int ny, int nx, const P& p) {
     EtaOut<T> o;
     T dxi = p.dxi;
     o.ux = (a.ur - a.ul) * dxi;
@@ -300,13 +322,13 @@ __device__ __forceinline__ EtaOut<T> cell_eta(const EtaIn<T>& a, T Bc, int i, in
     o.exy[3] = T(0.5) * ((a.ur - a.u_br) * dxi + (a.v_rb - a.vb) * dxi) * mbr;
     T e2 = T(0.25) * (o.exy[0] * o.exy[0] + o.exy[1] * o.exy[1] + o.exy[2] * o.exy[2] + o.exy[3] * o.exy[3]);
     o.eII = o.ux * o.ux + o.vy * o.vy + o.ux * o.vy + e2 + p.eps_reg;
-    o.eta = T(0.5) * Bc * M<T>::pow(o.eII, p.glen_exp);
+    o.eta = T(0.5) * Bc * glen_pow(o.eII, p);
     return o;
 }
 // Tangent of eta for a tangent (du, dv) of the same 12 faces.
 template <typename T>
-__device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>& d, T Bc, int i, int j, int ny,
-                                              int nx, const Phys<T>& p) {
+__device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>& d, int i, int j, int ny, int nx,
+                                              const Phys<T>& p) {
     T dxi = p.dxi;
     T dux = (d.ur - d.ul) * dxi;
     T dvy = (d.vt - d.vb) * dxi;
@@ -321,7 +343,7 @@ __device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>
     T de2sum = T(0.25) * (T(2) * e.exy[0] * de0 + T(2) * e.exy[1] * de1 + T(2) * e.exy[2] * de2 +
                           T(2) * e.exy[3] * de3);
     T deII = T(2) * e.ux * dux + T(2) * e.vy * dvy + (e.ux * dvy + e.vy * dux) + de2sum;
-    return T(0.5) * Bc * (p.glen_exp * M<T>::pow(e.eII, p.glen_exp - T(1)) * deII);
+    return p.glen_exp * e.eta * (deII * M<T>::rcp(e.eII));   // eta ~ eII^glen_exp
 }
 
 // Load the 12 faces around cell (i,j) from a u/v pair (clamped).

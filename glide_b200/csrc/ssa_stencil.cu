@@ -45,13 +45,13 @@ __device__ __forceinline__ T driving_s(T Hm, T Hp, T Sm, T Sp, T dxi, bool valid
 #endif
 // Ix: the element-index type of the per-field offsets (int when every field
 // has fewer than 2^31 elements, which keeps the address arithmetic 32-bit).
-template <typename T, typename Ix>
+template <typename T, typename Ix, typename P>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_RS_MINB64) residual_stream_kernel(
     T* __restrict__ o_u, T* __restrict__ o_v, T* __restrict__ o_H,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
     const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H,
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
-    const T* __restrict__ mask, const T* __restrict__ gamma, Geo g, Phys<T> p, int n_strips, int rows, int n_warps) {
+    const T* __restrict__ mask, const T* __restrict__ gamma, Geo g, P p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
     const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= n_warps) return;  // whole warp
@@ -232,14 +232,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
 #ifndef GLIDE_JS_MINB64
 #define GLIDE_JS_MINB64 1
 #endif
-template <typename T, bool ADD, typename Ix>
+template <typename T, bool ADD, typename Ix, typename P>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_JS_MINB64) jvp_stream_kernel(
     T* __restrict__ o_u, T* __restrict__ o_v, T* __restrict__ o_H,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
     const T* __restrict__ d_u, const T* __restrict__ d_v, const T* __restrict__ d_H,
     const T* __restrict__ base_u, const T* __restrict__ base_v, const T* __restrict__ base_H,
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
-    const T* __restrict__ mask, Geo g, Phys<T> p, int n_strips, int rows, int n_warps) {
+    const T* __restrict__ mask, Geo g, P p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
     const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= n_warps) return;  // whole warp
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
             da.v_lt = dvL1s; da.v_rt = dvR1s; da.v_lb = dvL2s; da.v_rb = dvR2s;
             const int ie = clampi(i + 1, 0, ny - 1);
             const EtaOut<T> e = cell_eta(a, Bp, ie, jcc, ny, nx, p);
-            const T deta = cell_eta_tangent(e, da, Bp, ie, jcc, ny, nx, p);
+            const T deta = cell_eta_tangent<T>(e, da, ie, jcc, ny, nx, p);
             etaHp = e.eta * Hp;
             detaHp = deta * Hp + e.eta * dHp;
         }
@@ -481,14 +481,14 @@ constexpr int VS_NT = 128;
 #ifndef GLIDE_VS_MINB64
 #define GLIDE_VS_MINB64 2
 #endif
-template <typename T, bool RF, typename Ix>
+template <typename T, bool RF, typename Ix, typename P>
 __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLIDE_VS_MINB64) vjp_stream_kernel(
     T* __restrict__ o_u, T* __restrict__ o_v, T* __restrict__ o_H,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
     const T* __restrict__ lu, const T* __restrict__ lv, const T* __restrict__ lH,
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta, const T* __restrict__ mask,
     const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H, int exact_boundary, Geo g,
-    Phys<T> p, int n_strips, int rows, int n_warps) {
+    P p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
     const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= n_warps) return;  // whole warp
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
             da.v_lt = lvL1s; da.v_rt = lvR1s; da.v_lb = lvL2s; da.v_rb = lvR2s;
             const int ie = clampi(i + 1, 0, ny - 1);
             const EtaOut<T> e = cell_eta(a, Bp, ie, jcc, ny, nx, p);
-            const T deta = cell_eta_tangent(e, da, Bp, ie, jcc, ny, nx, p);
+            const T deta = cell_eta_tangent<T>(e, da, ie, jcc, ny, nx, p);
             etaP = e.eta;
             etaHp = e.eta * Hp;
             detaHp = deta * Hp;
@@ -826,16 +826,19 @@ int launch_residual(const GlideLevelArgs* a, const void* f_u, const void* f_v, c
     Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     const StreamShape sh = stream_shape(g, 256);
     const dim3 grid(sh.blocks, g.nb);
-    auto go = [&](auto kernel) {
+    auto go = [&](auto kernel, const auto& p) {
         glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
             (T*)r_u, (T*)r_v, (T*)r_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u,
             (const T*)f_v, (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
             (const T*)a->gamma, g, p, sh.n_strips, sh.rows, sh.n_warps);
     };
-    if (index32(g))
-        go(residual_stream_kernel<T, int>);
-    else
-        go(residual_stream_kernel<T, int64_t>);
+    with_glen(a->params, p, [&](auto q) {
+        using P = decltype(q);
+        if (index32(g))
+            go(residual_stream_kernel<T, int, P>, q);
+        else
+            go(residual_stream_kernel<T, int64_t, P>, q);
+    });
     return (int)cudaGetLastError();
 }
 
@@ -847,17 +850,20 @@ int launch_jvp(const GlideLevelArgs* a, const void* d_u, const void* d_v, const 
     Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     const StreamShape sh = stream_shape(g, 256);
     const dim3 grid(sh.blocks, g.nb);
-    auto go = [&](auto kernel) {
+    auto go = [&](auto kernel, const auto& p) {
         glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
             (T*)j_u, (T*)j_v, (T*)j_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)d_u,
             (const T*)d_v, (const T*)d_H, (const T*)base_u, (const T*)base_v, (const T*)base_H, (const T*)a->bed,
             (const T*)a->B, (const T*)a->beta, (const T*)a->mask, g, p, sh.n_strips, sh.rows, sh.n_warps);
     };
     const bool i32 = index32(g);
-    if (base_u)
-        i32 ? go(jvp_stream_kernel<T, true, int>) : go(jvp_stream_kernel<T, true, int64_t>);
-    else
-        i32 ? go(jvp_stream_kernel<T, false, int>) : go(jvp_stream_kernel<T, false, int64_t>);
+    with_glen(a->params, p, [&](auto q) {
+        using P = decltype(q);
+        if (base_u)
+            i32 ? go(jvp_stream_kernel<T, true, int, P>, q) : go(jvp_stream_kernel<T, true, int64_t, P>, q);
+        else
+            i32 ? go(jvp_stream_kernel<T, false, int, P>, q) : go(jvp_stream_kernel<T, false, int64_t, P>, q);
+    });
     return (int)cudaGetLastError();
 }
 
@@ -869,17 +875,20 @@ int launch_vjp(const GlideLevelArgs* a, const void* l_u, const void* l_v, const 
     Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     const StreamShape sh = stream_shape(g, VS_NT);
     const dim3 grid(sh.blocks, g.nb);
-    auto go = [&](auto kernel) {
+    auto go = [&](auto kernel, const auto& p) {
         glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
             (T*)o_u, (T*)o_v, (T*)o_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)l_u,
             (const T*)l_v, (const T*)l_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
             (const T*)f_u, (const T*)f_v, (const T*)f_H, exact_boundary, g, p, sh.n_strips, sh.rows, sh.n_warps);
     };
     const bool i32 = index32(g);
-    if (f_u != nullptr)
-        i32 ? go(vjp_stream_kernel<T, true, int>) : go(vjp_stream_kernel<T, true, int64_t>);
-    else
-        i32 ? go(vjp_stream_kernel<T, false, int>) : go(vjp_stream_kernel<T, false, int64_t>);
+    with_glen(a->params, p, [&](auto q) {
+        using P = decltype(q);
+        if (f_u != nullptr)
+            i32 ? go(vjp_stream_kernel<T, true, int, P>, q) : go(vjp_stream_kernel<T, true, int64_t, P>, q);
+        else
+            i32 ? go(vjp_stream_kernel<T, false, int, P>, q) : go(vjp_stream_kernel<T, false, int64_t, P>, q);
+    });
     return (int)cudaGetLastError();
 }
 

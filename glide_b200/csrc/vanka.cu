@@ -34,9 +34,9 @@ template <typename T> struct Patch {
 
 // Fill the eta window of a VYxVX tile (+ ring) and the frozen patch of the
 // calling thread's cell.
-template <typename T>
+template <typename T, typename P>
 __device__ __forceinline__ void eta_window(T (*s_eta)[VX + 2], const T* u, const T* v, const T* B, int i0, int j0,
-                                           int ny, int nx, const Phys<T>& p) {
+                                           int ny, int nx, const P& p) {
     for (int k = threadIdx.x; k < (VY + 2) * (VX + 2); k += VNT) {
         int r = k / (VX + 2), c = k - r * (VX + 2);
         int ic = clampi(i0 - 1 + r, 0, ny - 1), jc = clampi(j0 - 1 + c, 0, nx - 1);
@@ -341,7 +341,7 @@ template <typename T> __device__ __forceinline__ void lu5_solve_pivot(T (&A)[25]
 
 // Per-cell Newton deltas.  scratch holds 5 cell arrays: 0.5*du_l, 0.5*du_r,
 // 0.5*dv_t, 0.5*dv_b, dH.
-template <typename T, bool LOCAL>
+template <typename T, bool LOCAL, typename P>
 #ifndef GLIDE_VANKA64_MIN_BLOCKS
 #define GLIDE_VANKA64_MIN_BLOCKS 2
 #endif
@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(VNT, sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS
     T* __restrict__ scratch, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
     const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H, const T* __restrict__ bed,
     const T* __restrict__ B, const T* __restrict__ beta, const T* __restrict__ gamma, const int* __restrict__ flags,
-    const int* __restrict__ any_active, int n_newton, T shift, T step, int pivot, Geo g, Phys<T> p) {
+    const int* __restrict__ any_active, int n_newton, T shift, T step, int pivot, Geo g, P p) {
     __shared__ T s_eta[VY + 2][VX + 2];
     const int ny = g.ny, nx = g.nx;
     const int bz = blockIdx.z;
@@ -372,9 +372,9 @@ __global__ void __launch_bounds__(VNT, sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS
 
     Frozen<T> F;
     {
-        Patch<T> P;
-        load_patch(P, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
-        make_frozen(F, P, ny, nx, p);
+        Patch<T> pt;
+        load_patch<T>(pt, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
+        make_frozen<T>(F, pt, ny, nx, p);
     }
     // 32-bit offsets within one field (the entry points bound a field below 2^31 elements)
     const int iu = i * (nx + 1) + j, ic32 = i * nx + j;
@@ -493,28 +493,37 @@ static inline dim3 cell_grid(const Geo& g) { return dim3((g.nx + VX - 1) / VX, (
 static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (g.ny + 1 + 7) / 8, g.nb); }
 
 template <typename T>
+static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton,
+                      double shift, double step, int pivot, const int* flags, const int* any_active, void* scratch,
+                      const Geo& g, cudaStream_t s) {
+    with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
+        using P = decltype(p);
+        auto go = [&](auto kernel) {
+            glide::count_launch(), kernel<<<cell_grid(g), VNT, 0, s>>>(
+                (T*)scratch, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u, (const T*)f_v,
+                (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, flags,
+                any_active, n_newton, T(shift), T(step), pivot, g, p);
+        };
+        flags ? go(vanka_cells_kernel<T, true, P>) : go(vanka_cells_kernel<T, false, P>);
+    });
+}
+
+template <typename T>
 int launch_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
                         int n_newton, double omega, double shift, const int* flags, const int* any_active,
                         void* scratch, cudaStream_t s, double newton_step, int pivot) {
     Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     T* u = (T*)a->u;
     T* v = (T*)a->v;
     T* H = (T*)a->H;
     for (int k = 0; k < n_iter; k++) {
-        if (flags) {
-            glide::count_launch(), vanka_cells_kernel<T, true><<<cell_grid(g), VNT, 0, s>>>(
-                (T*)scratch, u, v, H, (const T*)f_u, (const T*)f_v, (const T*)f_H, (const T*)a->bed,
-                (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, flags, any_active, n_newton, T(shift), T(newton_step), pivot, g, p);
-            glide::count_launch(), vanka_apply_kernel<T, true><<<face_grid(g), dim3(32, 8), 0, s>>>(u, v, H, (const T*)scratch, flags,
-                                                                               any_active, T(omega), g);
-        } else {
-            glide::count_launch(), vanka_cells_kernel<T, false><<<cell_grid(g), VNT, 0, s>>>(
-                (T*)scratch, u, v, H, (const T*)f_u, (const T*)f_v, (const T*)f_H, (const T*)a->bed,
-                (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, nullptr, nullptr, n_newton, T(shift), T(newton_step), pivot, g, p);
-            glide::count_launch(), vanka_apply_kernel<T, false><<<face_grid(g), dim3(32, 8), 0, s>>>(u, v, H, (const T*)scratch, nullptr,
-                                                                                nullptr, T(omega), g);
-        }
+        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, pivot, flags, any_active, scratch, g, s);
+        if (flags)
+            glide::count_launch(), vanka_apply_kernel<T, true><<<face_grid(g), dim3(32, 8), 0, s>>>(
+                u, v, H, (const T*)scratch, flags, any_active, T(omega), g);
+        else
+            glide::count_launch(), vanka_apply_kernel<T, false><<<face_grid(g), dim3(32, 8), 0, s>>>(
+                u, v, H, (const T*)scratch, nullptr, nullptr, T(omega), g);
     }
     return (int)cudaGetLastError();
 }
@@ -525,19 +534,8 @@ int launch_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v
                        int n_newton, double shift, const int* flags, const int* any_active, void* scratch,
                        cudaStream_t s, double newton_step) {
     Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
-    for (int k = 0; k < n_launch; k++) {
-        if (flags)
-            glide::count_launch(), vanka_cells_kernel<T, true><<<cell_grid(g), VNT, 0, s>>>(
-                (T*)scratch, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u, (const T*)f_v,
-                (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, flags,
-                any_active, n_newton, T(shift), T(newton_step), 0, g, p);
-        else
-            glide::count_launch(), vanka_cells_kernel<T, false><<<cell_grid(g), VNT, 0, s>>>(
-                (T*)scratch, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u, (const T*)f_v,
-                (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, nullptr,
-                nullptr, n_newton, T(shift), T(newton_step), 0, g, p);
-    }
+    for (int k = 0; k < n_launch; k++)
+        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, 0, flags, any_active, scratch, g, s);
     return (int)cudaGetLastError();
 }
 

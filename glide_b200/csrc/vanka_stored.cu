@@ -67,9 +67,9 @@ __device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __
 // marches down a chunk of rows with the rows in reach in registers and the
 // neighbouring columns in its lanes, as the residual does (ssa_stencil.cu).
 // --------------------------------------------------------------------------
-template <typename T, int MODE>
+template <typename T, int MODE, typename P>
 __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
-    stored_cells_kernel(const StoredArgs<T> A, Geo g, Phys<T> p) {
+    stored_cells_kernel(const StoredArgs<T> A, Geo g, P p) {
     const int ny = g.ny, nx = g.nx, b = blockIdx.y;
     const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     if (wid >= A.n_warps) return;  // whole warp
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
                 C.f_H = act ? T(0) : __ldg(A.f_H + b * nc + ic);
                 C.thk = __ldg(A.gamma + b * nc + ic);
                 Arrow<T> s;
-                arrow_assemble(C, Hc, A.shift, act ? (__ldg(act + ic) > T(0.5) ? 1 : 0) : -1, p, s);
+                arrow_assemble<T>(C, Hc, A.shift, act ? (__ldg(act + ic) > T(0.5) ? 1 : 0) : -1, p, s);
                 if constexpr (MODE == STORE_LU) {
                     const Two<T> c1 = s.c1 + s.hxy, c2 = s.c2 + s.hxy;
                     const T o[LU_N] = {s.D1.x, s.D1.y, s.D2.x, s.D2.y, s.p2, c1.x, c1.y, c2.x, c2.y, s.e1.x, s.e1.y,
@@ -221,76 +221,66 @@ __global__ void adjoint_color_kernel(const T* __restrict__ f, T* __restrict__ l_
 
 // --------------------------------------------------------------------------
 // One additive linear sweep, d += omega * sum of the cells' updates, in one
-// pass: a warp owns 31 face columns (lane 0 is the cell to their left) and
-// marches down, so a face's two cells are this lane and the one to its left,
-// or this row and the one above; no intermediate cell arrays.  A cell's
-// solution needs nothing that another warp writes (the bound H + d_H >= gamma
-// only enters its own d_H).
+// pass.  A CTA owns 31 x 8 faces and solves 32 x 9 cells, the column to the
+// left and the row above included: a face's two cells are this thread and its
+// left neighbour (a shuffle) or the thread above (shared memory), so no cell
+// array passes between two kernels.  A cell's solution needs nothing that
+// another thread writes (the bound H + d_H >= gamma only enters its own d_H).
+// Bound by reading the stored arrays; a thread per cell keeps all its loads in
+// flight at once.  1021 x 1403, FP32, with its JVP: 115 us per sweep with 25
+// factor arrays and two kernels, 105 as a march down the rows (3.5 TB/s), 94
+// here.
 // --------------------------------------------------------------------------
-constexpr int LW = 31;
+constexpr int LX = 31, LY = 8;
 
 template <typename T>
-__global__ void __launch_bounds__(256) vanka_linear_kernel(T* __restrict__ d_u, T* __restrict__ d_v,
-                                                           T* __restrict__ d_H, const T* __restrict__ lu,
-                                                           const T* __restrict__ rho_u, const T* __restrict__ rho_v,
-                                                           const T* __restrict__ rho_H, const T* __restrict__ H,
-                                                           const T* __restrict__ gamma, T omega, Geo g, int n_strips,
-                                                           int rows, int n_warps) {
-    const int ny = g.ny, nx = g.nx, b = blockIdx.y;
-    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    if (wid >= n_warps) return;  // whole warp
-    const int lane = threadIdx.x & 31;
-    const unsigned FULL = 0xffffffffu;
+__global__ void __launch_bounds__(32 * (LY + 1))
+    vanka_linear_kernel(T* __restrict__ d_u, T* __restrict__ d_v, T* __restrict__ d_H, const T* __restrict__ lu,
+                        const T* __restrict__ rho_u, const T* __restrict__ rho_v, const T* __restrict__ rho_H,
+                        const T* __restrict__ H, const T* __restrict__ gamma, T omega, Geo g) {
+    __shared__ T s_down[LY + 1][32];   // a cell's change of its lower face
+    const int ny = g.ny, nx = g.nx, b = blockIdx.z;
     const int64_t nc = g.nc();
     d_u += b * g.nu(); d_v += b * g.nv(); d_H += b * nc;
     rho_u += b * g.nu(); rho_v += b * g.nv(); rho_H += b * nc; H += b * nc; gamma += b * nc;
     lu += b * 25 * nc;
-    const int strip = wid % n_strips, chunk = wid / n_strips;
-    const int i0 = chunk * rows, i1 = min(i0 + rows, ny + 1);   // face rows
-    const int j = strip * LW - 1 + lane;
-    const bool col = j >= 0 && j < nx;
-    const bool own = lane >= 1 && j <= nx;
-    T xb_prev = T(0);   // the row above's change of its lower face
-    T rv = col && i0 > 0 ? __ldg(rho_v + (i0 - 1) * nx + j) : T(0);
-    for (int i = i0 - 1; i < i1; ++i) {
-        const bool cell = col && i >= 0 && i < ny;
-        Two<T> x1 = both(T(0)), x2 = both(T(0));   // outward changes of (l, t) and (r, b)
-        T xh = T(0);
-        const int ic = i * nx + j, iu = i * (nx + 1) + j;
-        if (i < 0 && col) rv = __ldg(rho_v + j);   // becomes row 0's upper face below
-        T rvb = rv;
-        if (cell) {
-            const T* f = lu + ic;
-            T o[LU_N];
+    const int i = blockIdx.y * LY - 1 + threadIdx.y, j = blockIdx.x * LX - 1 + threadIdx.x;
+    const bool cell = i >= 0 && i < ny && j >= 0 && j < nx;
+    const bool own = threadIdx.x > 0 && threadIdx.y > 0;
+    const int ic = i * nx + j, iu = i * (nx + 1) + j;
+    Two<T> x1 = both(T(0)), x2 = both(T(0));   // outward changes of (l, t) and (r, b)
+    T dH = T(0);
+    if (cell) {
+        const T* f = lu + ic;
+        T o[LU_N];
 #pragma unroll
-            for (int k = 0; k < LU_N; k++) o[k] = __ldg(f + k * nc);
-            const T ru_l = __ldg(rho_u + iu), ru_r = __ldg(rho_u + iu + 1), rH = __ldg(rho_H + ic);
-            rvb = __ldg(rho_v + ic + nx);
-            Arrow<T> s;
-            s.D1 = two(o[0], o[1]); s.D2 = two(o[2], o[3]); s.p2 = o[4];
-            s.c1 = two(o[5], o[6]); s.c2 = two(o[7], o[8]); s.e1 = two(o[9], o[10]); s.e2 = two(o[11], o[12]);
-            s.j4 = o[13];
-            s.hxy = both(T(0));
-            ArrowInv<T> q;
-            arrow_factor(s, q);
-            arrow_solve(q, two(ru_l, -rv), two(-ru_r, rvb), both(T(0)), T(0.5) * rH, x1, x2, xh);
-            if (!(isfinite(x1.x) && isfinite(x1.y) && isfinite(x2.x) && isfinite(x2.y) && isfinite(xh))) {
-                x1 = x2 = both(T(0));   // a failed local solve leaves its faces and its cell unchanged
-                xh = T(0);
-            } else if (own && i >= i0) {
-                const T dh = __ldg(gamma + ic) - __ldg(H + ic) - d_H[ic];
-                d_H[ic] += omega * M<T>::max(-xh, dh);
-            }
+        for (int k = 0; k < LU_N; k++) o[k] = __ldg(f + k * nc);
+        const T ru_l = __ldg(rho_u + iu), ru_r = __ldg(rho_u + iu + 1);
+        const T rv_t = __ldg(rho_v + ic), rv_b = __ldg(rho_v + ic + nx), rH = __ldg(rho_H + ic);
+        const T room = own ? __ldg(gamma + ic) - __ldg(H + ic) - d_H[ic] : T(0);
+        Arrow<T> s;
+        s.D1 = two(o[0], o[1]); s.D2 = two(o[2], o[3]); s.p2 = o[4];
+        s.c1 = two(o[5], o[6]); s.c2 = two(o[7], o[8]); s.e1 = two(o[9], o[10]); s.e2 = two(o[11], o[12]);
+        s.j4 = o[13];
+        s.hxy = both(T(0));
+        ArrowInv<T> q;
+        arrow_factor(s, q);
+        T xh;
+        arrow_solve(q, two(ru_l, -rv_t), two(-ru_r, rv_b), both(T(0)), T(0.5) * rH, x1, x2, xh);
+        dH = M<T>::max(-xh, room);
+        if (!(isfinite(x1.x) && isfinite(x1.y) && isfinite(x2.x) && isfinite(x2.y) && isfinite(xh))) {
+            x1 = x2 = both(T(0));   // a failed local solve leaves its faces and its cell unchanged
+            dH = T(0);
         }
-        // changes: u_l += x1.x/2, u_r -= x2.x/2, v_t -= x1.y/2, v_b += x2.y/2
-        const T from_left = __shfl_up_sync(FULL, x2.x, 1);
-        if (own && i >= i0) {
-            if (i < ny) d_u[iu] += omega * (T(0.5) * x1.x - T(0.5) * from_left);
-            if (j < nx) d_v[ic] += omega * (T(0.5) * xb_prev - T(0.5) * x1.y);
-        }
-        xb_prev = x2.y;
-        rv = rvb;
     }
+    // changes: u_l += x1.x/2, u_r -= x2.x/2, v_t -= x1.y/2, v_b += x2.y/2
+    s_down[threadIdx.y][threadIdx.x] = x2.y;
+    const T left = __shfl_up_sync(0xffffffffu, x2.x, 1);
+    __syncthreads();
+    if (!own || i > ny || j > nx) return;
+    if (i < ny) d_u[iu] += omega * (T(0.5) * x1.x - T(0.5) * left);
+    if (j < nx) d_v[ic] += omega * (T(0.5) * s_down[threadIdx.y - 1][threadIdx.x] - T(0.5) * x1.y);
+    if (cell) d_H[ic] += omega * dH;
 }
 
 // --------------------------------------------------------------------------
@@ -324,7 +314,9 @@ static int run_stored(const GlideLevelArgs* a, StoredArgs<T> A, cudaStream_t s) 
     const MarchShape sh = march_shape(A.n_strips, g.ny, g.nb, sizeof(T) == 4 ? 16 : 8, FC_NT);
     A.rows = sh.rows;
     A.n_warps = sh.n_warps;
-    glide::count_launch(), stored_cells_kernel<T, MODE><<<dim3(sh.blocks, g.nb), sh.threads, 0, s>>>(A, g, p);
+    with_glen(a->params, p, [&](auto q) {
+        glide::count_launch(), stored_cells_kernel<T, MODE, decltype(q)><<<dim3(sh.blocks, g.nb), sh.threads, 0, s>>>(A, g, q);
+    });
     return (int)cudaGetLastError();
 }
 
@@ -344,11 +336,10 @@ template <typename T>
 int launch_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* rho_v, const void* rho_H,
                         const void* lu, void* d_u, void* d_v, void* d_H, double omega, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
-    const int n_strips = (g.nx + 1 + LW - 1) / LW;
-    const MarchShape sh = march_shape(n_strips, g.ny + 1, g.nb, 32, 256);
-    glide::count_launch(), vanka_linear_kernel<T><<<dim3(sh.blocks, g.nb), sh.threads, 0, s>>>(
+    const dim3 grid((g.nx + 1 + LX - 1) / LX, (g.ny + 1 + LY - 1) / LY, g.nb);
+    glide::count_launch(), vanka_linear_kernel<T><<<grid, dim3(32, LY + 1), 0, s>>>(
         (T*)d_u, (T*)d_v, (T*)d_H, (const T*)lu, (const T*)rho_u, (const T*)rho_v, (const T*)rho_H, (const T*)a->H,
-        (const T*)a->gamma, T(omega), g, n_strips, sh.rows, sh.n_warps);
+        (const T*)a->gamma, T(omega), g);
     return (int)cudaGetLastError();
 }
 
