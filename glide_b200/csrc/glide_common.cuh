@@ -20,6 +20,57 @@ void count_launch();
 long long launch_total();
 
 // --------------------------------------------------------------------------
+// Chained launches.  A smoother is a chain of short kernels, each reading what
+// the one before wrote; between two of them the chip idles for the launch.  A
+// kernel launched with launch_chained() may start while its predecessor still
+// runs (programmatic stream serialization); chain_enter<true>(), its first
+// statement, lets its own successor do the same and then waits until the
+// predecessor has completed and its writes are visible.  Every thread of such
+// a kernel calls it before its first access, so completion is transitive along
+// the chain.  The predecessor's writes fall into the kernel's lifetime, so it
+// must not read them through the read-only path: ld<true>() loads without it,
+// and indices take chain_enter()'s zero, which keeps the compiler from moving
+// a load above the wait.  Kernels that fill the chip gain nothing and run with
+// CHAIN = false and read-only loads (2-3 % faster there): 200 sweeps of a 32^2
+// level, launched one by one: 2.87 ms plain, 2.17 ms chained.
+// --------------------------------------------------------------------------
+template <bool CHAIN> __device__ __forceinline__ int chain_enter() {
+    if constexpr (!CHAIN) return 0;
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    int zero = 0;
+    asm volatile("" : "+r"(zero)::"memory");
+    return zero;
+}
+template <bool CHAIN, typename T> __device__ __forceinline__ T ld(const T* p) {
+    if constexpr (CHAIN)
+        return __ldca(p);
+    else
+        return __ldg(p);
+}
+
+template <bool CHAIN, typename... KA, typename... A>
+inline void launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, cudaStream_t s, A&&... args) {
+    count_launch();
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &at;
+    if constexpr (CHAIN) {
+        // a captured graph issues its kernels back to back by itself (32^2: 8.1 us per sweep either way)
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        cudaStreamIsCapturing(s, &st);
+        c.numAttrs = st == cudaStreamCaptureStatusNone ? 1 : 0;
+    }
+    cudaLaunchKernelEx(&c, kernel, KA(args)...);
+}
+static inline int64_t blocks_of(dim3 g) { return int64_t(g.x) * g.y * g.z; }
+
+// --------------------------------------------------------------------------
 // precision helpers
 // --------------------------------------------------------------------------
 template <typename T> struct M;
@@ -124,17 +175,17 @@ __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? l
 // element counts: the entry points reject problems whose fields reach 2^31
 // elements (GLIDE_E_TOO_LARGE).
 // --------------------------------------------------------------------------
-template <typename T>
+template <bool CHAIN = false, typename T>
 __device__ __forceinline__ T ldu(const T* __restrict__ u, int i, int j, int ny, int nx) {
-    return __ldg(u + (clampi(i, 0, ny - 1) * (nx + 1) + clampi(j, 0, nx)));
+    return ld<CHAIN>(u + (clampi(i, 0, ny - 1) * (nx + 1) + clampi(j, 0, nx)));
 }
-template <typename T>
+template <bool CHAIN = false, typename T>
 __device__ __forceinline__ T ldv(const T* __restrict__ v, int i, int j, int ny, int nx) {
-    return __ldg(v + (clampi(i, 0, ny) * nx + clampi(j, 0, nx - 1)));
+    return ld<CHAIN>(v + (clampi(i, 0, ny) * nx + clampi(j, 0, nx - 1)));
 }
-template <typename T>
+template <bool CHAIN = false, typename T>
 __device__ __forceinline__ T ldc(const T* __restrict__ a, int i, int j, int ny, int nx) {
-    return __ldg(a + (clampi(i, 0, ny - 1) * nx + clampi(j, 0, nx - 1)));
+    return ld<CHAIN>(a + (clampi(i, 0, ny - 1) * nx + clampi(j, 0, nx - 1)));
 }
 
 // Stage a clamped window [r0, r0+R) x [c0, c0+C) of a (rows x cols) field
@@ -347,22 +398,22 @@ __device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>
 }
 
 // Load the 12 faces around cell (i,j) from a u/v pair (clamped).
-template <typename T>
+template <bool CHAIN = false, typename T>
 __device__ __forceinline__ EtaIn<T> eta_inputs(const T* __restrict__ u, const T* __restrict__ v, int i, int j,
                                                int ny, int nx) {
     EtaIn<T> a;
-    a.ul = ldu(u, i, j, ny, nx);
-    a.ur = ldu(u, i, j + 1, ny, nx);
-    a.vt = ldv(v, i, j, ny, nx);
-    a.vb = ldv(v, i + 1, j, ny, nx);
-    a.u_tl = ldu(u, i - 1, j, ny, nx);
-    a.u_tr = ldu(u, i - 1, j + 1, ny, nx);
-    a.u_bl = ldu(u, i + 1, j, ny, nx);
-    a.u_br = ldu(u, i + 1, j + 1, ny, nx);
-    a.v_lt = ldv(v, i, j - 1, ny, nx);
-    a.v_rt = ldv(v, i, j + 1, ny, nx);
-    a.v_lb = ldv(v, i + 1, j - 1, ny, nx);
-    a.v_rb = ldv(v, i + 1, j + 1, ny, nx);
+    a.ul = ldu<CHAIN>(u, i, j, ny, nx);
+    a.ur = ldu<CHAIN>(u, i, j + 1, ny, nx);
+    a.vt = ldv<CHAIN>(v, i, j, ny, nx);
+    a.vb = ldv<CHAIN>(v, i + 1, j, ny, nx);
+    a.u_tl = ldu<CHAIN>(u, i - 1, j, ny, nx);
+    a.u_tr = ldu<CHAIN>(u, i - 1, j + 1, ny, nx);
+    a.u_bl = ldu<CHAIN>(u, i + 1, j, ny, nx);
+    a.u_br = ldu<CHAIN>(u, i + 1, j + 1, ny, nx);
+    a.v_lt = ldv<CHAIN>(v, i, j - 1, ny, nx);
+    a.v_rt = ldv<CHAIN>(v, i, j + 1, ny, nx);
+    a.v_lb = ldv<CHAIN>(v, i + 1, j - 1, ny, nx);
+    a.v_rb = ldv<CHAIN>(v, i + 1, j + 1, ny, nx);
     return a;
 }
 

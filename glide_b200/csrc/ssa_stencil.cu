@@ -8,6 +8,8 @@
 // barrier is needed.  Every output has exactly one writer, so results are
 // deterministic (the reference scatters its VJP with float atomics,
 // glide/cuda/residuals.cu:617-1021).
+#include <type_traits>
+
 #include "glide_common.cuh"
 
 namespace glide {
@@ -43,9 +45,9 @@ __device__ __forceinline__ T driving_s(T Hm, T Hp, T Sm, T Sp, T dxi, bool valid
 #ifndef GLIDE_RS_MINB64
 #define GLIDE_RS_MINB64 2
 #endif
-// Ix: the element-index type of the per-field offsets (int when every field
-// has fewer than 2^31 elements, which keeps the address arithmetic 32-bit).
-template <typename T, typename Ix, typename P>
+// Offsets within a field are 32-bit: the entry points refuse fields of 2^31
+// elements.
+template <typename T, bool CHAIN, typename P>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_RS_MINB64) residual_stream_kernel(
     T* __restrict__ o_u, T* __restrict__ o_v, T* __restrict__ o_H,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
@@ -53,7 +55,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
     const T* __restrict__ mask, const T* __restrict__ gamma, Geo g, P p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
-    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32 + chain_enter<CHAIN>();
     if (wid >= n_warps) return;  // whole warp
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
@@ -75,9 +77,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
     const unsigned FULL = 0xffffffffu;
     const T dxi = p.dxi;
     const T rr = rho_ratio<T>();
-    auto U = [&](int r, int col) -> T { return __ldg(u + Ix(clampi(r, 0, ny - 1)) * (nx + 1) + col); };
-    auto Vf = [&](int r, int col) -> T { return __ldg(v + Ix(clampi(r, 0, ny)) * nx + col); };
-    auto Cell = [&](const T* a, int r) -> T { return __ldg(a + Ix(clampi(r, 0, ny - 1)) * nx + jcc); };
+    auto U = [&](int r, int col) -> T { return ld<CHAIN>(u + clampi(r, 0, ny - 1) * (nx + 1) + col); };
+    auto Vf = [&](int r, int col) -> T { return ld<CHAIN>(v + clampi(r, 0, ny) * nx + col); };
+    auto Cell = [&](const T* a, int r) -> T { return ld<CHAIN>(a + clampi(r, 0, ny - 1) * nx + jcc); };
 
     // state at the start of iteration i: u, v rows i and i+1; cell rows i-1 and i;
     // eta*H of row i; vertex sxy of row i; syy of row i-1
@@ -106,12 +108,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
         r.vL2 = first ? Vf(k + 2, jvL) : T(0);
         r.vR2 = last ? Vf(k + 2, jvR) : T(0);
         r.H = Cell(H, k + 1); r.bed = Cell(bed, k + 1); r.beta = Cell(beta, k + 1); r.B = Cell(B, k + 1);
-        const Ix ro = clampi(k, 0, ny - 1);
-        r.fu = __ldg(f_u + ro * (nx + 1) + jo);
-        r.fv = __ldg(f_v + ro * nx + jo);
-        r.fH = __ldg(f_H + ro * nx + jo);
-        r.m = __ldg(mask + ro * nx + jo);
-        r.gam = __ldg(gamma + ro * nx + jo);
+        const int ro = clampi(k, 0, ny - 1);
+        r.fu = ld<CHAIN>(f_u + ro * (nx + 1) + jo);
+        r.fv = ld<CHAIN>(f_v + ro * nx + jo);
+        r.fH = ld<CHAIN>(f_H + ro * nx + jo);
+        r.m = ld<CHAIN>(mask + ro * nx + jo);
+        r.gam = ld<CHAIN>(gamma + ro * nx + jo);
         return r;
     };
     RowIn nxt;
@@ -159,7 +161,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
             const T ScL = __shfl_up_sync(FULL, Sc, 1);
             const T becL = __shfl_up_sync(FULL, bec, 1), becR = __shfl_down_sync(FULL, bec, 1);
             if (own) {
-                const Ix ic = Ix(i) * nx + jc;
+                const int ic = i * nx + jc;
                 // ---- mass row (residuals.cu:50-84)
                 {
                     const T m = m_i;
@@ -182,12 +184,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
                     val += basal_drag_g(uL0, gcL, gcc, becL, bec, p).res -
                            driving_s(HcL, Hc, ScL, Sc, dxi, jc > 0 && jc < nx);
                     val -= fu_i;
-                    o_u[Ix(i) * (nx + 1) + jc] = val;
+                    o_u[i * (nx + 1) + jc] = val;
                     if (jc == nx - 1) {
                         T ve = (sxxR - sxx) * dxi + (sxy0R - sxy1R) * dxi;
                         ve += basal_drag_g(uR0s, gcc, gcR, bec, becR, p).res - T(0) * dxi;
-                        ve -= f_u[Ix(i) * (nx + 1) + nx];
-                        o_u[Ix(i) * (nx + 1) + nx] = ve;
+                        ve -= ld<CHAIN>(f_u + (i * (nx + 1) + nx));
+                        o_u[i * (nx + 1) + nx] = ve;
                     }
                 }
                 // ---- v-face (i, jc) and, at the bottom edge, (ny, jc)
@@ -200,8 +202,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
                     if (i == ny - 1) {
                         T ve = (syy - T(0)) * dxi + (sxy1R - sxy1) * dxi;
                         ve += basal_drag_g(v1, gcc, gp, bec, betap, p).res - T(0) * dxi;
-                        ve -= f_v[Ix(ny) * nx + jc];
-                        o_v[Ix(ny) * nx + jc] = ve;
+                        ve -= ld<CHAIN>(f_v + (ny * nx + jc));
+                        o_v[ny * nx + jc] = ve;
                     }
                 }
             }
@@ -232,7 +234,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_RS_MINB32 : GLIDE_
 #ifndef GLIDE_JS_MINB64
 #define GLIDE_JS_MINB64 1
 #endif
-template <typename T, bool ADD, typename Ix, typename P>
+template <typename T, bool ADD, bool CHAIN, typename P>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_JS_MINB64) jvp_stream_kernel(
     T* __restrict__ o_u, T* __restrict__ o_v, T* __restrict__ o_H,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
@@ -241,7 +243,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
     const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
     const T* __restrict__ mask, Geo g, P p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
-    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32 + chain_enter<CHAIN>();
     if (wid >= n_warps) return;  // whole warp
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
@@ -265,10 +267,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
     const T dxi = p.dxi;
     const T rr = rho_ratio<T>();
     auto Uf = [&](const T* a, int r, int col) -> T {
-        return __ldg(a + Ix(clampi(r, 0, ny - 1)) * (nx + 1) + col);
+        return ld<CHAIN>(a + clampi(r, 0, ny - 1) * (nx + 1) + col);
     };
-    auto Vf = [&](const T* a, int r, int col) -> T { return __ldg(a + Ix(clampi(r, 0, ny)) * nx + col); };
-    auto Cell = [&](const T* a, int r) -> T { return __ldg(a + Ix(clampi(r, 0, ny - 1)) * nx + jcc); };
+    auto Vf = [&](const T* a, int r, int col) -> T { return ld<CHAIN>(a + clampi(r, 0, ny) * nx + col); };
+    auto Cell = [&](const T* a, int r) -> T { return ld<CHAIN>(a + clampi(r, 0, ny - 1) * nx + jcc); };
     // slope factor of the surface max(bed, -rho H) + H with respect to H
     auto slope = [&](T Hx, T bx) -> T { return T(1) + (bx > -rr * Hx ? T(0) : -rr); };
 
@@ -303,12 +305,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
         r.dvR2 = last ? Vf(d_v, k + 2, jvR) : T(0);
         r.H = Cell(H, k + 1); r.bed = Cell(bed, k + 1); r.beta = Cell(beta, k + 1); r.B = Cell(B, k + 1);
         r.dH = Cell(d_H, k + 1);
-        const Ix ro = clampi(k, 0, ny - 1);
-        r.m = __ldg(mask + ro * nx + jo);
+        const int ro = clampi(k, 0, ny - 1);
+        r.m = ld<CHAIN>(mask + ro * nx + jo);
         if constexpr (ADD) {
-            r.bu = __ldg(base_u + ro * (nx + 1) + jo);
-            r.bv = __ldg(base_v + ro * nx + jo);
-            r.bH = __ldg(base_H + ro * nx + jo);
+            r.bu = ld<CHAIN>(base_u + ro * (nx + 1) + jo);
+            r.bv = ld<CHAIN>(base_v + ro * nx + jo);
+            r.bH = ld<CHAIN>(base_H + ro * nx + jo);
         } else {
             r.bu = r.bv = r.bH = T(0);
         }
@@ -389,7 +391,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
             const T ScL = __shfl_up_sync(FULL, Sc, 1), kHcL = __shfl_up_sync(FULL, kHc, 1);
             const T becL = __shfl_up_sync(FULL, bec, 1), becR = __shfl_down_sync(FULL, bec, 1);
             if (own) {
-                const Ix ic = Ix(i) * nx + jc;
+                const int ic = i * nx + jc;
                 // ---- mass row
                 {
                     const T m = cur.m;
@@ -416,13 +418,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
                     const T d_Hm = (T(0.5) * dS * dxi - Havg * kHcL * dxi) * w;
                     const T d_Hp = (T(0.5) * dS * dxi + Havg * kHc * dxi) * w;
                     val -= d_Hm * dHcL + d_Hp * dHc;
-                    o_u[Ix(i) * (nx + 1) + jc] = ADD ? cur.bu + val : val;
+                    o_u[i * (nx + 1) + jc] = ADD ? cur.bu + val : val;
                     if (jc == nx - 1) {
                         T ve = (dsxxR - dsxx) * dxi + (dsxy0R - dsxy1R) * dxi;
                         const BasalDrag<T> te = basal_drag_g(uR0s, gcc, gcR, bec, becR, p);
                         ve += te.d_vel * duR0s + te.d_H1 * dHc + te.d_H2 * dHcR;
-                        const Ix oe = Ix(i) * (nx + 1) + nx;
-                        o_u[oe] = ADD ? __ldg(base_u + oe) + ve : ve;
+                        const int oe = i * (nx + 1) + nx;
+                        o_u[oe] = ADD ? ld<CHAIN>(base_u + oe) + ve : ve;
                     }
                 }
                 // ---- v-face (i, jc) and, at the bottom edge, (ny, jc)
@@ -440,8 +442,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
                         T ve = (dsyy - T(0)) * dxi + (dsxy1R - dsxy1) * dxi;
                         const BasalDrag<T> te = basal_drag_g(v1, gcc, gp, bec, betap, p);
                         ve += te.d_vel * dv1 + te.d_H1 * dHc + te.d_H2 * dHp;
-                        const Ix oe = Ix(ny) * nx + jc;
-                        o_v[oe] = ADD ? __ldg(base_v + oe) + ve : ve;
+                        const int oe = ny * nx + jc;
+                        o_v[oe] = ADD ? ld<CHAIN>(base_v + oe) + ve : ve;
                     }
                 }
             }
@@ -481,7 +483,7 @@ constexpr int VS_NT = 128;
 #ifndef GLIDE_VS_MINB64
 #define GLIDE_VS_MINB64 2
 #endif
-template <typename T, bool RF, typename Ix, typename P>
+template <typename T, bool RF, bool CHAIN, typename P>
 __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLIDE_VS_MINB64) vjp_stream_kernel(
     T* __restrict__ o_u, T* __restrict__ o_v, T* __restrict__ o_H,
     const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
@@ -490,7 +492,7 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
     const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H, int exact_boundary, Geo g,
     P p, int n_strips, int rows, int n_warps) {
     const int ny = g.ny, nx = g.nx;
-    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
+    const int wid = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32 + chain_enter<CHAIN>();
     if (wid >= n_warps) return;  // whole warp
     const int lane = threadIdx.x & 31;
     const int b = blockIdx.y;
@@ -514,10 +516,10 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
     const T dxi = p.dxi;
     const T rr = rho_ratio<T>();
     auto Uf = [&](const T* a, int r, int col) -> T {
-        return __ldg(a + Ix(clampi(r, 0, ny - 1)) * (nx + 1) + col);
+        return ld<CHAIN>(a + clampi(r, 0, ny - 1) * (nx + 1) + col);
     };
-    auto Vf = [&](const T* a, int r, int col) -> T { return __ldg(a + Ix(clampi(r, 0, ny)) * nx + col); };
-    auto Cell = [&](const T* a, int r) -> T { return __ldg(a + Ix(clampi(r, 0, ny - 1)) * nx + jcc); };
+    auto Vf = [&](const T* a, int r, int col) -> T { return ld<CHAIN>(a + clampi(r, 0, ny) * nx + col); };
+    auto Cell = [&](const T* a, int r) -> T { return ld<CHAIN>(a + clampi(r, 0, ny - 1) * nx + jcc); };
     auto slope = [&](T Hx, T bx) -> T { return T(1) + (bx > -rr * Hx ? T(0) : -rr); };
 
     int i = i0 - 2;
@@ -557,10 +559,10 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
         r.H = Cell(H, k + 1); r.bed = Cell(bed, k + 1); r.beta = Cell(beta, k + 1); r.B = Cell(B, k + 1);
         r.lH = Cell(lH, k + 1); r.m = Cell(mask, k + 1);
         if constexpr (RF) {
-            const Ix ro = clampi(k, 0, ny - 1);
-            r.fu = __ldg(f_u + ro * (nx + 1) + jo);
-            r.fv = __ldg(f_v + ro * nx + jo);
-            r.fH = __ldg(f_H + ro * nx + jo);
+            const int ro = clampi(k, 0, ny - 1);
+            r.fu = ld<CHAIN>(f_u + ro * (nx + 1) + jo);
+            r.fv = ld<CHAIN>(f_v + ro * nx + jo);
+            r.fH = ld<CHAIN>(f_H + ro * nx + jo);
         } else {
             r.fu = r.fv = r.fH = T(0);
         }
@@ -680,7 +682,7 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
             const T W0R = __shfl_down_sync(FULL, W0, 1), W1R = __shfl_down_sync(FULL, W1, 1);
             const T ltR = __shfl_down_sync(FULL, ltc, 1);
             if (own) {
-                const Ix ic = Ix(i) * nx + jc;
+                const int ic = i * nx + jc;
                 // ---- H row
                 {
                     const Calving<T> cv = calving_g(Hc, gcc, p);
@@ -704,14 +706,14 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
                     const BasalDrag<T> tb = basal_drag_g(uL0, gcL, gcc, becL, bec, p);
                     const Flux<T> q = upwind_flux(uL0, HcL, Hc, jc > 0 && jc < nx);
                     val += luL0 * tb.d_vel + (ltL - ltc) * dxi * q.d_vel;
-                    o_u[Ix(i) * (nx + 1) + jc] = RF ? cur.fu - val : val;
+                    o_u[i * (nx + 1) + jc] = RF ? cur.fu - val : val;
                     if (jc == nx - 1) {
                         T ve = (dsxxR - dsxx) * dxi + (dsxy0R - dsxy1R) * dxi;
                         const BasalDrag<T> te = basal_drag_g(uR0s, gcc, gcR, bec, becR, p);
                         const Flux<T> qe = upwind_flux(uR0s, Hc, Hc, false);  // H(i, nx) clamps to H(i, nx-1)
                         ve += luR0s * te.d_vel + (ltc - ltR) * dxi * qe.d_vel;
-                        const Ix oe = Ix(i) * (nx + 1) + nx;
-                        o_u[oe] = RF ? __ldg(f_u + oe) - ve : ve;
+                        const int oe = i * (nx + 1) + nx;
+                        o_u[oe] = RF ? ld<CHAIN>(f_u + oe) - ve : ve;
                     }
                 }
                 // ---- v-face (i, jc) and, at the bottom edge, (ny, jc)
@@ -726,8 +728,8 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
                         const BasalDrag<T> te = basal_drag_g(v1, gcc, gp, bec, betap, p);
                         const Flux<T> qe = upwind_flux(v1, Hp, Hc, false);
                         ve += lv1 * te.d_vel + (ltp - ltc) * dxi * qe.d_vel;
-                        const Ix oe = Ix(ny) * nx + jc;
-                        o_v[oe] = RF ? __ldg(f_v + oe) - ve : ve;
+                        const int oe = ny * nx + jc;
+                        o_v[oe] = RF ? ld<CHAIN>(f_v + oe) - ve : ve;
                     }
                 }
             }
@@ -802,10 +804,6 @@ struct StreamShape {
     int n_strips, rows, n_warps, threads;
     unsigned blocks;
 };
-// 32-bit element offsets suffice when every field of one problem has fewer
-// than 2^31 elements (u and v have (ny+1)(nx+1) at most)
-static inline bool index32(const Geo& g) { return int64_t(g.ny + 1) * (g.nx + 1) < (int64_t(1) << 31); }
-
 static inline StreamShape stream_shape(const Geo& g, int max_threads) {
     StreamShape sh;
     sh.n_strips = (g.nx + SW - 1) / SW;
@@ -819,25 +817,28 @@ static inline StreamShape stream_shape(const Geo& g, int max_threads) {
     return sh;
 }
 
+// chained (see glide_common.cuh) while the march has at most one CTA per SM
+template <typename F> static void chain_if(dim3 grid, F&& go) {
+    if (blocks_of(grid) <= 148)
+        go(std::true_type{});
+    else
+        go(std::false_type{});
+}
+
 template <typename T>
 int launch_residual(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, void* r_u, void* r_v,
                     void* r_H, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     const StreamShape sh = stream_shape(g, 256);
     const dim3 grid(sh.blocks, g.nb);
-    auto go = [&](auto kernel, const auto& p) {
-        glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
-            (T*)r_u, (T*)r_v, (T*)r_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u,
-            (const T*)f_v, (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
-            (const T*)a->gamma, g, p, sh.n_strips, sh.rows, sh.n_warps);
-    };
-    with_glen(a->params, p, [&](auto q) {
-        using P = decltype(q);
-        if (index32(g))
-            go(residual_stream_kernel<T, int, P>, q);
-        else
-            go(residual_stream_kernel<T, int64_t, P>, q);
+    with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
+        chain_if(grid, [&](auto chain) {
+            constexpr bool CHAIN = decltype(chain)::value;
+            launch_chained<CHAIN>(residual_stream_kernel<T, CHAIN, decltype(p)>, grid, sh.threads, s, (T*)r_u, (T*)r_v,
+                                  (T*)r_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u,
+                                  (const T*)f_v, (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta,
+                                  (const T*)a->mask, (const T*)a->gamma, g, p, sh.n_strips, sh.rows, sh.n_warps);
+        });
     });
     return (int)cudaGetLastError();
 }
@@ -847,22 +848,21 @@ template <typename T>
 int launch_jvp(const GlideLevelArgs* a, const void* d_u, const void* d_v, const void* d_H, const void* base_u,
                const void* base_v, const void* base_H, void* j_u, void* j_v, void* j_H, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     const StreamShape sh = stream_shape(g, 256);
     const dim3 grid(sh.blocks, g.nb);
-    auto go = [&](auto kernel, const auto& p) {
-        glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
-            (T*)j_u, (T*)j_v, (T*)j_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)d_u,
-            (const T*)d_v, (const T*)d_H, (const T*)base_u, (const T*)base_v, (const T*)base_H, (const T*)a->bed,
-            (const T*)a->B, (const T*)a->beta, (const T*)a->mask, g, p, sh.n_strips, sh.rows, sh.n_warps);
-    };
-    const bool i32 = index32(g);
-    with_glen(a->params, p, [&](auto q) {
-        using P = decltype(q);
-        if (base_u)
-            i32 ? go(jvp_stream_kernel<T, true, int, P>, q) : go(jvp_stream_kernel<T, true, int64_t, P>, q);
-        else
-            i32 ? go(jvp_stream_kernel<T, false, int, P>, q) : go(jvp_stream_kernel<T, false, int64_t, P>, q);
+    with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
+        chain_if(grid, [&](auto chain) {
+            constexpr bool CHAIN = decltype(chain)::value;
+            auto go = [&](auto kernel) {
+                launch_chained<CHAIN>(kernel, grid, sh.threads, s, (T*)j_u, (T*)j_v, (T*)j_H, (const T*)a->u,
+                                      (const T*)a->v, (const T*)a->H, (const T*)d_u, (const T*)d_v, (const T*)d_H,
+                                      (const T*)base_u, (const T*)base_v, (const T*)base_H, (const T*)a->bed,
+                                      (const T*)a->B, (const T*)a->beta, (const T*)a->mask, g, p, sh.n_strips,
+                                      sh.rows, sh.n_warps);
+            };
+            base_u ? go(jvp_stream_kernel<T, true, CHAIN, decltype(p)>)
+                   : go(jvp_stream_kernel<T, false, CHAIN, decltype(p)>);
+        });
     });
     return (int)cudaGetLastError();
 }
@@ -872,22 +872,20 @@ int launch_vjp(const GlideLevelArgs* a, const void* l_u, const void* l_v, const 
                const void* f_v, const void* f_H, void* o_u, void* o_v, void* o_H, int exact_boundary,
                cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
     const StreamShape sh = stream_shape(g, VS_NT);
     const dim3 grid(sh.blocks, g.nb);
-    auto go = [&](auto kernel, const auto& p) {
-        glide::count_launch(), kernel<<<grid, sh.threads, 0, s>>>(
-            (T*)o_u, (T*)o_v, (T*)o_H, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)l_u,
-            (const T*)l_v, (const T*)l_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
-            (const T*)f_u, (const T*)f_v, (const T*)f_H, exact_boundary, g, p, sh.n_strips, sh.rows, sh.n_warps);
-    };
-    const bool i32 = index32(g);
-    with_glen(a->params, p, [&](auto q) {
-        using P = decltype(q);
-        if (f_u != nullptr)
-            i32 ? go(vjp_stream_kernel<T, true, int, P>, q) : go(vjp_stream_kernel<T, true, int64_t, P>, q);
-        else
-            i32 ? go(vjp_stream_kernel<T, false, int, P>, q) : go(vjp_stream_kernel<T, false, int64_t, P>, q);
+    with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
+        chain_if(grid, [&](auto chain) {
+            constexpr bool CHAIN = decltype(chain)::value;
+            auto go = [&](auto kernel) {
+                launch_chained<CHAIN>(kernel, grid, sh.threads, s, (T*)o_u, (T*)o_v, (T*)o_H, (const T*)a->u,
+                                      (const T*)a->v, (const T*)a->H, (const T*)l_u, (const T*)l_v, (const T*)l_H,
+                                      (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
+                                      (const T*)f_u, (const T*)f_v, (const T*)f_H, exact_boundary, g, p, sh.n_strips,
+                                      sh.rows, sh.n_warps);
+            };
+            f_u ? go(vjp_stream_kernel<T, true, CHAIN, decltype(p)>) : go(vjp_stream_kernel<T, false, CHAIN, decltype(p)>);
+        });
     });
     return (int)cudaGetLastError();
 }

@@ -12,11 +12,13 @@
 // memory; the neighbours' grounding sigmoids are hoisted out of the Newton
 // loop.  The local variant gates cells by the reference's 16x16-window /
 // stride-14 block rule (vanka.cu:875-888) through per-tile flags.
+#include <type_traits>
+
 #include "glide_common.cuh"
 
 namespace glide {
 
-constexpr int VX = 32, VY = 8, VNT = VX * VY;
+constexpr int VX = 32;   // tile width; a tile is VX x VY cells, VY = 8, 4 or 1 (see cell_tile)
 constexpr int REF_STRIDE = 14;   // reference block stride (glide/grid.py:182-188)
 constexpr int REF_WIN = 16;      // reference block (active cells + 1 ring)
 
@@ -34,18 +36,18 @@ template <typename T> struct Patch {
 
 // Fill the eta window of a VYxVX tile (+ ring) and the frozen patch of the
 // calling thread's cell.
-template <typename T, typename P>
+template <int VY, bool CHAIN, typename T, typename P>
 __device__ __forceinline__ void eta_window(T (*s_eta)[VX + 2], const T* u, const T* v, const T* B, int i0, int j0,
                                            int ny, int nx, const P& p) {
-    for (int k = threadIdx.x; k < (VY + 2) * (VX + 2); k += VNT) {
+    for (int k = threadIdx.x; k < (VY + 2) * (VX + 2); k += VX * VY) {
         int r = k / (VX + 2), c = k - r * (VX + 2);
         int ic = clampi(i0 - 1 + r, 0, ny - 1), jc = clampi(j0 - 1 + c, 0, nx - 1);
-        EtaIn<T> e = eta_inputs(u, v, ic, jc, ny, nx);
-        s_eta[r][c] = cell_eta(e, ldc(B, ic, jc, ny, nx), ic, jc, ny, nx, p).eta;
+        EtaIn<T> e = eta_inputs<CHAIN>(u, v, ic, jc, ny, nx);
+        s_eta[r][c] = cell_eta(e, ldc<CHAIN>(B, ic, jc, ny, nx), ic, jc, ny, nx, p).eta;
     }
 }
 
-template <typename T>
+template <bool CHAIN, typename T>
 __device__ __forceinline__ void load_patch(Patch<T>& P, T (*s_eta)[VX + 2], int r, int c, const T* u, const T* v,
                                            const T* H, const T* bed, const T* beta, int i, int j, int ny, int nx,
                                            const Phys<T>& p) {
@@ -56,27 +58,28 @@ __device__ __forceinline__ void load_patch(Patch<T>& P, T (*s_eta)[VX + 2], int 
 #pragma unroll
         for (int b = 0; b < 3; b++) {
             P.eta[a][b] = s_eta[r + a][c + b];
-            P.Hn[a][b] = ldc(H, i - 1 + a, j - 1 + b, ny, nx);
+            P.Hn[a][b] = ldc<CHAIN>(H, i - 1 + a, j - 1 + b, ny, nx);
         }
-    P.bed_c = ldc(bed, i, j, ny, nx); P.bed_l = ldc(bed, i, j - 1, ny, nx); P.bed_r = ldc(bed, i, j + 1, ny, nx);
-    P.bed_t = ldc(bed, i - 1, j, ny, nx); P.bed_b = ldc(bed, i + 1, j, ny, nx);
-    P.beta_c = ldc(beta, i, j, ny, nx); P.beta_l = ldc(beta, i, j - 1, ny, nx); P.beta_r = ldc(beta, i, j + 1, ny, nx);
-    P.beta_t = ldc(beta, i - 1, j, ny, nx); P.beta_b = ldc(beta, i + 1, j, ny, nx);
+    P.bed_c = ldc<CHAIN>(bed, i, j, ny, nx); P.bed_l = ldc<CHAIN>(bed, i, j - 1, ny, nx); P.bed_r = ldc<CHAIN>(bed, i, j + 1, ny, nx);
+    P.bed_t = ldc<CHAIN>(bed, i - 1, j, ny, nx); P.bed_b = ldc<CHAIN>(bed, i + 1, j, ny, nx);
+    P.beta_c = ldc<CHAIN>(beta, i, j, ny, nx); P.beta_l = ldc<CHAIN>(beta, i, j - 1, ny, nx); P.beta_r = ldc<CHAIN>(beta, i, j + 1, ny, nx);
+    P.beta_t = ldc<CHAIN>(beta, i - 1, j, ny, nx); P.beta_b = ldc<CHAIN>(beta, i + 1, j, ny, nx);
     P.g_l = sigmoid(P.bed_l + rho_ratio<T>() * P.Hn[1][0], p.sig_c);
     P.g_r = sigmoid(P.bed_r + rho_ratio<T>() * P.Hn[1][2], p.sig_c);
     P.g_t = sigmoid(P.bed_t + rho_ratio<T>() * P.Hn[0][1], p.sig_c);
     P.g_b = sigmoid(P.bed_b + rho_ratio<T>() * P.Hn[2][1], p.sig_c);
-    P.u_ll = ldu(u, i, j - 1, ny, nx); P.u_rr = ldu(u, i, j + 2, ny, nx);
-    P.u_tl = ldu(u, i - 1, j, ny, nx); P.u_tr = ldu(u, i - 1, j + 1, ny, nx);
-    P.u_bl = ldu(u, i + 1, j, ny, nx); P.u_br = ldu(u, i + 1, j + 1, ny, nx);
-    P.v_lt = ldv(v, i, j - 1, ny, nx); P.v_lb = ldv(v, i + 1, j - 1, ny, nx);
-    P.v_rt = ldv(v, i, j + 1, ny, nx); P.v_rb = ldv(v, i + 1, j + 1, ny, nx);
-    P.v_tt = ldv(v, i - 1, j, ny, nx); P.v_bb = ldv(v, i + 2, j, ny, nx);
+    P.u_ll = ldu<CHAIN>(u, i, j - 1, ny, nx); P.u_rr = ldu<CHAIN>(u, i, j + 2, ny, nx);
+    P.u_tl = ldu<CHAIN>(u, i - 1, j, ny, nx); P.u_tr = ldu<CHAIN>(u, i - 1, j + 1, ny, nx);
+    P.u_bl = ldu<CHAIN>(u, i + 1, j, ny, nx); P.u_br = ldu<CHAIN>(u, i + 1, j + 1, ny, nx);
+    P.v_lt = ldv<CHAIN>(v, i, j - 1, ny, nx); P.v_lb = ldv<CHAIN>(v, i + 1, j - 1, ny, nx);
+    P.v_rt = ldv<CHAIN>(v, i, j + 1, ny, nx); P.v_rb = ldv<CHAIN>(v, i + 1, j + 1, ny, nx);
+    P.v_tt = ldv<CHAIN>(v, i - 1, j, ny, nx); P.v_bb = ldv<CHAIN>(v, i + 2, j, ny, nx);
 }
 
+template <bool CHAIN>
 __device__ __forceinline__ bool ref_tile_on(const int* flags, int i, int j, int nx) {
     const int nbx = nx / REF_STRIDE + 1;
-    return flags[(i / REF_STRIDE) * nbx + j / REF_STRIDE] != 0;
+    return ld<CHAIN>(flags + (i / REF_STRIDE) * nbx + j / REF_STRIDE) != 0;
 }
 
 // Frozen per-cell coefficients of the forward local Newton loop: every term
@@ -341,50 +344,51 @@ template <typename T> __device__ __forceinline__ void lu5_solve_pivot(T (&A)[25]
 
 // Per-cell Newton deltas.  scratch holds 5 cell arrays: 0.5*du_l, 0.5*du_r,
 // 0.5*dv_t, 0.5*dv_b, dH.
-template <typename T, bool LOCAL, typename P>
+template <typename T, int VY, bool LOCAL, bool CHAIN, typename P>
 #ifndef GLIDE_VANKA64_MIN_BLOCKS
 #define GLIDE_VANKA64_MIN_BLOCKS 2
 #endif
 #ifndef GLIDE_VANKA32_MIN_BLOCKS
 #define GLIDE_VANKA32_MIN_BLOCKS 2
 #endif
-__global__ void __launch_bounds__(VNT, sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS : GLIDE_VANKA64_MIN_BLOCKS) vanka_cells_kernel(
+__global__ void __launch_bounds__(VX * VY, (sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS : GLIDE_VANKA64_MIN_BLOCKS) * (8 / VY)) vanka_cells_kernel(
     T* __restrict__ scratch, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
     const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H, const T* __restrict__ bed,
     const T* __restrict__ B, const T* __restrict__ beta, const T* __restrict__ gamma, const int* __restrict__ flags,
     const int* __restrict__ any_active, int n_newton, T shift, T step, int pivot, Geo g, P p) {
     __shared__ T s_eta[VY + 2][VX + 2];
+    const int zero = chain_enter<CHAIN>();
     const int ny = g.ny, nx = g.nx;
-    const int bz = blockIdx.z;
-    if (LOCAL && any_active[bz] == 0) return;
+    const int bz = blockIdx.z + zero;
+    if (LOCAL && ld<CHAIN>(any_active + bz) == 0) return;
     u += bz * g.nu(); v += bz * g.nv(); H += bz * g.nc(); f_u += bz * g.nu(); f_v += bz * g.nv();
     f_H += bz * g.nc(); bed += bz * g.nc(); B += bz * g.nc(); beta += bz * g.nc(); gamma += bz * g.nc();
     const int64_t nc = g.nc();
     scratch += bz * 5 * nc;
     if (LOCAL) flags += bz * int64_t(ny / REF_STRIDE + 1) * (nx / REF_STRIDE + 1);
-    const int i0 = blockIdx.y * VY, j0 = blockIdx.x * VX;
+    const int i0 = blockIdx.y * VY + zero, j0 = blockIdx.x * VX;
     const int r = threadIdx.x / VX, c = threadIdx.x % VX;
     const int i = i0 + r, j = j0 + c;
-    eta_window(s_eta, u, v, B, i0, j0, ny, nx, p);
+    eta_window<VY, CHAIN>(s_eta, u, v, B, i0, j0, ny, nx, p);
     __syncthreads();
     if (i >= ny || j >= nx) return;
-    if (LOCAL && !ref_tile_on(flags, i, j, nx)) return;
+    if (LOCAL && !ref_tile_on<CHAIN>(flags, i, j, nx)) return;
 
     Frozen<T> F;
     {
         Patch<T> pt;
-        load_patch<T>(pt, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
+        load_patch<CHAIN>(pt, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
         make_frozen<T>(F, pt, ny, nx, p);
     }
     // 32-bit offsets within one field (the entry points bound a field below 2^31 elements)
     const int iu = i * (nx + 1) + j, ic32 = i * nx + j;
-    const T ul0 = u[iu], ur0 = u[iu + 1];
-    const T vt0 = v[ic32], vb0 = v[ic32 + nx];
-    const T H0 = H[ic32];
-    const T fu_l = f_u[iu], fu_r = f_u[iu + 1];
-    const T fv_t = f_v[ic32], fv_b = f_v[ic32 + nx];
-    const T fH = f_H[ic32];
-    const T thk = gamma[ic32];
+    const T ul0 = ld<CHAIN>(u + iu), ur0 = ld<CHAIN>(u + iu + 1);
+    const T vt0 = ld<CHAIN>(v + ic32), vb0 = ld<CHAIN>(v + ic32 + nx);
+    const T H0 = ld<CHAIN>(H + ic32);
+    const T fu_l = ld<CHAIN>(f_u + iu), fu_r = ld<CHAIN>(f_u + iu + 1);
+    const T fv_t = ld<CHAIN>(f_v + ic32), fv_b = ld<CHAIN>(f_v + ic32 + nx);
+    const T fH = ld<CHAIN>(f_H + ic32);
+    const T thk = ld<CHAIN>(gamma + ic32);
     const T dti = T(1) / p.dt;
     T ul = ul0, ur = ur0, vt = vt0, vb = vb0, Hc = H0;
     for (int it = 0; it < n_newton; it++) {
@@ -414,34 +418,35 @@ __global__ void __launch_bounds__(VNT, sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS
 }
 
 // U += omega * delta, face delta = sum of the two adjacent cells' halves.
-template <typename T, bool LOCAL>
+template <typename T, bool LOCAL, bool CHAIN>
 __global__ void vanka_apply_kernel(T* __restrict__ u, T* __restrict__ v, T* __restrict__ H,
                                    const T* __restrict__ scratch, const int* __restrict__ flags,
                                    const int* __restrict__ any_active, T omega, Geo g) {
+    const int zero = chain_enter<CHAIN>();
     const int ny = g.ny, nx = g.nx;
-    const int bz = blockIdx.z;
-    if (LOCAL && any_active[bz] == 0) return;
+    const int bz = blockIdx.z + zero;
+    if (LOCAL && ld<CHAIN>(any_active + bz) == 0) return;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.y * blockDim.y + threadIdx.y + zero;
     if (i > ny || j > nx) return;
     const int64_t nc = g.nc();
     u += bz * g.nu(); v += bz * g.nv(); H += bz * g.nc();
     scratch += bz * 5 * nc;
     if (LOCAL) flags += bz * int64_t(ny / REF_STRIDE + 1) * (nx / REF_STRIDE + 1);
-    auto on = [&](int ii, int jj) { return !LOCAL || ref_tile_on(flags, ii, jj, nx); };
+    auto on = [&](int ii, int jj) { return !LOCAL || ref_tile_on<CHAIN>(flags, ii, jj, nx); };
     if (i < ny) {  // u-face (i,j), j in [0,nx]
         T d = T(0);
-        if (j < nx && on(i, j)) d += scratch[int64_t(i) * nx + j];                   // as u_l of cell (i,j)
-        if (j > 0 && on(i, j - 1)) d += scratch[nc + int64_t(i) * nx + j - 1];        // as u_r of cell (i,j-1)
+        if (j < nx && on(i, j)) d += ld<CHAIN>(scratch + int64_t(i) * nx + j);                   // as u_l of cell (i,j)
+        if (j > 0 && on(i, j - 1)) d += ld<CHAIN>(scratch + nc + int64_t(i) * nx + j - 1);        // as u_r of cell (i,j-1)
         u[int64_t(i) * (nx + 1) + j] += omega * d;
     }
     if (j < nx) {  // v-face (i,j), i in [0,ny]
         T d = T(0);
-        if (i < ny && on(i, j)) d += scratch[2 * nc + int64_t(i) * nx + j];
-        if (i > 0 && on(i - 1, j)) d += scratch[3 * nc + int64_t(i - 1) * nx + j];
+        if (i < ny && on(i, j)) d += ld<CHAIN>(scratch + 2 * nc + int64_t(i) * nx + j);
+        if (i > 0 && on(i - 1, j)) d += ld<CHAIN>(scratch + 3 * nc + int64_t(i - 1) * nx + j);
         v[int64_t(i) * nx + j] += omega * d;
     }
-    if (i < ny && j < nx && on(i, j)) H[int64_t(i) * nx + j] += omega * scratch[4 * nc + int64_t(i) * nx + j];
+    if (i < ny && j < nx && on(i, j)) H[int64_t(i) * nx + j] += omega * ld<CHAIN>(scratch + 4 * nc + int64_t(i) * nx + j);
 }
 
 // Local error indicator (glide/solver.py:148-154) and reference-tile flags.
@@ -450,18 +455,20 @@ template <typename T>
 __global__ void error_mask_kernel(T* __restrict__ err_mask, const T* __restrict__ r_u, const T* __restrict__ r_v,
                                   const T* __restrict__ r_H, const T* __restrict__ H, const T* __restrict__ gamma,
                                   T threshold, Geo g) {
+    const int zero = chain_enter<true>();
     const int ny = g.ny, nx = g.nx;
-    const int bz = blockIdx.z;
+    const int bz = blockIdx.z + zero;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.y * blockDim.y + threadIdx.y + zero;
     if (i >= ny || j >= nx) return;
     r_u += bz * g.nu(); r_v += bz * g.nv(); r_H += bz * g.nc(); H += bz * g.nc(); gamma += bz * g.nc();
     err_mask += bz * g.nc();
     const int64_t ic = int64_t(i) * nx + j;
-    T a = r_H[ic], b = H[ic] - gamma[ic];
+    T a = ld<true>(r_H + ic), b = ld<true>(H + ic) - ld<true>(gamma + ic);
     T fb = a + b - M<T>::sqrt(a * a + b * b);
-    T tot = M<T>::abs(r_u[int64_t(i) * (nx + 1) + j + 1]) + M<T>::abs(r_u[int64_t(i) * (nx + 1) + j]) +
-            M<T>::abs(r_v[int64_t(i + 1) * nx + j]) + M<T>::abs(r_v[ic]) + M<T>::abs(fb);
+    T tot = M<T>::abs(ld<true>(r_u + int64_t(i) * (nx + 1) + j + 1)) +
+            M<T>::abs(ld<true>(r_u + int64_t(i) * (nx + 1) + j)) + M<T>::abs(ld<true>(r_v + int64_t(i + 1) * nx + j)) +
+            M<T>::abs(ld<true>(r_v + ic)) + M<T>::abs(fb);
     err_mask[ic] = tot > threshold ? T(1) : T(0);
 }
 
@@ -489,8 +496,26 @@ __global__ void tile_flags_kernel(int* __restrict__ flags, int* __restrict__ any
 // --------------------------------------------------------------------------
 // launchers
 // --------------------------------------------------------------------------
-static inline dim3 cell_grid(const Geo& g) { return dim3((g.nx + VX - 1) / VX, (g.ny + VY - 1) / VY, g.nb); }
+static inline dim3 cell_grid(const Geo& g, int vy) { return dim3((g.nx + VX - 1) / VX, (g.ny + vy - 1) / vy, g.nb); }
 static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (g.ny + 1 + 7) / 8, g.nb); }
+
+// Tile height.  A cell's Newton loop is one long dependent chain, so on a grid
+// that leaves SMs idle a warp should share its scheduler with as few others as
+// possible: quarter-SM tiles of 4 rows up to 32 tiles of 8 (64^2), and up to 96
+// (128^2) single-row tiles of one warp, which the block scheduler spreads
+// evenly.  Microseconds per sweep of 10 Newton steps, FP32, 8 / 4 / 1 rows:
+// 32^2 10.3 / 8.3 / 8.7, 64^2 10.5 / 8.6 / 9.4, 128^2 11.6 / 12.7 / 9.5, 256^2
+// 15.8 / 16.6 / 17.8; FP64 at 128^2 26.7 / 27.2 / 18.8.
+static inline int cell_tile(const Geo& g) {
+    const int64_t tiles = blocks_of(cell_grid(g, 8));
+    return tiles <= 32 ? 4 : tiles <= 96 ? 1 : 8;
+}
+// The sweep's two kernels are chained while they fit the chip about once; not
+// with single-row tiles, whose CTAs would be placed around those of the kernel
+// before and lose their even spread (128^2: 12.9 us per sweep chained, 9.5 not).
+static inline bool sweep_chained(const Geo& g) {
+    return cell_tile(g) != 1 && blocks_of(cell_grid(g, 8)) <= 592;
+}
 
 template <typename T>
 static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton,
@@ -498,13 +523,27 @@ static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v,
                       const Geo& g, cudaStream_t s) {
     with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
         using P = decltype(p);
-        auto go = [&](auto kernel) {
-            glide::count_launch(), kernel<<<cell_grid(g), VNT, 0, s>>>(
-                (T*)scratch, (const T*)a->u, (const T*)a->v, (const T*)a->H, (const T*)f_u, (const T*)f_v,
-                (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, flags,
-                any_active, n_newton, T(shift), T(step), pivot, g, p);
+        auto go = [&](auto vy, auto chain) {
+            constexpr int VY = decltype(vy)::value;
+            constexpr bool CHAIN = decltype(chain)::value;
+            auto run = [&](auto kernel) {
+                launch_chained<CHAIN>(kernel, cell_grid(g, VY), VX * VY, s, (T*)scratch, (const T*)a->u,
+                                      (const T*)a->v, (const T*)a->H, (const T*)f_u, (const T*)f_v, (const T*)f_H,
+                                      (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, flags,
+                                      any_active, n_newton, T(shift), T(step), pivot, g, p);
+            };
+            flags ? run(vanka_cells_kernel<T, VY, true, CHAIN, P>) : run(vanka_cells_kernel<T, VY, false, CHAIN, P>);
         };
-        flags ? go(vanka_cells_kernel<T, true, P>) : go(vanka_cells_kernel<T, false, P>);
+        using std::integral_constant;
+        const int vy = cell_tile(g);
+        if (vy == 4)
+            go(integral_constant<int, 4>{}, std::true_type{});
+        else if (vy == 1)
+            go(integral_constant<int, 1>{}, std::false_type{});
+        else if (sweep_chained(g))
+            go(integral_constant<int, 8>{}, std::true_type{});
+        else
+            go(integral_constant<int, 8>{}, std::false_type{});
     });
 }
 
@@ -513,17 +552,17 @@ int launch_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_
                         int n_newton, double omega, double shift, const int* flags, const int* any_active,
                         void* scratch, cudaStream_t s, double newton_step, int pivot) {
     Geo g{a->ny, a->nx, a->nb};
-    T* u = (T*)a->u;
-    T* v = (T*)a->v;
-    T* H = (T*)a->H;
+    auto apply = [&](auto chain) {
+        constexpr bool CHAIN = decltype(chain)::value;
+        auto run = [&](auto kernel) {
+            launch_chained<CHAIN>(kernel, face_grid(g), dim3(32, 8), s, (T*)a->u, (T*)a->v, (T*)a->H,
+                                  (const T*)scratch, flags, any_active, T(omega), g);
+        };
+        flags ? run(vanka_apply_kernel<T, true, CHAIN>) : run(vanka_apply_kernel<T, false, CHAIN>);
+    };
     for (int k = 0; k < n_iter; k++) {
         run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, pivot, flags, any_active, scratch, g, s);
-        if (flags)
-            glide::count_launch(), vanka_apply_kernel<T, true><<<face_grid(g), dim3(32, 8), 0, s>>>(
-                u, v, H, (const T*)scratch, flags, any_active, T(omega), g);
-        else
-            glide::count_launch(), vanka_apply_kernel<T, false><<<face_grid(g), dim3(32, 8), 0, s>>>(
-                u, v, H, (const T*)scratch, nullptr, nullptr, T(omega), g);
+        sweep_chained(g) ? apply(std::true_type{}) : apply(std::false_type{});
     }
     return (int)cudaGetLastError();
 }
@@ -545,7 +584,7 @@ int launch_error_mask(const GlideLevelArgs* a, const void* r_u, const void* r_v,
     Geo g{a->ny, a->nx, a->nb};
     dim3 blk(32, 8);
     dim3 grd((g.nx + 31) / 32, (g.ny + 7) / 8, g.nb);
-    glide::count_launch(), error_mask_kernel<T><<<grd, blk, 0, s>>>((T*)err_mask, (const T*)r_u, (const T*)r_v, (const T*)r_H,
+    launch_chained<true>(error_mask_kernel<T>, grd, blk, s, (T*)err_mask, (const T*)r_u, (const T*)r_v, (const T*)r_H,
                                              (const T*)a->H, (const T*)a->gamma, T(threshold), g);
     if (flags) {
         cudaMemsetAsync(any_active, 0, sizeof(int) * g.nb, s);

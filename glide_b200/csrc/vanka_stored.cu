@@ -7,6 +7,8 @@
 // sweep (bound by reading them: the factors of an unstructured elimination are
 // 25), 18 for the adjoint (the solved form, without a reciprocal per sweep: its
 // levels are small and wait on latency).
+#include <type_traits>
+
 #include "cell_system.cuh"
 
 namespace glide {
@@ -46,7 +48,7 @@ template <typename T> __device__ __forceinline__ Arrow<T> transposed(const Arrow
 
 // lambda += omega * (half of each face's change, the full thickness change);
 // within one colour every face has one writer
-template <typename T>
+template <bool CHAIN, typename T>
 __device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __restrict__ ra_u,
                                                const T* __restrict__ ra_v, const T* __restrict__ ra_H,
                                                T* __restrict__ l_u, T* __restrict__ l_v, T* __restrict__ l_H, int i,
@@ -54,7 +56,8 @@ __device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __
     const int iu = i * (nx + 1) + j, ic = i * nx + j;
     Two<T> x1, x2;
     T xh;
-    arrow_solve(q, two(ra_u[iu], -ra_v[ic]), two(-ra_u[iu + 1], ra_v[ic + nx]), both(T(0)), ra_H[ic], x1, x2, xh);
+    arrow_solve(q, two(ld<CHAIN>(ra_u + iu), -ld<CHAIN>(ra_v + ic)),
+                two(-ld<CHAIN>(ra_u + iu + 1), ld<CHAIN>(ra_v + ic + nx)), both(T(0)), ld<CHAIN>(ra_H + ic), x1, x2, xh);
     l_u[iu] -= T(0.5) * omega * x1.x;
     l_u[iu + 1] += T(0.5) * omega * x2.x;
     l_v[ic] += T(0.5) * omega * x1.y;
@@ -183,7 +186,7 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
 #pragma unroll
                         for (int k = 0; k < ADJ_N; k++) out[k * nc] = o[k];
                     } else {
-                        adjoint_update(q, A.ra_u + b * g.nu(), A.ra_v + b * g.nv(), A.ra_H + b * nc,
+                        adjoint_update<false>(q, A.ra_u + b * g.nu(), A.ra_v + b * g.nv(), A.ra_H + b * nc,
                                        A.l_u + b * g.nu(), A.l_v + b * g.nv(), A.l_H + b * nc, i, jc, nx, A.omega);
                     }
                 }
@@ -198,24 +201,24 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
 }
 
 // One colour of the adjoint sweep from stored factors: a thread per cell of the colour.
-template <typename T>
+template <typename T, bool CHAIN>
 __global__ void adjoint_color_kernel(const T* __restrict__ f, T* __restrict__ l_u, T* __restrict__ l_v,
                                      T* __restrict__ l_H, const T* __restrict__ ra_u, const T* __restrict__ ra_v,
                                      const T* __restrict__ ra_H, int color, T omega, Geo g) {
     const int ny = g.ny, nx = g.nx, b = blockIdx.z;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y;
+    const int i = blockIdx.y * blockDim.y + threadIdx.y + chain_enter<CHAIN>();
     const int j = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((i + color) & 1);
     if (i >= ny || j >= nx) return;
     const int64_t nc = g.nc();
     f += b * ADJ_N * nc + int64_t(i) * nx + j;
     T o[ADJ_N];
 #pragma unroll
-    for (int k = 0; k < ADJ_N; k++) o[k] = __ldg(f + k * nc);
+    for (int k = 0; k < ADJ_N; k++) o[k] = ld<CHAIN>(f + k * nc);
     ArrowInv<T> q;
     q.i = two(o[0], o[1]); q.w1 = two(o[2], o[3]); q.w2 = two(o[4], o[5]); q.Cd = two(o[6], o[7]);
     q.k = two(o[8], o[9]); q.e = two(o[10], o[11]);
     q.b11 = o[12]; q.b12 = o[13]; q.b22 = o[14]; q.ag = o[15]; q.bg = o[16]; q.ih = o[17];
-    adjoint_update(q, ra_u + b * g.nu(), ra_v + b * g.nv(), ra_H + b * nc, l_u + b * g.nu(), l_v + b * g.nv(),
+    adjoint_update<CHAIN>(q, ra_u + b * g.nu(), ra_v + b * g.nv(), ra_H + b * nc, l_u + b * g.nu(), l_v + b * g.nv(),
                    l_H + b * nc, i, j, nx, omega);
 }
 
@@ -315,7 +318,7 @@ static int run_stored(const GlideLevelArgs* a, StoredArgs<T> A, cudaStream_t s) 
     A.rows = sh.rows;
     A.n_warps = sh.n_warps;
     with_glen(a->params, p, [&](auto q) {
-        glide::count_launch(), stored_cells_kernel<T, MODE, decltype(q)><<<dim3(sh.blocks, g.nb), sh.threads, 0, s>>>(A, g, q);
+        launch_chained<false>(stored_cells_kernel<T, MODE, decltype(q)>, dim3(sh.blocks, g.nb), sh.threads, s, A, g, q);
     });
     return (int)cudaGetLastError();
 }
@@ -337,8 +340,8 @@ int launch_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* 
                         const void* lu, void* d_u, void* d_v, void* d_H, double omega, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
     const dim3 grid((g.nx + 1 + LX - 1) / LX, (g.ny + 1 + LY - 1) / LY, g.nb);
-    glide::count_launch(), vanka_linear_kernel<T><<<grid, dim3(32, LY + 1), 0, s>>>(
-        (T*)d_u, (T*)d_v, (T*)d_H, (const T*)lu, (const T*)rho_u, (const T*)rho_v, (const T*)rho_H, (const T*)a->H,
+    launch_chained<false>(
+        vanka_linear_kernel<T>, grid, dim3(32, LY + 1), s, (T*)d_u, (T*)d_v, (T*)d_H, (const T*)lu, (const T*)rho_u, (const T*)rho_v, (const T*)rho_H, (const T*)a->H,
         (const T*)a->gamma, T(omega), g);
     return (int)cudaGetLastError();
 }
@@ -368,9 +371,12 @@ int launch_adjoint_color(const GlideLevelArgs* a, const void* factors, void* l_u
                          cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
     const dim3 blk(32, 4), grd(((g.nx + 1) / 2 + 31) / 32, (g.ny + 3) / 4, g.nb);
-    glide::count_launch(), adjoint_color_kernel<T><<<grd, blk, 0, s>>>(
-        (const T*)factors, (T*)l_u, (T*)l_v, (T*)l_H, (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, color, T(omega),
-        g);
+    auto go = [&](auto chain) {
+        constexpr bool CHAIN = decltype(chain)::value;
+        launch_chained<CHAIN>(adjoint_color_kernel<T, CHAIN>, grd, blk, s, (const T*)factors, (T*)l_u, (T*)l_v,
+                              (T*)l_H, (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, color, T(omega), g);
+    };
+    blocks_of(grd) <= 592 ? go(std::true_type{}) : go(std::false_type{});
     return (int)cudaGetLastError();
 }
 
