@@ -56,8 +56,8 @@ constexpr size_t CR_SMEM_SM = 227 * 1024;        // of one SM
 struct ConvRows {
     const __nv_bfloat16 *x0, *x1;   // x1: channels C0.. at full resolution (null without a second source)
     int C0, C1, up0;                // up0: x0 is (H/2, W/2), read at (y/2, x/2)
-    const __nv_bfloat16* W;
-    int ldw;
+    const void* W;                  // BF16, or FP32 (rounded to BF16 while it is staged)
+    int ldw, w32;
     void* out;
     int ldc, N;
     const float* bias;
@@ -106,7 +106,19 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
     for (int k = tid; k < kplanes * BN; k += CR_THREADS) {
         const int pl = k / BN, n = k - pl * BN;
         const bool ok = n0 + n < a.N && pl * 8 < 9 * C;
-        cp_async16(sB + uint32_t(k) * 16, ok ? a.W + int64_t(n0 + n) * a.ldw + pl * 8 : a.W, ok ? 16u : 0u);
+        const int64_t o = ok ? int64_t(n0 + n) * a.ldw + pl * 8 : 0;
+        if (a.w32) {
+            const float4* q = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(a.W) + o);
+            const float4 lo = ok ? __ldg(q) : make_float4(0, 0, 0, 0), hi = ok ? __ldg(q + 1) : make_float4(0, 0, 0, 0);
+            const __nv_bfloat162 h[4] = {__floats2bfloat162_rn(lo.x, lo.y), __floats2bfloat162_rn(lo.z, lo.w),
+                                         __floats2bfloat162_rn(hi.x, hi.y), __floats2bfloat162_rn(hi.z, hi.w)};
+            const uint32_t* w = reinterpret_cast<const uint32_t*>(h);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(sB + uint32_t(k) * 16), "r"(w[0]), "r"(w[1]),
+                         "r"(w[2]), "r"(w[3])
+                         : "memory");
+        } else {
+            cp_async16(sB + uint32_t(k) * 16, reinterpret_cast<const __nv_bfloat16*>(a.W) + o, ok ? 16u : 0u);
+        }
     }
     if (C8)
         for (int k = tid; k < S * 128; k += CR_THREADS)
@@ -310,31 +322,39 @@ template <int BN> int pick_conv_rows(const ConvRows& a, bool c8, size_t smem, cu
     }
 }
 
-// Launches the row march and returns its status, or returns -1000 where the
-// shape is not one of its own: C = 8 (one source) or C a multiple of 16, the
-// weights of 32 or 64 output channels and two staged rows within one SM's
-// shared memory (C <= 224), FP32 or BF16 stores, 16-byte aligned operands and
-// at least 64 columns, half of a tile's pixels.
-int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W, const void* Wt,
-                  int ldw, void* out, int ldc, int N, const float* bias, int relu, int out_mode, int* err,
-                  cudaStream_t s) {
+// The shapes of the row march: C = 8 (one source) or C a multiple of 16, the
+// weights of 32 output channels and two staged rows within one SM's shared
+// memory (C <= 224), and at least 64 columns, half of a tile's pixels.
+bool conv_rows_takes(int C0, int up0, int C1, int W, int N) {
     const int C = C0 + C1;
     const bool c8 = C == 8 && !C1 && !up0;
-    if (!(c8 || C % 16 == 0) || out_mode > 1 || W < 64 || ldw % 8 != 0) return -1000;
+    if (!(c8 || C % 16 == 0) || W < 64 || N < 1) return false;
+    const size_t stage = c8 ? CR_PLANES8 * CR_PLANE8 : size_t(C / 8) * CR_PLANE;
+    return size_t(c8 ? CR_PLANES8 : 9 * C / 8) * 32 * 16 + 128 + 2 * stage <= CR_SMEM_MAX;
+}
+
+// Launches the row march and returns its status, or returns -1000 where the
+// call is not one of its own: another shape, out_mode 2, operands that are not
+// 16-byte aligned.
+int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W, const void* Wt,
+                  int ldw, int w32, void* out, int ldc, int N, const float* bias, int relu, int out_mode, int* err,
+                  cudaStream_t s) {
+    if (!conv_rows_takes(C0, up0, C1, W, N) || out_mode > 1 || ldw % 8 != 0) return -1000;
+    const int C = C0 + C1;
+    const bool c8 = C == 8;
     if (((reinterpret_cast<uintptr_t>(x0) | reinterpret_cast<uintptr_t>(x1) | reinterpret_cast<uintptr_t>(Wt)) & 15))
         return -1000;
     ConvRows a{};
     a.x0 = (const __nv_bfloat16*)x0; a.x1 = (const __nv_bfloat16*)x1;
     a.C0 = C0; a.C1 = C1; a.up0 = up0;
-    a.W = (const __nv_bfloat16*)Wt; a.ldw = ldw;
+    a.W = Wt; a.ldw = ldw; a.w32 = w32;
     a.out = out; a.ldc = ldc; a.N = N; a.bias = bias; a.relu = relu; a.out_mode = out_mode; a.err = err;
     a.Bn = Bn; a.H = H; a.Wd = W;
     a.strips = (W + 127) / 128;
     const size_t stage = c8 ? CR_PLANES8 * CR_PLANE8 : size_t(C / 8) * CR_PLANE;
     const int kplanes = c8 ? CR_PLANES8 : 9 * C / 8;
     auto weights = [&](int bn) { return size_t(kplanes) * bn * 16 + 128; };
-    int bn = N > 32 && weights(64) + 2 * stage <= CR_SMEM_MAX ? 64 : 32;
-    if (weights(bn) + 2 * stage > CR_SMEM_MAX) return -1000;
+    const int bn = N > 32 && weights(64) + 2 * stage <= CR_SMEM_MAX ? 64 : 32;
     // as many resident CTAs as leave each at least four stages (or the one that fits)
     int occ = 1;
     for (int o = 512 / (CR_ACC * bn); o > 1; o--)
@@ -354,3 +374,19 @@ int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int B
 }
 
 }  // namespace glide
+
+extern "C" int glide_conv3x3_rows_ok(int C0, int up0, int C1, int W, int N) {
+    return C0 >= 8 && C1 >= 0 && C0 % 8 == 0 && C1 % 8 == 0 && glide::conv_rows_takes(C0, up0, C1, W, N) ? 1 : 0;
+}
+
+extern "C" int glide_conv3x3_rows_f32w(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W,
+                                       const float* Wt, void* out, int N, const float* bias, int relu, int* err,
+                                       void* stream) {
+    if (!x0 || !Wt || !out || (C1 > 0) != (x1 != nullptr)) return GLIDE_E_NULL;
+    if (Bn < 1 || H < 1 || W < 1 || !glide_conv3x3_rows_ok(C0, up0, C1, W, N) || (up0 && (H % 2 || W % 2)))
+        return GLIDE_E_SHAPE;
+    if (int64_t(Bn) * H * W >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
+    const int rc = glide::try_conv_rows(x0, C0, up0, x1, C1, Bn, H, W, Wt, 9 * (C0 + C1), 1, out, N, N, bias, relu, 1,
+                                        err, (cudaStream_t)stream);
+    return rc == -1000 ? GLIDE_E_SHAPE : rc;
+}

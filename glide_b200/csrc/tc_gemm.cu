@@ -30,7 +30,7 @@
 namespace glide {
 void count_launch();
 int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W, const void* Wt,
-                  int ldw, void* out, int ldc, int N, const float* bias, int relu, int out_mode, int* err,
+                  int ldw, int w32, void* out, int ldc, int N, const float* bias, int relu, int out_mode, int* err,
                   cudaStream_t s);
 }
 
@@ -636,7 +636,7 @@ extern "C" int glide_conv3x3_bf16(const void* x, int Bn, int H, int W, int C, co
     const int64_t M64 = int64_t(Bn) * H * W;
     if (M64 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
     const int M = int(M64), K = 9 * C;
-    const int rc = glide::try_conv_rows(x, C, 0, nullptr, 0, Bn, H, W, Wt, ldw, out, ldc, N, bias, relu, out_mode, err,
+    const int rc = glide::try_conv_rows(x, C, 0, nullptr, 0, Bn, H, W, Wt, ldw, 0, out, ldc, N, bias, relu, out_mode, err,
                                         (cudaStream_t)stream);
     if (rc != -1000) return rc;
     if (ldw % 8 == 0 && glide::al16(Wt))
@@ -661,7 +661,7 @@ extern "C" int glide_conv3x3_cat_bf16(const void* x0, int C0, int up0, const voi
     if (!glide::al16(x0) || !glide::al16(x1) || !glide::al16(Wt)) return GLIDE_E_SHAPE;
     const int64_t M64 = int64_t(Bn) * H * W;
     if (M64 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
-    const int rc = glide::try_conv_rows(x0, C0, up0, x1, C1, Bn, H, W, Wt, ldw, out, ldc, N, bias, relu, out_mode, err,
+    const int rc = glide::try_conv_rows(x0, C0, up0, x1, C1, Bn, H, W, Wt, ldw, 0, out, ldc, N, bias, relu, out_mode, err,
                                         (cudaStream_t)stream);
     if (rc != -1000) return rc;
     return glide::launch_pipe_n<true>((const __nv_bfloat16*)x0, 0, (const __nv_bfloat16*)Wt, ldw, out, ldc, int(M64), N,

@@ -96,6 +96,51 @@ __global__ void pool2_k(const uint4* __restrict__ x, uint4* __restrict__ y, int 
     y[idx] = *reinterpret_cast<const uint4*>(h);
 }
 
+// Network input of one cell per thread: H/1000, bed/1000, (log beta + 2.2)/0.7,
+// B/35 and four zeros, BF16.  Same roundings as glide_b200.guess.features in
+// torch (FP32, division by a constant as the product with its reciprocal).
+template <typename T>
+__global__ void guess_features_k(const T* __restrict__ H, const T* __restrict__ bed, const T* __restrict__ beta,
+                                 const T* __restrict__ B, uint4* __restrict__ x, int64_t n) {
+    const int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    float b = float(beta[k]);
+    b = b < 1e-8f ? 1e-8f : b;
+    const float f[4] = {__fmul_rn(float(H[k]), 1.0f / 1000.0f), __fmul_rn(float(bed[k]), 1.0f / 1000.0f),
+                        __fmul_rn(__fadd_rn(logf(b), 2.2f), 1.0f / 0.7f), __fmul_rn(float(B[k]), 1.0f / 35.0f)};
+    __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+    for (int e = 0; e < 8; e++) h[e] = __float2bfloat16(e < 4 ? f[e & 3] : 0.0f);
+    x[k] = *reinterpret_cast<const uint4*>(h);
+}
+
+// Cell velocities (ny, nx, 2) in units of scale -> staggered u (ny, nx+1) and v
+// (ny+1, nx) in FP64: FP32 averages of the two cells of a face, the cell's own
+// value on the boundary (glide_b200.guess.faces_from_cells in one pass).
+__global__ void guess_faces_k(const float2* __restrict__ p, double* __restrict__ u, double* __restrict__ v, int ny,
+                              int nx, float scale) {
+    const int b = blockIdx.z, j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y * blockDim.y + threadIdx.y;
+    if (i > ny || j > nx) return;
+    p += int64_t(b) * ny * nx;
+    u += int64_t(b) * ny * (nx + 1);
+    v += int64_t(b) * (ny + 1) * nx;
+    auto face = [&](float a, float c) {
+        return double(__fmul_rn(0.5f, __fadd_rn(__fmul_rn(c, scale), __fmul_rn(a, scale))));
+    };
+    if (i < ny) {
+        const float2* r = p + int64_t(i) * nx;
+        u[int64_t(i) * (nx + 1) + j] = j == 0    ? double(__fmul_rn(r[0].x, scale))
+                                       : j == nx ? double(__fmul_rn(r[nx - 1].x, scale))
+                                                 : face(r[j - 1].x, r[j].x);
+    }
+    if (j < nx) {
+        const float2* c = p + j;
+        v[int64_t(i) * nx + j] = i == 0    ? double(__fmul_rn(c[0].y, scale))
+                                 : i == ny ? double(__fmul_rn(c[int64_t(ny - 1) * nx].y, scale))
+                                           : face(c[int64_t(i - 1) * nx].y, c[int64_t(i) * nx].y);
+    }
+}
+
 static inline unsigned blocks_for(int64_t n) {
     int64_t b = (n + 255) / 256;
     return unsigned(b > 148 * 64 ? 148 * 64 : (b < 1 ? 1 : b));
@@ -136,5 +181,33 @@ extern "C" int glide_pool2_bf16(const void* x, void* y, int Bn, int H, int W, in
     if ((total + 255) / 256 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
     glide::count_launch(), glide::pool2_k<<<unsigned((total + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
         (const uint4*)x, (uint4*)y, H / 2, W / 2, C / 8, total);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int glide_guess_features(int dtype, const void* H, const void* bed, const void* beta, const void* B, void* x,
+                                    int64_t n, void* stream) {
+    if (dtype != GLIDE_F32 && dtype != GLIDE_F64) return GLIDE_E_DTYPE;
+    if (!H || !bed || !beta || !B || !x) return GLIDE_E_NULL;
+    if (n < 1 || (reinterpret_cast<uintptr_t>(x) & 15)) return GLIDE_E_SHAPE;
+    if ((n + 255) / 256 >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
+    const unsigned nb = unsigned((n + 255) / 256);
+    glide::count_launch();
+    if (dtype == GLIDE_F32)
+        glide::guess_features_k<float><<<nb, 256, 0, (cudaStream_t)stream>>>(
+            (const float*)H, (const float*)bed, (const float*)beta, (const float*)B, (uint4*)x, n);
+    else
+        glide::guess_features_k<double><<<nb, 256, 0, (cudaStream_t)stream>>>(
+            (const double*)H, (const double*)bed, (const double*)beta, (const double*)B, (uint4*)x, n);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int glide_guess_faces(const float* pred, double* u, double* v, int nb, int ny, int nx, double scale,
+                                 void* stream) {
+    if (!pred || !u || !v) return GLIDE_E_NULL;
+    if (nb < 1 || nb > 65535 || ny < 1 || nx < 1 || (reinterpret_cast<uintptr_t>(pred) & 7)) return GLIDE_E_SHAPE;
+    const dim3 grid((nx + 1 + 31) / 32, (ny + 1 + 7) / 8, nb);
+    if (grid.y > 65535) return GLIDE_E_TOO_LARGE;
+    glide::count_launch(), glide::guess_faces_k<<<grid, dim3(32, 8), 0, (cudaStream_t)stream>>>(
+        (const float2*)pred, u, v, ny, nx, float(scale));
     return (int)cudaGetLastError();
 }

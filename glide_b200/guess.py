@@ -62,6 +62,16 @@ def _lib():
         lib.glide_relu_grad_bf16.restype = C.c_int
         lib.glide_relu_grad_blocks.argtypes = [C.c_int64, C.c_int]
         lib.glide_relu_grad_blocks.restype = C.c_int
+        lib.glide_conv3x3_rows_ok.argtypes = [C.c_int] * 5
+        lib.glide_conv3x3_rows_ok.restype = C.c_int
+        lib.glide_conv3x3_rows_f32w.argtypes = ([C.c_void_p, C.c_int, C.c_int, C.c_void_p] + [C.c_int] * 4 +
+                                                [C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_int, C.c_void_p,
+                                                 C.c_void_p])
+        lib.glide_conv3x3_rows_f32w.restype = C.c_int
+        lib.glide_guess_features.argtypes = [C.c_int] + [C.c_void_p] * 5 + [C.c_int64, C.c_void_p]
+        lib.glide_guess_features.restype = C.c_int
+        lib.glide_guess_faces.argtypes = [C.c_void_p] * 3 + [C.c_int] * 3 + [C.c_double, C.c_void_p]
+        lib.glide_guess_faces.restype = C.c_int
         lib._guess_sigs = True
     return lib
 
@@ -136,9 +146,26 @@ def conv3x3_relu(x, W, b, relu=True):
     if (torch.is_grad_enabled() and (x.requires_grad or W.requires_grad or b.requires_grad)) or Cin % 8 != 0:
         return Conv3x3ReLU.apply(x, W, b, relu)
     Cout = W.shape[0]
-    y = torch.empty((Bn * H * Wd, Cout), dtype=torch.bfloat16, device=x.device)
-    conv3x3(x.contiguous(), W.detach().to(torch.bfloat16).contiguous(), y, bias=b.detach(), relu=relu, out_mode=1)
-    return y.view(Bn, H, Wd, Cout)
+    y = torch.empty((Bn, H, Wd, Cout), dtype=torch.bfloat16, device=x.device)
+    if not _rows_f32w(x.contiguous(), 0, None, W, b, relu, y):
+        conv3x3(x.contiguous(), W.detach().to(torch.bfloat16).contiguous(), y.view(-1, Cout), bias=b.detach(),
+                relu=relu, out_mode=1)
+    return y
+
+
+def _rows_f32w(x, up, skip, W, b, relu, y):
+    """y = relu(conv3x3(x | skip)) with the FP32 weights rounded inside the
+    kernel, where the row march takes the shape; False where it does not."""
+    lib = _lib()
+    C1 = 0 if skip is None else skip.shape[3]
+    if W.dtype != torch.float32 or not W.is_contiguous() or W.data_ptr() % 16 or \
+            not lib.glide_conv3x3_rows_ok(x.shape[3], up, C1, y.shape[2], y.shape[3]):
+        return False
+    N.check(lib.glide_conv3x3_rows_f32w(x.data_ptr(), x.shape[3], up, None if skip is None else skip.data_ptr(), C1,
+                                        y.shape[0], y.shape[1], y.shape[2], W.data_ptr(), y.data_ptr(), y.shape[3],
+                                        b.data_ptr(), int(relu), _err_flag(x.device).data_ptr(), N.stream_handle()),
+            "tensor-core conv3x3")
+    return True
 
 
 def conv3x3_up_cat(x, skip, W, b):
@@ -149,8 +176,10 @@ def conv3x3_up_cat(x, skip, W, b):
         return conv3x3_relu(torch.cat([_up(x), skip], dim=3), W, b)
     Bn, H, Wd, C1 = skip.shape
     x, skip = x.contiguous(), skip.contiguous()
-    Wb = W.detach().to(torch.bfloat16).contiguous()
     y = torch.empty((Bn, H, Wd, W.shape[0]), dtype=torch.bfloat16, device=x.device)
+    if _rows_f32w(x, 1, skip, W, b, True, y):
+        return y
+    Wb = W.detach().to(torch.bfloat16).contiguous()
     rc = _lib().glide_conv3x3_cat_bf16(x.data_ptr(), x.shape[3], 1, skip.data_ptr(), C1, Bn, H, Wd, Wb.data_ptr(),
                                        Wb.shape[1], y.data_ptr(), y.shape[3], y.shape[3], b.detach().data_ptr(), 1, 1,
                                        _err_flag(x.device).data_ptr(), N.stream_handle())
@@ -342,12 +371,26 @@ class UNet(torch.nn.Module):
 # features, targets and the guess interface
 # ---------------------------------------------------------------------------
 
+def _fusable(fs):
+    """One kernel reads these tensors as they are: CUDA, one dtype and shape, contiguous, not differentiated."""
+    a = fs[0]
+    return a.is_cuda and a.dtype in (torch.float32, torch.float64) and a.numel() > 0 and all(
+        t.dtype == a.dtype and t.device == a.device and t.shape == a.shape and t.is_contiguous() and
+        not (torch.is_grad_enabled() and t.requires_grad) for t in fs)
+
+
 def features(H, bed, beta, B):
     """(…, ny, nx) fields -> (B, ny, nx, IN_CH) BF16 normalised inputs."""
     def b3(t):
         t = torch.as_tensor(t)
         return t.unsqueeze(0) if t.dim() == 2 else t
-    H, bed, beta, B = (b3(t).float() for t in (H, bed, beta, B))
+    fs = [b3(t) for t in (H, bed, beta, B)]
+    if _fusable(fs):
+        x = torch.empty(fs[0].shape + (IN_CH,), dtype=torch.bfloat16, device=fs[0].device)
+        N.check(_lib().glide_guess_features(N.dtype_code(fs[0].dtype), *(t.data_ptr() for t in fs), x.data_ptr(),
+                                            fs[0].numel(), N.stream_handle()), "guess features")
+        return x
+    H, bed, beta, B = (t.float() for t in fs)
     logb = torch.log(torch.clamp(beta, min=1e-8))
     x = torch.stack([H / 1000.0, bed / 1000.0, (logb + 2.2) / 0.7, B / 35.0], dim=-1)
     pad = torch.zeros(x.shape[:-1] + (IN_CH - x.shape[-1],), device=x.device)
@@ -379,11 +422,18 @@ class GuessModel:
     @torch.no_grad()
     def predict(self, H, bed, beta, B):
         x = features(H, bed, beta, B)
-        pred = self.net(x)
-        u, v = faces_from_cells(pred.float())
+        pred = self.net(x).float()
+        if pred.is_cuda and pred.dim() == 4 and pred.shape[-1] == 2 and pred.is_contiguous():
+            nb, ny, nx, _ = pred.shape
+            u = torch.empty((nb, ny, nx + 1), dtype=torch.float64, device=pred.device)
+            v = torch.empty((nb, ny + 1, nx), dtype=torch.float64, device=pred.device)
+            N.check(_lib().glide_guess_faces(pred.data_ptr(), u.data_ptr(), v.data_ptr(), nb, ny, nx, VEL_SCALE,
+                                             N.stream_handle()), "guess faces")
+        else:
+            u, v = (t.double() for t in faces_from_cells(pred))
         if u.shape[0] == 1:
             u, v = u[0], v[0]
-        return u.double(), v.double()
+        return u, v
 
     def save(self, path=DEFAULT_WEIGHTS):
         torch.save(self.net.state_dict(), path)

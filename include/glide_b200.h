@@ -324,6 +324,18 @@ int glide_conv3x3_bf16(const void* x, int Bn, int H, int W, int C, const void* W
 int glide_conv3x3_cat_bf16(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W,
                            const void* Wt, int ldw, void* out, int ldc, int N, const float* bias, int relu,
                            int out_mode, int* err, void* stream);
+/* The same convolutions (x1 null and C1 = 0: one source) with FP32 weights
+ * (N, 9C), rounded to BF16 while they are staged, and BF16 output (..., N), for
+ * the shapes glide_conv3x3_rows_ok answers 1 for (others: GLIDE_E_SHAPE). */
+int glide_conv3x3_rows_ok(int C0, int up0, int C1, int W, int N);
+int glide_conv3x3_rows_f32w(const void* x0, int C0, int up0, const void* x1, int C1, int Bn, int H, int W,
+                            const float* Wt, void* out, int N, const float* bias, int relu, int* err, void* stream);
+/* Input and output of the learned guess: x (n, 8) BF16 from n cells' thickness,
+ * bed, beta and rate factor (dtype), and staggered FP64 u (nb, ny, nx+1), v
+ * (nb, ny+1, nx) from cell velocities pred (nb, ny, nx, 2) times scale. */
+int glide_guess_features(int dtype, const void* H, const void* bed, const void* beta, const void* B, void* x,
+                         int64_t n, void* stream);
+int glide_guess_faces(const float* pred, double* u, double* v, int nb, int ny, int nx, double scale, void* stream);
 /* Weight gradient of the same convolution: dW (N, 9C) FP32, dW[n, tap*C + c] =
  * sum over the pixels p of gz[p, n] * x[p shifted by tap, c] (zero outside the
  * image); gz (Bn*H*W, N) and x (Bn, H, W, C) BF16, N and C multiples of 8,

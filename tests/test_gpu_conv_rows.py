@@ -98,3 +98,58 @@ def test_relu_gradient_and_bias_sum(P, N, relu):
     assert torch.equal(gz.float(), ref)
     err = (db.double() - ref.double().sum(0)).abs()
     assert bool((err <= min(P, 4096) * 6e-8 * ref.double().abs().sum(0) + 1e-30).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_features_equal_torch(dtype):
+    """One-pass network input = the torch expression, bit for bit (values over
+    the geometry's ranges, beta down to 0 and below the clamp, infinities, NaN)."""
+    from glide_b200 import guess
+    g = torch.Generator(device="cuda").manual_seed(3)
+    f = [torch.randn(1, 211, 307, generator=g, device="cuda", dtype=torch.float64) * s for s in (1500.0, 600.0, 1.0, 40.0)]
+    f[2] = torch.exp(3 * f[2]) * 0.1
+    f[2].view(-1)[:5] = torch.tensor([0.0, -1.0, 1e-9, float("inf"), float("nan")], device="cuda")
+    f[0].view(-1)[:2] = torch.tensor([float("inf"), float("nan")], device="cuda")
+    f = [t.to(dtype) for t in f]
+    one = guess.features(*f)
+    ref = guess.features(*(t.transpose(1, 2).contiguous().transpose(1, 2) for t in f))   # not contiguous: torch path
+    same = (one == ref) | (one.isnan() & ref.isnan())
+    assert bool(same.all())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1), (1, 40, 33), (3, 17, 70)])
+def test_faces_equal_torch(shape):
+    from glide_b200 import guess
+
+    class Fixed(torch.nn.Module):
+        def __init__(self, p):
+            super().__init__()
+            self.p = p
+
+        def forward(self, x):
+            return self.p
+
+    g = torch.Generator(device="cuda").manual_seed(sum(shape))
+    p = torch.randn(*shape, 2, generator=g, device="cuda")
+    z = torch.ones(shape, device="cuda")
+    u, v = guess.GuessModel(Fixed(p)).predict(z, z, z, z)
+    ru, rv = guess.faces_from_cells(p)
+    if shape[0] == 1:
+        ru, rv = ru[0], rv[0]
+    assert torch.equal(u, ru.double()) and torch.equal(v, rv.double())
+
+
+@pytest.mark.parametrize("C,C1,N,W", [(8, 0, 32, 64), (32, 0, 40, 130), (64, 32, 32, 70), (128, 64, 64, 128)])
+def test_fp32_weights_equal_cast_weights(C, C1, N, W):
+    """Weights rounded while staged = weights cast to BF16 before."""
+    from glide_b200.guess import _rows_f32w, _up, conv3x3
+    g = torch.Generator(device="cuda").manual_seed(C + N)
+    up = 1 if C1 else 0
+    x = torch.randn(2, 6 >> up, W >> up, C, generator=g, device="cuda").to(torch.bfloat16)
+    skip = torch.randn(2, 6, W, C1, generator=g, device="cuda").to(torch.bfloat16) if C1 else None
+    Wf, b = torch.randn(N, 9 * (C + C1), generator=g, device="cuda"), torch.randn(N, generator=g, device="cuda")
+    y = torch.empty(2, 6, W, N, dtype=torch.bfloat16, device="cuda")
+    assert _rows_f32w(x, up, skip, Wf, b, True, y)
+    ref = torch.empty(2 * 6 * W, N, dtype=torch.bfloat16, device="cuda")
+    conv3x3(torch.cat([_up(x), skip], 3).contiguous() if C1 else x, Wf.to(torch.bfloat16), ref, bias=b, relu=True)
+    assert torch.equal(y.view(-1, N), ref)
