@@ -5,7 +5,7 @@
 //
 // What bounds it: the issue of narrow MMAs and, per row, the copy -> product ->
 // store latency that the ring and the resident CTAs have to cover.  1024^2,
-// 32 -> 32: 226 us as an implicit GEMM, 54 us here (134 MB, 2.5 TB/s); 512^2,
+// 32 -> 32: 226 us as an implicit GEMM, 52 us here (134 MB, 2.6 TB/s); 512^2,
 // 64 -> 64: 163 -> 37.
 //
 // The implicit GEMM of tc_gemm.cu gathers nine shifted copies of its 128
@@ -21,9 +21,12 @@
 // four-row ring of TMEM; a row's products are issued in the order ky, kx, c,
 // as the implicit GEMM issues them, so the results are the same bits.  Warps
 // are specialised: four copy rows (cp.async, zero-filled outside the image),
-// one thread issues the MMAs, four drain finished accumulators (bias, ReLU,
-// BF16 or FP32 stores), so copies, products and stores of different rows
-// overlap.  The input may be the channel concatenation of two tensors, the
+// two issue the MMAs, four drain finished accumulators (bias, ReLU, BF16 or
+// FP32 stores), so copies, products and stores of different rows overlap.  The
+// two MMA warps take the even and the odd output rows: one warp's issue (a
+// narrow MMA every 90 clocks, 40 needed) does not keep the pipe busy at 96
+// channels and more, where one CTA fits an SM (1024^2, 96 -> 32: 127 us with
+// one, 105 with two; 512^2, 192 -> 64: 136 -> 122; others within 3 %).  The input may be the channel concatenation of two tensors, the
 // first at half resolution (nearest upsampling): the copy warps read both
 // sources directly and neither the upsampled nor the joined tensor exists.
 //
@@ -44,7 +47,8 @@ void count_launch();
 
 constexpr int CR_PX = 130;                       // staged pixels of a row: 128 + one each side
 constexpr int CR_ROLE = 128;                     // copy threads = store threads
-constexpr int CR_THREADS = 2 * CR_ROLE + 32;
+constexpr int CR_MMA = 2;                        // MMA warps, one per parity of the output row
+constexpr int CR_THREADS = 2 * CR_ROLE + 32 * CR_MMA;
 constexpr int CR_ACC = 4;                        // accumulator rows in flight
 constexpr int CR_MAXST = 8;
 constexpr uint32_t CR_PLANE = CR_PX * 16;        // bytes of one 8-channel plane of a staged row
@@ -70,7 +74,7 @@ struct ConvRows {
 template <int BN, bool C8, int KS>
 __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a) {
     extern __shared__ __align__(128) uint8_t smem[];
-    __shared__ __align__(8) uint64_t full[CR_MAXST], empty[CR_MAXST], acc_full[CR_ACC], acc_empty[CR_ACC], drain;
+    __shared__ __align__(8) uint64_t full[CR_MAXST], empty[CR_MAXST], acc_full[CR_ACC], acc_empty[CR_ACC], drain[CR_MMA];
     __shared__ uint32_t tmem_slot;
     const int tid = threadIdx.x, warp = tid / 32, lane = tid & 31;
     const int C = a.C0 + a.C1, S = a.stages;
@@ -93,13 +97,13 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
     if (tid == 0) {
         for (int s = 0; s < S; s++) {
             mbar_init(&full[s], CR_ROLE);
-            mbar_init(&empty[s], 1);
+            mbar_init(&empty[s], CR_MMA);
         }
         for (int s = 0; s < CR_ACC; s++) {
             mbar_init(&acc_full[s], 1);
             mbar_init(&acc_empty[s], 4);
         }
-        mbar_init(&drain, 1);
+        for (int s = 0; s < CR_MMA; s++) mbar_init(&drain[s], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // weights: plane k/8, row n, 16 bytes
@@ -180,8 +184,9 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
         }
         cp_async_commit();
         cp_async_wait<0>();
-    } else if (warp == 8) {
+    } else if (warp >= 8) {
         // ---------------------------------------------------------------- products (the whole warp, lane 0 issues)
+        const int me = warp - 8;
         const uint32_t idesc = idesc_bf16_f32(128, BN), lead = lane == 0;
         const uint32_t a_hi = umma_hi(128), b_hi = umma_hi(128);
         for (int r = 0; r < n_in && ok; r++) {
@@ -190,6 +195,10 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
             const uint32_t st = sA + uint32_t(r % S) * stage_bytes;
             if constexpr (C8) {
                 const int slot = r % CR_ACC;
+                if ((r & 1) != me) {   // the other warp's row
+                    mma_commit_lead(&empty[r % S], lead);
+                    continue;
+                }
                 if (r >= CR_ACC && !mbar_wait_bounded(smem_u32(&acc_empty[slot]), uint32_t((r / CR_ACC - 1) & 1))) {
                     ok = false;
                     break;
@@ -208,7 +217,7 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
 #pragma unroll
                 for (int ky = 2; ky >= 0; ky--) {
                     const int yo = r - ky;
-                    if (yo < 0 || yo >= y1 - y0) continue;
+                    if (yo < 0 || yo >= y1 - y0 || (yo & 1) != me) continue;
                     const int slot = yo % CR_ACC;
                     if (ky == 0 && yo >= CR_ACC) {
                         if (!mbar_wait_bounded(smem_u32(&acc_empty[slot]), uint32_t((yo / CR_ACC - 1) & 1))) {
@@ -231,8 +240,8 @@ __global__ void __launch_bounds__(CR_THREADS) conv_rows_kernel(const ConvRows a)
             mma_commit_lead(&empty[r % S], lead);
         }
         // the MMAs in flight read shared memory: they end before the CTA does
-        mma_commit_lead(&drain, lead);
-        if (!mbar_wait_bounded(smem_u32(&drain), 0)) ok = false;
+        mma_commit_lead(&drain[me], lead);
+        if (!mbar_wait_bounded(smem_u32(&drain[me]), 0)) ok = false;
         __syncwarp();
     } else {
         // ---------------------------------------------------------------- store finished rows
@@ -309,7 +318,7 @@ template <int BN, bool C8, int KS> int launch_conv_rows(const ConvRows& a, size_
 // The narrow widths of the guess network have their K loop unrolled: with
 // every descriptor an immediate away from two bases the issuing warp comes
 // closer to the tensor pipe (about 90 clocks per MMA in a rolled loop, 40
-// needed; 1024^2, 96 -> 32: 160 -> 129 us).  At 192 channels the unrolled body
+// needed; 1024^2, 96 -> 32 with one MMA warp: 160 -> 129 us).  At 192 channels the unrolled body
 // is slower than the loop (512^2, 192 -> 64: 180 against 138 us).
 template <int BN> int pick_conv_rows(const ConvRows& a, bool c8, size_t smem, cudaStream_t s) {
     if (c8) return launch_conv_rows<BN, true, 0>(a, smem, s);
