@@ -16,7 +16,7 @@ PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 CSRC = PKG / "csrc"
 LIB = PKG / "libglide_b200.so"
-SOURCES = ["ssa_stencil.cu", "vanka.cu", "vanka_stored.cu", "transfer.cu", "driver.cu", "tc_gemm.cu", "unet_ops.cu",
+SOURCES = ["ssa_stencil.cu", "vanka.cu", "vanka_march.cu", "vanka_stored.cu", "transfer.cu", "driver.cu", "tc_gemm.cu", "unet_ops.cu",
            "vanka_noalloc.cu", "losses.cu", "krylov.cu", "conv_rows.cu",
            "conv_wgrad.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

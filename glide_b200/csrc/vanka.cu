@@ -1,14 +1,15 @@
 // Cell-patch Vanka smoothers (glide/cuda/vanka.cu) on B200.
 //
 // Forward sweep = two kernels:
-//   vanka_cells: one thread per cell runs the damped local Newton iterations
-//     on the cell's 5 unknowns (u_l, u_r, v_t, v_b, H_c) with the neighbours
-//     and the viscosity frozen, and stores half of each face change and the
-//     full H change per cell (deterministic, no atomics);
+//   the cell kernel runs the damped local Newton iterations on each cell's 5
+//     unknowns (u_l, u_r, v_t, v_b, H_c) with the neighbours and the viscosity
+//     frozen, and stores half of each face change and the full H change per
+//     cell (deterministic, no atomics): here a thread per cell of a tile
+//     (vanka_cells), in vanka_march.cu a march down rows; use_march chooses;
 //   vanka_apply: every face adds the halves of its two cells, U += omega*delta
 //     (the reference zero-fills a delta vector, scatters with atomicAdd and
 //     axpys on the host: glide/grid.py:305-317, vanka.cu:433-437).
-// The viscosity of the tile plus a one-cell ring is computed once into shared
+// In the tile form the viscosity of the tile plus a one-cell ring is computed once into shared
 // memory; the neighbours' grounding sigmoids are hoisted out of the Newton
 // loop.  The local variant gates cells by the reference's 16x16-window /
 // stride-14 block rule (vanka.cu:875-888) through per-tile flags.
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(VX * VY, (sizeof(T) == 4 ? GLIDE_VANKA32_MIN_B
         T J[25], rr[5], x[5];
         assemble_fast<T>(F, ul, ur, vt, vb, Hc, fu_l, fu_r, fv_t, fv_b, fH, thk, dti, p, J, rr);
         J[0] -= shift; J[6] -= shift; J[12] -= shift; J[18] -= shift; J[24] += shift;  // vanka.cu:406-410
-        if (pivot)
+        if (sizeof(T) == 8 || pivot)   // FP64 comes here for pivoted solves only
             lu5_solve_pivot(J, rr, x);
         else
             lu5_solve_fast(J, rr, x);
@@ -505,22 +506,43 @@ static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (
 // (128^2) single-row tiles of one warp, which the block scheduler spreads
 // evenly.  Microseconds per sweep of 10 Newton steps, FP32, 8 / 4 / 1 rows:
 // 32^2 10.3 / 8.3 / 8.7, 64^2 10.5 / 8.6 / 9.4, 128^2 11.6 / 12.7 / 9.5, 256^2
-// 15.8 / 16.6 / 17.8; FP64 at 128^2 26.7 / 27.2 / 18.8.
+// 15.8 / 16.6 / 17.8.
 static inline int cell_tile(const Geo& g) {
     const int64_t tiles = blocks_of(cell_grid(g, 8));
     return tiles <= 32 ? 4 : tiles <= 96 ? 1 : 8;
 }
+// Which form of the cell kernel: the march (vanka_march.cu) in FP64, and in
+// FP32 for sweeps of their own from 2^16 cells on.  The FP32 FAS cycle keeps
+// the tile form at every size although the march is faster there too (512^2:
+// 47 us per sweep of 10 Newton steps against 38): the two round differently, and
+// a few FP32 cycles amplify a rounding 1e3 to 1e4 times, so a step's answer
+// would move by up to 3e-4 between the forms.  Pivoted local solves exist in the
+// tile form only.  Microseconds per sweep, tile / march: FP32 of 10 steps 256^2
+// 16.1 / 13.3, 1024^2 174 / 136, of 2 steps 1024^2 73.5 / 50.3; 64^2 and below
+// within 10 % of each other; FP64 of 10 steps 32^2 16.5 / 13.3, 256^2 33.9 /
+// 26.2, 1024^2 408 / 348, of 2 steps 32^2 7.7 / 8.1, 1024^2 168 / 141.
+template <typename T> static inline bool use_march(const Geo& g, int pivot, bool cycle) {
+    if (pivot) return false;
+    return sizeof(T) == 8 || (!cycle && g.nc() * g.nb >= (int64_t(1) << 16));
+}
 // The sweep's two kernels are chained while they fit the chip about once; not
 // with single-row tiles, whose CTAs would be placed around those of the kernel
 // before and lose their even spread (128^2: 12.9 us per sweep chained, 9.5 not).
-static inline bool sweep_chained(const Geo& g) {
-    return cell_tile(g) != 1 && blocks_of(cell_grid(g, 8)) <= 592;
+static inline bool sweep_chained(const Geo& g, bool march) {
+    return (march || cell_tile(g) != 1) && blocks_of(cell_grid(g, 8)) <= 592;
 }
+template <typename T>
+void run_march(const GlideLevelArgs*, const void*, const void*, const void*, int, double, double, const int*,
+               const int*, void*, cudaStream_t);
 
 template <typename T>
 static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton,
                       double shift, double step, int pivot, const int* flags, const int* any_active, void* scratch,
-                      const Geo& g, cudaStream_t s) {
+                      const Geo& g, bool cycle, cudaStream_t s) {
+    if (use_march<T>(g, pivot, cycle)) {
+        run_march<T>(a, f_u, f_v, f_H, n_newton, shift, step, flags, any_active, scratch, s);
+        return;
+    }
     with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
         using P = decltype(p);
         auto go = [&](auto vy, auto chain) {
@@ -540,7 +562,7 @@ static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v,
             go(integral_constant<int, 4>{}, std::true_type{});
         else if (vy == 1)
             go(integral_constant<int, 1>{}, std::false_type{});
-        else if (sweep_chained(g))
+        else if (sweep_chained(g, false))
             go(integral_constant<int, 8>{}, std::true_type{});
         else
             go(integral_constant<int, 8>{}, std::false_type{});
@@ -550,7 +572,7 @@ static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v,
 template <typename T>
 int launch_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
                         int n_newton, double omega, double shift, const int* flags, const int* any_active,
-                        void* scratch, cudaStream_t s, double newton_step, int pivot) {
+                        void* scratch, cudaStream_t s, double newton_step, int pivot, bool cycle) {
     Geo g{a->ny, a->nx, a->nb};
     auto apply = [&](auto chain) {
         constexpr bool CHAIN = decltype(chain)::value;
@@ -560,9 +582,10 @@ int launch_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_
         };
         flags ? run(vanka_apply_kernel<T, true, CHAIN>) : run(vanka_apply_kernel<T, false, CHAIN>);
     };
+    const bool chained = sweep_chained(g, use_march<T>(g, pivot, cycle));
     for (int k = 0; k < n_iter; k++) {
-        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, pivot, flags, any_active, scratch, g, s);
-        sweep_chained(g) ? apply(std::true_type{}) : apply(std::false_type{});
+        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, pivot, flags, any_active, scratch, g, cycle, s);
+        chained ? apply(std::true_type{}) : apply(std::false_type{});
     }
     return (int)cudaGetLastError();
 }
@@ -574,7 +597,7 @@ int launch_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v
                        cudaStream_t s, double newton_step) {
     Geo g{a->ny, a->nx, a->nb};
     for (int k = 0; k < n_launch; k++)
-        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, 0, flags, any_active, scratch, g, s);
+        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, 0, flags, any_active, scratch, g, false, s);
     return (int)cudaGetLastError();
 }
 
@@ -605,7 +628,7 @@ int launch_tile_flags(const GlideLevelArgs* a, const void* err_mask, int* flags,
 
 #define INST(T)                                                                                                  \
     template int launch_vanka_sweeps<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,   \
-                                        double, double, const int*, const int*, void*, cudaStream_t, double, int);\
+                                        double, double, const int*, const int*, void*, cudaStream_t, double, int, bool);\
     template int launch_vanka_cells<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,     \
                                        double, const int*, const int*, void*, cudaStream_t, double);              \
     template int launch_error_mask<T>(const GlideLevelArgs*, const void*, const void*, const void*, double,       \
