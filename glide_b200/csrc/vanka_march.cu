@@ -287,7 +287,12 @@ __global__ void __launch_bounds__(VC_NT, VC_CTAS<T>)
 // Rows per warp: as few waves of resident warps as chunks of at most 32 rows
 // allow, the rows spread evenly over them (a chunk's two preparatory rows cost
 // about 10 % of a row of two Newton steps each).  Grids too small to fill the
-// chip take one row per warp and spread the warps over all SMs.
+// chip take one row per warp and spread the warps over all SMs.  A gated sweep
+// takes one row, two beyond four waves: which rows are active is not known here,
+// and only short chunks spread them over the chip (a quarter of the rows active,
+// 10 Newton steps, even chunks / these, tile form in brackets: FP32 512^2 29.2 /
+// 23.1 us (25), 1024^2 90.9 / 53.9 (77); FP64 512^2 77.4 / 49.7 (47), 1024^2
+// 281 / 114 (153)).
 template <typename T>
 void run_march(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton, double shift,
                double step, const int* flags, const int* any_active, void* scratch, cudaStream_t s) {
@@ -298,7 +303,9 @@ void run_march(const GlideLevelArgs* a, const void* f_u, const void* f_v, const 
     const int64_t units = int64_t(A.n_strips) * g.ny * g.nb;
     const int64_t waves = (units + 32 * resident - 1) / (32 * resident);
     const int64_t rows = (units + waves * resident - 1) / (waves * resident);
-    A.rows = int(rows < g.ny ? rows : g.ny);
+    const int64_t short_chunk = units > 4 * resident ? 2 : 1;
+    const int64_t most = flags && g.ny > short_chunk ? short_chunk : g.ny;
+    A.rows = int(rows < most ? rows : most);
     A.n_warps = A.n_strips * ((g.ny + A.rows - 1) / A.rows);
     const int64_t per_sm = (int64_t(A.n_warps) * g.nb + 147) / 148;
     const int threads = 32 * int(per_sm < VC_NT / 32 ? per_sm : VC_NT / 32);
