@@ -24,7 +24,7 @@ SYMBOLS = [
     "glide_mask_le", "glide_convert", "glide_norms", "glide_norm_parts", "glide_fascd_vcycle",
     "glide_adjoint_vcycle", "glide_restrict_parameters", "glide_graph_create", "glide_graph_launch",
     "glide_graph_destroy", "glide_launch_count", "glide_version", "glide_vanka_sweeps_noalloc",
-    "glide_noalloc_scratch_bytes", "glide_vanka_sweeps_ex", "glide_vanka_lu", "glide_vanka_linear",
+    "glide_noalloc_scratch_bytes", "glide_vanka_sweeps_ex", "glide_vanka_sweeps_work", "glide_vanka_lu", "glide_vanka_linear",
     "glide_misfit", "glide_tikhonov", "glide_loss_parts", "glide_jvp_add",
     "glide_linear_setup", "glide_linear_vcycle", "glide_vanka_lu_masked", "glide_newton_rhs", "glide_newton_update",
     "glide_active_mask", "glide_vanka_adjoint_sweeps", "glide_dots", "glide_dots_parts", "glide_combine",
@@ -54,7 +54,7 @@ class Level(C.Structure):
                 ("scratch", C.c_void_p), ("flags", C.c_void_p), ("any_active", C.c_void_p),
                 ("ls_tmp", C.c_void_p), ("ls_norms", C.c_void_p), ("norm_parts", C.c_void_p),
                 ("lu", C.c_void_p), ("lin_rhs", C.c_void_p), ("lin_rho", C.c_void_p), ("lin_d", C.c_void_p),
-                ("r_raw", C.c_void_p), ("adj_factors", C.c_void_p)]
+                ("r_raw", C.c_void_p), ("adj_factors", C.c_void_p), ("sweep_work", C.c_void_p)]
 
 LS_CANDIDATES = 4  # GLIDE_LS_CANDIDATES
 ADJ_FACTORS = 18   # GLIDE_ADJ_FACTORS
@@ -96,6 +96,7 @@ def load():
         "glide_grad_beta": [LA, vp, vp, vp, i, vp],
         "glide_vanka_sweeps": [LA, vp, vp, vp, i, i, d, d, vp, vp, vp, vp],
         "glide_vanka_sweeps_ex": [LA, vp, vp, vp, i, i, d, d, d, i, vp, vp, vp, vp],
+        "glide_vanka_sweeps_work": [LA, vp, vp, vp, i, i, d, d, d, i, vp, vp, vp, vp, vp],
         "glide_vanka_lu": [LA, vp, vp, d, vp],
         "glide_misfit": [i, i, d, vp, vp, vp, vp, i64, i64, vp, vp, vp, vp, vp],
         "glide_tikhonov": [i, vp, i, i, vp, vp, vp, vp],

@@ -22,7 +22,7 @@ int launch_jvp(const GlideLevelArgs*, const void*, const void*, const void*, con
                void*, void*, void*, cudaStream_t);
 template <typename T> int launch_vjp(const GlideLevelArgs*, const void*, const void*, const void*, const void*, const void*, const void*, void*, void*, void*, int, cudaStream_t);
 template <typename T> int launch_grad_beta(const GlideLevelArgs*, const void*, const void*, void*, int, cudaStream_t);
-template <typename T> int launch_vanka_sweeps(const GlideLevelArgs*, const void*, const void*, const void*, int, int, double, double, const int*, const int*, void*, cudaStream_t, double, int, bool cycle);
+template <typename T> int launch_vanka_sweeps(const GlideLevelArgs*, const void*, const void*, const void*, int, int, double, double, const int*, const int*, void*, cudaStream_t, double, int, bool cycle, void* work);
 template <typename T> int launch_vanka_lu(const GlideLevelArgs*, const void*, void*, double, cudaStream_t);
 template <typename T> int launch_vanka_linear(const GlideLevelArgs*, const void*, const void*, const void*, const void*, void*, void*, void*, double, cudaStream_t);
 template <typename T> int launch_adjoint_factors(const GlideLevelArgs*, void*, cudaStream_t);
@@ -72,7 +72,7 @@ static int check_level(const GlideLevelArgs* a) {
 // cycle: the sweeps of a FAS cycle (see use_march in vanka.cu)
 static int run_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
                       int n_newton, double newton_step, double omega, double shift, int pivoted_lu, const int* flags,
-                      const int* any_active, void* scratch, bool cycle, void* stream) {
+                      const int* any_active, void* scratch, bool cycle, void* work, void* stream) {
     int e = check_level(a);
     if (e) return e;
     if (!f_u || !f_v || !f_H || !scratch) return GLIDE_E_NULL;
@@ -81,9 +81,9 @@ static int run_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v,
     const int pv = pivoted_lu ? 1 : 0;
     return TDISPATCH(a->dtype,
                      launch_vanka_sweeps<float>(a, f_u, f_v, f_H, n_iter, n_newton, omega, shift, flags, any_active,
-                                                scratch, S(stream), newton_step, pv, cycle),
+                                                scratch, S(stream), newton_step, pv, cycle, work),
                      launch_vanka_sweeps<double>(a, f_u, f_v, f_H, n_iter, n_newton, omega, shift, flags,
-                                                 any_active, scratch, S(stream), newton_step, pv, cycle));
+                                                 any_active, scratch, S(stream), newton_step, pv, cycle, work));
 }
 
 extern "C" {
@@ -147,7 +147,14 @@ int glide_vanka_sweeps_ex(const GlideLevelArgs* a, const void* f_u, const void* 
                           int n_newton, double newton_step, double omega, double shift, int pivoted_lu,
                           const int* flags, const int* any_active, void* scratch, void* stream) {
     return run_sweeps(a, f_u, f_v, f_H, n_iter, n_newton, newton_step, omega, shift, pivoted_lu, flags, any_active,
-                      scratch, false, stream);
+                      scratch, false, nullptr, stream);
+}
+
+int glide_vanka_sweeps_work(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
+                            int n_newton, double newton_step, double omega, double shift, int pivoted_lu,
+                            const int* flags, const int* any_active, void* scratch, void* work, void* stream) {
+    return run_sweeps(a, f_u, f_v, f_H, n_iter, n_newton, newton_step, omega, shift, pivoted_lu, flags, any_active,
+                      scratch, false, work, stream);
 }
 
 int glide_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
@@ -353,7 +360,7 @@ int vanka(GlideLevel* L, int n_iter, const GlideSolverConfig* c, bool local, voi
     LevelView w = view(L);
     const double step = c->newton_step > 0.0 ? c->newton_step : GLIDE_REF_NEWTON_STEP;
     return run_sweeps(&L->a, w.u(L->f), w.v(L->f), w.H(L->f), n_iter, c->n_newton, step, c->omega, c->shift,
-                      c->pivoted_lu, local ? L->flags : nullptr, local ? L->any_active : nullptr, L->scratch, true, s);
+                      c->pivoted_lu, local ? L->flags : nullptr, local ? L->any_active : nullptr, L->scratch, true, L->sweep_work, s);
 }
 
 int fill_gamma(GlideLevel* L, double val, void* s) {

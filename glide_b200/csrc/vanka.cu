@@ -1,25 +1,37 @@
 // Cell-patch Vanka smoothers (glide/cuda/vanka.cu) on B200.
 //
-// Forward sweep = two kernels:
+// Forward sweep:
 //   the cell kernel runs the damped local Newton iterations on each cell's 5
 //     unknowns (u_l, u_r, v_t, v_b, H_c) with the neighbours and the viscosity
 //     frozen, and stores half of each face change and the full H change per
 //     cell (deterministic, no atomics): here a thread per cell of a tile
 //     (vanka_cells), in vanka_march.cu a march down rows; use_march chooses;
-//   vanka_apply: every face adds the halves of its two cells, U += omega*delta
+//   the update: every face adds the halves of its two cells, U += omega*delta
 //     (the reference zero-fills a delta vector, scatters with atomicAdd and
-//     axpys on the host: glide/grid.py:305-317, vanka.cu:433-437).
-// In the tile form the viscosity of the tile plus a one-cell ring is computed once into shared
-// memory; the neighbours' grounding sigmoids are hoisted out of the Newton
-// loop.  The local variant gates cells by the reference's 16x16-window /
-// stride-14 block rule (vanka.cu:875-888) through per-tile flags.
+//     axpys on the host: glide/grid.py:305-317, vanka.cu:433-437); by the next
+//     sweep's cell kernel as it reads the state, or by vanka_apply.
+// In the tile form the state in reach of a tile is read (and updated) once into
+// shared memory and the viscosity of the tile plus a one-cell ring computed
+// there; the neighbours' grounding sigmoids are hoisted out of the Newton loop.
+// The local variant gates cells by the reference's 16x16-window / stride-14
+// block rule (vanka.cu:875-888) through per-tile flags.
+//
+// What bounds the tile form: below about 200^2 the latency of one cell's chain
+// (0.33 us per Newton step, 3 us to read, assemble and store), above it
+// instruction issue (340 instructions per Newton step).
 #include <type_traits>
 
 #include "glide_common.cuh"
 
 namespace glide {
 
-constexpr int VX = 32;   // tile width; a tile is VX x VY cells, VY = 8, 4 or 1 (see cell_tile)
+// A tile is VX x VY cells, a CTA of four warps.  A cell's Newton loop is one long
+// dependent chain, so on a grid that leaves SMs idle a warp should share its
+// scheduler with as few others as possible, and on a large one small CTAs even
+// out the last wave: tiles of 8 rows took 8.9 us per sweep of 10 Newton steps
+// at 128^2 against 7.1 (FP32), 45.1 against 44.6 at 512^2, 176 against 172 at
+// 1024^2 (85 against 74 of 2 steps); single rows 9.1 at 128^2.
+constexpr int VX = 32, VY = 4;
 constexpr int REF_STRIDE = 14;   // reference block stride (glide/grid.py:182-188)
 constexpr int REF_WIN = 16;      // reference block (active cells + 1 ring)
 
@@ -35,31 +47,158 @@ template <typename T> struct Patch {
     int i, j;
 };
 
-// Fill the eta window of a VYxVX tile (+ ring) and the frozen patch of the
-// calling thread's cell.
-template <int VY, bool CHAIN, typename T, typename P>
-__device__ __forceinline__ void eta_window(T (*s_eta)[VX + 2], const T* u, const T* v, const T* B, int i0, int j0,
-                                           int ny, int nx, const P& p) {
-    for (int k = threadIdx.x; k < (VY + 2) * (VX + 2); k += VX * VY) {
-        int r = k / (VX + 2), c = k - r * (VX + 2);
-        int ic = clampi(i0 - 1 + r, 0, ny - 1), jc = clampi(j0 - 1 + c, 0, nx - 1);
-        EtaIn<T> e = eta_inputs<CHAIN>(u, v, ic, jc, ny, nx);
-        s_eta[r][c] = cell_eta(e, ldc<CHAIN>(B, ic, jc, ny, nx), ic, jc, ny, nx, p).eta;
+template <bool CHAIN>
+__device__ __forceinline__ bool ref_tile_on(const int* flags, int i, int j, int nx) {
+    const int nbx = nx / REF_STRIDE + 1;
+    return ld<CHAIN>(flags + (i / REF_STRIDE) * nbx + j / REF_STRIDE) != 0;
+}
+
+// The state a sweep starts from: U itself, or U plus the update of the sweep
+// before it (has; d*: that sweep's five cell arrays).  The update is
+// vanka_apply_kernel's, term by term, so both ways give the same bits.  Loads
+// and sums are apart, so that a thread has all its loads in flight at once: the
+// latency of this read is most of a small grid's sweep outside its Newton steps.
+template <typename T, bool LOCAL, bool CHAIN> struct State {
+    const T *u, *v, *H;
+    const T *du_l, *du_r, *dv_t, *dv_b, *dH;   // readable (any cell array) without an update
+    const int* flags;
+    T omega;
+    int ny, nx;
+    bool has;
+    struct In { T x, a, b; int fa, fb; };
+    __device__ __forceinline__ void two(In& q, const T* da, int ia, int ja, const T* db, int ib, int jb) const {
+        ia = min(ia, ny - 1); ja = min(ja, nx - 1); ib = max(ib, 0); jb = max(jb, 0);   // in range where unused
+        q.a = ld<CHAIN>(da + (ia * nx + ja));
+        q.b = ld<CHAIN>(db + (ib * nx + jb));
+        if (LOCAL) {
+            const int nbx = nx / REF_STRIDE + 1;
+            q.fa = ld<CHAIN>(flags + (ia / REF_STRIDE) * nbx + ja / REF_STRIDE);
+            q.fb = ld<CHAIN>(flags + (ib / REF_STRIDE) * nbx + jb / REF_STRIDE);
+        }
+    }
+    __device__ __forceinline__ T sum(const In& q, bool first, bool second) const {
+        T d = T(0);
+        d += first && (!LOCAL || q.fa) ? q.a : T(0);
+        d += second && (!LOCAL || q.fb) ? q.b : T(0);
+        return has ? q.x + omega * d : q.x;
+    }
+    // u-face (i,j): u_l of cell (i,j), u_r of cell (i,j-1)
+    __device__ __forceinline__ In loadU(int i, int j) const {
+        In q;
+        q.x = ld<CHAIN>(u + (i * (nx + 1) + j));
+        two(q, du_l, i, j, du_r, i, j - 1);
+        return q;
+    }
+    __device__ __forceinline__ T sumU(const In& q, int, int j) const { return sum(q, j < nx, j > 0); }
+    __device__ __forceinline__ In loadV(int i, int j) const {
+        In q;
+        q.x = ld<CHAIN>(v + (i * nx + j));
+        two(q, dv_t, i, j, dv_b, i - 1, j);
+        return q;
+    }
+    __device__ __forceinline__ T sumV(const In& q, int i, int) const { return sum(q, i < ny, i > 0); }
+    __device__ __forceinline__ In loadH(int i, int j) const {
+        In q;
+        q.x = ld<CHAIN>(H + (i * nx + j));
+        q.a = ld<CHAIN>(dH + (i * nx + j));
+        if (LOCAL) q.fa = ld<CHAIN>(flags + (i / REF_STRIDE) * (nx / REF_STRIDE + 1) + j / REF_STRIDE);
+        return q;
+    }
+    __device__ __forceinline__ T sumH(const In& q) const {
+        return has && (!LOCAL || q.fa) ? q.x + omega * q.a : q.x;
+    }
+};
+
+// The state in reach of a tile's cells, clamped at the domain's edges: entry
+// (r, c) of u is face (i0-2+r, j0-1+c), of v (i0-1+r, j0-2+c), of H cell
+// (i0-1+r, j0-1+c).
+template <typename T> struct Window {
+    T u[VY + 4][VX + 3], v[VY + 3][VX + 4], H[VY + 2][VX + 2], eta[VY + 2][VX + 2];
+};
+
+// Fill the state of the window; the tile's own entries also go to (ou, ov, oH)
+// unless null (faces belong to the cell right of / below them, a domain's last
+// face to its last tile).
+template <typename S, typename T>
+__device__ __forceinline__ void state_window(Window<T>& W, const S& st, T* ou, T* ov, T* oH, int i0, int j0) {
+    constexpr int NT = VX * VY, CU = VX + 3, CV = VX + 4, CH = VX + 2;
+    constexpr int NU = (VY + 4) * CU, NV = (VY + 3) * CV, NH = (VY + 2) * CH;
+    constexpr int KU = (NU + NT - 1) / NT, KV = (NV + NT - 1) / NT, KH = (NH + NT - 1) / NT;
+    const int ny = st.ny, nx = st.nx;
+    const int ie = min(i0 + VY, ny), je = min(j0 + VX, nx);
+    const bool lastr = ie == ny, lastc = je == nx;
+    typename S::In qu[KU], qv[KV], qh[KH];
+#pragma unroll
+    for (int m = 0; m < KU; m++) {
+        const int k = min(int(threadIdx.x) + m * NT, NU - 1), r = k / CU, c = k - r * CU;
+        qu[m] = st.loadU(clampi(i0 - 2 + r, 0, ny - 1), clampi(j0 - 1 + c, 0, nx));
+    }
+#pragma unroll
+    for (int m = 0; m < KV; m++) {
+        const int k = min(int(threadIdx.x) + m * NT, NV - 1), r = k / CV, c = k - r * CV;
+        qv[m] = st.loadV(clampi(i0 - 1 + r, 0, ny), clampi(j0 - 2 + c, 0, nx - 1));
+    }
+#pragma unroll
+    for (int m = 0; m < KH; m++) {
+        const int k = min(int(threadIdx.x) + m * NT, NH - 1), r = k / CH, c = k - r * CH;
+        qh[m] = st.loadH(clampi(i0 - 1 + r, 0, ny - 1), clampi(j0 - 1 + c, 0, nx - 1));
+    }
+#pragma unroll
+    for (int m = 0; m < KU; m++) {
+        const int k = min(int(threadIdx.x) + m * NT, NU - 1), r = k / CU, c = k - r * CU;
+        const int i = i0 - 2 + r, j = j0 - 1 + c;
+        const T x = st.sumU(qu[m], clampi(i, 0, ny - 1), clampi(j, 0, nx));
+        W.u[r][c] = x;
+        if (ou && i >= i0 && i < ie && j >= j0 && (j < je || (lastc && j == nx))) ou[i * (nx + 1) + j] = x;
+    }
+#pragma unroll
+    for (int m = 0; m < KV; m++) {
+        const int k = min(int(threadIdx.x) + m * NT, NV - 1), r = k / CV, c = k - r * CV;
+        const int i = i0 - 1 + r, j = j0 - 2 + c;
+        const T x = st.sumV(qv[m], clampi(i, 0, ny), clampi(j, 0, nx - 1));
+        W.v[r][c] = x;
+        if (ou && i >= i0 && (i < ie || (lastr && i == ny)) && j >= j0 && j < je) ov[i * nx + j] = x;
+    }
+#pragma unroll
+    for (int m = 0; m < KH; m++) {
+        const int k = min(int(threadIdx.x) + m * NT, NH - 1), r = k / CH, c = k - r * CH;
+        const int i = i0 - 1 + r, j = j0 - 1 + c;
+        const T x = st.sumH(qh[m]);
+        W.H[r][c] = x;
+        if (ou && i >= i0 && i < ie && j >= j0 && j < je) oH[i * nx + j] = x;
     }
 }
 
+// Fill the eta window of a VYxVX tile (+ ring).
+template <bool CHAIN, typename T, typename P>
+__device__ __forceinline__ void eta_window(Window<T>& W, const T* B, int i0, int j0, int ny, int nx, const P& p) {
+    for (int k = threadIdx.x; k < (VY + 2) * (VX + 2); k += VX * VY) {
+        int r = k / (VX + 2), c = k - r * (VX + 2);
+        int ic = clampi(i0 - 1 + r, 0, ny - 1), jc = clampi(j0 - 1 + c, 0, nx - 1);
+        const int a = ic - i0, b = jc - j0;
+        EtaIn<T> e;
+        e.ul = W.u[a + 2][b + 1];    e.ur = W.u[a + 2][b + 2];
+        e.vt = W.v[a + 1][b + 2];    e.vb = W.v[a + 2][b + 2];
+        e.u_tl = W.u[a + 1][b + 1];  e.u_tr = W.u[a + 1][b + 2];
+        e.u_bl = W.u[a + 3][b + 1];  e.u_br = W.u[a + 3][b + 2];
+        e.v_lt = W.v[a + 1][b + 1];  e.v_rt = W.v[a + 1][b + 3];
+        e.v_lb = W.v[a + 2][b + 1];  e.v_rb = W.v[a + 2][b + 3];
+        W.eta[r][c] = cell_eta(e, ldc<CHAIN>(B, ic, jc, ny, nx), ic, jc, ny, nx, p).eta;
+    }
+}
+
+// The frozen patch of cell (r, c) of the tile.
 template <bool CHAIN, typename T>
-__device__ __forceinline__ void load_patch(Patch<T>& P, T (*s_eta)[VX + 2], int r, int c, const T* u, const T* v,
-                                           const T* H, const T* bed, const T* beta, int i, int j, int ny, int nx,
-                                           const Phys<T>& p) {
+__device__ __forceinline__ void load_patch(Patch<T>& P, const Window<T>& W, int r, int c, const T* bed,
+                                           const T* beta, int i, int j, int ny, int nx, const Phys<T>& p) {
     P.i = i;
     P.j = j;
 #pragma unroll
     for (int a = 0; a < 3; a++)
 #pragma unroll
         for (int b = 0; b < 3; b++) {
-            P.eta[a][b] = s_eta[r + a][c + b];
-            P.Hn[a][b] = ldc<CHAIN>(H, i - 1 + a, j - 1 + b, ny, nx);
+            P.eta[a][b] = W.eta[r + a][c + b];
+            P.Hn[a][b] = W.H[r + a][c + b];
         }
     P.bed_c = ldc<CHAIN>(bed, i, j, ny, nx); P.bed_l = ldc<CHAIN>(bed, i, j - 1, ny, nx); P.bed_r = ldc<CHAIN>(bed, i, j + 1, ny, nx);
     P.bed_t = ldc<CHAIN>(bed, i - 1, j, ny, nx); P.bed_b = ldc<CHAIN>(bed, i + 1, j, ny, nx);
@@ -69,18 +208,12 @@ __device__ __forceinline__ void load_patch(Patch<T>& P, T (*s_eta)[VX + 2], int 
     P.g_r = sigmoid(P.bed_r + rho_ratio<T>() * P.Hn[1][2], p.sig_c);
     P.g_t = sigmoid(P.bed_t + rho_ratio<T>() * P.Hn[0][1], p.sig_c);
     P.g_b = sigmoid(P.bed_b + rho_ratio<T>() * P.Hn[2][1], p.sig_c);
-    P.u_ll = ldu<CHAIN>(u, i, j - 1, ny, nx); P.u_rr = ldu<CHAIN>(u, i, j + 2, ny, nx);
-    P.u_tl = ldu<CHAIN>(u, i - 1, j, ny, nx); P.u_tr = ldu<CHAIN>(u, i - 1, j + 1, ny, nx);
-    P.u_bl = ldu<CHAIN>(u, i + 1, j, ny, nx); P.u_br = ldu<CHAIN>(u, i + 1, j + 1, ny, nx);
-    P.v_lt = ldv<CHAIN>(v, i, j - 1, ny, nx); P.v_lb = ldv<CHAIN>(v, i + 1, j - 1, ny, nx);
-    P.v_rt = ldv<CHAIN>(v, i, j + 1, ny, nx); P.v_rb = ldv<CHAIN>(v, i + 1, j + 1, ny, nx);
-    P.v_tt = ldv<CHAIN>(v, i - 1, j, ny, nx); P.v_bb = ldv<CHAIN>(v, i + 2, j, ny, nx);
-}
-
-template <bool CHAIN>
-__device__ __forceinline__ bool ref_tile_on(const int* flags, int i, int j, int nx) {
-    const int nbx = nx / REF_STRIDE + 1;
-    return ld<CHAIN>(flags + (i / REF_STRIDE) * nbx + j / REF_STRIDE) != 0;
+    P.u_ll = W.u[r + 2][c];      P.u_rr = W.u[r + 2][c + 3];
+    P.u_tl = W.u[r + 1][c + 1];  P.u_tr = W.u[r + 1][c + 2];
+    P.u_bl = W.u[r + 3][c + 1];  P.u_br = W.u[r + 3][c + 2];
+    P.v_lt = W.v[r + 1][c + 1];  P.v_lb = W.v[r + 2][c + 1];
+    P.v_rt = W.v[r + 1][c + 3];  P.v_rb = W.v[r + 2][c + 3];
+    P.v_tt = W.v[r][c + 2];      P.v_bb = W.v[r + 3][c + 2];
 }
 
 // Frozen per-cell coefficients of the forward local Newton loop: every term
@@ -343,26 +476,28 @@ template <typename T> __device__ __forceinline__ void lu5_solve_pivot(T (&A)[25]
     }
 }
 
+// State of a sweep, and where its kernel puts it: (u, v, H) plus the update of
+// the sweep before from d (null: none), written to (ou, ov, oH) (null: not).
+template <typename T> struct SweepState {
+    const T *u, *v, *H, *d;
+    T *ou, *ov, *oH;
+    T omega;
+};
+
 // Per-cell Newton deltas.  scratch holds 5 cell arrays: 0.5*du_l, 0.5*du_r,
 // 0.5*dv_t, 0.5*dv_b, dH.
-template <typename T, int VY, bool LOCAL, bool CHAIN, typename P>
-#ifndef GLIDE_VANKA64_MIN_BLOCKS
-#define GLIDE_VANKA64_MIN_BLOCKS 2
-#endif
-#ifndef GLIDE_VANKA32_MIN_BLOCKS
-#define GLIDE_VANKA32_MIN_BLOCKS 2
-#endif
-__global__ void __launch_bounds__(VX * VY, (sizeof(T) == 4 ? GLIDE_VANKA32_MIN_BLOCKS : GLIDE_VANKA64_MIN_BLOCKS) * (8 / VY)) vanka_cells_kernel(
-    T* __restrict__ scratch, const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H,
-    const T* __restrict__ f_u, const T* __restrict__ f_v, const T* __restrict__ f_H, const T* __restrict__ bed,
-    const T* __restrict__ B, const T* __restrict__ beta, const T* __restrict__ gamma, const int* __restrict__ flags,
-    const int* __restrict__ any_active, int n_newton, T shift, T step, int pivot, Geo g, P p) {
-    __shared__ T s_eta[VY + 2][VX + 2];
-    const int zero = chain_enter<CHAIN>();
+template <typename T, bool LOCAL, typename P>
+__global__ void __launch_bounds__(VX * VY, 4) vanka_cells_kernel(
+    T* __restrict__ scratch, SweepState<T> q, const T* __restrict__ f_u, const T* __restrict__ f_v,
+    const T* __restrict__ f_H, const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
+    const T* __restrict__ gamma, const int* __restrict__ flags, const int* __restrict__ any_active, int n_newton,
+    T shift, T step, int pivot, Geo g, P p) {
+    __shared__ Window<T> W;
+    const int zero = chain_enter<true>();
     const int ny = g.ny, nx = g.nx;
     const int bz = blockIdx.z + zero;
-    if (LOCAL && ld<CHAIN>(any_active + bz) == 0) return;
-    u += bz * g.nu(); v += bz * g.nv(); H += bz * g.nc(); f_u += bz * g.nu(); f_v += bz * g.nv();
+    if (LOCAL && ld<true>(any_active + bz) == 0) return;
+    f_u += bz * g.nu(); f_v += bz * g.nv();
     f_H += bz * g.nc(); bed += bz * g.nc(); B += bz * g.nc(); beta += bz * g.nc(); gamma += bz * g.nc();
     const int64_t nc = g.nc();
     scratch += bz * 5 * nc;
@@ -370,26 +505,36 @@ __global__ void __launch_bounds__(VX * VY, (sizeof(T) == 4 ? GLIDE_VANKA32_MIN_B
     const int i0 = blockIdx.y * VY + zero, j0 = blockIdx.x * VX;
     const int r = threadIdx.x / VX, c = threadIdx.x % VX;
     const int i = i0 + r, j = j0 + c;
-    eta_window<VY, CHAIN>(s_eta, u, v, B, i0, j0, ny, nx, p);
+    const bool has = q.d;
+    const T* d = has ? q.d + bz * 5 * nc : q.H + bz * nc;
+    const int64_t ds = has ? nc : 0;
+    const State<T, LOCAL, true> st{q.u + bz * g.nu(), q.v + bz * g.nv(), q.H + bz * nc, d, d + ds, d + 2 * ds,
+                                    d + 3 * ds, d + 4 * ds, flags, q.omega, ny, nx, has};
+    T* ou = q.ou ? q.ou + bz * g.nu() : nullptr;
+    T *ov = q.ov + bz * g.nv(), *oH = q.oH + bz * nc;
+    const bool live = i < ny && j < nx && (!LOCAL || ref_tile_on<true>(flags, i, j, nx));
+    if (LOCAL && !ou && !__syncthreads_or(live)) return;
+    state_window(W, st, ou, ov, oH, i0, j0);
+    if (LOCAL ? !__syncthreads_or(live) : (__syncthreads(), false)) return;   // nothing to solve
+    eta_window<true>(W, B, i0, j0, ny, nx, p);
     __syncthreads();
-    if (i >= ny || j >= nx) return;
-    if (LOCAL && !ref_tile_on<CHAIN>(flags, i, j, nx)) return;
+    if (!live) return;
 
     Frozen<T> F;
     {
         Patch<T> pt;
-        load_patch<CHAIN>(pt, s_eta, r, c, u, v, H, bed, beta, i, j, ny, nx, p);
+        load_patch<true>(pt, W, r, c, bed, beta, i, j, ny, nx, p);
         make_frozen<T>(F, pt, ny, nx, p);
     }
     // 32-bit offsets within one field (the entry points bound a field below 2^31 elements)
     const int iu = i * (nx + 1) + j, ic32 = i * nx + j;
-    const T ul0 = ld<CHAIN>(u + iu), ur0 = ld<CHAIN>(u + iu + 1);
-    const T vt0 = ld<CHAIN>(v + ic32), vb0 = ld<CHAIN>(v + ic32 + nx);
-    const T H0 = ld<CHAIN>(H + ic32);
-    const T fu_l = ld<CHAIN>(f_u + iu), fu_r = ld<CHAIN>(f_u + iu + 1);
-    const T fv_t = ld<CHAIN>(f_v + ic32), fv_b = ld<CHAIN>(f_v + ic32 + nx);
-    const T fH = ld<CHAIN>(f_H + ic32);
-    const T thk = ld<CHAIN>(gamma + ic32);
+    const T ul0 = W.u[r + 2][c + 1], ur0 = W.u[r + 2][c + 2];
+    const T vt0 = W.v[r + 1][c + 2], vb0 = W.v[r + 2][c + 2];
+    const T H0 = W.H[r + 1][c + 1];
+    const T fu_l = ld<true>(f_u + iu), fu_r = ld<true>(f_u + iu + 1);
+    const T fv_t = ld<true>(f_v + ic32), fv_b = ld<true>(f_v + ic32 + nx);
+    const T fH = ld<true>(f_H + ic32);
+    const T thk = ld<true>(gamma + ic32);
     const T dti = T(1) / p.dt;
     T ul = ul0, ur = ur0, vt = vt0, vb = vb0, Hc = H0;
     for (int it = 0; it < n_newton; it++) {
@@ -418,9 +563,10 @@ __global__ void __launch_bounds__(VX * VY, (sizeof(T) == 4 ? GLIDE_VANKA32_MIN_B
     scratch[4 * nc + ic] = Hc - H0;
 }
 
-// U += omega * delta, face delta = sum of the two adjacent cells' halves.
+// (u, v, H) = (su, sv, sH) + omega * delta, face delta = sum of the two adjacent
+// cells' halves; the source is the target itself or a copy of it.
 template <typename T, bool LOCAL, bool CHAIN>
-__global__ void vanka_apply_kernel(T* __restrict__ u, T* __restrict__ v, T* __restrict__ H,
+__global__ void vanka_apply_kernel(T* u, T* v, T* H, const T* su, const T* sv, const T* sH,
                                    const T* __restrict__ scratch, const int* __restrict__ flags,
                                    const int* __restrict__ any_active, T omega, Geo g) {
     const int zero = chain_enter<CHAIN>();
@@ -432,22 +578,29 @@ __global__ void vanka_apply_kernel(T* __restrict__ u, T* __restrict__ v, T* __re
     if (i > ny || j > nx) return;
     const int64_t nc = g.nc();
     u += bz * g.nu(); v += bz * g.nv(); H += bz * g.nc();
+    su += bz * g.nu(); sv += bz * g.nv(); sH += bz * g.nc();
     scratch += bz * 5 * nc;
     if (LOCAL) flags += bz * int64_t(ny / REF_STRIDE + 1) * (nx / REF_STRIDE + 1);
     auto on = [&](int ii, int jj) { return !LOCAL || ref_tile_on<CHAIN>(flags, ii, jj, nx); };
     if (i < ny) {  // u-face (i,j), j in [0,nx]
+        const int64_t k = int64_t(i) * (nx + 1) + j;
         T d = T(0);
         if (j < nx && on(i, j)) d += ld<CHAIN>(scratch + int64_t(i) * nx + j);                   // as u_l of cell (i,j)
         if (j > 0 && on(i, j - 1)) d += ld<CHAIN>(scratch + nc + int64_t(i) * nx + j - 1);        // as u_r of cell (i,j-1)
-        u[int64_t(i) * (nx + 1) + j] += omega * d;
+        u[k] = su[k] + omega * d;
     }
     if (j < nx) {  // v-face (i,j), i in [0,ny]
+        const int64_t k = int64_t(i) * nx + j;
         T d = T(0);
-        if (i < ny && on(i, j)) d += ld<CHAIN>(scratch + 2 * nc + int64_t(i) * nx + j);
-        if (i > 0 && on(i - 1, j)) d += ld<CHAIN>(scratch + 3 * nc + int64_t(i - 1) * nx + j);
-        v[int64_t(i) * nx + j] += omega * d;
+        if (i < ny && on(i, j)) d += ld<CHAIN>(scratch + 2 * nc + k);
+        if (i > 0 && on(i - 1, j)) d += ld<CHAIN>(scratch + 3 * nc + k - nx);
+        v[k] = sv[k] + omega * d;
+        if (i < ny) {
+            T h = sH[k];
+            if (on(i, j)) h += omega * ld<CHAIN>(scratch + 4 * nc + k);
+            H[k] = h;
+        }
     }
-    if (i < ny && j < nx && on(i, j)) H[int64_t(i) * nx + j] += omega * ld<CHAIN>(scratch + 4 * nc + int64_t(i) * nx + j);
 }
 
 // Local error indicator (glide/solver.py:148-154) and reference-tile flags.
@@ -497,95 +650,92 @@ __global__ void tile_flags_kernel(int* __restrict__ flags, int* __restrict__ any
 // --------------------------------------------------------------------------
 // launchers
 // --------------------------------------------------------------------------
-static inline dim3 cell_grid(const Geo& g, int vy) { return dim3((g.nx + VX - 1) / VX, (g.ny + vy - 1) / vy, g.nb); }
+static inline dim3 cell_grid(const Geo& g) { return dim3((g.nx + VX - 1) / VX, (g.ny + VY - 1) / VY, g.nb); }
 static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (g.ny + 1 + 7) / 8, g.nb); }
 
-// Tile height.  A cell's Newton loop is one long dependent chain, so on a grid
-// that leaves SMs idle a warp should share its scheduler with as few others as
-// possible: quarter-SM tiles of 4 rows up to 32 tiles of 8 (64^2), and up to 96
-// (128^2) single-row tiles of one warp, which the block scheduler spreads
-// evenly.  Microseconds per sweep of 10 Newton steps, FP32, 8 / 4 / 1 rows:
-// 32^2 10.3 / 8.3 / 8.7, 64^2 10.5 / 8.6 / 9.4, 128^2 11.6 / 12.7 / 9.5, 256^2
-// 15.8 / 16.6 / 17.8.
-static inline int cell_tile(const Geo& g) {
-    const int64_t tiles = blocks_of(cell_grid(g, 8));
-    return tiles <= 32 ? 4 : tiles <= 96 ? 1 : 8;
-}
 // Which form of the cell kernel: the march (vanka_march.cu) in FP64, and in
 // FP32 for sweeps of their own from 2^16 cells on.  The FP32 FAS cycle keeps
-// the tile form at every size although the march is faster there too (512^2:
-// 47 us per sweep of 10 Newton steps against 38): the two round differently, and
+// the tile form at every size although the march is faster there too (512^2,
+// 10 Newton steps: 45 us per sweep against 38): the two round differently, and
 // a few FP32 cycles amplify a rounding 1e3 to 1e4 times, so a step's answer
 // would move by up to 3e-4 between the forms.  Pivoted local solves exist in the
-// tile form only.  Microseconds per sweep, tile / march: FP32 of 10 steps 256^2
-// 16.1 / 13.3, 1024^2 174 / 136, of 2 steps 1024^2 73.5 / 50.3; 64^2 and below
-// within 10 % of each other; FP64 of 10 steps 32^2 16.5 / 13.3, 256^2 33.9 /
-// 26.2, 1024^2 408 / 348, of 2 steps 32^2 7.7 / 8.1, 1024^2 168 / 141.
+// tile form only.  Microseconds per sweep, tile (one kernel per sweep) / march:
+// FP32 of 10 steps 256^2 14.1 / 13.4, 300^2 20.7 / 17.6, 1024^2 172 / 137, of 2
+// steps 256^2 6.4 / 7.8, 362^2 11.2 / 10.7, 1024^2 74.4 / 50.8; FP64, tile with
+// two kernels per sweep, of 10 steps 32^2 16.5 / 13.3, 256^2 33.9 / 26.2,
+// 1024^2 408 / 348, of 2 steps 32^2 7.7 / 8.1, 1024^2 168 / 141.
 template <typename T> static inline bool use_march(const Geo& g, int pivot, bool cycle) {
     if (pivot) return false;
     return sizeof(T) == 8 || (!cycle && g.nc() * g.nb >= (int64_t(1) << 16));
 }
-// The sweep's two kernels are chained while they fit the chip about once; not
-// with single-row tiles, whose CTAs would be placed around those of the kernel
-// before and lose their even spread (128^2: 12.9 us per sweep chained, 9.5 not).
-static inline bool sweep_chained(const Geo& g, bool march) {
-    return (march || cell_tile(g) != 1) && blocks_of(cell_grid(g, 8)) <= 592;
-}
+// The update kernel of a sweep is chained while it fits the chip about once.
+static inline bool apply_chained(const Geo& g) { return blocks_of(face_grid(g)) <= 592; }
 template <typename T>
 void run_march(const GlideLevelArgs*, const void*, const void*, const void*, int, double, double, const int*,
                const int*, void*, cudaStream_t);
 
 template <typename T>
+static SweepState<T> state_of(const GlideLevelArgs* a) {
+    return {(const T*)a->u, (const T*)a->v, (const T*)a->H, nullptr, nullptr, nullptr, nullptr, T(0)};
+}
+template <typename T>
 static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton,
                       double shift, double step, int pivot, const int* flags, const int* any_active, void* scratch,
-                      const Geo& g, bool cycle, cudaStream_t s) {
+                      const Geo& g, bool cycle, const SweepState<T>& q, cudaStream_t s) {
     if (use_march<T>(g, pivot, cycle)) {
         run_march<T>(a, f_u, f_v, f_H, n_newton, shift, step, flags, any_active, scratch, s);
         return;
     }
     with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
         using P = decltype(p);
-        auto go = [&](auto vy, auto chain) {
-            constexpr int VY = decltype(vy)::value;
-            constexpr bool CHAIN = decltype(chain)::value;
-            auto run = [&](auto kernel) {
-                launch_chained<CHAIN>(kernel, cell_grid(g, VY), VX * VY, s, (T*)scratch, (const T*)a->u,
-                                      (const T*)a->v, (const T*)a->H, (const T*)f_u, (const T*)f_v, (const T*)f_H,
-                                      (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->gamma, flags,
-                                      any_active, n_newton, T(shift), T(step), pivot, g, p);
-            };
-            flags ? run(vanka_cells_kernel<T, VY, true, CHAIN, P>) : run(vanka_cells_kernel<T, VY, false, CHAIN, P>);
+        auto run = [&](auto kernel) {
+            launch_chained<true>(kernel, cell_grid(g), VX * VY, s, (T*)scratch, q, (const T*)f_u, (const T*)f_v,
+                                 (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta,
+                                 (const T*)a->gamma, flags, any_active, n_newton, T(shift), T(step), pivot, g, p);
         };
-        using std::integral_constant;
-        const int vy = cell_tile(g);
-        if (vy == 4)
-            go(integral_constant<int, 4>{}, std::true_type{});
-        else if (vy == 1)
-            go(integral_constant<int, 1>{}, std::false_type{});
-        else if (sweep_chained(g, false))
-            go(integral_constant<int, 8>{}, std::true_type{});
-        else
-            go(integral_constant<int, 8>{}, std::false_type{});
+        flags ? run(vanka_cells_kernel<T, true, P>) : run(vanka_cells_kernel<T, false, P>);
     });
 }
 
+// work (GLIDE_SWEEP_WORK elements, or null): a second state and a second set of
+// cell arrays.  With them a sweep of the tile form is one kernel: it reads the
+// state before and the update of the sweep before, and passes the sum on from
+// one state to the other; one vanka_apply_kernel ends the call.  Microseconds per
+// sweep of 10 Newton steps, two kernels / one: 32^2 8.1 / 6.7, 64^2 9.0 / 7.0,
+// 256^2 16.1 / 14.1, 512^2 47.1 / 44.6, 1024^2 174 / 172; gated cycles gain most,
+// a 512^2 step of three cycles 32.0 / 25.8 ms.
 template <typename T>
 int launch_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
                         int n_newton, double omega, double shift, const int* flags, const int* any_active,
-                        void* scratch, cudaStream_t s, double newton_step, int pivot, bool cycle) {
+                        void* scratch, cudaStream_t s, double newton_step, int pivot, bool cycle, void* work) {
     Geo g{a->ny, a->nx, a->nb};
+    const bool chained = apply_chained(g), fused = work && !use_march<T>(g, pivot, cycle);
+    SweepState<T> q = state_of<T>(a);
+    q.omega = T(omega);
+    T* const first[3] = {(T*)a->u, (T*)a->v, (T*)a->H};
+    T *const wu = (T*)work, *const wv = wu + g.nu() * g.nb, *const wH = wv + g.nv() * g.nb;
+    T* const second[3] = {wu, wv, wH};
+    T *d = (T*)scratch, *d_next = fused ? wH + g.nc() * g.nb : d;
     auto apply = [&](auto chain) {
         constexpr bool CHAIN = decltype(chain)::value;
         auto run = [&](auto kernel) {
-            launch_chained<CHAIN>(kernel, face_grid(g), dim3(32, 8), s, (T*)a->u, (T*)a->v, (T*)a->H,
-                                  (const T*)scratch, flags, any_active, T(omega), g);
+            launch_chained<CHAIN>(kernel, face_grid(g), dim3(32, 8), s, (T*)a->u, (T*)a->v, (T*)a->H, q.u, q.v, q.H,
+                                  (const T*)d, flags, any_active, T(omega), g);
         };
         flags ? run(vanka_apply_kernel<T, true, CHAIN>) : run(vanka_apply_kernel<T, false, CHAIN>);
     };
-    const bool chained = sweep_chained(g, use_march<T>(g, pivot, cycle));
     for (int k = 0; k < n_iter; k++) {
-        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, pivot, flags, any_active, scratch, g, cycle, s);
-        chained ? apply(std::true_type{}) : apply(std::false_type{});
+        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, pivot, flags, any_active, d, g, cycle, q, s);
+        if (!fused || k == n_iter - 1) {
+            if (fused && q.ou) q.u = q.ou, q.v = q.ov, q.H = q.oH;
+            chained ? apply(std::true_type{}) : apply(std::false_type{});
+            continue;
+        }
+        if (q.ou) q.u = q.ou, q.v = q.ov, q.H = q.oH;   // this sweep's state; its update comes next
+        T* const* to = q.u == first[0] ? second : first;
+        q.ou = to[0], q.ov = to[1], q.oH = to[2];
+        q.d = d;
+        T* t = d; d = d_next; d_next = t;
     }
     return (int)cudaGetLastError();
 }
@@ -597,7 +747,7 @@ int launch_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v
                        cudaStream_t s, double newton_step) {
     Geo g{a->ny, a->nx, a->nb};
     for (int k = 0; k < n_launch; k++)
-        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, 0, flags, any_active, scratch, g, false, s);
+        run_cells<T>(a, f_u, f_v, f_H, n_newton, shift, newton_step, 0, flags, any_active, scratch, g, false, state_of<T>(a), s);
     return (int)cudaGetLastError();
 }
 
@@ -628,7 +778,7 @@ int launch_tile_flags(const GlideLevelArgs* a, const void* err_mask, int* flags,
 
 #define INST(T)                                                                                                  \
     template int launch_vanka_sweeps<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,   \
-                                        double, double, const int*, const int*, void*, cudaStream_t, double, int, bool);\
+                                        double, double, const int*, const int*, void*, cudaStream_t, double, int, bool, void*);\
     template int launch_vanka_cells<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,     \
                                        double, const int*, const int*, void*, cudaStream_t, double);              \
     template int launch_error_mask<T>(const GlideLevelArgs*, const void*, const void*, const void*, double,       \

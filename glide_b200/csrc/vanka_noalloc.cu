@@ -35,7 +35,7 @@
 namespace glide {
 template <typename T>
 int launch_vanka_sweeps(const GlideLevelArgs*, const void*, const void*, const void*, int, int, double, double,
-                        const int*, const int*, void*, cudaStream_t, double, int, bool cycle);
+                        const int*, const int*, void*, cudaStream_t, double, int, bool cycle, void* work);
 }
 
 namespace {
@@ -127,7 +127,7 @@ extern "C" int glide_vanka_sweeps_noalloc(const GlideLevelArgs* a, const void* f
     if (rc) return rc;
     return a->dtype == GLIDE_F32
                ? glide::launch_vanka_sweeps<float>(a, f_u, f_v, f_H, n_iter, n_newton, omega, shift, flags, any_active,
-                                                   scratch, (cudaStream_t)stream, GLIDE_REF_NEWTON_STEP, 0, false)
+                                                   scratch, (cudaStream_t)stream, GLIDE_REF_NEWTON_STEP, 0, false, nullptr)
                : glide::launch_vanka_sweeps<double>(a, f_u, f_v, f_H, n_iter, n_newton, omega, shift, flags,
-                                                    any_active, scratch, (cudaStream_t)stream, GLIDE_REF_NEWTON_STEP, 0, false);
+                                                    any_active, scratch, (cudaStream_t)stream, GLIDE_REF_NEWTON_STEP, 0, false, nullptr);
 }

@@ -76,6 +76,10 @@ class Grid:
         for name in ("H_prev", "chi", "phi", "bed", "beta", "B", "smb", "mask", "error_mask", "gamma"):
             setattr(self, name, self._cells())
         self._scratch = torch.zeros(5 * self.nb * self.nh, dtype=self.dtype, device=self.device)
+        # second state and cell arrays of the forward smoother (one kernel per sweep): FP32 grids
+        # up to 2^20 cells, 34 MB
+        fused = self.dtype == torch.float32 and self.nb * self.nh <= 1 << 20
+        self._sweep_work = self._scratch.new_empty(self.nb * (self.n_total + 5 * self.nh)) if fused else None
         nflags = (self.ny // 14 + 1) * (self.nx // 14 + 1) * self.nb
         self._flags = torch.zeros(nflags, dtype=torch.int32, device=self.device)
         self._any_active = torch.zeros(self.nb, dtype=torch.int32, device=self.device)
@@ -119,6 +123,8 @@ class Grid:
             L.norm_parts = self._norm_parts.data_ptr()
         if self._adj_factors is not None:
             L.adj_factors = self._adj_factors.data_ptr()
+        if self._sweep_work is not None:
+            L.sweep_work = self._sweep_work.data_ptr()
         return L
 
     def adjoint_factors(self):
@@ -212,10 +218,11 @@ class Grid:
         a = self.level_args()
         flags = self._flags.data_ptr() if local else None
         anyact = self._any_active.data_ptr() if local else None
-        N.check(self._lib.glide_vanka_sweeps_ex(C.byref(a), self.f_u.data_ptr(), self.f_v.data_ptr(),
-                                                self.f_H.data_ptr(), int(n_iter), int(n_inner), float(step),
-                                                float(omega), float(shift), int(bool(pivot)), flags, anyact,
-                                                self._scratch.data_ptr(), self._s()), "vanka")
+        work = None if self._sweep_work is None else self._sweep_work.data_ptr()
+        N.check(self._lib.glide_vanka_sweeps_work(C.byref(a), self.f_u.data_ptr(), self.f_v.data_ptr(),
+                                                  self.f_H.data_ptr(), int(n_iter), int(n_inner), float(step),
+                                                  float(omega), float(shift), int(bool(pivot)), flags, anyact,
+                                                  self._scratch.data_ptr(), work, self._s()), "vanka")
 
     def vanka_smooth(self, color=0, omega=1.0, n_inner=1, shift=1.0):
         """One ``vanka_smooth`` launch: adds the face/cell deltas into

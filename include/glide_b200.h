@@ -106,6 +106,14 @@ int glide_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_v
 int glide_vanka_sweeps_ex(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
                           int n_newton, double newton_step, double omega, double shift, int pivoted_lu,
                           const int* flags, const int* any_active, void* scratch, void* stream);
+/* glide_vanka_sweeps_ex with room for GLIDE_SWEEP_WORK(ny, nx, nb) elements of
+ * dtype: a sweep of the tile form is then one kernel instead of two.  work null:
+ * glide_vanka_sweeps_ex; the results are the same bits either way. */
+#define GLIDE_SWEEP_WORK(ny, nx, nb) \
+    ((int64_t)(nb) * ((int64_t)(ny) * ((nx) + 1) + (int64_t)((ny) + 1) * (nx) + 6 * (int64_t)(ny) * (nx)))
+int glide_vanka_sweeps_work(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_iter,
+                            int n_newton, double newton_step, double omega, double shift, int pivoted_lu,
+                            const int* flags, const int* any_active, void* scratch, void* work, void* stream);
 /* Same sweeps as glide_vanka_sweeps for callers that cannot allocate device
  * memory (no counterpart in the reference): the scratch lives in a fixed
  * 10 MiB device array inside the library (glide_noalloc_scratch_bytes()),
@@ -201,6 +209,8 @@ typedef struct GlideLevel {
     void* r_raw;            /* like U: residual at the linearisation state (active-set test) */
     /* adjoint smoother (may be null: the local matrices are then formed for every colour) */
     void* adj_factors;      /* GLIDE_ADJ_FACTORS * nc * nb */
+    /* forward smoother (may be null: a sweep is then two kernels) */
+    void* sweep_work;       /* GLIDE_SWEEP_WORK(ny, nx, nb) */
 } GlideLevel;
 
 /* Step sizes tried by the coarse-correction line search, best first on ties. */

@@ -1,5 +1,5 @@
-"""The forward sweep at sizes on both sides of its tile-height and chaining
-rules (tiles of 4, 1 and 8 rows), against the oracle; a chain of sweeps equals
+"""The forward sweep at sizes from one tile to many waves of them, on both sides
+of its march and chaining rules, against the oracle; a chain of sweeps equals
 the same sweeps with a synchronisation after each; FP64 1e-10, FP32 4e-4
 (tolerances of test_vanka_sweep)."""
 import pytest
