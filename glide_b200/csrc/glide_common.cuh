@@ -251,30 +251,8 @@ __device__ __forceinline__ ShearStress<T> shear_stress(T ut, T ub, T vl, T vr, T
 template <typename T> struct BasalDrag {
     T res, d_vel, d_H1, d_H2, d_beta1, d_beta2;
 };
-template <typename T>
-__device__ __forceinline__ BasalDrag<T> basal_drag(T vel, T H1, T H2, T bed1, T bed2, T beta1, T beta2,
-                                                   const Phys<T>& p) {
-    BasalDrag<T> o;
-    T z1 = bed1 + rho_ratio<T>() * H1, z2 = bed2 + rho_ratio<T>() * H2;
-    T g1 = sigmoid(z1, p.sig_c), g2 = sigmoid(z2, p.sig_c);
-    T be = T(0.5) * ((g1 * beta1 + (T(1) - g1) * p.water_drag) + (g2 * beta2 + (T(1) - g2) * p.water_drag));
-    o.res = -be * vel;
-    o.d_vel = -be;
-    o.d_beta1 = T(-0.5) * g1 * vel;
-    o.d_beta2 = T(-0.5) * g2 * vel;
-    if (p.gl_deriv) {
-        T s1 = p.sig_c * g1 * (T(1) - g1), s2 = p.sig_c * g2 * (T(1) - g2);
-        o.d_H1 = T(-0.5) * (rho_ratio<T>() * s1) * (beta1 - p.water_drag) * vel;
-        o.d_H2 = T(-0.5) * (rho_ratio<T>() * s2) * (beta2 - p.water_drag) * vel;
-    } else {
-        o.d_H1 = T(0);
-        o.d_H2 = T(0);
-    }
-    return o;
-}
-
-// Same drag with the two grounded fractions already known (the Vanka loop
-// hoists the neighbour's sigmoid out of its Newton iterations).
+// The drag of a face from the grounded fractions of its two cells (the Vanka
+// loop hoists the neighbour's sigmoid out of its Newton iterations).
 template <typename T>
 __device__ __forceinline__ BasalDrag<T> basal_drag_g(T vel, T g1, T g2, T beta1, T beta2, const Phys<T>& p) {
     BasalDrag<T> o;

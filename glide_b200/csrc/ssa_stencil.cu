@@ -754,36 +754,29 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
 template <typename T>
 __global__ void grad_beta_kernel(T* __restrict__ grad, const T* __restrict__ u, const T* __restrict__ v,
                                  const T* __restrict__ H, const T* __restrict__ lu, const T* __restrict__ lv,
-                                 const T* __restrict__ bed, const T* __restrict__ beta, int exact_boundary,
-                                 Geo g, Phys<T> p) {
+                                 const T* __restrict__ bed, int exact_boundary, Geo g, Phys<T> p) {
     const int ny = g.ny, nx = g.nx;
     const int b = blockIdx.z;
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = blockIdx.y * blockDim.y + threadIdx.y;
     if (i >= ny || j >= nx) return;
     u += b * g.nu(); v += b * g.nv(); H += b * g.nc(); lu += b * g.nu(); lv += b * g.nv();
-    bed += b * g.nc(); beta += b * g.nc(); grad += b * g.nc();
+    bed += b * g.nc(); grad += b * g.nc();
+    // d(drag)/d(beta) of a face is -velocity/2 times the cell's own grounded fraction: one sigmoid per cell
+    const T k = T(-0.5) * sigmoid(ldc(bed, i, j, ny, nx) + rho_ratio<T>() * ldc(H, i, j, ny, nx), p.sig_c);
     T acc = 0;
-    auto uface = [&](int jj) {
-        return basal_drag(ldu(u, i, jj, ny, nx), ldc(H, i, jj - 1, ny, nx), ldc(H, i, jj, ny, nx),
-                          ldc(bed, i, jj - 1, ny, nx), ldc(bed, i, jj, ny, nx), ldc(beta, i, jj - 1, ny, nx),
-                          ldc(beta, i, jj, ny, nx), p);
-    };
-    auto vface = [&](int ii) {
-        return basal_drag(ldv(v, ii, j, ny, nx), ldc(H, ii - 1, j, ny, nx), ldc(H, ii, j, ny, nx),
-                          ldc(bed, ii - 1, j, ny, nx), ldc(bed, ii, j, ny, nx), ldc(beta, ii - 1, j, ny, nx),
-                          ldc(beta, ii, j, ny, nx), p);
-    };
+    auto uface = [&](int jj) { return ldu(lu, i, jj, ny, nx) * (k * ldu(u, i, jj, ny, nx)); };
+    auto vface = [&](int ii) { return ldv(lv, ii, j, ny, nx) * (k * ldv(v, ii, j, ny, nx)); };
     // right face (i,j+1): this cell is its left cell (added when j+1 > 0: always)
-    acc += ldu(lu, i, j + 1, ny, nx) * uface(j + 1).d_beta1;
+    acc += uface(j + 1);
     // left face (i,j): this cell is its right cell (reference adds it only for j < nx-1)
-    if (exact_boundary || j < nx - 1) acc += ldu(lu, i, j, ny, nx) * uface(j).d_beta2;
-    if (exact_boundary && j == 0) acc += ldu(lu, i, 0, ny, nx) * uface(0).d_beta1;
-    if (exact_boundary && j == nx - 1) acc += ldu(lu, i, nx, ny, nx) * uface(nx).d_beta2;
-    acc += ldv(lv, i + 1, j, ny, nx) * vface(i + 1).d_beta1;
-    if (exact_boundary || i < ny - 1) acc += ldv(lv, i, j, ny, nx) * vface(i).d_beta2;
-    if (exact_boundary && i == 0) acc += ldv(lv, 0, j, ny, nx) * vface(0).d_beta1;
-    if (exact_boundary && i == ny - 1) acc += ldv(lv, ny, j, ny, nx) * vface(ny).d_beta2;
+    if (exact_boundary || j < nx - 1) acc += uface(j);
+    if (exact_boundary && j == 0) acc += uface(0);
+    if (exact_boundary && j == nx - 1) acc += uface(nx);
+    acc += vface(i + 1);
+    if (exact_boundary || i < ny - 1) acc += vface(i);
+    if (exact_boundary && i == 0) acc += vface(0);
+    if (exact_boundary && i == ny - 1) acc += vface(ny);
     grad[int64_t(i) * nx + j] = acc;
 }
 
@@ -898,8 +891,7 @@ int launch_grad_beta(const GlideLevelArgs* a, const void* l_u, const void* l_v, 
     dim3 blk(32, 8);
     dim3 grd((g.nx + 31) / 32, (g.ny + 7) / 8, g.nb);
     glide::count_launch(), grad_beta_kernel<T><<<grd, blk, 0, s>>>((T*)grad, (const T*)a->u, (const T*)a->v, (const T*)a->H,
-                                            (const T*)l_u, (const T*)l_v, (const T*)a->bed, (const T*)a->beta,
-                                            exact_boundary, g, p);
+                                            (const T*)l_u, (const T*)l_v, (const T*)a->bed, exact_boundary, g, p);
     return (int)cudaGetLastError();
 }
 
