@@ -448,19 +448,18 @@ def roofline(t, n):
     fp32_peak = 148 * 128 * 2 * 1.965e9 / 1e12
     t64, t32 = t.get("cells64"), t["cells32"]
     ach = hbm_obj(VANKA_ARRAYS, 4, t32)
-    roof = {"bound": "hbm", "kernel": "vanka_cells_kernel<float> (fine level, full sweep)",
+    roof = {"bound": "hbm", "kernel": "vanka_march_kernel<float> (fine level, full sweep)",
             "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": src,
             "traffic": VANKA32_DRAM_BYTES_1024 * scale,
-            "traffic_source": "ncu dram__bytes_read+write, one 1024^2 launch",
+            "traffic_source": "ncu dram__bytes_read+write, one 1024^2 launch of the tile form",
             "algorithmic_bytes": ncell * VANKA_ARRAYS * 4, "launch_ms": t32 * 1e3,
-            "limiter": "FP32 issue/latency (ncu at 1024^2: issue slots 61% active, 15 warps/SM at 128 registers, "
-                       "1687 instructions per cell: FP32 930, integer 466, memory 129)",
+            "limiter": "FP32 issue/latency (ncu at 1024^2, 10 Newton steps: issue slots 63% active, 13 warps/SM at 126 registers)",
             "alu": {"achieved_tflops": ncell * VANKA32_FLOPS_PER_CELL / t32 / 1e12, "peak_tflops": fp32_peak,
                     "frac": ncell * VANKA32_FLOPS_PER_CELL / t32 / 1e12 / fp32_peak,
                     "flops_per_cell": VANKA32_FLOPS_PER_CELL,
                     "peak_source": "nominal FP32 (148 SMs x 128 FFMA/clk)"}}
     if t64:
-        roof["fp64_cells"] = {"kernel": "vanka_cells_kernel<double> (fine level, FP64 finishing blocks)",
+        roof["fp64_cells"] = {"kernel": "vanka_march_kernel<double> (fine level, FP64 finishing blocks)",
                               "launch_ms": t64 * 1e3,
                               "achieved_tflops": ncell * VANKA64_FLOPS_PER_CELL / t64 / 1e12,
                               "frac_fp64_peak": ncell * VANKA64_FLOPS_PER_CELL / t64 / 1e12 / fp64_peak,

@@ -18,7 +18,7 @@
 //
 // What bounds the tile form: below about 200^2 the latency of one cell's chain
 // (0.33 us per Newton step, 3 us to read, assemble and store), above it
-// instruction issue (340 instructions per Newton step).
+// instruction issue (4,870 instructions per warp of 32 cells and 10 steps).
 #include <type_traits>
 
 #include "glide_common.cuh"

@@ -5,18 +5,17 @@
 // A warp owns 30 cell columns and marches down a chunk of rows with the rows
 // in reach in registers and the neighbouring columns in its lanes: every
 // viscosity, grounded fraction, surface and drag is computed once per launch
-// and every field read once per row, where a thread per cell of a tile takes 58
-// clamped loads, five sigmoids and two rounds of viscosities; a Newton step is
-// about 270 instructions instead of 340, with four reciprocals (two of them
-// independent) instead of five successive pivots.  The unknowns are the
+// and every field read once per row, where a thread per cell of a tile takes
+// five sigmoids and a ring of viscosities; 30 cells with 10 Newton steps are 2,590
+// warp instructions (32 cells of the tile form 4,870), with four reciprocals a
+// step (two of them independent) instead of five successive pivots.  The unknowns are the
 // increments of the face velocities over their values at the start, so the
 // differences of nearby velocities that the strain rates need are formed once,
 // from the unrounded state.
 //
-// What bounds it: in FP32 instruction issue (by count 105 of the 125 us that the
-// kernel takes at 1024^2 with 10 steps); in FP64 the FP64 pipe (155 of 335 us)
-// and the latency of a step's chain at two CTAs per SM.  Reading and writing a
-// cell's 13 values is 3 % of the time.  Figures of both forms: use_march in
+// What bounds it: instruction issue and the latency of a step's chain at the 13
+// (FP64: 8) warps that an SM's registers hold; FP32, 1024^2, 10 steps: issue slots
+// 63 % active, FMA pipe 44 %, DRAM 4 %.  Figures of both forms: use_march in
 // vanka.cu.
 #include <type_traits>
 

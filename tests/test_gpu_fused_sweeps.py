@@ -1,7 +1,7 @@
 """Sweeps that pass the state on inside the cell kernel (one kernel per sweep)
 give the bits of separate calls, each a cell kernel and an update: whole and
-gated, at sizes of every tile height, ragged, odd and even sweep counts, and a
-batch in which one scenario has no active cell."""
+gated, at edges of the tiles, odd and even sweep counts, and a batch in
+which one scenario has no active cell."""
 import pytest
 import torch
 
