@@ -416,10 +416,45 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloa
 // its own, 2x the L2 traffic and 8x the shared-memory writes, and the copies
 // set the pace (256^2, 384 -> 128: 274 us against 127).  The convolution's
 // input may be two tensors (see ConvShape).
+//
+// TAPS: the data gradient of a 3x3 layer, dx[y, x] = sum over the taps of
+// gz[y+1-ky, x+1-kx] W[tap].  Each tap's sum over the channels stays an FP32
+// number of its own (nine accumulators of BN columns) and the epilogue adds the
+// nine in FP32, tap after tap: what GEMM + col2im compute, without the (pixels x
+// 9 C) FP32 matrix between them.  B is the transposed weights, row tap * N + n.
 // --------------------------------------------------------------------------
 constexpr int RG_COPY = 256, RG_THREADS = RG_COPY + 32, RG_STAGES = 6;
 
-template <bool CONV, int BN>
+// The nine taps' sums of a warp's 32 pixels, added in tap order and stored as BF16.
+template <int BN>
+__device__ __forceinline__ void store_taps(uint32_t tmem, int warp, int lane, int m0, int n0, int M, int N,
+                                           __nv_bfloat16* C) {
+    const int row = m0 + warp * 32 + lane;
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += 8) {
+        uint32_t r[9][8];
+#pragma unroll
+        for (int t = 0; t < 9; t++)
+            asm volatile(
+                "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                : "=r"(r[t][0]), "=r"(r[t][1]), "=r"(r[t][2]), "=r"(r[t][3]), "=r"(r[t][4]), "=r"(r[t][5]),
+                  "=r"(r[t][6]), "=r"(r[t][7])
+                : "r"(tmem + (uint32_t(warp * 32) << 16) + uint32_t(t * BN + c0)));
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (row >= M || n0 + c0 >= N) continue;   // N is a multiple of 8
+        __align__(16) __nv_bfloat16 h[8];
+#pragma unroll
+        for (int e = 0; e < 8; e++) {
+            float x = 0.0f;
+#pragma unroll
+            for (int t = 0; t < 9; t++) x += __uint_as_float(r[t][e]);
+            h[e] = __float2bfloat16(x);
+        }
+        *reinterpret_cast<uint4*>(C + int64_t(row) * N + n0 + c0) = *reinterpret_cast<uint4*>(h);
+    }
+}
+
+template <bool CONV, int BN, bool TAPS = false>
 __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfloat16* __restrict__ A, int lda,
                                                                   const __nv_bfloat16* __restrict__ B, int ldb, void* C,
                                                                   int ldc, int M, int N, int K,
@@ -428,6 +463,8 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
     constexpr int A_BYTES = GM * GK * 2, B_BYTES = BN * GK * 2, STAGE = A_BYTES + B_BYTES;
     constexpr int AROWS = GM * 8 / RG_COPY, BROWS = BN * 8 / RG_COPY;   // 16-byte copies per thread and chunk
     constexpr int STEP = RG_COPY / 8;                                   // rows between a thread's copies
+    constexpr uint32_t COLS = TAPS ? 512 : BN;                          // TMEM columns
+    static_assert(!TAPS || (CONV && 9 * BN <= 512), "nine accumulators");
     extern __shared__ __align__(1024) uint8_t smem[];
     __shared__ __align__(8) uint64_t full[RG_STAGES], empty[RG_STAGES], done;
     __shared__ uint32_t tmem_slot;
@@ -436,7 +473,7 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
     const uint32_t sbase = (smem_u32(smem) + 1023u) & ~1023u;
     if (warp == RG_COPY / 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(uint32_t(BN)));
+                     "r"(COLS));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::);
     }
     if (threadIdx.x == 0) {
@@ -483,7 +520,8 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
             const int k = ch * GK + kc * 8;
             const bool kin = k < K;
             if (CONV) {
-                const int ky = tap / 3, dy = ky - 1, dx = tap - 3 * ky - 1;
+                const int ky = tap / 3, kx = tap - 3 * ky;
+                const int dy = TAPS ? 1 - ky : ky - 1, dx = TAPS ? 1 - kx : kx - 1;
                 const bool second = c >= cs.C0;
                 const int Cs = second ? cs.C - cs.C0 : cs.C0, cc = second ? c - cs.C0 : c;
                 const __nv_bfloat16* src0 = second ? cs.x1 : A;
@@ -497,6 +535,12 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
                     cp_async16(st + sw128_off(rsub + STEP * i, kc), in ? src0 + int64_t(pix) * Cs + cc : A,
                                in ? 16u : 0u);
                 }
+                if (TAPS) {   // one row per thread (BN = 32)
+                    const int n = n0 + rsub;
+                    const bool in = kin && n < N;
+                    cp_async16(st + A_BYTES + sw128_off(rsub, kc),
+                               in ? B + (int64_t(tap) * N + n) * cs.C + c : B, in ? 16u : 0u);
+                }
                 c += GK;
                 while (c >= cs.C) { c -= cs.C; tap++; }
             } else {
@@ -508,7 +552,7 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
                 }
             }
 #pragma unroll
-            for (int i = 0; i < BROWS; i++) {
+            for (int i = 0; i < (TAPS ? 0 : BROWS); i++) {
                 const int n = n0 + rsub + STEP * i;
                 const bool in = kin && n < N;
                 cp_async16(st + A_BYTES + sw128_off(rsub + STEP * i, kc), in ? B + int64_t(n) * ldb + k : B,
@@ -520,6 +564,7 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
         cp_async_wait<0>();
     } else {
         const uint32_t idesc = idesc_bf16_f32(GM, BN), lead = lane == 0, hi = umma_hi_sw128();
+        int tap = 0, c = 0;   // TAPS: a step's 16 columns lie in one tap (C is a multiple of 16)
         for (int ch = 0; ch < nchunks; ch++) {
             const int sl = ch % RG_STAGES;
             if (!mbar_wait_bounded(smem_u32(&full[sl]), uint32_t((ch / RG_STAGES) & 1))) { ok = false; break; }
@@ -527,8 +572,16 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
             const uint32_t st = sbase + uint32_t(sl * STAGE);
             const uint32_t a_lo = umma_lo(st, 16), b_lo = umma_lo(st + A_BYTES, 16);
 #pragma unroll
-            for (int s = 0; s < GK / 16; s++)
-                mma_bf16_lead(tmem, a_lo + s * 2, hi, b_lo + s * 2, hi, idesc, ch > 0 || s > 0, lead);
+            for (int s = 0; s < GK / 16; s++) {
+                if constexpr (TAPS) {
+                    if (tap == 9) break;
+                    mma_bf16_lead(tmem + uint32_t(tap * BN), a_lo + s * 2, hi, b_lo + s * 2, hi, idesc, c > 0, lead);
+                    c += 16;
+                    if (c == cs.C) { c = 0; tap++; }
+                } else {
+                    mma_bf16_lead(tmem, a_lo + s * 2, hi, b_lo + s * 2, hi, idesc, ch > 0 || s > 0, lead);
+                }
+            }
             mma_commit_lead(&empty[sl], lead);
         }
         mma_commit_lead(&done, lead);
@@ -538,15 +591,20 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
     if (!ok && lane == 0 && err) atomicExch(err, 1);
     ok = __syncthreads_and(ok ? 1 : 0) != 0;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok && warp < 4) store_tile<BN>(tmem, warp, lane, m0, n0, M, N, C, ldc, bias, relu, out_mode);
+    if (ok && warp < 4) {
+        if constexpr (TAPS)
+            store_taps<BN>(tmem, warp, lane, m0, n0, M, N, reinterpret_cast<__nv_bfloat16*>(C));
+        else
+            store_tile<BN>(tmem, warp, lane, m0, n0, M, N, C, ldc, bias, relu, out_mode);
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == RG_COPY / 32) {
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(uint32_t(BN)));
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS));
     }
 }
 
-template <bool CONV, int BN>
+template <bool CONV, int BN, bool TAPS = false>
 int launch_ring(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb, void* C, int ldc, int M, int N,
                 int K, const float* bias, int relu, int out_mode, int* err, ConvShape cs, cudaStream_t s) {
     constexpr int SMEM = RG_STAGES * (GM * GK * 2 + BN * GK * 2) + 1024;
@@ -555,14 +613,14 @@ int launch_ring(const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return GLIDE_E_SHAPE;
     if (!configured[dev]) {
-        const cudaError_t e = cudaFuncSetAttribute(tc_gemm_ring_kernel<CONV, BN>,
+        const cudaError_t e = cudaFuncSetAttribute(tc_gemm_ring_kernel<CONV, BN, TAPS>,
                                                    cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
         if (e != cudaSuccess) return int(e);
         configured[dev] = 1;
     }
     dim3 grid((M + GM - 1) / GM, (N + BN - 1) / BN);
-    count_launch(), tc_gemm_ring_kernel<CONV, BN><<<grid, RG_THREADS, SMEM, s>>>(A, lda, B, ldb, C, ldc, M, N, K, bias,
-                                                                                 relu, out_mode, err, cs);
+    count_launch(), tc_gemm_ring_kernel<CONV, BN, TAPS><<<grid, RG_THREADS, SMEM, s>>>(
+        A, lda, B, ldb, C, ldc, M, N, K, bias, relu, out_mode, err, cs);
     return int(cudaGetLastError());
 }
 
@@ -668,4 +726,16 @@ extern "C" int glide_conv3x3_cat_bf16(const void* x0, int C0, int up0, const voi
                                       9 * C, bias, relu, out_mode, err,
                                       glide::ConvShape{Bn, H, W, C, (const __nv_bfloat16*)x1, C0, up0},
                                       (cudaStream_t)stream);
+}
+
+extern "C" int glide_conv3x3_dgrad_bf16(const void* gz, const void* Wt, void* dx, int Bn, int H, int W, int C, int N,
+                                        int* err, void* stream) {
+    if (!gz || !Wt || !dx) return GLIDE_E_NULL;
+    if (Bn < 1 || H < 1 || W < 1 || C < 8 || C % 8 != 0 || N < 16 || N % 16 != 0) return GLIDE_E_SHAPE;
+    if (!glide::al16(gz) || !glide::al16(Wt) || !glide::al16(dx)) return GLIDE_E_SHAPE;
+    const int64_t P = int64_t(Bn) * H * W;
+    if (P >= (int64_t(1) << 31)) return GLIDE_E_TOO_LARGE;
+    return glide::launch_ring<true, 32, true>((const __nv_bfloat16*)gz, 0, (const __nv_bfloat16*)Wt, 0, dx, C, int(P), C,
+                                              9 * N, nullptr, 0, 1, err, glide::ConvShape{Bn, H, W, N, nullptr, N, 0},
+                                              (cudaStream_t)stream);
 }

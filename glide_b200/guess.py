@@ -58,6 +58,8 @@ def _lib():
         lib.glide_pool2_bf16.restype = C.c_int
         lib.glide_conv3x3_wgrad_bf16.argtypes = [C.c_void_p] * 3 + [C.c_int] * 5 + [C.c_void_p, C.c_void_p]
         lib.glide_conv3x3_wgrad_bf16.restype = C.c_int
+        lib.glide_conv3x3_dgrad_bf16.argtypes = [C.c_void_p] * 3 + [C.c_int] * 5 + [C.c_void_p, C.c_void_p]
+        lib.glide_conv3x3_dgrad_bf16.restype = C.c_int
         lib.glide_relu_grad_bf16.argtypes = [C.c_void_p] * 5 + [C.c_int64, C.c_int, C.c_int, C.c_void_p]
         lib.glide_relu_grad_bf16.restype = C.c_int
         lib.glide_relu_grad_blocks.argtypes = [C.c_int64, C.c_int]
@@ -199,13 +201,31 @@ def _relu_grad(gy, y, relu):
     return gz, db
 
 
+def _data_grad(gz, Wb, shape):
+    """dx of a 3x3 layer from gz (P, Cout): each tap's sum over Cout in FP32, the
+    nine added in FP32.  Output widths that are no multiple of 16 go through
+    dcol (P x 9Cin) = gz . W and col2im, the others compute the same numbers in
+    one kernel."""
+    Bn, H, Wd, Cin = shape
+    P, Cout = gz.shape
+    Wt = transpose(Wb)
+    if Cin % 8 == 0 and Cout % 16 == 0:
+        dx = torch.empty(shape, dtype=torch.bfloat16, device=gz.device)
+        N.check(_lib().glide_conv3x3_dgrad_bf16(gz.data_ptr(), Wt.data_ptr(), dx.data_ptr(), Bn, H, Wd, Cin, Cout,
+                                                _err_flag(gz.device).data_ptr(), N.stream_handle()), "data gradient")
+        return dx
+    dcol = torch.empty((P, 9 * Cin), dtype=torch.float32, device=gz.device)
+    gemm(gz, Wt, dcol, out_mode=0)
+    return col2im3(dcol, shape).to(torch.bfloat16)
+
+
 class Conv3x3ReLU(torch.autograd.Function):
     """y = relu(conv3x3(x, W) + b); x NHWC BF16, W (Cout, 9*Cin) FP32 master.
 
-    With Cin and Cout multiples of 8 no im2col matrix exists in either
-    direction: the forward product, the data gradient (the convolution of gz
-    with the flipped kernel) and the weight gradient gather their shifted
-    pixels themselves.  Other widths run im2col + GEMM."""
+    With Cin and Cout multiples of 8 no im2col matrix exists in the forward
+    product and the weight gradient, which gather their shifted pixels
+    themselves; the data gradient is _data_grad.  Other widths run im2col +
+    GEMM."""
 
     @staticmethod
     def forward(ctx, x, W, b, relu: bool):
@@ -239,11 +259,7 @@ class Conv3x3ReLU(torch.autograd.Function):
             N.check(_lib().glide_conv3x3_wgrad_bf16(gz.data_ptr(), src.data_ptr(), dW.data_ptr(), Bn, H, Wd, Cin, Cout,
                                                     _err_flag(gy.device).data_ptr(), N.stream_handle()),
                     "weight gradient")
-            # data gradient: gz convolved with the kernel flipped in both directions, channels exchanged
-            Wf = Wb.view(Cout, 3, 3, Cin).flip(1, 2).permute(3, 1, 2, 0).reshape(Cin, 9 * Cout)
-            dx = torch.empty((Bn, H, Wd, Cin), dtype=torch.bfloat16, device=gy.device)
-            conv3x3(gz.view(Bn, H, Wd, Cout), Wf, dx.view(P, Cin), out_mode=1)
-            return dx, dW, db, None
+            return _data_grad(gz, Wb, (Bn, H, Wd, Cin)), dW, db, None
         g = gy.reshape(P, Cout).float()
         if ctx.relu:
             g = g * (y > 0)
@@ -252,11 +268,7 @@ class Conv3x3ReLU(torch.autograd.Function):
         dW = torch.zeros((Cout, 9 * Cin), dtype=torch.float32, device=gy.device)
         gemm(transpose(gz), transpose(src), dW, out_mode=0)
         db = g.sum(0)
-        # data gradient: dcol (P x 9Cin) = gz (P x Cout) . W (Cout x 9Cin)
-        dcol = torch.empty((P, 9 * Cin), dtype=torch.float32, device=gy.device)
-        gemm(gz, transpose(Wb), dcol, out_mode=0)
-        dx = col2im3(dcol, (Bn, H, Wd, Cin))
-        return dx.to(torch.bfloat16), dW, db, None
+        return _data_grad(gz, Wb, (Bn, H, Wd, Cin)), dW, db, None
 
 
 class Conv1x1(torch.autograd.Function):

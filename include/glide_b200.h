@@ -353,6 +353,13 @@ int glide_guess_faces(const float* pred, double* u, double* v, int nb, int ny, i
  * glide_gemm_bf16 on the transposes of gz and of the im2col matrix. */
 int glide_conv3x3_wgrad_bf16(const void* gz, const void* x, float* dW, int Bn, int H, int W, int C, int N, int* err,
                              void* stream);
+/* Data gradient of the same convolution: dx (Bn, H, W, C) BF16, dx[y, x, c] = sum
+ * over the taps, in order, of the FP32 sum over n of gz[y+1-ky, x+1-kx, n] *
+ * W[n, tap*C + c]; Wt (9C, N): the transposed weights.  N a multiple of 16, C of
+ * 8, all 16-byte aligned.  Bit-identical to glide_gemm_bf16 (FP32 out) followed
+ * by glide_col2im3_f32 and rounding to BF16. */
+int glide_conv3x3_dgrad_bf16(const void* gz, const void* Wt, void* dx, int Bn, int H, int W, int C, int N, int* err,
+                             void* stream);
 /* Backward of bias + ReLU of a (P, N) BF16 layer output y: gz = gy where y > 0
  * (gy itself without relu; y may then be null) and db[n] = the sum of gz over
  * p.  N a multiple of 8 (at most 2048), 16-byte aligned; parts:

@@ -1,0 +1,27 @@
+"""Data gradient of the training layer: every tap's sum over the output
+channels is an FP32 number of its own and the nine are added tap after tap, as
+col2im adds the product of gz and the transposed weights.  The same bits as
+that pair, at ragged pixel counts, channel tiles and output widths (multiples
+of 16 in one kernel, others by GEMM and col2im)."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("Bn,H,W,Cin,Cout", [(1, 1, 3, 8, 16), (2, 9, 13, 40, 48), (1, 20, 66, 64, 128), (2, 8, 32, 192, 256),
+                                             (3, 30, 128, 32, 32), (1, 7, 384, 16, 96), (2, 5, 37, 72, 24)])
+def test_data_gradient_adds_the_taps_in_order(Bn, H, W, Cin, Cout):
+    from glide_b200.guess import Conv3x3ReLU, _err_flag, col2im3, gemm, transpose
+    g = torch.Generator(device="cuda").manual_seed(H + W + Cin + Cout)
+    x = torch.randn(Bn, H, W, Cin, generator=g, device="cuda").to(torch.bfloat16).requires_grad_()
+    Wf = torch.randn(Cout, 9 * Cin, generator=g, device="cuda") * 0.1
+    b = torch.randn(Cout, generator=g, device="cuda")
+    y = Conv3x3ReLU.apply(x, Wf, b, True)
+    gy = torch.randn(Bn, H, W, Cout, generator=g, device="cuda").to(torch.bfloat16)
+    dx, = torch.autograd.grad(y, x, gy)
+    gz = (gy * (y > 0)).reshape(-1, Cout)
+    dcol = torch.empty(Bn * H * W, 9 * Cin, device="cuda")
+    gemm(gz, transpose(Wf.to(torch.bfloat16)), dcol, out_mode=0)
+    assert torch.equal(dx, col2im3(dcol, (Bn, H, W, Cin)).to(torch.bfloat16))
+    assert int(_err_flag(x.device).item()) == 0
