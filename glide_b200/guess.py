@@ -157,10 +157,16 @@ def conv3x3_relu(x, W, b, relu=True):
 
 def _rows_f32w(x, up, skip, W, b, relu, y):
     """y = relu(conv3x3(x | skip)) with the FP32 weights rounded inside the
-    kernel, where the row march takes the shape; False where it does not."""
+    kernel, where the row march takes the shape; False where it does not.  The
+    entry point sees addresses only: types, the weights' width (it assumes
+    9 Cin) and the bias are checked here, and what does not fit is left to
+    conv3x3, which refuses it or takes its pitch."""
     lib = _lib()
     C1 = 0 if skip is None else skip.shape[3]
-    if W.dtype != torch.float32 or not W.is_contiguous() or W.data_ptr() % 16 or \
+    if x.dtype != torch.bfloat16 or (skip is not None and skip.dtype != torch.bfloat16) or \
+            W.dtype != torch.float32 or W.shape != (y.shape[3], 9 * (x.shape[3] + C1)) or \
+            not W.is_contiguous() or W.data_ptr() % 16 or \
+            b.dtype != torch.float32 or not b.is_contiguous() or b.numel() < y.shape[3] or \
             not lib.glide_conv3x3_rows_ok(x.shape[3], up, C1, y.shape[2], y.shape[3]):
         return False
     N.check(lib.glide_conv3x3_rows_f32w(x.data_ptr(), x.shape[3], up, None if skip is None else skip.data_ptr(), C1,
