@@ -176,14 +176,29 @@ def _rows_f32w(x, up, skip, W, b, relu, y):
     return True
 
 
+def _in_place(x, skip, W):
+    """Whether the two sources can be read as they are: BF16, skip at twice the
+    resolution of x, 16-byte aligned channels in both, weights without padding."""
+    return x.dim() == 4 and skip.dim() == 4 and x.dtype == skip.dtype == torch.bfloat16 and \
+        x.device == skip.device and x.numel() > 0 and skip.numel() > 0 and \
+        skip.shape[:3] == (x.shape[0], 2 * x.shape[1], 2 * x.shape[2]) and \
+        x.shape[3] % 8 == 0 and skip.shape[3] % 8 == 0 and W.dim() == 2 and \
+        W.shape[1] == 9 * (x.shape[3] + skip.shape[3]) and not any(t.data_ptr() % 16 for t in (x, skip, W))
+
+
 def conv3x3_up_cat(x, skip, W, b):
     """conv3x3_relu(cat([_up(x), skip]), W, b).  Without autograd recording the
-    convolution reads both tensors directly (bit-identical)."""
-    if (torch.is_grad_enabled() and any(t.requires_grad for t in (x, skip, W, b))) or \
-            x.shape[3] % 8 != 0 or skip.shape[3] % 8 != 0:
-        return conv3x3_relu(torch.cat([_up(x), skip], dim=3), W, b)
+    convolution reads both tensors directly where it can (bit-identical); what
+    does not fit is joined first, so that torch.cat refuses what it refuses."""
+    if not (torch.is_grad_enabled() and any(t.requires_grad for t in (x, skip, W, b))):
+        x, skip = x.contiguous(), skip.contiguous()
+        if _in_place(x, skip, W):
+            return _conv_two_sources(x, skip, W, b)
+    return conv3x3_relu(torch.cat([_up(x), skip], dim=3), W, b)
+
+
+def _conv_two_sources(x, skip, W, b):
     Bn, H, Wd, C1 = skip.shape
-    x, skip = x.contiguous(), skip.contiguous()
     y = torch.empty((Bn, H, Wd, W.shape[0]), dtype=torch.bfloat16, device=x.device)
     if _rows_f32w(x, 1, skip, W, b, True, y):
         return y

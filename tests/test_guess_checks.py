@@ -62,3 +62,51 @@ def test_conv_row_march_needs_a_plain_bias(lib, b):
     x, W, _ = _layer()
     guess.conv3x3_relu(x, W, b)
     assert not lib.args("glide_conv3x3_rows_f32w")
+
+
+def _sources(h=2, w=32, C0=32, C1=32, dtype=torch.bfloat16, **skip):
+    s = dict(Bn=1, H=2 * h, W=2 * w, C=C1, dtype=dtype) | skip
+    return (torch.zeros(1, h, w, C0, dtype=dtype), torch.zeros(s["Bn"], s["H"], s["W"], s["C"], dtype=s["dtype"]),
+            torch.zeros(32, 9 * (C0 + s["C"])), torch.zeros(32))
+
+
+def test_two_sources_are_read_in_place(lib):
+    guess.conv3x3_up_cat(*_sources())
+    (a,) = lib.args("glide_conv3x3_rows_f32w")
+    assert a[2] == 1 and a[4] == 32
+
+
+@pytest.mark.parametrize("skip", [dict(Bn=2), dict(H=6), dict(W=66), dict(W=128), dict(H=3)])
+def test_two_sources_of_unequal_sizes_are_refused(lib, skip):
+    """As torch.cat refuses them."""
+    with pytest.raises(RuntimeError):
+        guess.conv3x3_up_cat(*_sources(**skip))
+    assert not [n for n, _ in lib.calls if n.startswith("glide_conv3x3") and n != "glide_conv3x3_rows_ok"]
+
+
+@pytest.mark.parametrize("x,skip", [(torch.float32, torch.float32), (torch.bfloat16, torch.float32),
+                                    (torch.float16, torch.bfloat16)])
+def test_two_sources_of_other_types_are_refused(lib, x, skip):
+    a, s, W, b = _sources(dtype=x)
+    with pytest.raises(AssertionError):
+        guess.conv3x3_up_cat(a, s.to(skip), W, b)
+    assert not lib.args("glide_conv3x3_rows_f32w") and not lib.args("glide_conv3x3_cat_bf16")
+
+
+@pytest.mark.parametrize("which", ["x", "skip", "no skip channels", "padded weights"])
+def test_two_sources_that_need_the_joined_tensor(lib, which):
+    """What only the concatenation can serve still runs on it."""
+    x, skip, W, b = _sources(C1=0) if which == "no skip channels" else _sources()
+
+    def shifted(t):   # contiguous, 2 bytes off a 16-byte boundary
+        return torch.zeros(t.numel() + 1, dtype=t.dtype)[1:].view(t.shape)
+
+    if which == "x":
+        x = shifted(x)
+    if which == "skip":
+        skip = shifted(skip)
+    if which == "padded weights":
+        W = torch.zeros(32, W.shape[1] + 8)
+    guess.conv3x3_up_cat(x, skip, W, b)
+    assert not lib.args("glide_conv3x3_cat_bf16") and all(a[3] is None for a in lib.args("glide_conv3x3_rows_f32w"))
+    assert lib.args("glide_conv3x3_rows_f32w") or lib.args("glide_conv3x3_bf16")
