@@ -321,9 +321,24 @@ class Conv1x1(torch.autograd.Function):
         return dx.view(Bn, H, Wd, Cin).to(torch.bfloat16), dW, g.sum(0)
 
 
+def _plain(*ts):
+    """Whether a kernel may read these tensors by address: ordinary contiguous
+    tensors on the current device that nothing differentiates, maps or traces
+    (torch's own operations serve all of that)."""
+    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack():
+        return False
+    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and
+               not torch._C._functorch.is_functorch_wrapped_tensor(t) and
+               t.is_cuda and t.get_device() == torch.cuda.current_device() and
+               t.layout == torch.strided and t.is_contiguous() and t.numel() > 0 and not t.is_neg() and
+               not (torch.is_grad_enabled() and t.requires_grad) and
+               torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in ts)
+
+
 def _pool(x):
     Bn, H, W, Cc = x.shape
-    if not (torch.is_grad_enabled() and x.requires_grad) and Cc % 8 == 0 and x.is_contiguous():
+    if _plain(x) and x.dtype == torch.bfloat16 and Cc % 8 == 0 and H % 2 == 0 and W % 2 == 0 and \
+            x.data_ptr() % 16 == 0:
         y = torch.empty((Bn, H // 2, W // 2, Cc), dtype=torch.bfloat16, device=x.device)
         N.check(_lib().glide_pool2_bf16(x.data_ptr(), y.data_ptr(), Bn, H, W, Cc, N.stream_handle()), "pool")
         return y

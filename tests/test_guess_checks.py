@@ -110,3 +110,21 @@ def test_two_sources_that_need_the_joined_tensor(lib, which):
     guess.conv3x3_up_cat(x, skip, W, b)
     assert not lib.args("glide_conv3x3_cat_bf16") and all(a[3] is None for a in lib.args("glide_conv3x3_rows_f32w"))
     assert lib.args("glide_conv3x3_rows_f32w") or lib.args("glide_conv3x3_bf16")
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+def test_pool_on_the_host_is_torch(lib, dtype):
+    x = torch.arange(1 * 4 * 6 * 8, dtype=torch.float32).view(1, 4, 6, 8).to(dtype)
+    ref = torch.nn.functional.avg_pool2d(x.float().permute(0, 3, 1, 2), 2).permute(0, 2, 3, 1)
+    assert torch.equal(guess._pool(x), ref.to(torch.bfloat16)) and not lib.calls
+
+
+@pytest.mark.parametrize("shape", [(1, 3, 4, 8), (1, 4, 5, 8)])
+def test_pool_refuses_odd_sizes(lib, shape):
+    with pytest.raises(RuntimeError):
+        guess._pool(torch.zeros(shape, dtype=torch.bfloat16))
+    assert not lib.calls
+
+
+def test_pool_of_an_empty_batch(lib):
+    assert guess._pool(torch.zeros(0, 4, 4, 8, dtype=torch.bfloat16)).shape == (0, 2, 2, 8) and not lib.calls
