@@ -419,21 +419,14 @@ class UNet(torch.nn.Module):
 # features, targets and the guess interface
 # ---------------------------------------------------------------------------
 
-def _fusable(fs):
-    """One kernel reads these tensors as they are: CUDA, one dtype and shape, contiguous, not differentiated."""
-    a = fs[0]
-    return a.is_cuda and a.dtype in (torch.float32, torch.float64) and a.numel() > 0 and all(
-        t.dtype == a.dtype and t.device == a.device and t.shape == a.shape and t.is_contiguous() and
-        not (torch.is_grad_enabled() and t.requires_grad) for t in fs)
-
-
 def features(H, bed, beta, B):
     """(…, ny, nx) fields -> (B, ny, nx, IN_CH) BF16 normalised inputs."""
     def b3(t):
         t = torch.as_tensor(t)
         return t.unsqueeze(0) if t.dim() == 2 else t
     fs = [b3(t) for t in (H, bed, beta, B)]
-    if _fusable(fs):
+    if _plain(*fs) and fs[0].dtype in (torch.float32, torch.float64) and \
+            all(t.dtype == fs[0].dtype and t.shape == fs[0].shape for t in fs):
         x = torch.empty(fs[0].shape + (IN_CH,), dtype=torch.bfloat16, device=fs[0].device)
         N.check(_lib().glide_guess_features(N.dtype_code(fs[0].dtype), *(t.data_ptr() for t in fs), x.data_ptr(),
                                             fs[0].numel(), N.stream_handle()), "guess features")
@@ -471,7 +464,8 @@ class GuessModel:
     def predict(self, H, bed, beta, B):
         x = features(H, bed, beta, B)
         pred = self.net(x).float()
-        if pred.is_cuda and pred.dim() == 4 and pred.shape[-1] == 2 and pred.is_contiguous():
+        if _plain(pred) and pred.dim() == 4 and pred.shape[-1] == 2 and pred.data_ptr() % 8 == 0 and \
+                pred.shape[0] <= 65535 and pred.shape[1] <= 8 * 65535 - 8:
             nb, ny, nx, _ = pred.shape
             u = torch.empty((nb, ny, nx + 1), dtype=torch.float64, device=pred.device)
             v = torch.empty((nb, ny + 1, nx), dtype=torch.float64, device=pred.device)
