@@ -240,6 +240,13 @@ def _data_grad(gz, Wb, shape):
     return col2im3(dcol, shape).to(torch.bfloat16)
 
 
+def _aligned(t):
+    """t as the 16-byte loads of the training layer want it: contiguous, copied
+    where it starts off a 16-byte boundary."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
 class Conv3x3ReLU(torch.autograd.Function):
     """y = relu(conv3x3(x, W) + b); x NHWC BF16, W (Cout, 9*Cin) FP32 master.
 
@@ -257,6 +264,7 @@ class Conv3x3ReLU(torch.autograd.Function):
         y = torch.empty((Bn * H * Wd, Cout), dtype=torch.bfloat16, device=x.device)
         ctx.implicit = Cin % 8 == 0 and Cout % 8 == 0 and Cout <= 2048
         if ctx.implicit:
+            x = _aligned(x)
             conv3x3(x, Wb, y, bias=b, relu=relu, out_mode=1)
             ctx.save_for_backward(x, Wb, y)
         else:
@@ -274,8 +282,8 @@ class Conv3x3ReLU(torch.autograd.Function):
         Cout = Wb.shape[0]
         P = Bn * H * Wd
         if ctx.implicit:
-            gy = gy.reshape(P, Cout).to(torch.bfloat16).contiguous()
-            gz, db = _relu_grad(gy, y.reshape(P, Cout), ctx.relu)
+            src, Wb, y = _aligned(src), _aligned(Wb), _aligned(y.reshape(P, Cout))   # hooks may have moved them
+            gz, db = _relu_grad(_aligned(gy.reshape(P, Cout).to(torch.bfloat16)), y, ctx.relu)
             dW = torch.empty((Cout, 9 * Cin), dtype=torch.float32, device=gy.device)
             N.check(_lib().glide_conv3x3_wgrad_bf16(gz.data_ptr(), src.data_ptr(), dW.data_ptr(), Bn, H, Wd, Cin, Cout,
                                                     _err_flag(gy.device).data_ptr(), N.stream_handle()),

@@ -25,3 +25,30 @@ def test_data_gradient_adds_the_taps_in_order(Bn, H, W, Cin, Cout):
     gemm(gz, transpose(Wf.to(torch.bfloat16)), dcol, out_mode=0)
     assert torch.equal(dx, col2im3(dcol, (Bn, H, W, Cin)).to(torch.bfloat16))
     assert int(_err_flag(x.device).item()) == 0
+
+
+@pytest.mark.parametrize("which", ["x", "gy", "y"])
+def test_training_layer_takes_unaligned_slices(which):
+    """Inputs and gradients that start off a 16-byte boundary (a slice of a flat
+    buffer) give the bits of aligned copies."""
+    from glide_b200.guess import Conv3x3ReLU
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(1, 9, 20, 16, generator=g, device="cuda").to(torch.bfloat16)
+    Wf, b = torch.randn(32, 9 * 16, generator=g, device="cuda") * 0.1, torch.randn(32, generator=g, device="cuda")
+    gy = torch.randn(1, 9, 20, 32, generator=g, device="cuda").to(torch.bfloat16)
+
+    def shifted(t):
+        s = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:].view(t.shape)
+        return s.copy_(t)
+
+    def run(x, gy):
+        x, W, bb = x.detach().requires_grad_(), Wf.clone().requires_grad_(), b.clone().requires_grad_()
+        y = Conv3x3ReLU.apply(x, W, bb, True)
+        if which == "y":   # a hook may keep what is saved for backward anywhere
+            with torch.autograd.graph.saved_tensors_hooks(lambda t: t, shifted):
+                y = Conv3x3ReLU.apply(x, W, bb, True)
+        return [y.detach(), *torch.autograd.grad(y, (x, W, bb), gy)]
+
+    ref = run(x, gy)
+    got = run(shifted(x) if which == "x" else x, shifted(gy) if which == "gy" else gy)
+    assert all(torch.equal(p, q) for p, q in zip(got, ref))
