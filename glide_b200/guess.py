@@ -266,7 +266,8 @@ class Conv3x3ReLU(torch.autograd.Function):
         if ctx.implicit:
             x = _aligned(x)
             conv3x3(x, Wb, y, bias=b, relu=relu, out_mode=1)
-            ctx.save_for_backward(x, Wb, y)
+            # an input that is not differentiated is often a buffer which the caller fills again
+            ctx.save_for_backward(x if ctx.needs_input_grad[0] else x.clone(), Wb, y)
         else:
             col = im2col3(x)
             gemm(col, Wb, y, bias=b, relu=relu, out_mode=1)

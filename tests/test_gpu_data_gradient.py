@@ -52,3 +52,17 @@ def test_training_layer_takes_unaligned_slices(which):
     ref = run(x, gy)
     got = run(shifted(x) if which == "x" else x, shifted(gy) if which == "gy" else gy)
     assert all(torch.equal(p, q) for p, q in zip(got, ref))
+
+
+def test_input_buffer_may_be_refilled_before_backward():
+    """The weight gradient belongs to the input of the forward pass, also when
+    the caller has put the next batch into the same buffer since."""
+    from glide_b200.guess import Conv3x3ReLU
+    g = torch.Generator(device="cuda").manual_seed(6)
+    x = torch.randn(2, 8, 16, 8, generator=g, device="cuda").to(torch.bfloat16)
+    b, gy = torch.zeros(16, device="cuda"), torch.ones(2, 8, 16, 16, device="cuda", dtype=torch.bfloat16)
+    Wf = (torch.randn(16, 72, generator=g, device="cuda") * 0.1).requires_grad_()
+    ref, = torch.autograd.grad(Conv3x3ReLU.apply(x, Wf, b, True), Wf, gy)
+    y = Conv3x3ReLU.apply(x, Wf, b, True)
+    x.zero_()
+    assert torch.equal(torch.autograd.grad(y, Wf, gy)[0], ref)
