@@ -22,7 +22,8 @@ SYMBOLS = [
     "glide_error_mask",
     "glide_tile_flags", "glide_vanka_adjoint", "glide_restrict", "glide_prolong", "glide_lincomb", "glide_fill",
     "glide_mask_le", "glide_convert", "glide_norms", "glide_norm_parts", "glide_fascd_vcycle",
-    "glide_adjoint_vcycle", "glide_restrict_parameters", "glide_graph_create", "glide_graph_launch",
+    "glide_adjoint_vcycle", "glide_fascd_vcycle_work", "glide_adjoint_vcycle_work", "glide_restrict_parameters",
+    "glide_graph_create", "glide_graph_create_work", "glide_graph_launch",
     "glide_graph_destroy", "glide_launch_count", "glide_version", "glide_vanka_sweeps_noalloc",
     "glide_noalloc_scratch_bytes", "glide_vanka_sweeps_ex", "glide_vanka_sweeps_work", "glide_vanka_lu", "glide_vanka_linear",
     "glide_misfit", "glide_tikhonov", "glide_loss_parts", "glide_jvp_add",
@@ -54,7 +55,12 @@ class Level(C.Structure):
                 ("scratch", C.c_void_p), ("flags", C.c_void_p), ("any_active", C.c_void_p),
                 ("ls_tmp", C.c_void_p), ("ls_norms", C.c_void_p), ("norm_parts", C.c_void_p),
                 ("lu", C.c_void_p), ("lin_rhs", C.c_void_p), ("lin_rho", C.c_void_p), ("lin_d", C.c_void_p),
-                ("r_raw", C.c_void_p), ("adj_factors", C.c_void_p), ("sweep_work", C.c_void_p)]
+                ("r_raw", C.c_void_p)]
+
+
+class LevelWork(C.Structure):
+    _fields_ = [("adj_factors", C.c_void_p), ("sweep_work", C.c_void_p)]
+
 
 LS_CANDIDATES = 4  # GLIDE_LS_CANDIDATES
 ADJ_FACTORS = 18   # GLIDE_ADJ_FACTORS
@@ -117,6 +123,10 @@ def load():
         "glide_norm_parts": [i64],
         "glide_fascd_vcycle": [C.POINTER(Level), i, i, i, C.POINTER(SolverConfig), vp],
         "glide_adjoint_vcycle": [C.POINTER(Level), i, i, C.POINTER(SolverConfig), vp],
+        "glide_fascd_vcycle_work": [C.POINTER(Level), C.POINTER(LevelWork), i, i, i, C.POINTER(SolverConfig), vp],
+        "glide_adjoint_vcycle_work": [C.POINTER(Level), C.POINTER(LevelWork), i, i, C.POINTER(SolverConfig), vp],
+        "glide_graph_create_work": [C.POINTER(Level), C.POINTER(LevelWork), i, C.POINTER(SolverConfig), i,
+                                    C.POINTER(C.c_void_p)],
         "glide_restrict_parameters": [C.POINTER(Level), i, i, vp],
         "glide_graph_create": [C.POINTER(Level), i, C.POINTER(SolverConfig), i, C.POINTER(C.c_void_p)],
         "glide_graph_launch": [vp, vp],

@@ -356,11 +356,12 @@ LevelView view(GlideLevel* L) {
         if (_e) return _e;      \
     } while (0)
 
-int vanka(GlideLevel* L, int n_iter, const GlideSolverConfig* c, bool local, void* s) {
+int vanka(GlideLevel* L, const GlideLevelWork* W, int n_iter, const GlideSolverConfig* c, bool local, void* s) {
     LevelView w = view(L);
     const double step = c->newton_step > 0.0 ? c->newton_step : GLIDE_REF_NEWTON_STEP;
     return run_sweeps(&L->a, w.u(L->f), w.v(L->f), w.H(L->f), n_iter, c->n_newton, step, c->omega, c->shift,
-                      c->pivoted_lu, local ? L->flags : nullptr, local ? L->any_active : nullptr, L->scratch, true, L->sweep_work, s);
+                      c->pivoted_lu, local ? L->flags : nullptr, local ? L->any_active : nullptr, L->scratch, true,
+                      W ? W->sweep_work : nullptr, s);
 }
 
 int fill_gamma(GlideLevel* L, double val, void* s) {
@@ -408,8 +409,9 @@ int line_search_correction(GlideLevel* L, GlideLevel* C, const GlideSolverConfig
                                                                                    S(s));
 }
 
-int fascd(GlideLevel* lv, int n, int k, bool finest, const GlideSolverConfig* c, void* s) {
+int fascd(GlideLevel* lv, const GlideLevelWork* wk, int n, int k, bool finest, const GlideSolverConfig* c, void* s) {
     GlideLevel* L = &lv[k];
+    const GlideLevelWork* W = wk ? &wk[k] : nullptr;
     LevelView w = view(L);
     const int64_t ncb = w.nc * w.nb, ntb = w.ntot * w.nb;
     if (finest) {
@@ -418,7 +420,7 @@ int fascd(GlideLevel* lv, int n, int k, bool finest, const GlideSolverConfig* c,
     }
     if (k == n - 1) {
         TRY(gamma_from(L, L->chi, s));
-        TRY(vanka(L, c->n_coarse, c, false, s));
+        TRY(vanka(L, W, c->n_coarse, c, false, s));
         return fill_gamma(L, c->thklim, s);
     }
     GlideLevel* C = &lv[k + 1];
@@ -426,7 +428,7 @@ int fascd(GlideLevel* lv, int n, int k, bool finest, const GlideSolverConfig* c,
     // chi_c = maxpool(chi); gamma = w_H + (inject(-chi_c) + chi)   (solver.py:101-108)
     TRY((wc.dt == GLIDE_F32 ? launch_constraint_down<float> : launch_constraint_down<double>)(
         C->chi, (void*)L->a.gamma, L->chi, w.H(L->w), C->a.ny, C->a.nx, C->a.nb, (cudaStream_t)s));
-    TRY(vanka(L, c->n_smooth, c, false, s));
+    TRY(vanka(L, W, c->n_smooth, c, false, s));
     TRY(fill_gamma(L, c->thklim, s));
     // restrict the state, child.w = child.U   (solver.py:113-117)
     TRY(restrict3(L, C, L->U, C->U, s));
@@ -435,7 +437,7 @@ int fascd(GlideLevel* lv, int n, int k, bool finest, const GlideSolverConfig* c,
     TRY(glide_residual(&L->a, w.u(L->f), w.v(L->f), w.H(L->f), w.u(L->r), w.v(L->r), w.H(L->r), s));
     TRY(restrict3(L, C, L->r, C->r, s));
     TRY(glide_residual(&C->a, wc.u(C->r), wc.v(C->r), wc.H(C->r), wc.u(C->f), wc.v(C->f), wc.H(C->f), s));
-    TRY(fascd(lv, n, k + 1, false, c, s));
+    TRY(fascd(lv, wk, n, k + 1, false, c, s));
     // U += P(U_c - w_c): bilinear for u and v, injection for H   (solver.py:131-140)
     TRY(glide_lincomb(wc.dt, C->z, C->U, 1.0, C->w, -1.0, wc.ntot * wc.nb, s));
     if (finest && c->coarse_line_search && L->ls_tmp && L->ls_norms && L->norm_parts) {
@@ -449,12 +451,12 @@ int fascd(GlideLevel* lv, int n, int k, bool finest, const GlideSolverConfig* c,
     }
     // post-smoothing and local error-driven smoothing   (solver.py:143-157)
     TRY(gamma_from(L, L->chi, s));
-    TRY(vanka(L, c->n_smooth, c, false, s));
+    TRY(vanka(L, W, c->n_smooth, c, false, s));
     for (int it = 0; it < c->n_local_outer; it++) {
         TRY(glide_residual(&L->a, w.u(L->f), w.v(L->f), w.H(L->f), w.u(L->r), w.v(L->r), w.H(L->r), s));
         TRY(glide_error_mask(&L->a, w.u(L->r), w.v(L->r), w.H(L->r), c->err_threshold, L->err_mask, L->flags,
                              L->any_active, s));
-        TRY(vanka(L, c->n_local, c, true, s));
+        TRY(vanka(L, W, c->n_local, c, true, s));
     }
     return fill_gamma(L, c->thklim, s);
 }
@@ -476,11 +478,11 @@ int adj_residual(GlideLevel* L, int exact, void* s) {
                      w.u(L->r_adj), w.v(L->r_adj), w.H(L->r_adj), exact, s);
 }
 
-int vanka_adj(GlideLevel* L, int n_iter, double omega, int exact, void* s) {
+int vanka_adj(GlideLevel* L, const GlideLevelWork* W, int n_iter, double omega, int exact, void* s) {
     LevelView w = view(L);
     return glide_vanka_adjoint_sweeps(&L->a, w.u(L->lam), w.v(L->lam), w.H(L->lam), w.u(L->f_adj), w.v(L->f_adj),
                                       w.H(L->f_adj), w.u(L->r_adj), w.v(L->r_adj), w.H(L->r_adj), n_iter, omega, exact,
-                                      L->adj_factors, s);
+                                      W ? W->adj_factors : nullptr, s);
 }
 
 int restrict_params(GlideLevel* L, GlideLevel* C, void* s) {
@@ -494,30 +496,31 @@ int restrict_params(GlideLevel* L, GlideLevel* C, void* s) {
     return 0;
 }
 
-int adjoint(GlideLevel* lv, int n, int k, const GlideSolverConfig* c, void* s) {
+int adjoint(GlideLevel* lv, const GlideLevelWork* wk, int n, int k, const GlideSolverConfig* c, void* s) {
     GlideLevel* L = &lv[k];
+    const GlideLevelWork* W = wk ? &wk[k] : nullptr;
     LevelView w = view(L);
     const int ex = c->exact_adjoint;
     if (k == n - 1) {
         TRY(mask_on(L, c, s));
-        TRY(vanka_adj(L, c->adj_coarse, c->adj_omega, ex, s));
+        TRY(vanka_adj(L, W, c->adj_coarse, c->adj_omega, ex, s));
         return mask_off(L, s);
     }
     GlideLevel* C = &lv[k + 1];
     LevelView wc = view(C);
     TRY(mask_on(L, c, s));
-    TRY(vanka_adj(L, c->adj_smooth, c->adj_omega, ex, s));
+    TRY(vanka_adj(L, W, c->adj_smooth, c->adj_omega, ex, s));
     TRY(mask_off(L, s));
     TRY(adj_residual(L, ex, s));                               // solver.py:187-189 (mask = 0)
     TRY(restrict_params(L, C, s));                             // solver.py:193
     TRY(restrict3(L, C, L->r_adj, C->f_adj, s));               // solver.py:196-199
     TRY(glide_fill(wc.dt, C->lam, 0.0, wc.ntot * wc.nb, s));   // solver.py:200
-    TRY(adjoint(lv, n, k + 1, c, s));
+    TRY(adjoint(lv, wk, n, k + 1, c, s));
     TRY(glide_prolong(w.dt, 0, 1, 1, wc.u(C->lam), w.u(L->lam), C->a.ny, C->a.nx, C->a.nb, s));
     TRY(glide_prolong(w.dt, 1, 1, 1, wc.v(C->lam), w.v(L->lam), C->a.ny, C->a.nx, C->a.nb, s));
     TRY(glide_prolong(w.dt, 2, 1, 1, wc.H(C->lam), w.H(L->lam), C->a.ny, C->a.nx, C->a.nb, s));
     TRY(mask_on(L, c, s));
-    TRY(vanka_adj(L, c->adj_smooth, c->adj_omega, ex, s));
+    TRY(vanka_adj(L, W, c->adj_smooth, c->adj_omega, ex, s));
     return mask_off(L, s);
 }
 
@@ -599,19 +602,29 @@ struct GraphHandle {
 
 extern "C" {
 
-int glide_fascd_vcycle(GlideLevel* levels, int n_levels, int k0, int finest, const GlideSolverConfig* cfg,
-                       void* stream) {
+int glide_fascd_vcycle_work(GlideLevel* levels, const GlideLevelWork* work, int n_levels, int k0, int finest,
+                            const GlideSolverConfig* cfg, void* stream) {
     int e = check_levels(levels, n_levels);
     if (e) return e;
     if (!cfg || k0 < 0 || k0 >= n_levels) return GLIDE_E_SHAPE;
-    return fascd(levels, n_levels, k0, finest != 0, cfg, stream);
+    return fascd(levels, work, n_levels, k0, finest != 0, cfg, stream);
+}
+
+int glide_fascd_vcycle(GlideLevel* levels, int n_levels, int k0, int finest, const GlideSolverConfig* cfg,
+                       void* stream) {
+    return glide_fascd_vcycle_work(levels, nullptr, n_levels, k0, finest, cfg, stream);
+}
+
+int glide_adjoint_vcycle_work(GlideLevel* levels, const GlideLevelWork* work, int n_levels, int k0,
+                              const GlideSolverConfig* cfg, void* stream) {
+    int e = check_levels(levels, n_levels);
+    if (e) return e;
+    if (!cfg || k0 < 0 || k0 >= n_levels) return GLIDE_E_SHAPE;
+    return adjoint(levels, work, n_levels, k0, cfg, stream);
 }
 
 int glide_adjoint_vcycle(GlideLevel* levels, int n_levels, int k0, const GlideSolverConfig* cfg, void* stream) {
-    int e = check_levels(levels, n_levels);
-    if (e) return e;
-    if (!cfg || k0 < 0 || k0 >= n_levels) return GLIDE_E_SHAPE;
-    return adjoint(levels, n_levels, k0, cfg, stream);
+    return glide_adjoint_vcycle_work(levels, nullptr, n_levels, k0, cfg, stream);
 }
 
 int glide_restrict_parameters(GlideLevel* levels, int n_levels, int k0, void* stream) {
@@ -638,7 +651,8 @@ int glide_linear_vcycle(GlideLevel* levels, int n_levels, const GlideSolverConfi
     return lin_vcycle(levels, n_levels, 0, cfg, stream);
 }
 
-int glide_graph_create(GlideLevel* levels, int n_levels, const GlideSolverConfig* cfg, int kind, void** graph_out) {
+int glide_graph_create_work(GlideLevel* levels, const GlideLevelWork* work, int n_levels, const GlideSolverConfig* cfg,
+                            int kind, void** graph_out) {
     int e = check_levels(levels, n_levels);
     if (e) return e;
     if (!cfg || !graph_out) return GLIDE_E_NULL;
@@ -650,8 +664,8 @@ int glide_graph_create(GlideLevel* levels, int n_levels, const GlideSolverConfig
     int rc = 0;
     if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) rc = GLIDE_E_GRAPH;
     if (!rc) {
-        rc = kind == 0   ? fascd(levels, n_levels, 0, true, cfg, s)
-             : kind == 1 ? adjoint(levels, n_levels, 0, cfg, s)
+        rc = kind == 0   ? fascd(levels, work, n_levels, 0, true, cfg, s)
+             : kind == 1 ? adjoint(levels, work, n_levels, 0, cfg, s)
                          : lin_vcycle(levels, n_levels, 0, cfg, s);
         cudaError_t ce = cudaStreamEndCapture(s, &h->g);
         if (!rc && ce != cudaSuccess) rc = GLIDE_E_GRAPH;
@@ -664,6 +678,10 @@ int glide_graph_create(GlideLevel* levels, int n_levels, const GlideSolverConfig
     }
     *graph_out = h;
     return 0;
+}
+
+int glide_graph_create(GlideLevel* levels, int n_levels, const GlideSolverConfig* cfg, int kind, void** graph_out) {
+    return glide_graph_create_work(levels, nullptr, n_levels, cfg, kind, graph_out);
 }
 
 int glide_graph_launch(void* graph, void* stream) {

@@ -121,11 +121,11 @@ class Grid:
                 self._ls_norms = torch.zeros(3 * N.LS_CANDIDATES + 1, dtype=torch.float64, device=self.device)
             L.ls_tmp, L.ls_norms = self._ls_tmp.data_ptr(), self._ls_norms.data_ptr()
             L.norm_parts = self._norm_parts.data_ptr()
-        if self._adj_factors is not None:
-            L.adj_factors = self._adj_factors.data_ptr()
-        if self._sweep_work is not None:
-            L.sweep_work = self._sweep_work.data_ptr()
         return L
+
+    def native_work(self) -> N.LevelWork:
+        """The smoothers' room that this level has so far."""
+        return N.LevelWork(*(None if t is None else t.data_ptr() for t in (self._adj_factors, self._sweep_work)))
 
     def adjoint_factors(self):
         """Buffer of the adjoint smoother's local systems, made on first use

@@ -345,7 +345,8 @@ class AdjointKrylov:
         else:
             gc.f_adj.copy_(self.pin)
         gc.Lambda.zero_()
-        N.check(lib.glide_adjoint_vcycle(ph._native, ph._nlev, 0, C.byref(self._cfg), s), "adjoint_vcycle")
+        N.check(lib.glide_adjoint_vcycle_work(ph._native, ph._work, ph._nlev, 0, C.byref(self._cfg), s),
+                "adjoint_vcycle")
         if self.mixed:
             N.check(lib.glide_convert(N.F64, self.pout.data_ptr(), gc.Lambda.data_ptr(), self.n, 1, s), "convert")
         else:

@@ -36,7 +36,7 @@ import torch
 
 from . import _native as N
 from .grid import Grid
-from .solver import REFERENCE, SolverSettings, native_levels, restrict_parameters_to_hierarchy
+from .solver import REFERENCE, SolverSettings, native_levels, native_work, restrict_parameters_to_hierarchy
 
 RHO_ICE = 917.0
 G = 9.81
@@ -233,6 +233,7 @@ class IcePhysics:
             self.grid32 = None
             self._solve_grids = gs
         self._native, self._nlev = native_levels(self._solve_grids[0])
+        self._work = native_work(self._solve_grids[0])
 
     def _shape(self):
         return (self.ny, self.nx) if self.batch == 1 else (self.batch, self.ny, self.nx)
@@ -290,14 +291,15 @@ class IcePhysics:
             g.dt = float(dt)
         # dt is passed to the kernels by value: rebuild the level descriptors
         self._native, self._nlev = native_levels(self._solve_grids[0])
+        self._work = native_work(self._solve_grids[0])
 
     def _cfg(self):
         return self.settings.native(self.thklim)
 
     def _vcycle_native(self):
         cfg = self._cfg()
-        N.check(self.kernels.glide_fascd_vcycle(self._native, self._nlev, 0, 1, C.byref(cfg), N.stream_handle()),
-                "fascd_vcycle")
+        N.check(self.kernels.glide_fascd_vcycle_work(self._native, self._work, self._nlev, 0, 1, C.byref(cfg),
+                                                     N.stream_handle()), "fascd_vcycle")
 
     def _dc_step(self):
         """Mixed precision: one FP32 FASCD cycle as the correction solver of the
@@ -782,9 +784,9 @@ class IcePhysics:
             g.f_adj_H.copy_(-_as_tensor(dL_dH, g.dtype, self.device))
             g.Lambda.zero_()
             cfg = st.native(self.thklim)
-            for level, lg in zip(self._native, self._solve_grids):
-                f = lg.adjoint_factors()
-                level.adj_factors = None if f is None else f.data_ptr()
+            for lg in self._solve_grids:
+                lg.adjoint_factors()
+            self._work = native_work(self._solve_grids[0])
             if tol is not None and self.adjoint_krylov > 0:
                 from .newton import AdjointKrylov
                 if self._ak is None or self._ak.m != self.adjoint_krylov:
@@ -819,8 +821,8 @@ class IcePhysics:
                 if self.precision == "mixed":
                     self._adjoint_dc_step(cfg)
                 else:
-                    N.check(self.kernels.glide_adjoint_vcycle(self._native, self._nlev, 0, C.byref(cfg),
-                                                              N.stream_handle()), "adjoint_vcycle")
+                    N.check(self.kernels.glide_adjoint_vcycle_work(self._native, self._work, self._nlev, 0,
+                                                                   C.byref(cfg), N.stream_handle()), "adjoint_vcycle")
                 info["vcycles"] = k + 1
                 if tol is None:
                     continue
@@ -881,7 +883,8 @@ class IcePhysics:
         N.check(lib.glide_convert(N.F32, g32.U.data_ptr(), g64.U.data_ptr(), n, 0, s), "convert")
         N.check(lib.glide_convert(N.F32, g32.f_adj.data_ptr(), g64.r_adj.data_ptr(), n, 0, s), "convert")
         g32.Lambda.zero_()
-        N.check(lib.glide_adjoint_vcycle(self._native, self._nlev, 0, C.byref(cfg), s), "adjoint_vcycle")
+        N.check(lib.glide_adjoint_vcycle_work(self._native, self._work, self._nlev, 0, C.byref(cfg), s),
+                "adjoint_vcycle")
         N.check(lib.glide_convert(N.F64, g64.Lambda.data_ptr(), g32.Lambda.data_ptr(), n, 1, s), "convert")
 
     def reset_solution(self):

@@ -80,6 +80,12 @@ def native_levels(grid):
     return arr, len(gs)
 
 
+def native_work(grid):
+    """The smoothers' room of every level, for the ``_work`` entry points."""
+    gs = hierarchy(grid)
+    return (N.LevelWork * len(gs))(*(g.native_work() for g in gs))
+
+
 def restrict_parameters(grid):
     """bed, B, beta, H_prev, smb to the child (glide/solver.py:53-61)."""
     if grid.child is None:
@@ -103,12 +109,13 @@ def fascd_vcycle(grid, thklim, finest=False, settings: SolverSettings = REFERENC
     """One FASCD V-cycle (glide/solver.py:71-157)."""
     arr, n = native_levels(grid)
     cfg = settings.native(thklim)
-    N.check(N.load().glide_fascd_vcycle(arr, n, 0, int(bool(finest)), C.byref(cfg), N.stream_handle()),
-            "fascd_vcycle")
+    N.check(N.load().glide_fascd_vcycle_work(arr, native_work(grid), n, 0, int(bool(finest)), C.byref(cfg),
+                                             N.stream_handle()), "fascd_vcycle")
 
 
 def adjoint_vcycle(grid, settings: SolverSettings = REFERENCE, thklim=0.1):
     """One adjoint V-cycle (glide/solver.py:160-220)."""
     arr, n = native_levels(grid)
     cfg = settings.native(thklim)
-    N.check(N.load().glide_adjoint_vcycle(arr, n, 0, C.byref(cfg), N.stream_handle()), "adjoint_vcycle")
+    N.check(N.load().glide_adjoint_vcycle_work(arr, native_work(grid), n, 0, C.byref(cfg), N.stream_handle()),
+            "adjoint_vcycle")

@@ -207,11 +207,17 @@ typedef struct GlideLevel {
     void* lin_rho;          /* like U: linear residual g + J d */
     void* lin_d;            /* like U: correction d */
     void* r_raw;            /* like U: residual at the linearisation state (active-set test) */
-    /* adjoint smoother (may be null: the local matrices are then formed for every colour) */
-    void* adj_factors;      /* GLIDE_ADJ_FACTORS * nc * nb */
-    /* forward smoother (may be null: a sweep is then two kernels) */
-    void* sweep_work;       /* GLIDE_SWEEP_WORK(ny, nx, nb) */
 } GlideLevel;
+
+/* Room that the smoothers of one level can use; an array of them, one per
+ * level, beside the levels (GlideLevel keeps the layout that its callers were
+ * built with). */
+typedef struct GlideLevelWork {
+    void* adj_factors;      /* GLIDE_ADJ_FACTORS * nc * nb; null: the adjoint smoother forms its local
+                               matrices for every colour */
+    void* sweep_work;       /* GLIDE_SWEEP_WORK(ny, nx, nb); null: a forward sweep of the tile form is
+                               two kernels */
+} GlideLevelWork;
 
 /* Step sizes tried by the coarse-correction line search, best first on ties. */
 #define GLIDE_LS_CANDIDATES 4
@@ -245,6 +251,11 @@ typedef struct GlideSolverConfig {
 int glide_fascd_vcycle(GlideLevel* levels, int n_levels, int k0, int finest, const GlideSolverConfig* cfg,
                        void* stream);
 int glide_adjoint_vcycle(GlideLevel* levels, int n_levels, int k0, const GlideSolverConfig* cfg, void* stream);
+/* The same cycles with work (n_levels entries, or null); results as without. */
+int glide_fascd_vcycle_work(GlideLevel* levels, const GlideLevelWork* work, int n_levels, int k0, int finest,
+                            const GlideSolverConfig* cfg, void* stream);
+int glide_adjoint_vcycle_work(GlideLevel* levels, const GlideLevelWork* work, int n_levels, int k0,
+                              const GlideSolverConfig* cfg, void* stream);
 /* restrict bed, B, beta, H_prev, smb from every level to its child (glide/solver.py:53-68) */
 int glide_restrict_parameters(GlideLevel* levels, int n_levels, int k0, void* stream);
 
@@ -290,6 +301,8 @@ int glide_combine(int dtype, int64_t n, int k, const void* V, int64_t ldv, const
  * 2 = linear V-cycle (glide_linear_vcycle).
  * The graph keeps the device pointers it was built with. */
 int glide_graph_create(GlideLevel* levels, int n_levels, const GlideSolverConfig* cfg, int kind, void** graph_out);
+int glide_graph_create_work(GlideLevel* levels, const GlideLevelWork* work, int n_levels, const GlideSolverConfig* cfg,
+                            int kind, void** graph_out);
 int glide_graph_launch(void* graph, void* stream);
 int glide_graph_destroy(void* graph);
 
