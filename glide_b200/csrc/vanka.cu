@@ -654,7 +654,8 @@ static inline dim3 cell_grid(const Geo& g) { return dim3((g.nx + VX - 1) / VX, (
 static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (g.ny + 1 + 7) / 8, g.nb); }
 
 // Which form of the cell kernel: the march (vanka_march.cu) in FP64, and in
-// FP32 for sweeps of their own from 2^16 cells on.  The FP32 FAS cycle keeps
+// FP32 for sweeps of their own from 2^16 cells of a problem on (whatever its
+// batch: the two forms round differently).  The FP32 FAS cycle keeps
 // the tile form at every size although the march is faster there too (512^2,
 // 10 Newton steps: 45 us per sweep against 38): the two round differently, and
 // a few FP32 cycles amplify a rounding 1e3 to 1e4 times, so a step's answer
@@ -666,7 +667,7 @@ static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (
 // 1024^2 408 / 348, of 2 steps 32^2 7.7 / 8.1, 1024^2 168 / 141.
 template <typename T> static inline bool use_march(const Geo& g, int pivot, bool cycle) {
     if (pivot) return false;
-    return sizeof(T) == 8 || (!cycle && g.nc() * g.nb >= (int64_t(1) << 16));
+    return sizeof(T) == 8 || (!cycle && g.nc() >= (int64_t(1) << 16));
 }
 // The update kernel of a sweep is chained while it fits the chip about once.
 static inline bool apply_chained(const Geo& g) { return blocks_of(face_grid(g)) <= 592; }
