@@ -541,7 +541,7 @@ __global__ void __launch_bounds__(VX * VY, 4) vanka_cells_kernel(
         T J[25], rr[5], x[5];
         assemble_fast<T>(F, ul, ur, vt, vb, Hc, fu_l, fu_r, fv_t, fv_b, fH, thk, dti, p, J, rr);
         J[0] -= shift; J[6] -= shift; J[12] -= shift; J[18] -= shift; J[24] += shift;  // vanka.cu:406-410
-        if (sizeof(T) == 8 || pivot)   // FP64 comes here for pivoted solves only
+        if (pivot)
             lu5_solve_pivot(J, rr, x);
         else
             lu5_solve_fast(J, rr, x);
@@ -653,21 +653,36 @@ __global__ void tile_flags_kernel(int* __restrict__ flags, int* __restrict__ any
 static inline dim3 cell_grid(const Geo& g) { return dim3((g.nx + VX - 1) / VX, (g.ny + VY - 1) / VY, g.nb); }
 static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (g.ny + 1 + 7) / 8, g.nb); }
 
-// Which form of the cell kernel: the march (vanka_march.cu) in FP64, and in
-// FP32 for sweeps of their own from 2^16 cells of a problem on (whatever its
-// batch: the two forms round differently).  The FP32 FAS cycle keeps
-// the tile form at every size although the march is faster there too (512^2,
-// 10 Newton steps: 45 us per sweep against 38): the two round differently, and
-// a few FP32 cycles amplify a rounding 1e3 to 1e4 times, so a step's answer
-// would move by up to 3e-4 between the forms.  Pivoted local solves exist in the
-// tile form only.  Microseconds per sweep, tile (one kernel per sweep) / march:
-// FP32 of 10 steps 256^2 14.1 / 13.4, 300^2 20.7 / 17.6, 1024^2 172 / 137, of 2
-// steps 256^2 6.4 / 7.8, 362^2 11.2 / 10.7, 1024^2 74.4 / 50.8; FP64, tile with
-// two kernels per sweep, of 10 steps 32^2 16.5 / 13.3, 256^2 33.9 / 26.2,
-// 1024^2 408 / 348, of 2 steps 32^2 7.7 / 8.1, 1024^2 168 / 141.
-template <typename T> static inline bool use_march(const Geo& g, int pivot, bool cycle) {
+// Which form of the cell kernel: the tile, or the march (vanka_march.cu), whose
+// cells cost less and whose warps need more of them: it pays from a size on that
+// falls with the number of Newton steps and rises when only some rows are
+// active.  The problem's own size decides, whatever its batch, because the two
+// round differently.  So the FP32 FAS cycle keeps the tile at every size: a few
+// FP32 cycles amplify a rounding 1e3 to 1e4 times, and a step's answer would move
+// by up to 3e-4 between the forms.  Pivoted local solves exist in the tile only.
+//
+// Microseconds per sweep, tile (one kernel per sweep) / march, at both sides of
+// the lines.  FP32, 10 steps: 181^2 13.9 / 13.1, 256^2 14.6 / 15.0, 300^2
+// 21.3 / 20.1, 512^2 45.4 / 43.3, 1024^2 172 / 142; 7 steps: 420^2 26.2 / 27.4,
+// 600^2 48.9 / 47.1; 2 steps: 512^2 19.1 / 21.0, 600^2 25.7 / 27.3, 724^2
+// 36.2 / 31.4, 1024^2 75.1 / 55.7.  FP64, 10 steps: 16^2 15.9 / 14.1, 256^2
+// 33.7 / 29.3, 1024^2 410 / 353; 2 steps: 32^2 7.7 / 9.1, 256^2 13.9 / 15.0, 300^2
+// 21.8 / 18.1.  Gated, a quarter (2 %) of the rows active, FP32, 2 steps: 512^2
+// 13.6 / 20.1 (11.1 / 15.6), 724^2 24.0 / 27.9 (18.6 / 20.2), 1024^2 44.8 / 36.3
+// (33.3 / 27.3); FP64, 2 steps: 512^2 20.8 / 28.3 (15.1 / 19.9), 724^2 40.5 / 42.3
+// (23.9 / 24.3), 850^2 55.1 / 47.6 (30.5 / 26.1); FP64, 10 steps: 450^2
+// 38.1 / 34.2 (24.0 / 34.1), 512^2 39.4 / 53.2 (27.4 / 34.0), 600^2 63.5 / 54.6
+// (31.9 / 36.2), 724^2 77.4 / 79.2 (35.9 / 38.6), 850^2 106 / 89 (42.5 / 40.4).
+template <typename T>
+static inline bool use_march(const Geo& g, int n_newton, bool gated, int pivot, bool cycle) {
     if (pivot) return false;
-    return sizeof(T) == 8 || (!cycle && g.nc() >= (int64_t(1) << 16));
+    const int64_t nc = g.nc(), k = int64_t(1) << 16;
+    if constexpr (sizeof(T) == 8) {
+        const bool few = n_newton <= 2;
+        return gated ? nc >= 8 * k || (!few && nc < 4 * k) : !few || nc > k;
+    }
+    if (cycle) return false;
+    return nc >= (gated ? 8 * k : n_newton < 8 ? 6 * k : k);
 }
 // The update kernel of a sweep is chained while it fits the chip about once.
 static inline bool apply_chained(const Geo& g) { return blocks_of(face_grid(g)) <= 592; }
@@ -683,7 +698,7 @@ template <typename T>
 static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton,
                       double shift, double step, int pivot, const int* flags, const int* any_active, void* scratch,
                       const Geo& g, bool cycle, const SweepState<T>& q, cudaStream_t s) {
-    if (use_march<T>(g, pivot, cycle)) {
+    if (use_march<T>(g, n_newton, flags, pivot, cycle)) {
         run_march<T>(a, f_u, f_v, f_H, n_newton, shift, step, flags, any_active, scratch, s);
         return;
     }
@@ -710,7 +725,7 @@ int launch_vanka_sweeps(const GlideLevelArgs* a, const void* f_u, const void* f_
                         int n_newton, double omega, double shift, const int* flags, const int* any_active,
                         void* scratch, cudaStream_t s, double newton_step, int pivot, bool cycle, void* work) {
     Geo g{a->ny, a->nx, a->nb};
-    const bool chained = apply_chained(g), fused = work && !use_march<T>(g, pivot, cycle);
+    const bool chained = apply_chained(g), fused = work && !use_march<T>(g, n_newton, flags, pivot, cycle);
     SweepState<T> q = state_of<T>(a);
     q.omega = T(omega);
     T* const first[3] = {(T*)a->u, (T*)a->v, (T*)a->H};
