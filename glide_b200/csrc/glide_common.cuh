@@ -68,6 +68,12 @@ inline void launch_chained(void (*kernel)(KA...), dim3 grid, dim3 block, cudaStr
     }
     cudaLaunchKernelEx(&c, kernel, KA(args)...);
 }
+// A launch has at most 65,535 rows of blocks: taller grids go in pieces, each
+// told the block row it starts at.
+template <typename F> inline void by_block_rows(dim3 grid, F&& launch) {
+    for (unsigned y0 = 0; y0 < grid.y; y0 += 65535u)
+        launch(dim3(grid.x, grid.y - y0 < 65535u ? grid.y - y0 : 65535u, grid.z), int(y0));
+}
 static inline int64_t blocks_of(dim3 g) { return int64_t(g.x) * g.y * g.z; }
 
 // --------------------------------------------------------------------------

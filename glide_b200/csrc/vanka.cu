@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(VX * VY, 4) vanka_cells_kernel(
     T* __restrict__ scratch, SweepState<T> q, const T* __restrict__ f_u, const T* __restrict__ f_v,
     const T* __restrict__ f_H, const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
     const T* __restrict__ gamma, const int* __restrict__ flags, const int* __restrict__ any_active, int n_newton,
-    T shift, T step, int pivot, Geo g, P p) {
+    T shift, T step, int pivot, int y0, Geo g, P p) {
     __shared__ Window<T> W;
     const int zero = chain_enter<true>();
     const int ny = g.ny, nx = g.nx;
@@ -502,7 +502,7 @@ __global__ void __launch_bounds__(VX * VY, 4) vanka_cells_kernel(
     const int64_t nc = g.nc();
     scratch += bz * 5 * nc;
     if (LOCAL) flags += bz * int64_t(ny / REF_STRIDE + 1) * (nx / REF_STRIDE + 1);
-    const int i0 = blockIdx.y * VY + zero, j0 = blockIdx.x * VX;
+    const int i0 = (blockIdx.y + y0) * VY + zero, j0 = blockIdx.x * VX;
     const int r = threadIdx.x / VX, c = threadIdx.x % VX;
     const int i = i0 + r, j = j0 + c;
     const bool has = q.d;
@@ -705,9 +705,12 @@ static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v,
     with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
         using P = decltype(p);
         auto run = [&](auto kernel) {
-            launch_chained<true>(kernel, cell_grid(g), VX * VY, s, (T*)scratch, q, (const T*)f_u, (const T*)f_v,
-                                 (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta,
-                                 (const T*)a->gamma, flags, any_active, n_newton, T(shift), T(step), pivot, g, p);
+            by_block_rows(cell_grid(g), [&](dim3 grid, int y0) {
+                launch_chained<true>(kernel, grid, VX * VY, s, (T*)scratch, q, (const T*)f_u, (const T*)f_v,
+                                     (const T*)f_H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta,
+                                     (const T*)a->gamma, flags, any_active, n_newton, T(shift), T(step), pivot, y0, g,
+                                     p);
+            });
         };
         flags ? run(vanka_cells_kernel<T, true, P>) : run(vanka_cells_kernel<T, false, P>);
     });

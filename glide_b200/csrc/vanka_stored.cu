@@ -204,9 +204,9 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
 template <typename T, bool CHAIN>
 __global__ void adjoint_color_kernel(const T* __restrict__ f, T* __restrict__ l_u, T* __restrict__ l_v,
                                      T* __restrict__ l_H, const T* __restrict__ ra_u, const T* __restrict__ ra_v,
-                                     const T* __restrict__ ra_H, int color, T omega, Geo g) {
+                                     const T* __restrict__ ra_H, int color, T omega, int y0, Geo g) {
     const int ny = g.ny, nx = g.nx, b = blockIdx.z;
-    const int i = blockIdx.y * blockDim.y + threadIdx.y + chain_enter<CHAIN>();
+    const int i = (blockIdx.y + y0) * blockDim.y + threadIdx.y + chain_enter<CHAIN>();
     const int j = 2 * (blockIdx.x * blockDim.x + threadIdx.x) + ((i + color) & 1);
     if (i >= ny || j >= nx) return;
     const int64_t nc = g.nc();
@@ -373,8 +373,10 @@ int launch_adjoint_color(const GlideLevelArgs* a, const void* factors, void* l_u
     const dim3 blk(32, 4), grd(((g.nx + 1) / 2 + 31) / 32, (g.ny + 3) / 4, g.nb);
     auto go = [&](auto chain) {
         constexpr bool CHAIN = decltype(chain)::value;
-        launch_chained<CHAIN>(adjoint_color_kernel<T, CHAIN>, grd, blk, s, (const T*)factors, (T*)l_u, (T*)l_v,
-                              (T*)l_H, (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, color, T(omega), g);
+        by_block_rows(grd, [&](dim3 grid, int y0) {
+            launch_chained<CHAIN>(adjoint_color_kernel<T, CHAIN>, grid, blk, s, (const T*)factors, (T*)l_u, (T*)l_v,
+                                  (T*)l_H, (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, color, T(omega), y0, g);
+        });
     };
     blocks_of(grd) <= 592 ? go(std::true_type{}) : go(std::false_type{});
     return (int)cudaGetLastError();
