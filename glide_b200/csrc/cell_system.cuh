@@ -88,15 +88,23 @@ template <typename T> struct ArrowInv {
 // sign, and the mass row gives the thickness.  Four reciprocals (two of them
 // independent) instead of the five successive pivots of an unstructured 5x5
 // elimination, and no subtraction of nearly equal pivots; a row with D = 0 is
-// fine as long as its pair's sum is not 0.
-template <typename T>
+// fine as long as its pair's sum is not 0.  IEEE: correctly rounded reciprocals
+// also in FP32 (the adjoint, whose systems are not iterated on), else M<T>::rcp
+// as the forward Newton steps and the linear factors take it.
+template <bool IEEE, typename T> __device__ __forceinline__ T reciprocal(T x) {
+    if constexpr (IEEE)
+        return T(1) / x;
+    else
+        return M<T>::rcp(x);
+}
+template <bool IEEE = false, typename T>
 __device__ __forceinline__ void arrow_factor(const Arrow<T>& s, ArrowInv<T>& q) {
     const Two<T> ds = s.D1 + s.D2;
-    q.i = two(M<T>::rcp(ds.x), M<T>::rcp(ds.y));
+    q.i = two(reciprocal<IEEE>(ds.x), reciprocal<IEEE>(ds.y));
     q.w1 = s.D1 * q.i;
     q.w2 = s.D2 * q.i;
     const Two<T> xy = s.D1 * q.w2;
-    const T id = M<T>::rcp(xy.x * xy.y + s.p2 * (T(3) * s.p2 + T(2) * (xy.x + xy.y)));
+    const T id = reciprocal<IEEE>(xy.x * xy.y + s.p2 * (T(3) * s.p2 + T(2) * (xy.x + xy.y)));
     q.b11 = (xy.x + T(2) * s.p2) * id;
     q.b22 = (xy.y + T(2) * s.p2) * id;
     q.b12 = s.p2 * id;
@@ -107,7 +115,7 @@ __device__ __forceinline__ void arrow_factor(const Arrow<T>& s, ArrowInv<T>& q) 
     q.k = fma2(s.e2, both(T(-1)), s.e1) * q.i;
     q.e = fma2(s.e1, q.w2, s.e2 * q.w1);
     const Two<T> t = fma2(q.k, q.Cd, q.e * two(q.ag, q.bg));
-    q.ih = M<T>::rcp(s.j4 + (t.x + t.y));
+    q.ih = reciprocal<IEEE>(s.j4 + (t.x + t.y));
 }
 
 template <typename T>

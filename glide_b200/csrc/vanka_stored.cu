@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
                     for (int k = 0; k < LU_N; k++) out[k * nc] = o[k];
                 } else {
                     ArrowInv<T> q;
-                    arrow_factor(transposed(s), q);
+                    arrow_factor<true>(transposed(s), q);
                     if constexpr (MODE == STORE_ADJOINT) {
                         const T o[ADJ_N] = {q.i.x, q.i.y, q.w1.x, q.w1.y, q.w2.x, q.w2.y, q.Cd.x, q.Cd.y, q.k.x,
                                             q.k.y, q.e.x, q.e.y, q.b11, q.b12, q.b22, q.ag, q.bg, q.ih};
