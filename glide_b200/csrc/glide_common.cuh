@@ -360,9 +360,12 @@ __device__ __forceinline__ EtaOut<T> cell_eta(const EtaIn<T>& a, T Bc, int i, in
     o.eta = T(0.5) * Bc * glen_pow(o.eII, p);
     return o;
 }
-// Tangent of eta for a tangent (du, dv) of the same 12 faces.
+// Tangent of eta for a tangent (du, dv) of the same 12 faces.  FP64 takes it from
+// eta (a quarter of the error of a second power, which costs as much as the rest
+// of the row); FP32's power is two hardware approximations, and one of its own
+// keeps its error apart from eta's.
 template <typename T>
-__device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>& d, int i, int j, int ny, int nx,
+__device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>& d, T Bc, int i, int j, int ny, int nx,
                                               const Phys<T>& p) {
     T dxi = p.dxi;
     T dux = (d.ur - d.ul) * dxi;
@@ -378,6 +381,7 @@ __device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>
     T de2sum = T(0.25) * (T(2) * e.exy[0] * de0 + T(2) * e.exy[1] * de1 + T(2) * e.exy[2] * de2 +
                           T(2) * e.exy[3] * de3);
     T deII = T(2) * e.ux * dux + T(2) * e.vy * dvy + (e.ux * dvy + e.vy * dux) + de2sum;
+    if constexpr (sizeof(T) == 4) return T(0.5) * Bc * (p.glen_exp * M<T>::pow(e.eII, p.glen_exp - T(1)) * deII);
     return p.glen_exp * e.eta * (deII * M<T>::rcp(e.eII));   // eta ~ eII^glen_exp
 }
 

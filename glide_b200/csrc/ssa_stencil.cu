@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? GLIDE_JS_MINB32 : GLIDE_
             da.v_lt = dvL1s; da.v_rt = dvR1s; da.v_lb = dvL2s; da.v_rb = dvR2s;
             const int ie = clampi(i + 1, 0, ny - 1);
             const EtaOut<T> e = cell_eta(a, Bp, ie, jcc, ny, nx, p);
-            const T deta = cell_eta_tangent<T>(e, da, ie, jcc, ny, nx, p);
+            const T deta = cell_eta_tangent<T>(e, da, Bp, ie, jcc, ny, nx, p);
             etaHp = e.eta * Hp;
             detaHp = deta * Hp + e.eta * dHp;
         }
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(VS_NT, sizeof(T) == 4 ? GLIDE_VS_MINB32 : GLID
             da.v_lt = lvL1s; da.v_rt = lvR1s; da.v_lb = lvL2s; da.v_rb = lvR2s;
             const int ie = clampi(i + 1, 0, ny - 1);
             const EtaOut<T> e = cell_eta(a, Bp, ie, jcc, ny, nx, p);
-            const T deta = cell_eta_tangent<T>(e, da, ie, jcc, ny, nx, p);
+            const T deta = cell_eta_tangent<T>(e, da, Bp, ie, jcc, ny, nx, p);
             etaP = e.eta;
             etaHp = e.eta * Hp;
             detaHp = deta * Hp;
