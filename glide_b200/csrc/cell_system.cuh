@@ -88,7 +88,9 @@ template <typename T> struct ArrowInv {
 // sign, and the mass row gives the thickness.  Four reciprocals (two of them
 // independent) instead of the five successive pivots of an unstructured 5x5
 // elimination, and no subtraction of nearly equal pivots; a row with D = 0 is
-// fine as long as its pair's sum is not 0.  IEEE: correctly rounded reciprocals
+// fine as long as its pair's sum is not 0.  The determinant is taken in units of
+// the two pair sums: a product of two drags leaves FP32's range from 2e19 on,
+// their quotients do not.  IEEE: correctly rounded reciprocals
 // also in FP32 (the adjoint, whose systems are not iterated on), else M<T>::rcp
 // as the forward Newton steps and the linear factors take it.
 template <bool IEEE, typename T> __device__ __forceinline__ T reciprocal(T x) {
@@ -103,19 +105,20 @@ __device__ __forceinline__ void arrow_factor(const Arrow<T>& s, ArrowInv<T>& q) 
     q.i = two(reciprocal<IEEE>(ds.x), reciprocal<IEEE>(ds.y));
     q.w1 = s.D1 * q.i;
     q.w2 = s.D2 * q.i;
-    const Two<T> xy = s.D1 * q.w2;
-    const T id = reciprocal<IEEE>(xy.x * xy.y + s.p2 * (T(3) * s.p2 + T(2) * (xy.x + xy.y)));
-    q.b11 = (xy.x + T(2) * s.p2) * id;
-    q.b22 = (xy.y + T(2) * s.p2) * id;
-    q.b12 = s.p2 * id;
+    const Two<T> w = q.w1 * q.w2, t = both(s.p2) * q.i, a = fma2(both(T(2)), t, w);
+    const T id = reciprocal<IEEE>(w.x * a.y + t.x * (T(3) * t.y + T(2) * w.y));
+    const Two<T> n = q.i * both(id);
+    q.b11 = a.x * n.y;
+    q.b22 = a.y * n.x;
+    q.b12 = t.x * n.y;
     const Two<T> g = fma2(s.c1, q.w2, fma2(s.c2, q.w1, s.hxy));
     q.ag = q.b22 * g.x - q.b12 * g.y;
     q.bg = q.b11 * g.y - q.b12 * g.x;
     q.Cd = fma2(s.c2, both(T(-1)), s.c1);
     q.k = fma2(s.e2, both(T(-1)), s.e1) * q.i;
     q.e = fma2(s.e1, q.w2, s.e2 * q.w1);
-    const Two<T> t = fma2(q.k, q.Cd, q.e * two(q.ag, q.bg));
-    q.ih = reciprocal<IEEE>(s.j4 + (t.x + t.y));
+    const Two<T> m = fma2(q.k, q.Cd, q.e * two(q.ag, q.bg));
+    q.ih = reciprocal<IEEE>(s.j4 + (m.x + m.y));
 }
 
 template <typename T>
