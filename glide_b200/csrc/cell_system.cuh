@@ -184,9 +184,9 @@ __device__ __forceinline__ void arrow_assemble(const Cell<T>& C, T h, T shift, i
     // half of the mass row: upwind fluxes, calving (flux.cu:39-64, :187-211)
     {
         const T cal = T(0.5) * p.calving_rate * (T(1) - g);
-        // a velocity of +0 takes the cell to the left of / below the face (copysign, flux.cu:53)
-        s.e1 = C.W_1 * two(C.n_1.x > T(0) ? h : C.H_1.x, neg(C.n_1.y) ? C.H_1.y : h);
-        s.e2 = C.W_2 * two(neg(C.n_2.x) ? C.H_2.x : h, C.n_2.y > T(0) ? h : C.H_2.y);
+        // inward by the sign bit, a zero's too (copysign, flux.cu:53): the neighbour's thickness
+        s.e1 = C.W_1 * two(neg(C.n_1.x) ? C.H_1.x : h, neg(C.n_1.y) ? C.H_1.y : h);
+        s.e2 = C.W_2 * two(neg(C.n_2.x) ? C.H_2.x : h, neg(C.n_2.y) ? C.H_2.y : h);
         const Two<T> o = fma2(C.W_1, two(M<T>::max(C.n_1.x, T(0)), M<T>::max(C.n_1.y, T(0))),
                               C.W_2 * two(M<T>::max(C.n_2.x, T(0)), M<T>::max(C.n_2.y, T(0))));
         s.j4 = (hdti + cal) - (o.x + o.y);

@@ -93,9 +93,9 @@ __device__ __forceinline__ void newton_assemble(const Cell<T>& C, Two<T> R1, Two
     // half of the mass row: upwind fluxes, calving (flux.cu:39-64, :187-211)
     {
         const T cal = T(0.5) * p.calving_rate * (T(1) - g);
-        // a velocity of +0 takes the cell to the left of / below the face (copysign, flux.cu:53)
-        s.e1 = C.W_1 * two(n1.x > T(0) ? h : C.H_1.x, neg(n1.y) ? C.H_1.y : h);
-        s.e2 = C.W_2 * two(neg(n2.x) ? C.H_2.x : h, n2.y > T(0) ? h : C.H_2.y);
+        // inward by the sign bit, a zero's too (copysign, flux.cu:53): the neighbour's thickness
+        s.e1 = C.W_1 * two(neg(n1.x) ? C.H_1.x : h, neg(n1.y) ? C.H_1.y : h);
+        s.e2 = C.W_2 * two(neg(n2.x) ? C.H_2.x : h, neg(n2.y) ? C.H_2.y : h);
         const Two<T> t = fma2(s.e1, n1, s.e2 * n2);
         r4 = h * (hdti + cal) - T(0.5) * C.f_H - (t.x + t.y);
         const Two<T> o = fma2(C.W_1, two(M<T>::max(n1.x, T(0)), M<T>::max(n1.y, T(0))),
@@ -124,7 +124,7 @@ template <typename T>
 __device__ __forceinline__ void newton_cell(const Cell<T>& C, Two<T> R1, Two<T> R2, T H0, int n_newton, T shift,
                                             T step, const Phys<T>& p, Two<T>& d1, Two<T>& d2, T& dh) {
     const T hdti = T(0.5) / p.dt;
-    d1 = d2 = both(T(0));
+    d1 = d2 = both(T(-0.0));   // x + (-0) keeps the sign of a zero velocity x
     T h = H0;
     for (int it = 0; it < n_newton; it++) {
         Arrow<T> s;
