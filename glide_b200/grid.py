@@ -76,9 +76,9 @@ class Grid:
         for name in ("H_prev", "chi", "phi", "bed", "beta", "B", "smb", "mask", "error_mask", "gamma"):
             setattr(self, name, self._cells())
         self._scratch = torch.zeros(5 * self.nb * self.nh, dtype=self.dtype, device=self.device)
-        # second state and cell arrays of the forward smoother (one kernel per sweep): up to 34 MB,
-        # 2^20 cells in FP32
-        fused = self.nb * self.nh * self._scratch.element_size() <= 1 << 22
+        # second state and cell arrays of the forward smoother (one kernel per sweep): FP32 grids
+        # up to 2^20 cells, 34 MB
+        fused = self.dtype == torch.float32 and self.nb * self.nh <= 1 << 20
         self._sweep_work = self._scratch.new_empty(self.nb * (self.n_total + 5 * self.nh)) if fused else None
         nflags = (self.ny // 14 + 1) * (self.nx // 14 + 1) * self.nb
         self._flags = torch.zeros(nflags, dtype=torch.int32, device=self.device)
