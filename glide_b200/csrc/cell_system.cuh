@@ -205,4 +205,37 @@ __device__ __forceinline__ void arrow_assemble(const Cell<T>& C, T h, T shift, i
     }
 }
 
+// J^T x = b of one cell in the arrow form: the velocity block is symmetric, the
+// thickness column and the mass row change places (the mass row is stored at
+// half its size).
+template <typename T> __device__ __forceinline__ Arrow<T> transposed(const Arrow<T>& s) {
+    Arrow<T> t = s;
+    t.c1 = s.e1 + s.e1;
+    t.c2 = s.e2 + s.e2;
+    t.e1 = s.c1 + two(s.hxy.x, s.hxy.y);
+    t.e2 = s.c2 + two(s.hxy.x, s.hxy.y);
+    t.hxy = both(T(0));
+    t.j4 = T(2) * s.j4;
+    return t;
+}
+
+// lambda += omega * (half of each face's change, the full thickness change);
+// within one colour every face has one writer
+template <bool CHAIN, typename T>
+__device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __restrict__ ra_u,
+                                               const T* __restrict__ ra_v, const T* __restrict__ ra_H,
+                                               T* __restrict__ l_u, T* __restrict__ l_v, T* __restrict__ l_H, int i,
+                                               int j, int nx, T omega) {
+    const int iu = i * (nx + 1) + j, ic = i * nx + j;
+    Two<T> x1, x2;
+    T xh;
+    arrow_solve(q, two(ld<CHAIN>(ra_u + iu), -ld<CHAIN>(ra_v + ic)),
+                two(-ld<CHAIN>(ra_u + iu + 1), ld<CHAIN>(ra_v + ic + nx)), both(T(0)), ld<CHAIN>(ra_H + ic), x1, x2, xh);
+    l_u[iu] -= T(0.5) * omega * x1.x;
+    l_u[iu + 1] += T(0.5) * omega * x2.x;
+    l_v[ic] += T(0.5) * omega * x1.y;
+    l_v[ic + nx] -= T(0.5) * omega * x2.y;
+    l_H[ic] += omega * xh;
+}
+
 }  // namespace glide

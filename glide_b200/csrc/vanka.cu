@@ -21,7 +21,7 @@
 // instruction issue (4,870 instructions per warp of 32 cells and 10 steps).
 #include <type_traits>
 
-#include "glide_common.cuh"
+#include "cell_system.cuh"
 
 namespace glide {
 
@@ -603,6 +603,87 @@ __global__ void vanka_apply_kernel(T* u, T* v, T* H, const T* su, const T* sv, c
     }
 }
 
+// --------------------------------------------------------------------------
+// Adjoint Vanka, one colour (glide/cuda/vanka.cu:441-840), forming the cells'
+// systems as it goes: for calls without room for stored ones (vanka_stored.cu).
+// lambda changes in place; within one colour every face has one writer.  The
+// tile's state and viscosities come from shared memory and half of the threads
+// take a cell of the colour each: whole warps solve, the others are done.
+// --------------------------------------------------------------------------
+template <typename T>
+__device__ __forceinline__ Cell<T> patch_cell(const Patch<T>& P, T ul, T ur, T vt, T vb, int ny, int nx,
+                                              const Phys<T>& p) {
+    const T d2 = p.dxi * p.dxi, q = T(0.25) * d2, rr = rho_ratio<T>();
+    const T wl = P.j > 0 ? T(1) : T(0), wr = P.j + 1 < nx ? T(1) : T(0);
+    const T wt = P.i > 0 ? T(1) : T(0), wb = P.i + 1 < ny ? T(1) : T(0);
+    T e[3][3];
+#pragma unroll
+    for (int a = 0; a < 3; a++)
+#pragma unroll
+        for (int b = 0; b < 3; b++) e[a][b] = P.eta[a][b] * P.Hn[a][b];
+    auto surface = [&](T bed, T H) { return -(M<T>::max(bed, -rr * H) + H); };
+    auto drag = [&](T g, T beta) { return T(0.5) * (g * beta + (T(1) - g) * p.water_drag); };
+    Cell<T> C;
+    C.H_1 = two(P.Hn[1][0], P.Hn[0][1]);
+    C.H_2 = two(P.Hn[1][2], P.Hn[2][1]);
+    C.Z_1 = two(surface(P.bed_l, C.H_1.x), surface(P.bed_t, C.H_1.y));
+    C.Z_2 = two(surface(P.bed_r, C.H_2.x), surface(P.bed_b, C.H_2.y));
+    C.B_1 = two(drag(P.g_l, P.beta_l), drag(P.g_t, P.beta_t));
+    C.B_2 = two(drag(P.g_r, P.beta_r), drag(P.g_b, P.beta_b));
+    C.bed = P.bed_c;
+    C.beta = P.beta_c;
+    C.n_1 = two(-ul, vt);
+    C.n_2 = two(ur, -vb);
+    C.D0 = two(ur - ul, vt - vb);
+    C.E = T(2) * d2 * P.eta[1][1];
+    const T e4 = q * P.eta[1][1];
+    C.ew_p = two(e4 * wt * wl, e4 * wb * wr);
+    C.ew_q = two(e4 * wb * wl, e4 * wt * wr);
+    C.S_p = two(q * (e[0][0] + e[0][1] + e[1][0]) * wt * wl, q * (e[1][2] + e[2][1] + e[2][2]) * wb * wr);
+    C.S_q = two(q * (e[1][0] + e[2][0] + e[2][1]) * wb * wl, q * (e[0][1] + e[0][2] + e[1][2]) * wt * wr);
+    C.X_p = two((P.u_tl - ul) + (vt - P.v_lt), (ur - P.u_br) + (P.v_rb - vb));
+    C.X_q = two((P.u_bl - ul) + (P.v_lb - vb), (ur - P.u_tr) + (vt - P.v_rt));
+    C.K_1 = two(T(4) * d2 * e[1][0] * wl, T(4) * d2 * e[0][1] * wt);
+    C.K_2 = two(T(4) * d2 * e[1][2] * wr, T(4) * d2 * e[2][1] * wb);
+    C.W_1 = two(T(-0.5) * p.dxi * wl, T(-0.5) * p.dxi * wt);
+    C.W_2 = two(T(-0.5) * p.dxi * wr, T(-0.5) * p.dxi * wb);
+    C.f_H = C.thk = T(0);   // the active set is given
+    return C;
+}
+
+template <typename T, typename P>
+__global__ void __launch_bounds__(VX * VY, 4) vanka_adjoint_kernel(
+    T* l_u, T* l_v, T* l_H, const T* __restrict__ ra_u, const T* __restrict__ ra_v, const T* __restrict__ ra_H,
+    const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H, const T* __restrict__ bed,
+    const T* __restrict__ B, const T* __restrict__ beta, const T* __restrict__ mask, int color, T omega, int y0, Geo g,
+    P p) {
+    __shared__ Window<T> W;
+    const int zero = chain_enter<true>();
+    const int ny = g.ny, nx = g.nx, bz = blockIdx.z + zero;
+    const int64_t nc = g.nc();
+    u += bz * g.nu(); v += bz * g.nv(); H += bz * nc;
+    bed += bz * nc; B += bz * nc; beta += bz * nc;
+    const int i0 = (blockIdx.y + y0) * VY + zero, j0 = blockIdx.x * VX;
+    const State<T, false, true> st{u, v, H, H, H, H, H, H, nullptr, T(0), ny, nx, false};
+    state_window(W, st, (T*)nullptr, (T*)nullptr, (T*)nullptr, i0, j0);
+    __syncthreads();
+    eta_window<true>(W, B, i0, j0, ny, nx, p);
+    __syncthreads();
+    const int r = threadIdx.x / (VX / 2), c = 2 * (threadIdx.x % (VX / 2)) + ((i0 + r + j0 + color) & 1);
+    const int i = i0 + r, j = j0 + c;
+    if (r >= VY || i >= ny || j >= nx) return;
+    Patch<T> pt;
+    load_patch<true>(pt, W, r, c, bed, beta, i, j, ny, nx, p);
+    const Cell<T> C = patch_cell<T>(pt, W.u[r + 2][c + 1], W.u[r + 2][c + 2], W.v[r + 1][c + 2], W.v[r + 2][c + 2], ny,
+                                    nx, p);
+    Arrow<T> s;
+    arrow_assemble<T>(C, W.H[r + 1][c + 1], T(0), ld<true>(mask + bz * nc + i * nx + j) > T(0.5) ? 1 : 0, p, s);
+    ArrowInv<T> q;
+    arrow_factor<true>(transposed(s), q);
+    adjoint_update<true>(q, ra_u + bz * g.nu(), ra_v + bz * g.nv(), ra_H + bz * nc, l_u + bz * g.nu(),
+                         l_v + bz * g.nv(), l_H + bz * nc, i, j, nx, omega);
+}
+
 // Local error indicator (glide/solver.py:148-154) and reference-tile flags.
 // err = |r_u(l)| + |r_u(r)| + |r_v(t)| + |r_v(b)| + |FB(r_H, H-gamma)| > threshold
 template <typename T>
@@ -769,6 +850,21 @@ int launch_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v
 }
 
 template <typename T>
+int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
+                         const void* ra_H, int color, double omega, cudaStream_t s) {
+    Geo g{a->ny, a->nx, a->nb};
+    with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
+        by_block_rows(cell_grid(g), [&](dim3 grid, int y0) {
+            launch_chained<true>(vanka_adjoint_kernel<T, decltype(p)>, grid, VX * VY, s, (T*)l_u, (T*)l_v, (T*)l_H,
+                                 (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, (const T*)a->u, (const T*)a->v,
+                                 (const T*)a->H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
+                                 color, T(omega), y0, g, p);
+        });
+    });
+    return (int)cudaGetLastError();
+}
+
+template <typename T>
 int launch_error_mask(const GlideLevelArgs* a, const void* r_u, const void* r_v, const void* r_H, double threshold,
                       void* err_mask, int* flags, int* any_active, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
@@ -798,6 +894,8 @@ int launch_tile_flags(const GlideLevelArgs* a, const void* err_mask, int* flags,
                                         double, double, const int*, const int*, void*, cudaStream_t, double, int, bool, void*);\
     template int launch_vanka_cells<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,     \
                                        double, const int*, const int*, void*, cudaStream_t, double);              \
+    template int launch_vanka_adjoint<T>(const GlideLevelArgs*, void*, void*, void*, const void*, const void*,   \
+                                         const void*, int, double, cudaStream_t);                                \
     template int launch_error_mask<T>(const GlideLevelArgs*, const void*, const void*, const void*, double,       \
                                       void*, int*, int*, cudaStream_t);                                           \
     template int launch_tile_flags<T>(const GlideLevelArgs*, const void*, int*, int*, cudaStream_t);

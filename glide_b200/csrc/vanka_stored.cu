@@ -18,52 +18,15 @@ constexpr int FC_NT = 128;
 constexpr int LU_N = 14;        // D1, D2, p2, c1, c2, e1, e2, j4
 constexpr int ADJ_N = 18;       // i, w1, w2, Cd, k, e, b11, b12, b22, ag, bg, ih
 
-enum { STORE_LU = 0, STORE_ADJOINT = 1, SOLVE_ADJOINT = 2 };
+enum { STORE_LU = 0, STORE_ADJOINT = 1 };
 
 template <typename T> struct StoredArgs {
     const T *u, *v, *H, *f_H, *bed, *B, *beta, *gamma;
     const T* act;               // active set; null: tested with f_H
     T* out;                     // stored arrays
     T shift;
-    T *l_u, *l_v, *l_H;         // SOLVE_ADJOINT: multiplier, adjoint residual, colour
-    const T *ra_u, *ra_v, *ra_H;
-    T omega;
-    int color;
     int n_strips, rows, n_warps;
 };
-
-// J^T x = b of one cell in the arrow form: the velocity block is symmetric, the
-// thickness column and the mass row change places (the mass row is stored at
-// half its size).
-template <typename T> __device__ __forceinline__ Arrow<T> transposed(const Arrow<T>& s) {
-    Arrow<T> t = s;
-    t.c1 = s.e1 + s.e1;
-    t.c2 = s.e2 + s.e2;
-    t.e1 = s.c1 + two(s.hxy.x, s.hxy.y);
-    t.e2 = s.c2 + two(s.hxy.x, s.hxy.y);
-    t.hxy = both(T(0));
-    t.j4 = T(2) * s.j4;
-    return t;
-}
-
-// lambda += omega * (half of each face's change, the full thickness change);
-// within one colour every face has one writer
-template <bool CHAIN, typename T>
-__device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __restrict__ ra_u,
-                                               const T* __restrict__ ra_v, const T* __restrict__ ra_H,
-                                               T* __restrict__ l_u, T* __restrict__ l_v, T* __restrict__ l_H, int i,
-                                               int j, int nx, T omega) {
-    const int iu = i * (nx + 1) + j, ic = i * nx + j;
-    Two<T> x1, x2;
-    T xh;
-    arrow_solve(q, two(ld<CHAIN>(ra_u + iu), -ld<CHAIN>(ra_v + ic)),
-                two(-ld<CHAIN>(ra_u + iu + 1), ld<CHAIN>(ra_v + ic + nx)), both(T(0)), ld<CHAIN>(ra_H + ic), x1, x2, xh);
-    l_u[iu] -= T(0.5) * omega * x1.x;
-    l_u[iu + 1] += T(0.5) * omega * x2.x;
-    l_v[ic] += T(0.5) * omega * x1.y;
-    l_v[ic + nx] -= T(0.5) * omega * x2.y;
-    l_H[ic] += omega * xh;
-}
 
 // --------------------------------------------------------------------------
 // The march: a warp owns SW cell columns (lane l holds column j0 - 1 + l) and
@@ -162,7 +125,7 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
             C.K_2 = two(T(4) * d2 * eR * wr, T(4) * d2 * ep * wb);
             C.W_1 = two(T(-0.5) * dxi * wl, T(-0.5) * dxi * wt);
             C.W_2 = two(T(-0.5) * dxi * wr, T(-0.5) * dxi * wb);
-            if (own && (MODE != SOLVE_ADJOINT || ((i + jc) & 1) == A.color)) {
+            if (own) {
                 const int ic = i * nx + jc;
                 const T* act = A.act ? A.act + b * nc : nullptr;
                 C.f_H = act ? T(0) : __ldg(A.f_H + b * nc + ic);
@@ -179,16 +142,11 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
                 } else {
                     ArrowInv<T> q;
                     arrow_factor<true>(transposed(s), q);
-                    if constexpr (MODE == STORE_ADJOINT) {
-                        const T o[ADJ_N] = {q.i.x, q.i.y, q.w1.x, q.w1.y, q.w2.x, q.w2.y, q.Cd.x, q.Cd.y, q.k.x,
-                                            q.k.y, q.e.x, q.e.y, q.b11, q.b12, q.b22, q.ag, q.bg, q.ih};
-                        T* out = A.out + b * ADJ_N * nc + ic;
+                    const T o[ADJ_N] = {q.i.x, q.i.y, q.w1.x, q.w1.y, q.w2.x, q.w2.y, q.Cd.x, q.Cd.y, q.k.x,
+                                        q.k.y, q.e.x, q.e.y, q.b11, q.b12, q.b22, q.ag, q.bg, q.ih};
+                    T* out = A.out + b * ADJ_N * nc + ic;
 #pragma unroll
-                        for (int k = 0; k < ADJ_N; k++) out[k * nc] = o[k];
-                    } else {
-                        adjoint_update<false>(q, A.ra_u + b * g.nu(), A.ra_v + b * g.nv(), A.ra_H + b * nc,
-                                       A.l_u + b * g.nu(), A.l_v + b * g.nv(), A.l_H + b * nc, i, jc, nx, A.omega);
-                    }
+                    for (int k = 0; k < ADJ_N; k++) out[k * nc] = o[k];
                 }
             }
         }
@@ -346,18 +304,6 @@ int launch_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* 
     return (int)cudaGetLastError();
 }
 
-template <typename T>
-int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
-                         const void* ra_H, int color, double omega, cudaStream_t s) {
-    StoredArgs<T> A{};
-    A.act = (const T*)a->mask;
-    A.l_u = (T*)l_u; A.l_v = (T*)l_v; A.l_H = (T*)l_H;
-    A.ra_u = (const T*)ra_u; A.ra_v = (const T*)ra_v; A.ra_H = (const T*)ra_H;
-    A.omega = T(omega);
-    A.color = color;
-    return run_stored<T, SOLVE_ADJOINT>(a, A, s);
-}
-
 template <typename T> int launch_adjoint_factors(const GlideLevelArgs* a, void* factors, cudaStream_t s) {
     StoredArgs<T> A{};
     A.act = (const T*)a->mask;
@@ -386,8 +332,6 @@ int launch_adjoint_color(const GlideLevelArgs* a, const void* factors, void* l_u
     template int launch_vanka_lu<T>(const GlideLevelArgs*, const void*, void*, double, cudaStream_t);               \
     template int launch_vanka_linear<T>(const GlideLevelArgs*, const void*, const void*, const void*, const void*,  \
                                         void*, void*, void*, double, cudaStream_t);                                 \
-    template int launch_vanka_adjoint<T>(const GlideLevelArgs*, void*, void*, void*, const void*, const void*,      \
-                                         const void*, int, double, cudaStream_t);                                   \
     template int launch_adjoint_factors<T>(const GlideLevelArgs*, void*, cudaStream_t);                             \
     template int launch_adjoint_color<T>(const GlideLevelArgs*, const void*, void*, void*, void*, const void*,      \
                                          const void*, const void*, int, double, cudaStream_t);
