@@ -238,4 +238,38 @@ __device__ __forceinline__ void adjoint_update(const ArrowInv<T>& q, const T* __
     l_H[ic] += omega * xh;
 }
 
+// What the sweeps with stored systems read, one array of nc cells after the
+// other: the matrix for the linear sweep, the solved form for the adjoint.
+constexpr int LU_N = 14;    // D1, D2, p2, c1, c2, e1, e2, j4
+constexpr int LU_ROOM = 25; // arrays per problem in the caller's buffer
+constexpr int ADJ_N = 18;   // i, w1, w2, Cd, k, e, b11, b12, b22, ag, bg, ih
+template <typename T> __device__ __forceinline__ void store_matrix(T* out, int64_t nc, const Arrow<T>& s) {
+    const Two<T> c1 = s.c1 + s.hxy, c2 = s.c2 + s.hxy;
+    const T o[LU_N] = {s.D1.x, s.D1.y, s.D2.x, s.D2.y, s.p2, c1.x, c1.y, c2.x, c2.y, s.e1.x, s.e1.y,
+                       s.e2.x, s.e2.y, s.j4};
+#pragma unroll
+    for (int k = 0; k < LU_N; k++) out[k * nc] = o[k];
+}
+template <typename T> __device__ __forceinline__ void store_solved(T* out, int64_t nc, const ArrowInv<T>& q) {
+    const T o[ADJ_N] = {q.i.x, q.i.y, q.w1.x, q.w1.y, q.w2.x, q.w2.y, q.Cd.x, q.Cd.y, q.k.x,
+                        q.k.y, q.e.x, q.e.y, q.b11, q.b12, q.b22, q.ag, q.bg, q.ih};
+#pragma unroll
+    for (int k = 0; k < ADJ_N; k++) out[k * nc] = o[k];
+}
+
+// Which cells' systems a kernel forms, and what becomes of them.
+enum { STORE_LU = 0, STORE_ADJOINT = 1, SOLVE_ADJOINT = 2 };
+template <typename T> struct StoredArgs {
+    const T *u, *v, *H, *f_H, *bed, *B, *beta, *gamma;
+    const T* act;               // active set; null: tested with f_H
+    T* out;                     // stored arrays
+    T shift;
+    T *l_u, *l_v, *l_H;         // SOLVE_ADJOINT: multiplier, adjoint residual, colour
+    const T *ra_u, *ra_v, *ra_H;
+    T omega;
+    int color;
+    int n_strips, rows, n_warps;   // march
+    int y0;                        // tile
+};
+
 }  // namespace glide

@@ -604,11 +604,14 @@ __global__ void vanka_apply_kernel(T* u, T* v, T* H, const T* su, const T* sv, c
 }
 
 // --------------------------------------------------------------------------
-// Adjoint Vanka, one colour (glide/cuda/vanka.cu:441-840), forming the cells'
-// systems as it goes: for calls without room for stored ones (vanka_stored.cu).
-// lambda changes in place; within one colour every face has one writer.  The
-// tile's state and viscosities come from shared memory and half of the threads
-// take a cell of the colour each: whole warps solve, the others are done.
+// The cells' systems in arrow form, a thread per cell of a tile whose state and
+// viscosities come from shared memory: stored for the linear sweeps (vanka_stored.cu
+// has the march for large FP32 levels and the adjoint), or solved at once for one
+// colour of the adjoint Vanka (glide/cuda/vanka.cu:441-840), for calls without
+// room for stored systems.  Then lambda changes in place (within one colour every
+// face has one writer) and half of the threads take a cell of the colour each:
+// whole warps solve, the others are done.  One colour at 512^2, march / this: FP32
+// 18.0 / 10.5 us, FP64 25.8 / 19.3; 256^2 9.8 / 5.0 and 13.7 / 6.2.
 // --------------------------------------------------------------------------
 template <typename T>
 __device__ __forceinline__ Cell<T> patch_cell(const Patch<T>& P, T ul, T ur, T vt, T vb, int ny, int nx,
@@ -651,37 +654,42 @@ __device__ __forceinline__ Cell<T> patch_cell(const Patch<T>& P, T ul, T ur, T v
     return C;
 }
 
-template <typename T, typename P>
-__global__ void __launch_bounds__(VX * VY, 4) vanka_adjoint_kernel(
-    T* l_u, T* l_v, T* l_H, const T* __restrict__ ra_u, const T* __restrict__ ra_v, const T* __restrict__ ra_H,
-    const T* __restrict__ u, const T* __restrict__ v, const T* __restrict__ H, const T* __restrict__ bed,
-    const T* __restrict__ B, const T* __restrict__ beta, const T* __restrict__ mask, int color, T omega, int y0, Geo g,
-    P p) {
+template <typename T, int MODE, typename P>
+__global__ void __launch_bounds__(VX * VY, 4) cell_systems_kernel(const StoredArgs<T> A, Geo g, P p) {
     __shared__ Window<T> W;
     const int zero = chain_enter<true>();
     const int ny = g.ny, nx = g.nx, bz = blockIdx.z + zero;
     const int64_t nc = g.nc();
-    u += bz * g.nu(); v += bz * g.nv(); H += bz * nc;
-    bed += bz * nc; B += bz * nc; beta += bz * nc;
-    const int i0 = (blockIdx.y + y0) * VY + zero, j0 = blockIdx.x * VX;
+    const T *u = A.u + bz * g.nu(), *v = A.v + bz * g.nv(), *H = A.H + bz * nc;
+    const int i0 = (blockIdx.y + A.y0) * VY + zero, j0 = blockIdx.x * VX;
     const State<T, false, true> st{u, v, H, H, H, H, H, H, nullptr, T(0), ny, nx, false};
     state_window(W, st, (T*)nullptr, (T*)nullptr, (T*)nullptr, i0, j0);
     __syncthreads();
-    eta_window<true>(W, B, i0, j0, ny, nx, p);
+    eta_window<true>(W, A.B + bz * nc, i0, j0, ny, nx, p);
     __syncthreads();
-    const int r = threadIdx.x / (VX / 2), c = 2 * (threadIdx.x % (VX / 2)) + ((i0 + r + j0 + color) & 1);
+    int r = threadIdx.x / VX, c = threadIdx.x % VX;
+    if (MODE == SOLVE_ADJOINT) {
+        r = threadIdx.x / (VX / 2);
+        c = 2 * (threadIdx.x % (VX / 2)) + ((i0 + r + j0 + A.color) & 1);
+    }
     const int i = i0 + r, j = j0 + c;
     if (r >= VY || i >= ny || j >= nx) return;
+    const int64_t ic = i * nx + j;
     Patch<T> pt;
-    load_patch<true>(pt, W, r, c, bed, beta, i, j, ny, nx, p);
-    const Cell<T> C = patch_cell<T>(pt, W.u[r + 2][c + 1], W.u[r + 2][c + 2], W.v[r + 1][c + 2], W.v[r + 2][c + 2], ny,
-                                    nx, p);
+    load_patch<true>(pt, W, r, c, A.bed + bz * nc, A.beta + bz * nc, i, j, ny, nx, p);
+    Cell<T> C = patch_cell<T>(pt, W.u[r + 2][c + 1], W.u[r + 2][c + 2], W.v[r + 1][c + 2], W.v[r + 2][c + 2], ny, nx, p);
+    C.f_H = A.act ? T(0) : ld<true>(A.f_H + bz * nc + ic);
+    C.thk = A.act ? T(0) : ld<true>(A.gamma + bz * nc + ic);
     Arrow<T> s;
-    arrow_assemble<T>(C, W.H[r + 1][c + 1], T(0), ld<true>(mask + bz * nc + i * nx + j) > T(0.5) ? 1 : 0, p, s);
-    ArrowInv<T> q;
-    arrow_factor<true>(transposed(s), q);
-    adjoint_update<true>(q, ra_u + bz * g.nu(), ra_v + bz * g.nv(), ra_H + bz * nc, l_u + bz * g.nu(),
-                         l_v + bz * g.nv(), l_H + bz * nc, i, j, nx, omega);
+    arrow_assemble<T>(C, W.H[r + 1][c + 1], A.shift, A.act ? (ld<true>(A.act + bz * nc + ic) > T(0.5) ? 1 : 0) : -1, p, s);
+    if constexpr (MODE == STORE_LU) {
+        store_matrix(A.out + bz * LU_ROOM * nc + ic, nc, s);
+    } else {
+        ArrowInv<T> q;
+        arrow_factor<true>(transposed(s), q);
+        adjoint_update<true>(q, A.ra_u + bz * g.nu(), A.ra_v + bz * g.nv(), A.ra_H + bz * nc, A.l_u + bz * g.nu(),
+                             A.l_v + bz * g.nv(), A.l_H + bz * nc, i, j, nx, A.omega);
+    }
 }
 
 // Local error indicator (glide/solver.py:148-154) and reference-tile flags.
@@ -849,19 +857,29 @@ int launch_vanka_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v
     return (int)cudaGetLastError();
 }
 
-template <typename T>
-int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
-                         const void* ra_H, int color, double omega, cudaStream_t s) {
+template <typename T, int MODE> int run_tile(const GlideLevelArgs* a, StoredArgs<T> A, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
+    A.u = (const T*)a->u; A.v = (const T*)a->v; A.H = (const T*)a->H;
+    A.bed = (const T*)a->bed; A.B = (const T*)a->B; A.beta = (const T*)a->beta; A.gamma = (const T*)a->gamma;
     with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto p) {
         by_block_rows(cell_grid(g), [&](dim3 grid, int y0) {
-            launch_chained<true>(vanka_adjoint_kernel<T, decltype(p)>, grid, VX * VY, s, (T*)l_u, (T*)l_v, (T*)l_H,
-                                 (const T*)ra_u, (const T*)ra_v, (const T*)ra_H, (const T*)a->u, (const T*)a->v,
-                                 (const T*)a->H, (const T*)a->bed, (const T*)a->B, (const T*)a->beta, (const T*)a->mask,
-                                 color, T(omega), y0, g, p);
+            A.y0 = y0;
+            launch_chained<true>(cell_systems_kernel<T, MODE, decltype(p)>, grid, VX * VY, s, A, g, p);
         });
     });
     return (int)cudaGetLastError();
+}
+
+template <typename T>
+int launch_vanka_adjoint(const GlideLevelArgs* a, void* l_u, void* l_v, void* l_H, const void* ra_u, const void* ra_v,
+                         const void* ra_H, int color, double omega, cudaStream_t s) {
+    StoredArgs<T> A{};
+    A.act = (const T*)a->mask;
+    A.l_u = (T*)l_u; A.l_v = (T*)l_v; A.l_H = (T*)l_H;
+    A.ra_u = (const T*)ra_u; A.ra_v = (const T*)ra_v; A.ra_H = (const T*)ra_H;
+    A.omega = T(omega);
+    A.color = color;
+    return run_tile<T, SOLVE_ADJOINT>(a, A, s);
 }
 
 template <typename T>
@@ -894,6 +912,7 @@ int launch_tile_flags(const GlideLevelArgs* a, const void* err_mask, int* flags,
                                         double, double, const int*, const int*, void*, cudaStream_t, double, int, bool, void*);\
     template int launch_vanka_cells<T>(const GlideLevelArgs*, const void*, const void*, const void*, int, int,     \
                                        double, const int*, const int*, void*, cudaStream_t, double);              \
+    template int run_tile<T, STORE_LU>(const GlideLevelArgs*, StoredArgs<T>, cudaStream_t);                       \
     template int launch_vanka_adjoint<T>(const GlideLevelArgs*, void*, void*, void*, const void*, const void*,   \
                                          const void*, int, double, cudaStream_t);                                \
     template int launch_error_mask<T>(const GlideLevelArgs*, const void*, const void*, const void*, double,       \

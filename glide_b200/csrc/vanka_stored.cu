@@ -15,19 +15,6 @@ namespace glide {
 
 constexpr int SW = 30;          // cell columns per warp of the march
 constexpr int FC_NT = 128;
-constexpr int LU_N = 14;        // D1, D2, p2, c1, c2, e1, e2, j4
-constexpr int ADJ_N = 18;       // i, w1, w2, Cd, k, e, b11, b12, b22, ag, bg, ih
-
-enum { STORE_LU = 0, STORE_ADJOINT = 1 };
-
-template <typename T> struct StoredArgs {
-    const T *u, *v, *H, *f_H, *bed, *B, *beta, *gamma;
-    const T* act;               // active set; null: tested with f_H
-    T* out;                     // stored arrays
-    T shift;
-    int n_strips, rows, n_warps;
-};
-
 // --------------------------------------------------------------------------
 // The march: a warp owns SW cell columns (lane l holds column j0 - 1 + l) and
 // marches down a chunk of rows with the rows in reach in registers and the
@@ -133,20 +120,11 @@ __global__ void __launch_bounds__(FC_NT, sizeof(T) == 4 ? 4 : 2)
                 Arrow<T> s;
                 arrow_assemble<T>(C, Hc, A.shift, act ? (__ldg(act + ic) > T(0.5) ? 1 : 0) : -1, p, s);
                 if constexpr (MODE == STORE_LU) {
-                    const Two<T> c1 = s.c1 + s.hxy, c2 = s.c2 + s.hxy;
-                    const T o[LU_N] = {s.D1.x, s.D1.y, s.D2.x, s.D2.y, s.p2, c1.x, c1.y, c2.x, c2.y, s.e1.x, s.e1.y,
-                                       s.e2.x, s.e2.y, s.j4};
-                    T* out = A.out + b * 25 * nc + ic;
-#pragma unroll
-                    for (int k = 0; k < LU_N; k++) out[k * nc] = o[k];
+                    store_matrix(A.out + b * LU_ROOM * nc + ic, nc, s);
                 } else {
                     ArrowInv<T> q;
                     arrow_factor<true>(transposed(s), q);
-                    const T o[ADJ_N] = {q.i.x, q.i.y, q.w1.x, q.w1.y, q.w2.x, q.w2.y, q.Cd.x, q.Cd.y, q.k.x,
-                                        q.k.y, q.e.x, q.e.y, q.b11, q.b12, q.b22, q.ag, q.bg, q.ih};
-                    T* out = A.out + b * ADJ_N * nc + ic;
-#pragma unroll
-                    for (int k = 0; k < ADJ_N; k++) out[k * nc] = o[k];
+                    store_solved(A.out + b * ADJ_N * nc + ic, nc, q);
                 }
             }
         }
@@ -204,7 +182,7 @@ __global__ void __launch_bounds__(32 * (LY + 1))
     const int64_t nc = g.nc();
     d_u += b * g.nu(); d_v += b * g.nv(); d_H += b * nc;
     rho_u += b * g.nu(); rho_v += b * g.nv(); rho_H += b * nc; H += b * nc; gamma += b * nc;
-    lu += b * 25 * nc;
+    lu += b * LU_ROOM * nc;
     const int i = blockIdx.y * LY - 1 + threadIdx.y, j = blockIdx.x * LX - 1 + threadIdx.x;
     const bool cell = i >= 0 && i < ny && j >= 0 && j < nx;
     const bool own = threadIdx.x > 0 && threadIdx.y > 0;
@@ -252,12 +230,12 @@ struct MarchShape {
     int rows, n_warps, threads;
     unsigned blocks;
 };
+// As few rows as fill the resident warps once.
 static inline MarchShape march_shape(int n_strips, int lines, int nb, int warps_per_sm, int max_threads) {
     const int64_t units = int64_t(n_strips) * lines * nb;
-    const int64_t few = (units + 148 * 4 - 1) / (148 * 4), many = (units + 148 * warps_per_sm - 1) / (148 * warps_per_sm);
+    const int64_t rows = (units + 148 * warps_per_sm - 1) / (148 * warps_per_sm);
     MarchShape sh;
-    // short chunks on small grids, as in ssa_stencil.cu
-    sh.rows = int(few < 8 ? few : many < 8 ? 8 : many > 64 ? 64 : many);
+    sh.rows = int(rows > 64 ? 64 : rows);
     sh.n_warps = n_strips * ((lines + sh.rows - 1) / sh.rows);
     const int64_t per_sm = (int64_t(sh.n_warps) * nb + 147) / 148;
     sh.threads = 32 * int(per_sm < max_threads / 32 ? per_sm : max_threads / 32);
@@ -265,19 +243,31 @@ static inline MarchShape march_shape(int n_strips, int lines, int nb, int warps_
     return sh;
 }
 
+template <typename T, int MODE> int run_tile(const GlideLevelArgs*, StoredArgs<T>, cudaStream_t);   // vanka.cu
+
+// Linear factors by the tile (vanka.cu), in FP32 from 2^18 cells of a problem on by
+// the march; tile / march: FP32 256^2 3.9 / 4.8 us, 512^2 9.3 / 8.9, 1024^2 33.0 / 27.5;
+// FP64 181^2 4.4 / 7.1, 256^2 5.8 / 7.4, 512^2 16.1 / 18.1, 1024^2 76 / 88.  The adjoint's by
+// the march, which takes no shared memory: behind a kernel that does, its chained VJPs
+// and colours run slower than the tile saves (40 sweeps at 256^2 FP64 1.39 / 1.20 ms,
+// one by one; 1.15 / 1.16 ms from a graph).
 template <typename T, int MODE>
 static int run_stored(const GlideLevelArgs* a, StoredArgs<T> A, cudaStream_t s) {
     Geo g{a->ny, a->nx, a->nb};
-    Phys<T> p = make_phys<T>(a->params, a->dx, a->dt);
+    if constexpr (MODE == STORE_LU) {
+        if (sizeof(T) == 8 || g.nc() < (int64_t(1) << 18)) return run_tile<T, MODE>(a, A, s);
+    }
     A.u = (const T*)a->u; A.v = (const T*)a->v; A.H = (const T*)a->H;
     A.bed = (const T*)a->bed; A.B = (const T*)a->B; A.beta = (const T*)a->beta; A.gamma = (const T*)a->gamma;
     A.n_strips = (g.nx + SW - 1) / SW;
     const MarchShape sh = march_shape(A.n_strips, g.ny, g.nb, sizeof(T) == 4 ? 16 : 8, FC_NT);
     A.rows = sh.rows;
     A.n_warps = sh.n_warps;
-    with_glen(a->params, p, [&](auto q) {
-        launch_chained<false>(stored_cells_kernel<T, MODE, decltype(q)>, dim3(sh.blocks, g.nb), sh.threads, s, A, g, q);
-    });
+    if constexpr (MODE != STORE_LU || sizeof(T) == 4)
+        with_glen(a->params, make_phys<T>(a->params, a->dx, a->dt), [&](auto q) {
+            launch_chained<false>(stored_cells_kernel<T, MODE, decltype(q)>, dim3(sh.blocks, g.nb), sh.threads, s, A, g,
+                                  q);
+        });
     return (int)cudaGetLastError();
 }
 
