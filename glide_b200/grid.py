@@ -129,10 +129,15 @@ class Grid:
 
     def adjoint_factors(self):
         """Buffer of the adjoint smoother's local systems, made on first use
-        and kept with the level; None while a CUDA graph that would own a new
-        allocation is being captured (the sweeps then form them per colour)."""
+        and kept with the level (2.4 GB at 4096^2 FP64); None while a CUDA graph
+        that would own a new allocation is being captured, and where there is no
+        memory for it: the sweeps then form them per colour."""
         if self._adj_factors is None and not torch.cuda.is_current_stream_capturing():
-            self._adj_factors = torch.empty(N.ADJ_FACTORS * self.nb * self.nh, dtype=self.dtype, device=self.device)
+            try:
+                self._adj_factors = torch.empty(N.ADJ_FACTORS * self.nb * self.nh, dtype=self.dtype,
+                                                device=self.device)
+            except torch.OutOfMemoryError:
+                pass
         return self._adj_factors
 
     def newton_buffers(self):

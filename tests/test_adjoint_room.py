@@ -1,0 +1,33 @@
+"""The adjoint smoother's room is a convenience: without memory for it, or inside a
+capture, the sweeps form their systems as they go (host checks on a stand-in)."""
+from types import SimpleNamespace
+
+import torch
+
+from glide_b200 import grid as G
+
+
+def _level():
+    return SimpleNamespace(_adj_factors=None, nb=1, nh=6, dtype=torch.float32, device=torch.device("cpu"))
+
+
+def test_room_is_made_once():
+    g = _level()
+    a = G.Grid.adjoint_factors(g)
+    assert a.numel() == 18 * 6 and G.Grid.adjoint_factors(g) is a
+
+
+def test_no_memory_is_no_room(monkeypatch):
+    def empty(*a, **k):
+        raise torch.OutOfMemoryError("CUDA out of memory")
+    g = _level()
+    with monkeypatch.context() as m:
+        m.setattr(torch, "empty", empty)
+        assert G.Grid.adjoint_factors(g) is None
+    assert G.Grid.adjoint_factors(g) is not None   # asked again when there is memory
+
+
+def test_capture_makes_no_room(monkeypatch):
+    g = _level()
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: True)
+    assert G.Grid.adjoint_factors(g) is None
