@@ -2,9 +2,15 @@
 capture, the sweeps form their systems as they go (host checks on a stand-in)."""
 from types import SimpleNamespace
 
+import pytest
 import torch
 
 from glide_b200 import grid as G
+
+
+@pytest.fixture(autouse=True)
+def no_capture(monkeypatch):
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
 
 
 def _level():
