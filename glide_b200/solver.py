@@ -116,6 +116,8 @@ def fascd_vcycle(grid, thklim, finest=False, settings: SolverSettings = REFERENC
 def adjoint_vcycle(grid, settings: SolverSettings = REFERENCE, thklim=0.1):
     """One adjoint V-cycle (glide/solver.py:160-220)."""
     arr, n = native_levels(grid)
+    for g in hierarchy(grid):
+        g.adjoint_factors()
     cfg = settings.native(thklim)
     N.check(N.load().glide_adjoint_vcycle_work(arr, native_work(grid), n, 0, C.byref(cfg), N.stream_handle()),
             "adjoint_vcycle")
