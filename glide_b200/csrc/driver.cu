@@ -481,7 +481,8 @@ int adj_residual(GlideLevel* L, int exact, void* s) {
 int vanka_adj(GlideLevel* L, const GlideLevelWork* W, int n_iter, double omega, int exact, void* s) {
     LevelView w = view(L);
     return glide_vanka_adjoint_sweeps(&L->a, w.u(L->lam), w.v(L->lam), w.H(L->lam), w.u(L->f_adj), w.v(L->f_adj),
-                                      w.H(L->f_adj), w.u(L->r_adj), w.v(L->r_adj), w.H(L->r_adj), n_iter, omega, exact,
+                                      w.H(L->f_adj), w.u(L->r_adj), w.v(L->r_adj), w.H(L->r_adj), n_iter > 0 ? n_iter : 0,
+                                      omega, exact,
                                       W ? W->adj_factors : nullptr, s);
 }
 

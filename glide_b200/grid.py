@@ -299,12 +299,13 @@ class Grid:
 
     def vanka_sweep_adjoint(self, n_iter, omega=0.5, exact_boundary=False):
         """glide/grid.py:319-330."""
+        n_iter = len(range(n_iter))   # a negative count is no sweep
         a = self.level_args()
         factors = self.adjoint_factors()
         N.check(self._lib.glide_vanka_adjoint_sweeps(
             C.byref(a), self.lambda_u.data_ptr(), self.lambda_v.data_ptr(), self.lambda_H.data_ptr(),
             self.f_adj_u.data_ptr(), self.f_adj_v.data_ptr(), self.f_adj_H.data_ptr(), self.r_adj_u.data_ptr(),
-            self.r_adj_v.data_ptr(), self.r_adj_H.data_ptr(), int(n_iter), float(omega), int(exact_boundary),
+            self.r_adj_v.data_ptr(), self.r_adj_H.data_ptr(), n_iter, float(omega), int(exact_boundary),
             None if factors is None else factors.data_ptr(), self._s()), "adjoint sweeps")
 
     def compute_mask(self, tol=1e-1):
