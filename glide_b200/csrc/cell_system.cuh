@@ -1,6 +1,6 @@
-// One cell's local Vanka problem and its solution (terms of
-// glide/cuda/vanka.cu:56-404), for the kernels that form a cell's matrix once:
-// the stored factors of the linear sweeps and the adjoint smoother.
+// One cell's local Vanka problem in arrow form and its solution (terms of
+// glide/cuda/vanka.cu:56-404): the march of the forward sweeps, the stored systems of
+// the linear sweeps and the adjoint smoother.
 #pragma once
 #include "glide_common.cuh"
 

@@ -30,9 +30,11 @@ long long launch_total();
 // the chain.  The predecessor's writes fall into the kernel's lifetime, so it
 // must not read them through the read-only path: ld<true>() loads without it,
 // and indices take chain_enter()'s zero, which keeps the compiler from moving
-// a load above the wait.  Kernels that fill the chip gain nothing and run with
-// CHAIN = false and read-only loads (2-3 % faster there): 200 sweeps of a 32^2
-// level, launched one by one: 2.87 ms plain, 2.17 ms chained.
+// a load above the wait.  200 sweeps of a 32^2 level, launched one by one: 2.87 ms
+// plain, 2.17 ms chained.  The marches and the updates that fill the chip gain
+// nothing and run with CHAIN = false and read-only loads (2-3 % faster there); the
+// tiles, which load a window at once, are chained at every size (FP32 sweeps of
+// 1024^2 with 2 / 10 Newton steps 76.6 / 174.6 us, 82.6 / 177.4 unchained).
 // --------------------------------------------------------------------------
 template <bool CHAIN> __device__ __forceinline__ int chain_enter() {
     if constexpr (!CHAIN) return 0;
@@ -176,34 +178,14 @@ struct Geo {
 __device__ __forceinline__ int clampi(int x, int lo, int hi) { return x < lo ? lo : (x > hi ? hi : x); }
 
 // --------------------------------------------------------------------------
-// clamped global accessors (same semantics as glide/cuda/common.cu:78-125:
+// clamped access to a cell field (same semantics as glide/cuda/common.cu:78-125:
 // every index is clamped to the field's own extent).  Offsets are 32-bit
 // element counts: the entry points reject problems whose fields reach 2^31
 // elements (GLIDE_E_TOO_LARGE).
 // --------------------------------------------------------------------------
 template <bool CHAIN = false, typename T>
-__device__ __forceinline__ T ldu(const T* __restrict__ u, int i, int j, int ny, int nx) {
-    return ld<CHAIN>(u + (clampi(i, 0, ny - 1) * (nx + 1) + clampi(j, 0, nx)));
-}
-template <bool CHAIN = false, typename T>
-__device__ __forceinline__ T ldv(const T* __restrict__ v, int i, int j, int ny, int nx) {
-    return ld<CHAIN>(v + (clampi(i, 0, ny) * nx + clampi(j, 0, nx - 1)));
-}
-template <bool CHAIN = false, typename T>
 __device__ __forceinline__ T ldc(const T* __restrict__ a, int i, int j, int ny, int nx) {
     return ld<CHAIN>(a + (clampi(i, 0, ny - 1) * nx + clampi(j, 0, nx - 1)));
-}
-
-// Stage a clamped window [r0, r0+R) x [c0, c0+C) of a (rows x cols) field
-// into shared memory (row-major, leading dimension C).
-template <typename T>
-__device__ __forceinline__ void stage(T* __restrict__ s, const T* __restrict__ g, int rows, int cols, int r0,
-                                      int c0, int R, int C, int tid, int nthreads) {
-    for (int k = tid; k < R * C; k += nthreads) {
-        int r = k / C, c = k - r * C;
-        int gi = clampi(r0 + r, 0, rows - 1), gj = clampi(c0 + c, 0, cols - 1);
-        s[k] = __ldg(g + int64_t(gi) * cols + gj);
-    }
 }
 
 // --------------------------------------------------------------------------
@@ -277,26 +259,6 @@ __device__ __forceinline__ BasalDrag<T> basal_drag_g(T vel, T g1, T g2, T beta1,
     return o;
 }
 
-// Driving stress H_avg (S_p - S_m)/dx on a face (stress.cu:406-436, :481-510);
-// x-faces: m = left, p = right; y-faces: m = bottom (row i), p = top (row i-1).
-template <typename T> struct Driving {
-    T res, d_Hm, d_Hp;
-};
-template <typename T>
-__device__ __forceinline__ Driving<T> driving(T Hm, T Hp, T bedm, T bedp, T dxi, bool valid) {
-    Driving<T> o;
-    T w = valid ? T(1) : T(0);
-    T Havg = T(0.5) * (Hm + Hp);
-    T bm = M<T>::max(bedm, -rho_ratio<T>() * Hm), bp = M<T>::max(bedp, -rho_ratio<T>() * Hp);
-    T dbm = bedm > -rho_ratio<T>() * Hm ? T(0) : -rho_ratio<T>();
-    T dbp = bedp > -rho_ratio<T>() * Hp ? T(0) : -rho_ratio<T>();
-    T dS = (bp + Hp) - (bm + Hm);
-    o.res = Havg * dS * dxi * w;
-    o.d_Hm = (T(0.5) * dS * dxi - Havg * (T(1) + dbm) * dxi) * w;
-    o.d_Hp = (T(0.5) * dS * dxi + Havg * (T(1) + dbp) * dxi) * w;
-    return o;
-}
-
 // Upwind face flux (flux.cu:39-64, :110-135).  For x-faces a = left cell,
 // b = right cell, q = H_avg u - 0.5|u|(H_b - H_a).  For y-faces a = bottom
 // (row i), b = top (row i-1), q = H_avg v - 0.5|v|(H_top - H_bottom).
@@ -326,9 +288,6 @@ template <typename T> __device__ __forceinline__ Calving<T> calving_g(T H, T g, 
     o.d_H = -p.calving_rate * (T(1) - g);
     if (p.gl_deriv) o.d_H += p.calving_rate * H * (rho_ratio<T>() * (p.sig_c * g * (T(1) - g)));
     return o;
-}
-template <typename T> __device__ __forceinline__ Calving<T> calving(T H, T bed, const Phys<T>& p) {
-    return calving_g(H, sigmoid(bed + rho_ratio<T>() * H, p.sig_c), p);
 }
 
 // Cell viscosity from its 4 faces and the 8 neighbouring faces of the 4
@@ -383,31 +342,6 @@ __device__ __forceinline__ T cell_eta_tangent(const EtaOut<T>& e, const EtaIn<T>
     T deII = T(2) * e.ux * dux + T(2) * e.vy * dvy + (e.ux * dvy + e.vy * dux) + de2sum;
     if constexpr (sizeof(T) == 4) return T(0.5) * Bc * (p.glen_exp * M<T>::pow(e.eII, p.glen_exp - T(1)) * deII);
     return p.glen_exp * e.eta * (deII * M<T>::rcp(e.eII));   // eta ~ eII^glen_exp
-}
-
-// Load the 12 faces around cell (i,j) from a u/v pair (clamped).
-template <bool CHAIN = false, typename T>
-__device__ __forceinline__ EtaIn<T> eta_inputs(const T* __restrict__ u, const T* __restrict__ v, int i, int j,
-                                               int ny, int nx) {
-    EtaIn<T> a;
-    a.ul = ldu<CHAIN>(u, i, j, ny, nx);
-    a.ur = ldu<CHAIN>(u, i, j + 1, ny, nx);
-    a.vt = ldv<CHAIN>(v, i, j, ny, nx);
-    a.vb = ldv<CHAIN>(v, i + 1, j, ny, nx);
-    a.u_tl = ldu<CHAIN>(u, i - 1, j, ny, nx);
-    a.u_tr = ldu<CHAIN>(u, i - 1, j + 1, ny, nx);
-    a.u_bl = ldu<CHAIN>(u, i + 1, j, ny, nx);
-    a.u_br = ldu<CHAIN>(u, i + 1, j + 1, ny, nx);
-    a.v_lt = ldv<CHAIN>(v, i, j - 1, ny, nx);
-    a.v_rt = ldv<CHAIN>(v, i, j + 1, ny, nx);
-    a.v_lb = ldv<CHAIN>(v, i + 1, j - 1, ny, nx);
-    a.v_rb = ldv<CHAIN>(v, i + 1, j + 1, ny, nx);
-    return a;
-}
-
-// error reporting from kernels: set a device flag, never trap
-__device__ __forceinline__ void set_error(int* flag, int code) {
-    if (flag) atomicCAS(flag, 0, code);
 }
 
 }  // namespace glide

@@ -1,7 +1,8 @@
 // BF16 tensor-core GEMM on the 5th-generation tensor cores (tcgen05 + TMEM)
-// for the learned initial guess: 3x3 convolutions as GEMMs, either on an
-// explicit im2col matrix (training, whose weight gradient needs it) or with
-// the im2col done while staging the A tile (inference, no im2col buffer).
+// for the learned initial guess: 3x3 convolutions as GEMMs with the im2col done
+// while staging the A tile, where conv_rows.cu does not take the shape, their data
+// gradient, and plain products (the head; layers whose widths are no multiple of 8,
+// on an explicit im2col matrix).
 //
 //   C[M,N] (+)= A[M,K] * B[N,K]^T   (A, B: BF16, K-major; accumulate FP32 in TMEM)
 //   epilogue: + bias[N], ReLU, store FP32 or BF16, or add into FP32 C.
@@ -206,7 +207,7 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_kernel(const __nv_bfloat16* 
 }
 
 // --------------------------------------------------------------------------
-// Pipelined form (what aligned GEMMs and every convolution run): a ring of
+// Pipelined form (aligned operands, up to 8 chunks): a ring of
 // PSTAGES shared-memory stages filled by 16-byte cp.async copies (zero-filled
 // outside the matrix or the image, so the implicit im2col needs no branch
 // around the copy), so the copies of the next chunks are in flight while the
@@ -220,8 +221,6 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_kernel(const __nv_bfloat16* 
 // once for 128 outputs.  The epilogue stores 8 BF16 outputs per 16-byte
 // store where the row allows it.
 // --------------------------------------------------------------------------
-constexpr int PSTAGES_MAX = 4;
-
 // Bias, ReLU and store of the 32 rows of one warp (warps 0..3) of a finished tile.
 template <int BN>
 __device__ __forceinline__ void store_tile(uint32_t tmem, int warp, int lane, int m0, int n0, int M, int N, void* C,
@@ -273,7 +272,7 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloa
     constexpr int A_BYTES = GM * GK * 2, B_BYTES = BN * GK * 2, STAGE = A_BYTES + B_BYTES;
     constexpr int AROWS = GM / 16, BROWS = BN / 16;   // rows per thread and chunk
     extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ __align__(8) uint64_t mbar[PSTAGES_MAX];
+    __shared__ __align__(8) uint64_t mbar[PSTAGES];
     __shared__ uint32_t tmem_slot;
 
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;

@@ -219,7 +219,7 @@ __device__ __forceinline__ void load_patch(Patch<T>& P, const Window<T>& W, int 
 // Frozen per-cell coefficients of the forward local Newton loop: every term
 // that depends only on neighbour values (fixed during a cell's iterations) is
 // evaluated once here, so the loop only evaluates what depends on the cell's
-// own 5 unknowns.  Same formulas as assemble<T,true>; the neighbour normal
+// own 5 unknowns; the neighbour normal
 // stresses are kept as k*(x - x_far) + c so no cancellation is introduced.
 template <typename T> struct Frozen {
     T eta_c, ec;                       // eta of the cell, 0.25*eta
@@ -287,7 +287,7 @@ __device__ __forceinline__ void make_frozen(Frozen<T>& F, const Patch<T>& P, int
 }
 
 // One local Newton step's matrix and residual from the frozen coefficients
-// (same terms and order of rows/columns as assemble<T,true>).
+// (terms of glide/cuda/vanka.cu:56-404; rows and columns u_l, u_r, v_t, v_b, H_c).
 template <typename T>
 __device__ __forceinline__ void assemble_fast(const Frozen<T>& F, T ul, T ur, T vt, T vb, T Hc, T fu_l, T fu_r,
                                               T fv_t, T fv_b, T fH, T thk, T dti, const Phys<T>& p, T (&J)[25],

@@ -31,8 +31,8 @@ constexpr int VC_NT = 128;
 template <typename T> constexpr int VC_CTAS = sizeof(T) == 4 ? 4 : 2;
 constexpr int REF_STRIDE = 14;  // reference block stride (glide/grid.py:182-188)
 
-__device__ __forceinline__ bool tile_on(const int* flags, int i, int j, int nx) {
-    return flags[(i / REF_STRIDE) * (nx / REF_STRIDE + 1) + j / REF_STRIDE] != 0;
+template <bool CHAIN> __device__ __forceinline__ bool tile_on(const int* flags, int i, int j, int nx) {
+    return ld<CHAIN>(flags + (i / REF_STRIDE) * (nx / REF_STRIDE + 1) + j / REF_STRIDE) != 0;
 }
 
 // Matrix and residual at the iterate (n + d, h); R: minus the residual terms
@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(VC_NT, VC_CTAS<T>)
         bool any = false;
         if (own)
             for (int i = i0; i < i1 && !any; i += (i1 - 1 - i > 0 ? min(REF_STRIDE, i1 - 1 - i) : 1))
-                any = tile_on(flags, i, jc, nx);
+                any = tile_on<CHAIN>(flags, i, jc, nx);
         if (!__any_sync(FULL, any)) return;
     }
     const T dxi = p.dxi, d2 = p.dxi * p.dxi, rr = rho_ratio<T>();
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(VC_NT, VC_CTAS<T>)
         const T bp = gp * betap + (T(1) - gp) * p.water_drag;
 
         bool on = own;
-        if (LOCAL) on = on && i >= i0 && tile_on(flags, i, jc, nx);
+        if (LOCAL) on = on && i >= i0 && tile_on<CHAIN>(flags, i, jc, nx);
         if (i >= i0 && (!LOCAL || __any_sync(FULL, on))) {  // warp-uniform
             Cell<T> C;
             const T wl = jc > 0 ? T(1) : T(0), wr = jc + 1 < nx ? T(1) : T(0);

@@ -10,13 +10,14 @@ Network: 4 resolution levels, 32 base channels (32-64-128-256), two 3x3
 conv + ReLU per level, 2x average pooling down, nearest upsampling and skip
 concatenation up, a 1x1 head to 2 channels.  Activations are NHWC BF16,
 weights are kept in FP32 for the optimiser and cast to BF16 for the
-products.  Every convolution runs on the tcgen05 BF16 GEMM with FP32
-accumulation in TMEM: in training (forward, data gradient, weight gradient)
-as im2col + ``glide_gemm_bf16``, in inference as an implicit GEMM that
-gathers the im2col rows while staging each tile (``glide_conv3x3_bf16``);
-bias and ReLU are fused into the GEMM epilogue.
-Pooling, upsampling, concatenation and the optimiser are element-wise torch
-glue.  This part has no counterpart in the reference.
+products.  Every convolution runs on the tcgen05 tensor cores with FP32
+accumulation in TMEM, without an im2col matrix in either direction
+(``glide_conv3x3_bf16`` and its ``cat``, ``rows_f32w``, ``dgrad`` and ``wgrad``
+forms; widths that are no multiple of 8 run im2col + ``glide_gemm_bf16``); bias and
+ReLU are fused into the epilogue.  In inference the decoder's upsampling and
+concatenation are read in place and pooling is one pass; in training they and the
+optimiser are element-wise torch glue.  This part has no counterpart in the
+reference.
 """
 from __future__ import annotations
 
@@ -141,9 +142,9 @@ def transpose(x):
 
 def conv3x3_relu(x, W, b, relu=True):
     """relu(conv3x3(x, W) + b).  With autograd recording (training) this is
-    Conv3x3ReLU, which keeps the im2col matrix for the weight gradient; without
-    (inference) the im2col is gathered inside the GEMM when Cin % 8 == 0, with a
-    bit-identical result."""
+    Conv3x3ReLU, which keeps x for the weight gradient; without (inference) the
+    weights are rounded inside the kernel where the row march takes the shape, with
+    a bit-identical result."""
     Bn, H, Wd, Cin = x.shape
     if (torch.is_grad_enabled() and (x.requires_grad or W.requires_grad or b.requires_grad)) or Cin % 8 != 0:
         return Conv3x3ReLU.apply(x, W, b, relu)

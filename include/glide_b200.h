@@ -137,7 +137,8 @@ size_t glide_noalloc_scratch_bytes(void);
  * (room for 25 * ny * nx * nb elements; the contents are private).  glide_vanka_linear makes one
  * additive sweep for the correction d of the linear problem r + J d = 0:
  * rho = r + J d is the caller's linear residual; d += omega * (face average
- * of -A^-1 rho), with H + d_H kept >= gamma.  scratch as for the sweeps. */
+ * of -A^-1 rho), with H + d_H kept >= gamma.  scratch is not used (it held the
+ * cells' updates); a null pointer is refused as before. */
 int glide_vanka_lu(const GlideLevelArgs* a, const void* f_H, void* lu, double shift, void* stream);
 int glide_vanka_linear(const GlideLevelArgs* a, const void* rho_u, const void* rho_v, const void* rho_H,
                        const void* lu, void* d_u, void* d_v, void* d_H, double omega, void* scratch, void* stream);
