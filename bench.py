@@ -394,9 +394,11 @@ def time_fast_and_e2e(fast, fdev, host, args, world, flush, n, keep=None):
 
 def kernel_timings(runner, launches=20):
     """Average launch durations (CUDA events on the launching stream) on the
-    solved 1024^2 state of the fast path: the fine-level Vanka cell kernel in
-    FP64 (the finishing sweeps) and FP32 (the V-cycle smoothing), with the
-    fast path's local Newton settings, and the residual stencil in both."""
+    solved 1024^2 state of the fast path: the fine-level Vanka cell kernel of
+    whole sweeps (the finishing blocks', in FP64 and FP32: the march; the FP32
+    V-cycle smooths with the tile form, which no entry point launches alone),
+    with the fast path's local Newton settings, and the residual stencil in
+    both."""
     import ctypes as C
     import torch
     from glide_b200 import _native as N
@@ -429,9 +431,9 @@ def kernel_timings(runner, launches=20):
 
 
 def roofline(t, n):
-    """Roofline object of the dominant kernel (the FP32 Vanka cell kernel: the
-    V-cycle smoothing and the FP32 finishing blocks, half of the fast path's
-    kernel time) plus the FP64 cell kernel and the residual stencils."""
+    """Roofline object of the FP32 Vanka cell kernel of the finishing blocks (the
+    V-cycle's smoothing does the same sweep in the tile form) plus the FP64
+    cell kernel and the residual stencils."""
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))
@@ -448,10 +450,10 @@ def roofline(t, n):
     fp32_peak = 148 * 128 * 2 * 1.965e9 / 1e12
     t64, t32 = t.get("cells64"), t["cells32"]
     ach = hbm_obj(VANKA_ARRAYS, 4, t32)
-    roof = {"bound": "hbm", "kernel": "vanka_march_kernel<float> (fine level, full sweep)",
+    roof = {"bound": "hbm", "kernel": "vanka_march_kernel<float> (fine level, whole sweep of a finishing block)",
             "achieved": ach, "peak": hbm, "unit": "GB/s", "frac": ach / hbm, "peak_source": src,
             "traffic": VANKA32_DRAM_BYTES_1024 * scale,
-            "traffic_source": "ncu dram__bytes_read+write, one 1024^2 launch of the tile form",
+            "traffic_source": "ncu dram__bytes_read+write, one 1024^2 launch",
             "algorithmic_bytes": ncell * VANKA_ARRAYS * 4, "launch_ms": t32 * 1e3,
             "limiter": "FP32 issue/latency (ncu at 1024^2, 10 Newton steps: issue slots 63% active, 13 warps/SM at 126 registers)",
             "alu": {"achieved_tflops": ncell * VANKA32_FLOPS_PER_CELL / t32 / 1e12, "peak_tflops": fp32_peak,
@@ -704,12 +706,12 @@ def oracle_check(cases, sols, workers=None):
     return {name: [r[j] for r in rels] for j, name in enumerate(names)}
 
 
-# Per-cell figures of the fine-level Vanka cell kernel with 2 local Newton
-# iterations, from ncu op counts of one 1024^2 launch (dadd + dmul + 2 dfma,
-# fadd + fmul + 2 ffma per cell), and its DRAM bytes per launch.
-VANKA64_FLOPS_PER_CELL = 1611.0
-VANKA32_FLOPS_PER_CELL = 1324.0
-VANKA32_DRAM_BYTES_1024 = 43.98e6
+# Per-cell figures of the fine-level Vanka march with 2 local Newton iterations,
+# from ncu op counts of one 1024^2 launch (dadd + dmul + 2 dfma; fadd + fmul + 2 ffma
+# and twice their paired forms), and its DRAM bytes per launch.
+VANKA64_FLOPS_PER_CELL = 950.0
+VANKA32_FLOPS_PER_CELL = 753.0
+VANKA32_DRAM_BYTES_1024 = 42.7e6
 # algorithmic arrays per cell: Vanka reads u, v, H, f_u, f_v, f_H, bed, B,
 # beta, gamma and writes 5 delta arrays; the residual reads 11 and writes 3
 VANKA_ARRAYS = 15
