@@ -364,9 +364,14 @@ int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int B
     const int kplanes = c8 ? CR_PLANES8 : 9 * C / 8;
     auto weights = [&](int bn) { return size_t(kplanes) * bn * 16 + 128; };
     const int bn = N > 32 && weights(64) + 2 * stage <= CR_SMEM_MAX ? 64 : 32;
-    // as many resident CTAs as leave each at least four stages (or the one that fits)
+    // as many CTAs per SM as shared memory and TMEM leave at least four stages each (or the one
+    // that fits); registers hold two of 32 channels or one of 64 at a time, which is what an image
+    // of few rows should be cut for: more CTAs would be a second wave of single rows, each staging
+    // three (eight 64^2 images, 16 -> 32: 18.4 us, 9.1 with two per SM; before the march 14.3)
+    const int64_t total = int64_t(Bn) * a.strips * H * ((N + bn - 1) / bn);
+    const int most = 512 / (CR_ACC * bn);
     int occ = 1;
-    for (int o = 512 / (CR_ACC * bn); o > 1; o--)
+    for (int o = total < 4 * 148 * most ? most / 2 : most; o > 1; o--)
         if (weights(bn) + 4 * stage + 1024 <= CR_SMEM_SM / o) {
             occ = o;
             break;
@@ -374,7 +379,6 @@ int try_conv_rows(const void* x0, int C0, int up0, const void* x1, int C1, int B
     const size_t room = occ > 1 ? CR_SMEM_SM / occ - 1024 : CR_SMEM_MAX;
     int64_t st = int64_t((room - weights(bn)) / stage);
     a.stages = int(st < CR_MAXST ? st : CR_MAXST);
-    const int64_t total = int64_t(Bn) * a.strips * H * ((N + bn - 1) / bn);
     int64_t rows = (total + 148 * occ - 1) / (148 * occ);
     a.rows = int(rows < H ? rows : H);
     a.chunks = (H + a.rows - 1) / a.rows;
