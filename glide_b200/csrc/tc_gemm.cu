@@ -424,11 +424,20 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloa
 // --------------------------------------------------------------------------
 constexpr int RG_COPY = 256, RG_THREADS = RG_COPY + 32, RG_STAGES = 6;
 
-// The nine taps' sums of a warp's 32 pixels, added in tap order and stored as BF16.
+// The nine taps' sums of a warp's 32 pixels, added in tap order and stored as BF16;
+// a tap outside the image is left out (its products are with zeros, but a weight
+// need not be finite).
 template <int BN>
 __device__ __forceinline__ void store_taps(uint32_t tmem, int warp, int lane, int m0, int n0, int M, int N,
-                                           __nv_bfloat16* C) {
+                                           __nv_bfloat16* C, const ConvShape& cs) {
     const int row = m0 + warp * 32 + lane;
+    const int t0 = row / cs.W, px = row - t0 * cs.W, py = t0 % cs.H;
+    uint32_t inside = 0;
+#pragma unroll
+    for (int t = 0; t < 9; t++) {
+        const int y = py + 1 - t / 3, x = px + 1 - t % 3;
+        if (y >= 0 && y < cs.H && x >= 0 && x < cs.W) inside |= 1u << t;
+    }
 #pragma unroll 1
     for (int c0 = 0; c0 < BN; c0 += 8) {
         uint32_t r[9][8];
@@ -446,7 +455,7 @@ __device__ __forceinline__ void store_taps(uint32_t tmem, int warp, int lane, in
         for (int e = 0; e < 8; e++) {
             float x = 0.0f;
 #pragma unroll
-            for (int t = 0; t < 9; t++) x += __uint_as_float(r[t][e]);
+            for (int t = 0; t < 9; t++) x += inside >> t & 1 ? __uint_as_float(r[t][e]) : 0.0f;
             h[e] = __float2bfloat16(x);
         }
         *reinterpret_cast<uint4*>(C + int64_t(row) * N + n0 + c0) = *reinterpret_cast<uint4*>(h);
@@ -592,7 +601,7 @@ __global__ void __launch_bounds__(RG_THREADS) tc_gemm_ring_kernel(const __nv_bfl
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     if (ok && warp < 4) {
         if constexpr (TAPS)
-            store_taps<BN>(tmem, warp, lane, m0, n0, M, N, reinterpret_cast<__nv_bfloat16*>(C));
+            store_taps<BN>(tmem, warp, lane, m0, n0, M, N, reinterpret_cast<__nv_bfloat16*>(C), cs);
         else
             store_tile<BN>(tmem, warp, lane, m0, n0, M, N, C, ldc, bias, relu, out_mode);
     }

@@ -66,3 +66,21 @@ def test_input_buffer_may_be_refilled_before_backward():
     y = Conv3x3ReLU.apply(x, Wf, b, True)
     x.zero_()
     assert torch.equal(torch.autograd.grad(y, Wf, gy)[0], ref)
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_border_pixels_do_not_see_taps_outside(bad):
+    """A tap outside the image adds nothing, whatever its weight."""
+    from glide_b200.guess import _data_grad, col2im3, gemm, transpose
+    g = torch.Generator(device="cuda").manual_seed(3)
+    shape, Cout = (2, 5, 7, 8), 16
+    W = torch.randn(Cout, 9, 8, generator=g, device="cuda")
+    W[3, 0, 2] = bad
+    Wb = W.view(Cout, 72).to(torch.bfloat16)
+    gz = torch.randn(70, Cout, generator=g, device="cuda").to(torch.bfloat16)
+    dx = _data_grad(gz, Wb, shape)
+    dcol = torch.empty(70, 72, device="cuda")
+    gemm(gz, transpose(Wb), dcol, out_mode=0)
+    ref = col2im3(dcol, shape).to(torch.bfloat16)
+    assert torch.equal(dx.isnan(), ref.isnan()) and torch.equal(dx[~ref.isnan()], ref[~ref.isnan()])
+    assert bool(ref[..., 2].isfinite().any()) and not bool(ref[..., 2].isfinite().all())
