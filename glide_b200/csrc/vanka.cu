@@ -485,8 +485,10 @@ template <typename T> struct SweepState {
 };
 
 // Per-cell Newton deltas.  scratch holds 5 cell arrays: 0.5*du_l, 0.5*du_r,
-// 0.5*dv_t, 0.5*dv_b, dH.
-template <typename T, bool LOCAL, typename P>
+// 0.5*dv_t, 0.5*dv_b, dH.  FP64 has an instance for either local solve (PLAIN: not
+// pivoted, gated sweeps only; a branch between them costs 3 %: 512^2, 10 pivoted
+// steps 180 / 185 us), FP32 one for both.
+template <typename T, bool LOCAL, bool PLAIN, typename P>
 __global__ void __launch_bounds__(VX * VY, 4) vanka_cells_kernel(
     T* __restrict__ scratch, SweepState<T> q, const T* __restrict__ f_u, const T* __restrict__ f_v,
     const T* __restrict__ f_H, const T* __restrict__ bed, const T* __restrict__ B, const T* __restrict__ beta,
@@ -541,7 +543,7 @@ __global__ void __launch_bounds__(VX * VY, 4) vanka_cells_kernel(
         T J[25], rr[5], x[5];
         assemble_fast<T>(F, ul, ur, vt, vb, Hc, fu_l, fu_r, fv_t, fv_b, fH, thk, dti, p, J, rr);
         J[0] -= shift; J[6] -= shift; J[12] -= shift; J[18] -= shift; J[24] += shift;  // vanka.cu:406-410
-        if (pivot)
+        if (sizeof(T) == 8 ? !PLAIN : pivot != 0)
             lu5_solve_pivot(J, rr, x);
         else
             lu5_solve_fast(J, rr, x);
@@ -799,7 +801,10 @@ static void run_cells(const GlideLevelArgs* a, const void* f_u, const void* f_v,
                                      p);
             });
         };
-        flags ? run(vanka_cells_kernel<T, true, P>) : run(vanka_cells_kernel<T, false, P>);
+        if constexpr (sizeof(T) == 8) {
+            if (!pivot) return run(vanka_cells_kernel<T, true, true, P>);   // gated: use_march
+        }
+        flags ? run(vanka_cells_kernel<T, true, false, P>) : run(vanka_cells_kernel<T, false, false, P>);
     });
 }
 
