@@ -753,23 +753,23 @@ static inline dim3 face_grid(const Geo& g) { return dim3((g.nx + 1 + 31) / 32, (
 // by up to 3e-4 between the forms.  Pivoted local solves exist in the tile only.
 //
 // Microseconds per sweep at both sides of the lines, tile / march; FP32 tile sweeps
-// are one kernel each, FP64 ones two (room for one would be 34 MB more per level,
-// for the few grids between the lines).  FP32, 10 steps: 181^2 13.9 / 13.1, 256^2
-// 14.6 / 15.0, 300^2 21.3 / 20.1, 512^2 45.4 / 43.3, 1024^2 172 / 142; 7 steps: 420^2
-// 26.2 / 27.4, 600^2 48.9 / 47.1; 2 steps: 512^2 19.1 / 21.0, 600^2 25.7 / 27.3, 724^2
-// 36.2 / 31.4, 1024^2 75.1 / 55.7.  FP64: the march at every size, 10 steps: 32^2
-// 27.7 (before the march) / 14.3, 1024^2 410 / 353; 2 steps: 32^2 9.4 / 9.1, 256^2
-// 17.1 / 15.0, 1024^2 164 / 146.  Gated, a quarter (2 %) of the rows active, where the
-// march's chunks of two rows need a second wave: FP32, 2 steps: 512^2 13.6 / 20.1
-// (11.1 / 15.6), 724^2 24.0 / 27.9 (18.6 / 20.2), 1024^2 44.8 / 36.3 (33.3 / 27.3);
-// FP64, 2 steps: 450^2 23.4 / 20.2 (19.8 / 19.7), 512^2 23.9 / 27.9 (18.0 / 19.8), 724^2
-// 38.4 / 42.3 (24.3 / 24.5), 850^2 51.7 / 48.0 (27.6 / 26.0); 10 steps: 450^2 42.5 / 34.1,
-// 512^2 43.4 / 52.2 (32.4 / 34.2), 600^2 63.9 / 54.6.
+// are one kernel each, FP64 ones two (room for one would be 34 MB more per level).
+// FP32, 10 steps: 181^2 13.9 / 13.1, 256^2 14.6 / 15.0, 300^2 21.3 / 20.1, 512^2
+// 45.4 / 43.3, 1024^2 172 / 142; 7 steps: 420^2 26.2 / 27.4, 600^2 48.9 / 47.1; 2 steps:
+// 512^2 19.1 / 21.0, 600^2 25.7 / 27.3, 724^2 36.2 / 31.4, 1024^2 75.1 / 55.7.  FP64, the
+// march: 10 steps: 32^2 17.4 / 14.9, 256^2 32.6 / 29.9, 1024^2 352 / 352; 2 steps: 32^2
+// 9.7 / 9.7, 512^2 40.5 / 38.1, 1024^2 147 / 146.  Gated, a quarter (2 %) of the rows
+// active, where the march's chunks of one or two rows repeat their preparatory rows or
+// need a second wave: FP32, 2 steps: 512^2 13.6 / 20.1 (11.1 / 15.6), 724^2 24.0 / 27.9
+// (18.6 / 20.2), 1024^2 44.8 / 36.3 (33.3 / 27.3); FP64, 2 steps: 256^2 15.0 / 14.4
+// (13.9 / 13.5), 450^2 21.0 / 20.2 (17.5 / 19.7), 512^2 20.9 / 28.1 (16.2 / 20.1), 2048^2
+// 235 / 281 (104 / 120); 10 steps: 450^2 38.1 / 34.2 (29.7 / 34.1), 512^2 38.3 / 52.5
+// (26.3 / 34.1), 1024^2 116 / 118 (47.9 / 47.7), 2048^2 444 / 481 (125 / 141).
 template <typename T>
 static inline bool use_march(const Geo& g, int n_newton, bool gated, int pivot, bool cycle) {
     if (pivot) return false;
     const int64_t nc = g.nc(), k = int64_t(1) << 16;
-    if constexpr (sizeof(T) == 8) return !gated || nc < 4 * k || nc >= (n_newton < 8 ? 8 : 5) * k;
+    if constexpr (sizeof(T) == 8) return !gated || nc < 4 * k;
     if (cycle) return false;
     return nc >= (gated ? 8 * k : n_newton < 8 ? 6 * k : k);
 }

@@ -289,9 +289,8 @@ __global__ void __launch_bounds__(VC_NT, VC_CTAS<T>)
 // chip take one row per warp and spread the warps over all SMs.  A gated sweep
 // takes one row, two beyond four waves: which rows are active is not known here,
 // and only short chunks spread them over the chip (a quarter of the rows active,
-// 10 Newton steps: even chunks / these at 1024^2 FP32 90.9 / 53.9 us, FP64
-// 281 / 114; one row / two at 1024^2 FP32 60.9 / 56.7, FP64 133 / 116, at 256^2 FP64
-// 21.8 / 27.8).
+// 10 Newton steps: even chunks / these at 1024^2 FP32 90.9 / 53.9 us; one row / two at
+// 1024^2 FP32 60.9 / 56.7, at 256^2 FP64 21.8 / 27.8).
 template <typename T>
 void run_march(const GlideLevelArgs* a, const void* f_u, const void* f_v, const void* f_H, int n_newton, double shift,
                double step, const int* flags, const int* any_active, void* scratch, cudaStream_t s) {
