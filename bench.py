@@ -455,7 +455,7 @@ def roofline(t, n):
             "traffic": VANKA32_DRAM_BYTES_1024 * scale,
             "traffic_source": "ncu dram__bytes_read+write, one 1024^2 launch",
             "algorithmic_bytes": ncell * VANKA_ARRAYS * 4, "launch_ms": t32 * 1e3,
-            "limiter": "FP32 issue/latency (ncu at 1024^2, 10 Newton steps: issue slots 63% active, 13 warps/SM at 126 registers)",
+            "limiter": "FP32 issue/latency (ncu at 1024^2, 10 Newton steps: issue slots 62% active, 13 warps/SM at 127 registers)",
             "alu": {"achieved_tflops": ncell * VANKA32_FLOPS_PER_CELL / t32 / 1e12, "peak_tflops": fp32_peak,
                     "frac": ncell * VANKA32_FLOPS_PER_CELL / t32 / 1e12 / fp32_peak,
                     "flops_per_cell": VANKA32_FLOPS_PER_CELL,

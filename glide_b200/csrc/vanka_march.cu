@@ -15,7 +15,7 @@
 //
 // What bounds it: instruction issue and the latency of a step's chain at the 13
 // (FP64: 8) warps that an SM's registers hold; FP32, 1024^2, 10 steps: issue slots
-// 63 % active, FMA pipe 44 %, DRAM 4 %.  Figures of both forms: use_march in
+// 62 % active, FMA pipe 43 %, DRAM 4 %.  Figures of both forms: use_march in
 // vanka.cu.
 #include <type_traits>
 
