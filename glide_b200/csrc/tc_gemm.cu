@@ -421,6 +421,8 @@ __global__ void __launch_bounds__(GTHREADS) tc_gemm_pipe_kernel(const __nv_bfloa
 // number of its own (nine accumulators of BN columns) and the epilogue adds the
 // nine in FP32, tap after tap: what GEMM + col2im compute, without the (pixels x
 // 9 C) FP32 matrix between them.  B is the transposed weights, row tap * N + n.
+// Bound by latency at one CTA per SM (288 of TMEM's 512 columns); eight 256^2
+// patches, 32 -> 32: 157 us, GEMM + col2im 1,322; eight 32^2, 256 -> 256: 96 and 204.
 // --------------------------------------------------------------------------
 constexpr int RG_COPY = 256, RG_THREADS = RG_COPY + 32, RG_STAGES = 6;
 
