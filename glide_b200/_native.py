@@ -161,8 +161,11 @@ def check(rc: int, what: str = "glide call"):
 
 
 def stream_handle(stream=None) -> int:
-    s = torch.cuda.current_stream() if stream is None else stream
-    return s.cuda_stream
+    """The stream's address; of the current device's current stream without one
+    (asked for by number: a Stream object costs 3 us, a tenth of a small call)."""
+    if stream is None:
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return stream.cuda_stream
 
 
 def ptr(t) -> int:

@@ -27,6 +27,7 @@ import os
 from pathlib import Path
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _native as N
 
@@ -150,8 +151,9 @@ def conv3x3_relu(x, W, b, relu=True):
         return Conv3x3ReLU.apply(x, W, b, relu)
     Cout = W.shape[0]
     y = torch.empty((Bn, H, Wd, Cout), dtype=torch.bfloat16, device=x.device)
-    if not _rows_f32w(x.contiguous(), 0, None, W, b, relu, y):
-        conv3x3(x.contiguous(), W.detach().to(torch.bfloat16).contiguous(), y.view(-1, Cout), bias=b.detach(),
+    x = x.contiguous()
+    if not _rows_f32w(x, 0, None, W, b, relu, y):
+        conv3x3(x, W.detach().to(torch.bfloat16).contiguous(), y.view(-1, Cout), bias=b.detach(),
                 relu=relu, out_mode=1)
     return y
 
@@ -163,28 +165,30 @@ def _rows_f32w(x, up, skip, W, b, relu, y):
     9 Cin) and the bias are checked here, and what does not fit is left to
     conv3x3, which refuses it or takes its pitch."""
     lib = _lib()
-    C1 = 0 if skip is None else skip.shape[3]
-    if x.dtype != torch.bfloat16 or (skip is not None and skip.dtype != torch.bfloat16) or \
-            W.dtype != torch.float32 or W.shape != (y.shape[3], 9 * (x.shape[3] + C1)) or \
-            not W.is_contiguous() or W.data_ptr() % 16 or \
-            b.dtype != torch.float32 or not b.is_contiguous() or b.numel() < y.shape[3] or \
-            not lib.glide_conv3x3_rows_ok(x.shape[3], up, C1, y.shape[2], y.shape[3]):
+    Bn, H, Wd, Cout = y.shape
+    C0, C1 = x.shape[3], 0 if skip is None else skip.shape[3]
+    w = W.data_ptr()
+    if x.dtype is not torch.bfloat16 or (C1 and skip.dtype is not torch.bfloat16) or \
+            W.dtype is not torch.float32 or W.shape != (Cout, 9 * (C0 + C1)) or w % 16 or not W.is_contiguous() or \
+            b.dtype is not torch.float32 or b.numel() < Cout or not b.is_contiguous() or \
+            not lib.glide_conv3x3_rows_ok(C0, up, C1, Wd, Cout):
         return False
-    N.check(lib.glide_conv3x3_rows_f32w(x.data_ptr(), x.shape[3], up, None if skip is None else skip.data_ptr(), C1,
-                                        y.shape[0], y.shape[1], y.shape[2], W.data_ptr(), y.data_ptr(), y.shape[3],
-                                        b.data_ptr(), int(relu), _err_flag(x.device).data_ptr(), N.stream_handle()),
-            "tensor-core conv3x3")
+    N.check(lib.glide_conv3x3_rows_f32w(x.data_ptr(), C0, up, skip.data_ptr() if C1 else None, C1, Bn, H, Wd, w,
+                                        y.data_ptr(), Cout, b.data_ptr(), int(relu), _err_flag(x.device).data_ptr(),
+                                        N.stream_handle()), "tensor-core conv3x3")
     return True
 
 
 def _in_place(x, skip, W):
     """Whether the two sources can be read as they are: BF16, skip at twice the
     resolution of x, 16-byte aligned channels in both, weights without padding."""
-    return x.dim() == 4 and skip.dim() == 4 and x.dtype == skip.dtype == torch.bfloat16 and \
-        x.device == skip.device and x.numel() > 0 and skip.numel() > 0 and \
-        skip.shape[:3] == (x.shape[0], 2 * x.shape[1], 2 * x.shape[2]) and \
-        x.shape[3] % 8 == 0 and skip.shape[3] % 8 == 0 and W.dim() == 2 and \
-        W.shape[1] == 9 * (x.shape[3] + skip.shape[3]) and not any(t.data_ptr() % 16 for t in (x, skip, W))
+    if x.dtype is not torch.bfloat16 or skip.dtype is not torch.bfloat16 or x.dim() != 4 or skip.dim() != 4:
+        return False
+    n, h, w, c0 = x.shape
+    m, H, Wd, c1 = skip.shape
+    return m == n and H == 2 * h and Wd == 2 * w and n * h * w * c0 * c1 > 0 and c0 % 8 == 0 and c1 % 8 == 0 and \
+        W.dim() == 2 and W.shape[1] == 9 * (c0 + c1) and x.device == skip.device and \
+        (x.data_ptr() | skip.data_ptr() | W.data_ptr()) % 16 == 0
 
 
 def conv3x3_up_cat(x, skip, W, b):
@@ -335,14 +339,15 @@ def _plain(*ts):
     """Whether a kernel may read these tensors by address: ordinary contiguous
     tensors on the current device that nothing differentiates, maps or traces
     (torch's own operations serve all of that)."""
-    if torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack():
+    if torch._C._len_torch_dispatch_stack() or torch.compiler.is_compiling() or torch.jit.is_tracing():
         return False
-    return all(type(t) in (torch.Tensor, torch.nn.Parameter) and
+    dual = forward_ad._current_level >= 0
+    return all(t.is_cuda and type(t) in (torch.Tensor, torch.nn.Parameter) and
                not torch._C._functorch.is_functorch_wrapped_tensor(t) and
-               t.is_cuda and t.get_device() == torch.cuda.current_device() and
-               t.layout == torch.strided and t.is_contiguous() and t.numel() > 0 and not t.is_neg() and
-               not (torch.is_grad_enabled() and t.requires_grad) and
-               torch.autograd.forward_ad.unpack_dual(t).tangent is None for t in ts)
+               t.layout is torch.strided and t.is_contiguous() and t.numel() > 0 and not t.is_neg() and
+               not (t.requires_grad and torch.is_grad_enabled()) and
+               not (dual and forward_ad.unpack_dual(t).tangent is not None) and
+               t.get_device() == torch.cuda.current_device() for t in ts)
 
 
 def _pool(x):
